@@ -158,42 +158,53 @@ __device__ __forceinline__ unsigned make_idesc_tf32(int n) {
 }
 
 // The four K-slices of one stage (descriptor low words advance by 2 = 32 bytes), one predicate set-up.
-__device__ __forceinline__ void umma_tf32_x4(unsigned tmem_d, unsigned long long a_desc, unsigned long long b_desc,
+__device__ __forceinline__ void umma_tf32_x4(unsigned leader, unsigned tmem_d, unsigned long long a_desc, unsigned long long b_desc,
                                              unsigned idesc, unsigned accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "{\n\t.reg .pred p, q, e;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "setp.eq.b32 q, 0, 0;\n\t"
       "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\t"
       "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], a1, b1, %3, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], a2, b2, %3, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], a3, b3, %3, q;\n\t}"
-      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], a1, b1, %3, q;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], a2, b2, %3, q;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], a3, b3, %3, q;\n\t}"
+      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 // Same with a caller-given advance of the A descriptor per K-slice (in 16-byte units) and only the first `nks`
 // (1..4) slices issued: a chunk that holds fewer than 32 real channels needs no MMA on its zero padding.
-__device__ __forceinline__ void umma_tf32_step(unsigned tmem_d, unsigned long long a_desc, unsigned long long b_desc,
+__device__ __forceinline__ void umma_tf32_step(unsigned leader, unsigned tmem_d, unsigned long long a_desc, unsigned long long b_desc,
                                                unsigned idesc, unsigned accumulate, unsigned long long a_step, unsigned nks) {
   asm volatile(
-      "{\n\t.reg .pred p, q, r1, r2, r3;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "{\n\t.reg .pred p, q, e, r1, r2, r3;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "setp.ne.b32 e, %7, 0;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "setp.eq.b32 q, 0, 0;\n\t"
-      "setp.gt.u32 r1, %6, 1;\n\tsetp.gt.u32 r2, %6, 2;\n\tsetp.gt.u32 r3, %6, 3;\n\t"
+      "setp.gt.and.u32 r1, %6, 1, e;\n\tsetp.gt.and.u32 r2, %6, 2, e;\n\tsetp.gt.and.u32 r3, %6, 3, e;\n\t"
       "add.u64 a1, %1, %5;\n\tadd.u64 a2, a1, %5;\n\tadd.u64 a3, a2, %5;\n\t"
       "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
       "@r1 tcgen05.mma.cta_group::1.kind::tf32 [%0], a1, b1, %3, q;\n\t"
       "@r2 tcgen05.mma.cta_group::1.kind::tf32 [%0], a2, b2, %3, q;\n\t"
       "@r3 tcgen05.mma.cta_group::1.kind::tf32 [%0], a3, b3, %3, q;\n\t}"
-      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "l"(a_step), "r"(nks)
+      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "l"(a_step), "r"(nks), "r"(leader)
       : "memory");
 }
-__device__ __forceinline__ void umma_commit(unsigned long long *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+__device__ __forceinline__ void umma_commit(unsigned leader, unsigned long long *bar) {
+  asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+               "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(leader)
                : "memory");
+}
+// 1 in one lane of a converged warp, 0 in the others.  The single-thread roles (MMA issue) run their loops with the whole
+// warp and predicate only the tcgen05 instructions: inside `if (lane == 0)` the compiler cannot keep the descriptors in
+// uniform registers, and an instruction then takes 77 clocks to issue whatever its size instead of the 40-64 of its operands.
+__device__ __forceinline__ unsigned elect_one() {
+  unsigned r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
 }
 // ---- thread-block cluster helpers (K-split variant of the halo kernel) ----
 __device__ __forceinline__ unsigned cluster_ctarank() {
@@ -669,7 +680,7 @@ conv_tc_halo_kernel(const TcParams p, const __grid_constant__ CUtensorMap map_in
   __shared__ unsigned s_tmem_base;
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // the shuffle tells the compiler that `warp` is uniform
   // K-split: the CS CTAs of a cluster work on the same item, CTA `crank` reducing chunks [ch_lo, ch_hi); a cluster has
   // at most one item (the host sizes the grid so), hence `bid` / `nblk` below index clusters, not CTAs.
   const unsigned CS = KSPLIT ? (unsigned)p.ksplit : 1u;
@@ -814,7 +825,8 @@ conv_tc_halo_kernel(const TcParams p, const __grid_constant__ CUtensorMap map_in
   } else if (warp == 2 || warp == 3) {
     // =========================== MMA issuers ===========================
     const unsigned me = (unsigned)warp - 2u;
-    if (lane == 0 && me < NI) {
+    if (me < NI) {
+      const unsigned leader = elect_one();
       const unsigned idesc = make_idesc_tf32(NB);
       const unsigned long long b_hi = make_smem_desc(0) & 0xFFFFFFFF00000000ull;
       const unsigned b_lo_flags = (unsigned)(make_smem_desc(0) & 0xFFFF0000ull);
@@ -855,21 +867,21 @@ conv_tc_halo_kernel(const TcParams p, const __grid_constant__ CUtensorMap map_in
             for (int j = 0; j < p.tps; ++j, b_addr += b_bytes) {
               const unsigned a_lo = a_lo_flags | ((tap_addr & 0x3FFFFu) >> 4);
               const unsigned b_lo = b_lo_flags | ((b_addr & 0x3FFFFu) >> 4);
-              umma_tf32_step(tmem_d, a_hi | a_lo, b_hi | b_lo, idesc, accumulate, a_step, nks);
+              umma_tf32_step(leader, tmem_d, a_hi | a_lo, b_hi | b_lo, idesc, accumulate, a_step, nks);
               accumulate = 1u;
               tap_addr += 16u;
               if (++kx == (unsigned)p.k) { kx = 0; row_addr += 2u * row_bytes; tap_addr = row_addr; }
             }
-            umma_commit(&b_empty[slot]);
+            umma_commit(leader, &b_empty[slot]);
             issued = true;
           }
           if (!ok) break;
           // the halo buffer is free once the MMAs of both issuers have read it
-          if (issued) umma_commit(&a_empty[abuf]);
-          else mbar_arrive(&a_empty[abuf]);
+          if (issued) umma_commit(leader, &a_empty[abuf]);
+          else if (leader) mbar_arrive(&a_empty[abuf]);
         }
         if (!ok) break;
-        umma_commit(&acc_full[buf]);
+        umma_commit(leader, &acc_full[buf]);
         if (me == 0 && item_idx == 0) TC_TRACE(9);
       }
     }
@@ -976,7 +988,7 @@ conv_tc_kernel(const TcParams p, const __grid_constant__ TcMaps maps) {
   __shared__ unsigned s_tmem_base;
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // the shuffle tells the compiler that `warp` is uniform
   // K-split: `bid` / `nblk` index clusters; a cluster has at most one item (the host sizes the grid so)
   const unsigned CS = KSPLIT ? (unsigned)p.ksplit : 1u;
   const unsigned crank = CS > 1u ? cluster_ctarank() : 0u;
@@ -1112,7 +1124,8 @@ conv_tc_kernel(const TcParams p, const __grid_constant__ TcMaps maps) {
     // =========================== MMA issuer ===========================
     // Same care as the producer: a lean loop issues an MMA every ~70 cycles, one that rebuilds descriptors and
     // divides by the stage count needs ~250.  Descriptors are pre-built; a stage only adds its address.
-    if (lane == 0) {
+    {
+      const unsigned leader = elect_one();
       const unsigned idesc = make_idesc_tf32(NB);
       const unsigned smem_base = smem_u32(smem);
       const unsigned long long desc_hi = make_smem_desc(0) & 0xFFFFFFFF00000000ull;   // stride, version, swizzle
@@ -1134,14 +1147,14 @@ conv_tc_kernel(const TcParams p, const __grid_constant__ TcMaps maps) {
           const unsigned a_lo = desc_lo_flags | ((stage_addr & 0x3FFFFu) >> 4);
           const unsigned b_lo = desc_lo_flags | (((stage_addr + A_STAGE_BYTES) & 0x3FFFFu) >> 4);
           // 4 x (K = 8 tf32 = 32 bytes = 2 descriptor units) inside the 128-byte swizzled row
-          umma_tf32_x4(tmem_d, desc_hi | a_lo, desc_hi | b_lo, idesc, accumulate);
+          umma_tf32_x4(leader, tmem_d, desc_hi | a_lo, desc_hi | b_lo, idesc, accumulate);
           accumulate = 1u;
-          umma_commit(&empty_bar[s]);  // arrives once the MMAs above have finished reading the stage
+          umma_commit(leader, &empty_bar[s]);  // arrives once the MMAs above have finished reading the stage
           stage_addr += (unsigned)stage_bytes;
           if (++s == (unsigned)p.stages) { s = 0; stage_addr = smem_base; parity ^= 1u; }
         }
         if (!ok) break;
-        umma_commit(&acc_full[buf]);
+        umma_commit(leader, &acc_full[buf]);
         if (item_idx == 0) TC_TRACE(8);
       }
     }

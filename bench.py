@@ -911,9 +911,9 @@ def main():
                          "per window); the headline is e2depth")
     ap.add_argument("--tensor-cores", default="auto", choices=["auto", "off"],
                     help="off keeps every convolution on the FP32 path (secondary measurements)")
-    ap.add_argument("--ksplit", action=argparse.BooleanOptionalAction, default=True,
-                    help="small-image tensor-core layers run as clusters that split the input channels (default); "
-                         "--no-ksplit keeps one thread block per work item")
+    ap.add_argument("--ksplit", action=argparse.BooleanOptionalAction, default=False,
+                    help="small-image tensor-core layers run as clusters that split the input channels instead of on "
+                         "CTA pairs (slower)")
     ap.add_argument("--own-tiles", action=argparse.BooleanOptionalAction, default=None,
                     help="tensor-core convolutions find their active tiles themselves instead of reading a list made by "
                          "a dilation launch in front of them (default: the library's setting)")

@@ -62,13 +62,14 @@ enum {
    * points below except the one-off packing kernels); mie_set_option stores a value (0 resets), mie_get_option reads
    * it modulo 2^31 */
   MIE_OPT_LAUNCH_COUNT = 4,
-  /* 1 (default): small-image layers with long reductions run the tensor-core kernel as clusters of 2 or 4 thread
-   * blocks that split the input channels of a work item and exchange partial sums through distributed shared
-   * memory; 0: one thread block per work item */
+  /* 1: small-image layers with long reductions run the tensor-core kernels as clusters of 2 or 4 thread blocks that
+   * split the input channels of a work item and exchange partial sums through distributed shared memory; 0 (default):
+   * the CTA-pair kernel takes them, which measured faster at every such layer */
   MIE_OPT_TC_KSPLIT = 5,
-  /* which tensor-core kernels honour mie_conv_args.own_tiles, as a bit mask: 1 the per-tap kernel, 2 the per-tap kernel as
-   * clusters, 4 the halo kernel, 8 the halo kernel as clusters; the others get the separate dilation launch from the
-   * entry point.  Default 7: the clustered halo kernel measured slower with the mode than without */
+  /* which tensor-core kernels honour mie_conv_args.own_tiles, as a bit mask: 1 the per-tap kernel and the CTA-pair kernel
+   * with stride 2, 2 the per-tap kernel as clusters, 4 the CTA-pair kernel with stride 1, 8 layers whose tiles are
+   * finished by several blocks (the CTA-pair kernel with more than one column block, the halo kernel as clusters); the
+   * others get the separate dilation launch from the entry point.  Default 7: kind 8 measured slower with the mode */
   MIE_OPT_TC_OWN_KERNELS = 6
 };
 int mie_set_option(int option, int value);
@@ -227,7 +228,16 @@ typedef struct mie_conv_args {
    * mie_tiles_dilate launch from the entry point instead. */
   int own_tiles;
   void *own_scratch;
+  /* Dense evaluation (`refresh`) in fp32 precision on the tensor cores, both or neither: the filter packed by
+   * mie_pack_conv_weights_exact, and the second field of mie_split_exact (`in` is then its first one, same pixel stride).
+   * Taken for k in {3, 5, 7} without a second input when the fields are 16-byte aligned; else, and with either null, the
+   * FP32 kernel runs (on `in` as given: pass the unsplit field there).  Every output tile has to be listed. */
+  const float *wpacked_exact;
+  const float *in_lo;
 } mie_conv_args;
+
+/* Host only: 1 if mie_conv_tiles would run these arguments in fp32 precision on the tensor cores, else 0. */
+int mie_conv_is_exact(const mie_conv_args *args /* host */);
 
 int mie_conv_tiles(const mie_conv_args *args /* host */, void *stream);
 
@@ -242,6 +252,12 @@ int mie_conv_cluster_size(const mie_conv_args *args /* host */);
 /* Host helper (no device work): floats needed for the packed copy of a [cout,cin,k,k] filter, and
  * the padded extents the kernels assume. */
 int mie_conv_pack_dims(int cin, int cout, int k, int *cin_pad, int *cout_pad, int64_t *n_floats);
+
+/* Fp32 precision on the tensor cores: hi = v rounded to TF32, lo = v - hi rounded to TF32 (together v to 2^-24), for a dense
+ * field of `pixels` pixels, and for a filter as [tap][32-channel chunk][hi rows | lo rows][32]. */
+int mie_split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, void *stream);
+int mie_conv_pack_dims_exact(int cin, int cout, int k, int64_t *n_floats /* host */);
+int mie_pack_conv_weights_exact(const float *w_oihw, int cout, int cin, int k, float *wpacked, void *stream);
 
 /* Same for the tensor-core copy: cin padded to 32, layout [k*k][cin_pad/32][cout_pad][32]. */
 int mie_conv_pack_dims_tc(int cin, int cout, int k, int *cin_pad, int *cout_pad, int64_t *n_floats);
@@ -352,6 +368,10 @@ int mie_cat2(const float *a, int64_t a_ps, const uint64_t *a_bits, int ca, const
  * (incr_modules/mask_incr_functional.py:41-42). */
 int mie_accumulate(float *y, int64_t y_ps, const float *d, int64_t d_ps, const uint64_t *d_bits, int N,
                    int C, int H, int W, void *stream);
+/* The same, and kept = d with kept_bits = d_bits: the state delta that the next step is given (recurrent feedback), in one
+ * pass.  C and the pixel strides multiples of 4, 16-byte aligned fields. */
+int mie_accumulate_keep(float *y, int64_t y_ps, const float *d, int64_t d_ps, const uint64_t *d_bits, float *kept, int64_t k_ps,
+                        uint64_t *kept_bits, int N, int C, int H, int W, void *stream);
 
 /* ---------------------------------------------------------------------------------------------
  * The steps either side of the network in the reference's driver loop.

@@ -51,6 +51,7 @@ class ConvArgs(C.Structure):
         ("in2", _vp), ("in2_ps", _i64),
         ("accum", _vp), ("accum_ps", _i64),
         ("own_tiles", _i), ("own_scratch", _vp),
+        ("wpacked_exact", _vp), ("in_lo", _vp),
     ]
 
 
@@ -74,6 +75,10 @@ SIGNATURES = {
     "mie_pack_conv_weights": (_i, [_vp, _i, _i, _i, _vp, _vp]),
     "mie_conv_pack_dims_tc": (_i, [_i, _i, _i, C.POINTER(_i), C.POINTER(_i), C.POINTER(_i64)]),
     "mie_pack_conv_weights_tc": (_i, [_vp, _i, _i, _i, _vp, _vp]),
+    "mie_conv_is_exact": (_i, [C.POINTER(ConvArgs)]),
+    "mie_split_exact": (_i, [_vp, _i64, _i, _i64, _vp, _vp, _i64, _vp]),
+    "mie_conv_pack_dims_exact": (_i, [_i, _i, _i, C.POINTER(_i64)]),
+    "mie_pack_conv_weights_exact": (_i, [_vp, _i, _i, _i, _vp, _vp]),
     "mie_activation_increment": (_i, [_vp, _vp, _vp, _i64, _i, _vp]),
     "mie_conv_increment_workspace_bytes": (_i64, [_i, _i, _i, _i, _i, _i, _i]),
     "mie_conv_increment_ext": (_i, [_vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _i64, _vp]),
@@ -86,6 +91,7 @@ SIGNATURES = {
     "mie_add": (_i, [_vp, _i64, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _i, _i, _i, _i, _vp, _vp]),
     "mie_cat2": (_i, [_vp, _i64, _vp, _i, _vp, _i64, _vp, _i, _vp, _i64, _vp, _i, _i, _i, _vp, _vp]),
     "mie_accumulate": (_i, [_vp, _i64, _vp, _i64, _vp, _i, _i, _i, _i, _vp]),
+    "mie_accumulate_keep": (_i, [_vp, _i64, _vp, _i64, _vp, _vp, _i64, _vp, _i, _i, _i, _i, _vp]),
     "mie_delta_mask": (_i, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i, _i, _i, _i, _f, _vp, _i64, _vp, _vp, _vp]),
     "mie_events_to_voxel": (_i, [_vp, _i, _i, _i, _i, _vp, _i64, _i, _i, _i, _i, _vp]),
     "mie_events_to_count_image": (_i, [_vp, _i, _i, _i, _vp, _i64, _i, _i, _i, _i, _vp]),

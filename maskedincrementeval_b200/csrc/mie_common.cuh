@@ -82,7 +82,7 @@ static inline void launch_chained_cluster(void (*kernel)(KArgs...), dim3 grid, d
 
 static inline int divup(int a, int b) { return (a + b - 1) / b; }
 static inline int64_t divup64(int64_t a, int64_t b) { return (a + b - 1) / b; }
-static inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+__host__ __device__ static inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 __device__ __forceinline__ float act_apply(int op, float x) {
   // expf/tanhf are the accurate libm-class device functions (no fast-math): parity with

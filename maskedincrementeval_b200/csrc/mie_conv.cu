@@ -18,6 +18,8 @@ using namespace mie;
 namespace mie {
 bool tc_eligible(const mie_conv_args *a);
 int launch_conv_tc(const mie_conv_args *a, cudaStream_t st);
+bool exact_takes(const mie_conv_args *a);
+int launch_conv_exact(const mie_conv_args *a, cudaStream_t st);
 }  // namespace mie
 
 namespace {
@@ -555,6 +557,8 @@ extern "C" int mie_pack_conv_weights(const float *w_oihw, int cout, int cin, int
   return check_launch();
 }
 
+extern "C" int mie_conv_is_exact(const mie_conv_args *a) { return (a && exact_takes(a)) ? 1 : 0; }
+
 extern "C" int mie_conv_uses_tensor_cores(const mie_conv_args *a) { return (a && tc_eligible(a)) ? 1 : 0; }
 
 extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
@@ -585,6 +589,7 @@ extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
     b.own_tiles = 0;
     return mie_conv_tiles(&b, stream);
   }
+  if (exact_takes(a)) return tail_after_launch(launch_conv_exact(a, (cudaStream_t)stream), a->tail, true, stream);
   if (tc_eligible(a)) return tail_after_launch(launch_conv_tc(a, (cudaStream_t)stream), a->tail, true, stream);
 
   ConvParams p;

@@ -1,0 +1,459 @@
+// Dense evaluation (the refresh pass) in fp32 precision on the tensor cores, on CTA pairs like mie_conv_pair.cu.
+//
+// Every operand is two TF32 numbers, hi = round(v) and lo = round(v - hi) (round to nearest: together they hold v to 2^-24),
+// and a product is hi*hi + hi*lo + lo*hi; the dropped lo*lo is 2^-24 of it.  The input comes as two fields (mie_split_exact),
+// the filter as two arrays of rows.  Per filter tap two instructions per K-slice:
+//     hi(input) x [hi(filter) | lo(filter)]  ->  N = 2 CB columns,      lo(input) x hi(filter)  ->  N = CB columns.
+// What keeps the result at fp32 level is where the sums are rounded: the tensor core truncates each time it adds to an
+// accumulator (1.7e-8 of the value per addition, always towards zero: 3e-5 after the 2400 additions of a 256-channel 5x5
+// layer).  So the first product starts from zero again with every ring stage (at most 16 additions) and the epilogue warps
+// add the partial sums to registers, rounded to nearest, while the next stage runs; the second product is 2^-12 of the first
+// and stays in its accumulator for the whole work item.  Against a float64 convolution the error is that of the CUDA-core
+// FP32 kernel or below it (see tests/test_gpu_exact.py).
+// Epilogue: reservoir = conv + bias (+ addend), output = f(reservoir), every pixel of a listed tile marked.
+#include "mie_pair.cuh"
+
+using namespace mie;
+
+namespace mie {
+namespace {
+
+constexpr int EXACT_THREADS = 384;
+constexpr int EXACT_MAX_STAGES = 8;
+constexpr int EXACT_MAX_HALOS = 4;
+
+struct ExactParams {
+  int cin, cout, cout_pad, n_chunks, n, hout, wout;
+  const int32_t *list; int32_t *counts; int max_tiles;
+  float *out; int64_t out_ps; unsigned int *out_bits32;
+  int act; float *res; int64_t res_ps; const float *addend; int64_t addend_ps; const float *bias;
+  int cb, stages, halos, tps, wp;
+  unsigned spin_limit;
+  mie_tail_job tail;
+  PairTaps t;
+};
+struct ExactMaps {
+  CUtensorMap hi[4], lo[4], w;
+};
+
+__device__ __forceinline__ void tmem_add16(unsigned taddr, float *acc) {
+  unsigned r[16];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                 "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) acc[i] += __uint_as_float(r[i]);
+}
+
+// HW: channels per epilogue set (CB = 2 HW channels per block)
+template <int HW>
+__global__ void __launch_bounds__(EXACT_THREADS, 1)
+conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr int CB = 2 * HW;
+  constexpr unsigned half_bytes = HW * 128u, tap_bytes = 2u * half_bytes;   // this block's rows of one tap: [hi | lo] of its half of the channels
+  const unsigned row_bytes = (unsigned)p.wp * 128u;
+  const unsigned halo_bytes = ((unsigned)p.wp * 2u * row_bytes + 1023u) & ~1023u;
+  const unsigned stage_bytes = tap_bytes * (unsigned)p.tps;
+  __shared__ unsigned long long b_full[EXACT_MAX_STAGES], b_empty[EXACT_MAX_STAGES], a_full[EXACT_MAX_HALOS], a_empty[EXACT_MAX_HALOS],
+      seg_full[2], seg_empty[2], item_full[2], item_empty[2];
+  __shared__ unsigned s_tmem_base;
+  __shared__ int s_abort;
+
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const unsigned crank = cluster_ctarank();
+  const int bid = (int)(blockIdx.x >> 1), nblk = (int)(gridDim.x >> 1);
+  const int THo = (p.hout + 7) >> 3, TWo = (p.wout + 7) >> 3;
+  const int ntiles_total = p.n * THo * TWo;
+  // columns: two segment buffers of 2 CB (hi and lo of the filter), two item buffers of CB (lo of the input)
+  constexpr unsigned tmem_cols = CB == 64 ? 512u : 256u, item_col = 4u * CB;
+
+  if (tid == 0) {
+    for (int s = 0; s < p.stages; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
+    for (int s = 0; s < p.halos; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&seg_full[b], 1); mbar_init(&seg_empty[b], 16); mbar_init(&item_full[b], 1); mbar_init(&item_empty[b], 16); }
+    s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(tmem_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const unsigned tmem_base = s_tmem_base;
+  pair_cluster_sync();
+  grid_dependency_wait();
+  grid_dependency_trigger();
+
+  const int n_active = __shfl_sync(0xffffffffu, min(p.counts[0], p.max_tiles), 0);
+  const int n_cblk = p.cout_pad / CB, n_items = ((n_active + 3) >> 2) * n_cblk;
+  const unsigned b_base = smem_u32(smem), a_base = b_base + (((unsigned)p.stages * stage_bytes + 1023u) & ~1023u);
+  const int nv = p.t.nviews;
+
+  if (warp == 0) {
+    // =========================== halo producer: hi views, then lo views of a chunk ===========================
+    const unsigned leader = elect_one();
+    unsigned s = 0, parity = 0;
+    bool first_lap = true, ok = true;
+    for (int item = bid; item < n_items && ok; item += nblk) {
+      const int e = 4 * (item / n_cblk) + 2 * (int)crank;
+      int tx8[2], ty8[2], tn[2];
+      bool have[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        int t = __shfl_sync(0xffffffffu, e + i < n_active ? p.list[e + i] : -1, 0);
+        have[i] = e + i < n_active;
+        if (have[i] && (t < 0 || t >= ntiles_total)) {      // reported, skipped by the epilogue; tile 0 stands in for it here
+          if (leader) atomicOr(&p.counts[3], MIE_ERR_BAD_TILE);
+          t = 0;
+        }
+        tx8[i] = have[i] ? (t % TWo) * 8 : 0; ty8[i] = have[i] ? ((t / TWo) % THo) * 8 : 0; tn[i] = have[i] ? t / (TWo * THo) : 0;
+      }
+      const unsigned tx_bytes = (unsigned)min(4, n_active - 4 * (item / n_cblk)) * (unsigned)p.wp * row_bytes;
+      for (int chunk = 0; chunk < p.n_chunks && ok; ++chunk)
+        for (int u = 0; u < 2 * nv; ++u) {
+          if (!first_lap) ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[s], parity, &s_abort, p.spin_limit));
+          if (!ok) break;
+          const int v = u < nv ? u : u - nv;
+          const unsigned bar = mapa_shared(smem_u32(&a_full[s]), 0);
+          if (leader) {
+            if (crank == 0u)
+              asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&a_full[s])), "r"(tx_bytes) : "memory");
+            const CUtensorMap *map = u < nv ? &maps.hi[v] : &maps.lo[v];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              if (have[i]) {
+                unsigned dst = a_base + s * halo_bytes + (unsigned)i * row_bytes;
+                for (int r = 0; r < p.wp; ++r, dst += 2u * row_bytes) tma_load_4d_pair(dst, map, bar, chunk * 32, tx8[i] + p.t.x0[v], ty8[i] + p.t.y0[v] + r, tn[i]);
+              }
+          }
+          __syncwarp();
+          if (++s == (unsigned)p.halos) { s = 0; if (!first_lap) parity ^= 1u; first_lap = false; }
+        }
+    }
+    for (int i = 0; i < p.halos && ok; ++i) {       // nothing may signal this block's barriers after it has left
+      if (first_lap && (unsigned)i >= s) break;
+      if (first_lap) ok = mbar_wait(&a_empty[i], 0u, &s_abort, p.spin_limit);
+      else {
+        ok = mbar_wait(&a_empty[s], parity, &s_abort, p.spin_limit);
+        if (++s == (unsigned)p.halos) { s = 0; parity ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    // =========================== filter producer ===========================
+    const unsigned leader = elect_one();
+    unsigned s = 0, parity = 0, stage_addr = b_base;
+    bool first_lap = true, ok = true;
+    for (int item = bid; item < n_items && ok; item += nblk) {
+      const int row = (item % n_cblk) * CB + (int)crank * HW;
+      for (int chunk = 0; chunk < p.n_chunks && ok; ++chunk)
+        for (int u = 0; u < 2 * nv && ok; ++u) {
+          const int v = u < nv ? u : u - nv;
+          for (int i = p.t.first[v]; i < p.t.first[v + 1]; i += p.tps) {
+            if (!first_lap) ok = __all_sync(0xffffffffu, mbar_wait(&b_empty[s], parity, &s_abort, p.spin_limit));
+            if (!ok) break;
+            const int nt = min(p.tps, p.t.first[v + 1] - i);
+            if (leader) {
+              if (crank == 0u)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&b_full[s])),
+                             "r"((unsigned)nt * 2u * (u < nv ? tap_bytes : half_bytes)) : "memory");
+              const unsigned bar = mapa_shared(smem_u32(&b_full[s]), 0);
+              for (int k = 0; k < nt; ++k) {
+                const unsigned dst = stage_addr + (unsigned)k * tap_bytes;
+                tma_load_4d_pair(dst, &maps.w, bar, 0, row, chunk, (int)p.t.tap[i + k]);
+                if (u < nv) tma_load_4d_pair(dst + half_bytes, &maps.w, bar, 0, p.cout_pad + row, chunk, (int)p.t.tap[i + k]);
+              }
+            }
+            __syncwarp();
+            stage_addr += stage_bytes;
+            if (++s == (unsigned)p.stages) { s = 0; stage_addr = b_base; if (!first_lap) parity ^= 1u; first_lap = false; }
+          }
+        }
+    }
+    for (int i = 0; i < p.stages && ok; ++i) {
+      if (first_lap && (unsigned)i >= s) break;
+      if (first_lap) ok = mbar_wait(&b_empty[i], 0u, &s_abort, p.spin_limit);
+      else {
+        ok = mbar_wait(&b_empty[s], parity, &s_abort, p.spin_limit);
+        if (++s == (unsigned)p.stages) { s = 0; parity ^= 1u; }
+      }
+    }
+  } else if (warp == 2) {
+    // =========================== MMA issuer (first block of the pair) ===========================
+    if (crank == 0u) {
+      const unsigned id0 = (make_idesc_tf32(0) & ~(31u << 24)) | (16u << 24);       // M = 256
+      const unsigned id_hi = id0 | ((unsigned)(2 * CB >> 3) << 17), id_lo = id0 | ((unsigned)(CB >> 3) << 17);
+      const unsigned long long b_tmpl = make_smem_desc(0), a_tmpl = make_smem_desc(0, row_bytes);
+      const unsigned long long b_hi = b_tmpl & 0xFFFFFFFF00000000ull, a_hi = a_tmpl & 0xFFFFFFFF00000000ull;
+      const unsigned lo_flags = (unsigned)(b_tmpl & 0xFFFF0000ull);
+      unsigned bs = 0, bpar = 0, as = 0, apar = 0, item_idx = 0, seg = 0, stage_addr = b_base;
+      bool ok = true;
+      for (int item = bid; item < n_items && ok; item += nblk, ++item_idx) {
+        const unsigned buf = item_idx & 1u;
+        if (item_idx >= 2 && !__all_sync(0xffffffffu, mbar_wait_cluster(&item_empty[buf], ((item_idx >> 1) - 1) & 1u, &s_abort, p.spin_limit))) break;
+        unsigned started = 0;          // the item accumulator holds something
+        for (int chunk = 0; chunk < p.n_chunks && ok; ++chunk) {
+          const unsigned nks = (unsigned)min(4, (p.cin - chunk * 32 + 7) >> 3);
+          for (int u = 0; u < 2 * nv && ok; ++u) {
+            const bool lo = u >= nv;
+            const int v = lo ? u - nv : u, end = p.t.first[v + 1];
+            if (!__all_sync(0xffffffffu, mbar_wait(&a_full[as], apar, &s_abort, p.spin_limit))) { ok = false; break; }
+            const unsigned halo = lo_flags | ((a_base + as * halo_bytes) >> 4);
+            for (int i = p.t.first[v]; i < end; i += p.tps) {
+              const int nt = min(p.tps, end - i);
+              if (!__all_sync(0xffffffffu, mbar_wait(&b_full[bs], bpar, &s_abort, p.spin_limit))) { ok = false; break; }
+              if (!lo && seg >= 2 && !__all_sync(0xffffffffu, mbar_wait_cluster(&seg_empty[seg & 1u], ((seg >> 1) - 1) & 1u, &s_abort, p.spin_limit))) { ok = false; break; }
+              tc_fence_after();
+              const unsigned d = tmem_base + (lo ? item_col + buf * CB : (seg & 1u) * (2u * CB));
+              unsigned b_lo = lo_flags | (stage_addr >> 4);
+              for (int k = 0; k < nt; ++k, b_lo += tap_bytes >> 4)
+                pair_mma(d, a_hi | (halo + (unsigned)p.t.off[i + k] * 8u), b_hi | b_lo, lo ? id_lo : id_hi, lo ? (started | (unsigned)k) : (unsigned)k, nks);
+              pair_commit(&b_empty[bs]);
+              if (lo) started = 1u;
+              else { pair_commit(&seg_full[seg & 1u]); ++seg; }
+              stage_addr += stage_bytes;
+              if (++bs == (unsigned)p.stages) { bs = 0; bpar ^= 1u; stage_addr = b_base; }
+            }
+            if (!ok) break;
+            pair_commit(&a_empty[as]);
+            if (++as == (unsigned)p.halos) { as = 0; apar ^= 1u; }
+          }
+        }
+        if (!ok) break;
+        pair_commit(&item_full[buf]);
+      }
+    }
+  } else if (warp >= 4) {
+    // =========================== epilogue: set `set` takes channels [set * HW, set * HW + HW) of the block ===========================
+    const int q = warp & 3, set = (warp - 4) >> 2;
+    const int slot = (lane >> 3) & 1, prow = 2 * q + (lane >> 4), pcol = lane & 7;
+    const unsigned lane_base = tmem_base + ((unsigned)(q * 32) << 16);
+    int segs_per_chunk = 0;
+    for (int v = 0; v < nv; ++v) segs_per_chunk += (p.t.first[v + 1] - p.t.first[v] + p.tps - 1) / p.tps;
+    const int segs = segs_per_chunk * p.n_chunks;
+    unsigned item_idx = 0, seg = 0;
+    bool ok = true;
+    for (int item = bid; item < n_items && ok; item += nblk, ++item_idx) {
+      const int quad = item / n_cblk, cb = item - quad * n_cblk;
+      const unsigned buf = item_idx & 1u;
+      const int e = 4 * quad + 2 * (int)crank + slot;
+      int t = e < n_active ? p.list[e] : -1;
+      if (t >= ntiles_total) t = -1;
+      const int tx = (t >= 0) ? (t % TWo) * 8 : 0, ty = (t >= 0) ? ((t / TWo) % THo) * 8 : 0, n = (t >= 0) ? t / (TWo * THo) : 0;
+      const bool valid = t >= 0 && ty + prow < p.hout && tx + pcol < p.wout;
+      const int64_t pix = valid ? (int64_t)(n * p.hout + ty + prow) * p.wout + tx + pcol : 0;
+      float acc[HW];
+#pragma unroll
+      for (int i = 0; i < HW; ++i) acc[i] = 0.0f;
+      for (int s = 0; s < segs; ++s, ++seg) {
+        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&seg_full[seg & 1u], (seg >> 1) & 1u, &s_abort, p.spin_limit)))) break;
+        tc_fence_after();
+        const unsigned c = lane_base + (seg & 1u) * (2u * CB) + (unsigned)set * CB;     // [hi | lo] columns of this set's channels
+#pragma unroll
+        for (int g = 0; g < HW; g += 16) {
+          tmem_add16(c + g, acc + g);
+          tmem_add16(c + HW + g, acc + g);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&seg_empty[seg & 1u]), 0));
+      }
+      if (!ok) break;
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait(&item_full[buf], (item_idx >> 1) & 1u, &s_abort, p.spin_limit)))) break;
+      tc_fence_after();
+#pragma unroll
+      for (int g = 0; g < HW; g += 16) tmem_add16(lane_base + item_col + buf * CB + (unsigned)(set * HW + g), acc + g);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&item_empty[buf]), 0));
+      const int co = cb * CB + set * HW;
+      if (valid) {
+#pragma unroll
+        for (int h = 0; h < HW / 4; ++h) {
+          const int c = co + 4 * h;
+          if (c >= p.cout) break;
+          float4 v = make_float4(acc[4 * h], acc[4 * h + 1], acc[4 * h + 2], acc[4 * h + 3]);
+          if (p.bias) v = f4add(v, make_float4(__ldg(p.bias + c), __ldg(p.bias + c + 1), __ldg(p.bias + c + 2), __ldg(p.bias + c + 3)));
+          if (p.addend) v = f4add(v, *reinterpret_cast<const float4 *>(p.addend + pix * p.addend_ps + c));
+          if (p.act != MIE_ACT_NONE) {
+            *reinterpret_cast<float4 *>(p.res + pix * p.res_ps + c) = v;
+            v = make_float4(act_apply(p.act, v.x), act_apply(p.act, v.y), act_apply(p.act, v.z), act_apply(p.act, v.w));
+          }
+          *reinterpret_cast<float4 *>(p.out + pix * p.out_ps + c) = v;
+        }
+      }
+      // every pixel written is marked; ballot bytes: [tile 0 row 2q][tile 1 row 2q][tile 0 row 2q+1][tile 1 row 2q+1]
+      const unsigned bal = __ballot_sync(0xffffffffu, valid);
+      if ((lane == 0 || lane == 8) && t >= 0) {
+        const unsigned rows = ((bal >> lane) & 0xFFu) | (((bal >> (16 + lane)) & 0xFFu) << 8);
+        if (rows) atomicOr(p.out_bits32 + 2 * (size_t)t + (q >> 1), rows << ((q & 1) * 16));
+      }
+    }
+  }
+
+  // ---- teardown ----
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (s_abort) {
+    if (tid == 0) atomicOr(&p.counts[3], MIE_ERR_WAIT_EXPIRED);
+    if (warp == 0) { const long long t0 = clock64(); while (clock64() - t0 < 2000000) { } }
+    __syncthreads();
+  }
+  pair_cluster_sync();
+  if (warp == 2) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+  }
+  run_tail_job(p.tail);
+}
+
+}  // namespace
+
+bool exact_takes(const mie_conv_args *a) {
+  return a->refresh && !a->head && a->wpacked_exact && a->in_lo && a->k >= 3 && a->k <= 7 && (a->stride == 1 || a->stride == 2) && !a->in2 && !a->accum &&
+         a->in_ps % 4 == 0 && aligned16(a->in) && aligned16(a->in_lo) && aligned16(a->wpacked_exact) && a->cout % 4 == 0 && a->out_ps % 4 == 0 &&
+         aligned16(a->out) && (!a->res || (a->res_ps % 4 == 0 && aligned16(a->res))) && (!a->addend || (a->addend_ps % 4 == 0 && aligned16(a->addend))) &&
+         a->cout_pad % 32 == 0;
+}
+
+int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
+  ExactParams p;
+  memset(&p, 0, sizeof(p));
+  p.spin_limit = g_opt_spin_limit;
+  p.cin = a->cin; p.cout = a->cout; p.cout_pad = a->cout_pad; p.n_chunks = divup(a->cin, 32);
+  p.n = a->n; p.hout = a->hout; p.wout = a->wout;
+  p.list = a->list; p.counts = a->counts; p.max_tiles = a->max_tiles;
+  p.out = a->out; p.out_ps = a->out_ps; p.out_bits32 = reinterpret_cast<unsigned int *>(a->out_bits);
+  p.act = a->act; p.res = a->res; p.res_ps = a->res_ps; p.addend = a->addend; p.addend_ps = a->addend_ps; p.bias = a->bias;
+  p.tail = tail_for_kernel(a->tail);
+  pair_make_taps(a->k, a->stride, a->pad, &p.t, &p.wp);
+  const int quads = divup(a->max_tiles, 4), clusters_max = MIE_SM_COUNT / 2;
+  // 64 channels per block (107 clocks per K-slice and tap) unless blocks of 32 (82) take fewer clocks over all rounds
+  p.cb = 32;
+  if (a->cout_pad % 64 == 0 &&
+      (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 107 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 82)
+    p.cb = 64;
+  const int halo_bytes = (p.wp * 2 * p.wp * 128 + 1023) & ~1023, budget = 222 * 1024;
+  p.tps = 4;                       // additions into one segment accumulator: 4 taps x 4 K-slices
+  const int stage_bytes = p.tps * p.cb * 128;
+  p.halos = EXACT_MAX_HALOS;
+  while (p.halos > 2 && budget - p.halos * halo_bytes < 3 * stage_bytes) --p.halos;
+  p.stages = (budget - p.halos * halo_bytes) / stage_bytes;
+  if (p.stages > EXACT_MAX_STAGES) p.stages = EXACT_MAX_STAGES;
+  if (p.stages < 2) return MIE_EUNSUPPORTED;
+  const size_t smem = (size_t)((p.stages * stage_bytes + 1023) & ~1023) + (size_t)p.halos * halo_bytes + 1024;
+
+  ExactMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  const int s = a->stride;
+  const cuuint32_t box_in[4] = {32, (cuuint32_t)p.wp, 1, 1};
+  for (int v = 0; v < p.t.nviews; ++v) {
+    const int py = s == 2 ? v >> 1 : 0, px = s == 2 ? v & 1 : 0;
+    const cuuint64_t dims[4] = {(cuuint64_t)a->cin, (cuuint64_t)((a->win - px + s - 1) / s), (cuuint64_t)((a->hin - py + s - 1) / s), (cuuint64_t)a->n};
+    const cuuint64_t str[3] = {(cuuint64_t)a->in_ps * 4 * s, (cuuint64_t)a->win * a->in_ps * 4 * s, (cuuint64_t)a->hin * a->win * a->in_ps * 4};
+    const int64_t off = ((int64_t)py * a->win + px) * a->in_ps;
+    if (!tc_encode(&maps.hi[v], 4, a->in + off, dims, str, box_in, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !tc_encode(&maps.lo[v], 4, a->in_lo + off, dims, str, box_in, CU_TENSOR_MAP_SWIZZLE_128B))
+      return MIE_EINVAL;
+  }
+  {
+    // [tap][chunk][hi rows | lo rows][32]
+    const cuuint64_t rows = 2 * (cuuint64_t)a->cout_pad, nch = (cuuint64_t)p.n_chunks;
+    const cuuint64_t dims[4] = {32, rows, nch, (cuuint64_t)(a->k * a->k)};
+    const cuuint64_t str[3] = {128, rows * 128, nch * rows * 128};
+    const cuuint32_t box_w[4] = {32, (cuuint32_t)(p.cb / 2), 1, 1};
+    if (!tc_encode(&maps.w, 4, a->wpacked_exact, dims, str, box_w, CU_TENSOR_MAP_SWIZZLE_128B)) return MIE_EINVAL;
+  }
+  const int64_t items = (int64_t)quads * (a->cout_pad / p.cb);
+  const int clusters = (int)(items < clusters_max ? items : clusters_max);
+  static int smem_set[2][MAX_DEVICES] = {{0}};
+  auto launch = [&](auto kernel, int i) {
+    const int r = ensure_dynamic_smem(kernel, smem_set[i], smem);
+    if (r != MIE_OK) return r;
+    launch_chained_cluster(kernel, dim3((unsigned)(2 * clusters)), dim3(EXACT_THREADS), smem, st, 2, p, maps);
+    return check_launch();
+  };
+  return p.cb == 64 ? launch(conv_exact_kernel<32>, 1) : launch(conv_exact_kernel<16>, 0);
+}
+
+// Round to nearest TF32 (10 mantissa bits); NaN and infinity pass through.
+__device__ __forceinline__ float round_tf32(float v) {
+  unsigned r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
+  return __uint_as_float(r);
+}
+
+// hi = round(v), lo = round(v - hi): one pass over a dense field, a thread per four channels of a pixel.  HBM bound.
+__global__ void __launch_bounds__(256) split_exact_kernel(const float *__restrict__ in, int64_t in_ps, int C, int64_t pixels, float *__restrict__ hi,
+                                                          float *__restrict__ lo, int64_t out_ps, int quads, int vec) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const int64_t total = pixels * quads;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t px = i / quads;
+    const int c = (int)(i - px * quads) * 4;
+    float v[4];
+    if (vec) {
+      const float4 x = *reinterpret_cast<const float4 *>(in + px * in_ps + c);
+      v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = c + j < C ? in[px * in_ps + c + j] : 0.0f;
+    }
+    float h[4], l[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { h[j] = round_tf32(v[j]); l[j] = round_tf32(v[j] - h[j]); }
+    *reinterpret_cast<float4 *>(hi + px * out_ps + c) = make_float4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<float4 *>(lo + px * out_ps + c) = make_float4(l[0], l[1], l[2], l[3]);
+  }
+}
+
+// [tap][chunk][hi: cout_pad rows | lo: cout_pad rows][32] <- w[cout][cin][ky][kx], zero padded
+__global__ void pack_weights_exact_kernel(const float *__restrict__ w, int cout, int cin, int k, int nch, int cout_pad, float *__restrict__ wp, int64_t total) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int cl = (int)(i % 32);
+    int64_t rest = i / 32;
+    const int row = (int)(rest % (2 * cout_pad));
+    rest /= 2 * cout_pad;
+    const int ci = (int)(rest % nch) * 32 + cl, tap = (int)(rest / nch), co = row < cout_pad ? row : row - cout_pad;
+    float v = 0.0f;
+    if (co < cout && ci < cin) v = w[((int64_t)co * cin + ci) * k * k + tap];
+    const float h = round_tf32(v);
+    wp[i] = row < cout_pad ? h : round_tf32(v - h);
+  }
+}
+
+}  // namespace mie
+
+extern "C" int mie_split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, void *stream) {
+  if (!in || !hi || !lo || C <= 0 || pixels <= 0 || in_ps < C || out_ps < (C + 3) / 4 * 4 || out_ps % 4) return MIE_EINVAL;
+  if (!aligned16(hi) || !aligned16(lo)) return MIE_EALIGN;
+  const int quads = divup(C, 4), vec = C % 4 == 0 && in_ps % 4 == 0 && aligned16(in);
+  int64_t blocks = divup64(pixels * quads, 256);
+  if (blocks > MIE_SM_COUNT * 16) blocks = MIE_SM_COUNT * 16;
+  launch_chained(split_exact_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, in, in_ps, C, pixels, hi, lo, out_ps, quads, vec);
+  return check_launch();
+}
+
+extern "C" int mie_conv_pack_dims_exact(int cin, int cout, int k, int64_t *n_floats) {
+  if (cin <= 0 || cout <= 0 || k <= 0 || !n_floats) return MIE_EINVAL;
+  *n_floats = (int64_t)k * k * divup(cin, 32) * 2 * (divup(cout, 32) * 32) * 32;
+  return MIE_OK;
+}
+
+extern "C" int mie_pack_conv_weights_exact(const float *w_oihw, int cout, int cin, int k, float *wpacked, void *stream) {
+  int64_t total;
+  if (!w_oihw || !wpacked) return MIE_EINVAL;
+  const int s = mie_conv_pack_dims_exact(cin, cout, k, &total);
+  if (s != MIE_OK) return s;
+  int64_t blocks = divup64(total, 256);
+  if (blocks > MIE_SM_COUNT * 8) blocks = MIE_SM_COUNT * 8;
+  pack_weights_exact_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(w_oihw, cout, cin, k, divup(cin, 32), divup(cout, 32) * 32, wpacked, total);
+  return check_launch();
+}

@@ -22,7 +22,7 @@
 // clock, so it takes 39 / 43 / 64 / 128 clocks for N = 32 / 64 / 128 / 256 (measured with resident operands) where the
 // tensor core itself needs 16 / 32 / 64 / 128.  The filter taps written by TMA share that port: 20.5 / 24.6 / 32.8 / 49 KB
 // per tap and chunk in all.
-#include "mie_tc.cuh"
+#include "mie_pair.cuh"
 
 using namespace mie;
 
@@ -33,15 +33,6 @@ constexpr int PAIR_THREADS = 384;
 constexpr int PAIR_MAX_STAGES = 12;
 constexpr int PAIR_MAX_HALOS = 4;
 constexpr int PAIR_SLAB_BYTES = 128 * 128;    // 32 channels of the 128 pixels of a block, as two tiles of 64 rows of 128 bytes
-
-// The reduction of one channel chunk: for every view of the input a halo origin (relative to the tile's first pixel, in
-// view pixels) and its taps, each an index into the filter and an offset into the halo in units of 128 bytes.
-struct PairTaps {
-  int nviews;
-  int first[5];
-  int x0[4], y0[4];
-  unsigned char tap[49], off[49];
-};
 
 struct PairParams {
   TcParams c;
@@ -55,44 +46,6 @@ struct PairParams {
 struct PairMaps {
   CUtensorMap in[4], w, out, res, emitted;
 };
-
-__device__ __forceinline__ void tma_load_4d_pair(unsigned smem_addr, const CUtensorMap *map, unsigned bar_cluster_addr, int c0, int c1,
-                                                 int c2, int c3) {
-  // .cta_group::2: the barrier may lie in the other block of the pair
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(smem_addr), "l"(reinterpret_cast<unsigned long long>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-
-// Up to four K-slices (8 channels = 32 bytes each) of one tap.  Called by a converged warp; the electing happens inside the
-// asm block, next to the instructions it guards, so that the predicate stays uniform for the compiler.
-__device__ __forceinline__ void pair_mma(unsigned tmem_d, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc, unsigned accumulate,
-                                         unsigned nks) {
-  asm volatile(
-      "{\n\t.reg .pred p, q, e, r1, r2, r3;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.eq.b32 q, 0, 0;\n\t"
-      "setp.gt.and.u32 r1, %5, 1, e;\n\tsetp.gt.and.u32 r2, %5, 2, e;\n\tsetp.gt.and.u32 r3, %5, 3, e;\n\t"
-      "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\t"
-      "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t"
-      "@r1 tcgen05.mma.cta_group::2.kind::tf32 [%0], a1, b1, %3, q;\n\t"
-      "@r2 tcgen05.mma.cta_group::2.kind::tf32 [%0], a2, b2, %3, q;\n\t"
-      "@r3 tcgen05.mma.cta_group::2.kind::tf32 [%0], a3, b3, %3, q;\n\t}"
-      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(nks)
-      : "memory");
-}
-// Arrives on the barrier at the same offset in both blocks once the instructions issued so far have completed.
-__device__ __forceinline__ void pair_commit(unsigned long long *bar) {
-  asm volatile("{\n\t.reg .pred e;\n\t.reg .b16 m;\n\telect.sync _|e, 0xffffffff;\n\tmov.b16 m, 3;\n\t"
-               "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void pair_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
 
 // 16 accumulator columns of this lane's row; two accumulators (taddr2 != taddr) are added.
 __device__ __forceinline__ void tmem_ld16_pair(unsigned taddr, unsigned taddr2, float *v) {
@@ -585,36 +538,9 @@ int launch_conv_pair(const mie_conv_args *a, cudaStream_t st) {
   p.head = tail_for_kernel(a->head);
   p.nb = pair_block_width(a);
 
-  // views and taps
   const int s = a->stride, k = a->k;
-  int lo[2] = {0, 0}, span = k;                 // first offset of a parity, largest number of offsets of a parity
-  if (s == 2) {
-    int cnt[2] = {0, 0};
-    for (int i = 0; i < k; ++i) {
-      const int d = i - a->pad, par = d & 1, off = (d - par) / 2;
-      if (!cnt[par]++) lo[par] = off;           // offsets ascend with i
-    }
-    span = cnt[0] > cnt[1] ? cnt[0] : cnt[1];
-  }
-  P.wp = P.hp = 8 + span - 1;
-  P.t.nviews = s == 2 ? 4 : 1;
-  int nt = 0;
-  for (int v = 0; v < P.t.nviews; ++v) {
-    const int py = v >> 1, px = v & 1;
-    P.t.first[v] = nt;
-    P.t.y0[v] = s == 2 ? lo[py] : -a->pad;
-    P.t.x0[v] = s == 2 ? lo[px] : -a->pad;
-    for (int ky = 0; ky < k; ++ky)
-      for (int kx = 0; kx < k; ++kx) {
-        const int dy = ky - a->pad, dx = kx - a->pad;
-        if (s == 2 && ((dy & 1) != py || (dx & 1) != px)) continue;
-        const int oy = s == 2 ? (dy - py) / 2 - lo[py] : ky, ox = s == 2 ? (dx - px) / 2 - lo[px] : kx;
-        P.t.tap[nt] = (unsigned char)(ky * k + kx);
-        P.t.off[nt] = (unsigned char)(oy * 2 * P.wp + ox);
-        ++nt;
-      }
-  }
-  P.t.first[P.t.nviews] = nt;
+  pair_make_taps(k, s, a->pad, &P.t, &P.wp);
+  P.hp = P.wp;
 
   // Shared memory: epilogue slabs, halo buffers, and the filter ring in what is left.  Taps per stage: enough that a stage
   // lasts several times the 120 clocks its barriers cost the issuer.
@@ -669,10 +595,13 @@ int launch_conv_pair(const mie_conv_args *a, cudaStream_t st) {
   const int64_t items = ((int64_t)a->max_tiles + 3) / 4 * n_cblk;
   int64_t clusters = items < MIE_SM_COUNT / 2 ? items : MIE_SM_COUNT / 2;
   if (a->own_tiles) {
-    // whole groups of n_cblk clusters; a group's share of the tiles must fit the list in its shared memory
+    // Not where several clusters finish a tile (kind 8, off by default): its word then goes through a scratch word and a
+    // ticket per epilogue warp, which costs more than the launch it saves (gates 0 / 1 / 2, one stream: 27.8 / 25.6 / 24.0 us
+    // against 23.6 / 23.1 / 22.2 us with the dilation launch).  Layers of 64 channels in two blocks keep the mode.
+    // Whole groups of n_cblk clusters; a group's share of the tiles must fit the list in its shared memory
     const int64_t groups = clusters / n_cblk, sp = ((int64_t)a->max_tiles + 1) / 2;
     const int64_t ntiles = (int64_t)a->n * divup(a->hout, 8) * divup(a->wout, 8);
-    if ((g_opt_own_kernels & (s == 2 ? 1 : 4)) && groups >= 1 && 2 * ((sp + groups - 1) / groups) <= OWN_MAX && a->max_tiles == ntiles) {
+    if ((g_opt_own_kernels & (n_cblk > 1 && a->cout_pad > 64 ? 8 : s == 2 ? 1 : 4)) && groups >= 1 && 2 * ((sp + groups - 1) / groups) <= OWN_MAX && a->max_tiles == ntiles) {
       p.own = 1;
       p.head = *a->head;
       p.own_words = static_cast<unsigned long long *>(a->own_scratch);

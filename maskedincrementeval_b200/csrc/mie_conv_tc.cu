@@ -977,7 +977,7 @@ bool tc_encode(CUtensorMap *m, int rank, const void *base, const cuuint64_t *dim
 int g_opt_tc_thresholded = 1;               // MIE_OPT_TC_THRESHOLDED
 unsigned g_opt_spin_limit = SPIN_LIMIT;     // MIE_OPT_TC_SPIN_LIMIT
 int g_opt_withhold_loads = 0;               // MIE_OPT_TC_WITHHOLD_LOADS
-int g_opt_ksplit = 1;                       // MIE_OPT_TC_KSPLIT
+int g_opt_ksplit = 0;                       // MIE_OPT_TC_KSPLIT (off: the CTA-pair kernel is faster at every shape the rule accepts)
 int g_opt_own_kernels = 7;                  // MIE_OPT_TC_OWN_KERNELS
 
 namespace {

@@ -34,7 +34,8 @@ extern "C" const char *mie_last_cuda_error(void) { return g_cuda_err; }
 // ---------------------------------------------------------------------------------------------
 // mask words from a delta tensor or an explicit mask tensor: one warp per 8x8 tile
 // ---------------------------------------------------------------------------------------------
-template <typename T, bool VEC4>
+// Any channel count, element by element (odd counts, strides or alignments).
+template <typename T>
 __global__ void __launch_bounds__(256) mask_words_kernel(const T *__restrict__ src, int64_t ps, int C, int N,
                                                          int H, int W, float thr, uint64_t *__restrict__ bits) {
   grid_dependency_wait();
@@ -47,38 +48,69 @@ __global__ void __launch_bounds__(256) mask_words_kernel(const T *__restrict__ s
     const int tx = t % TW, ty = (t / TW) % TH, n = t / (TW * TH);
     const int rows = min(8, H - ty * 8), cols = min(8, W - tx * 8);
     unsigned lo = 0, hi = 0;
-    if (VEC4) {
-      // C % 4 == 0, ps % 4 == 0, base 16-byte aligned: each float4 lies inside one pixel
-      const int c4 = C >> 2;
-      const int per_row = cols * c4;
-      const int total = rows * per_row;
-#pragma unroll 4
-      for (int i = lane; i < total; i += 32) {   // independent 16-byte loads: four in flight per lane
-        const int r = i / per_row, rem = i - r * per_row;
-        const int px = rem / c4, q = rem - px * c4;
-        const float4 v = *reinterpret_cast<const float4 *>(
-            reinterpret_cast<const float *>(src) + ((int64_t)(n * H + ty * 8 + r) * W + tx * 8 + px) * ps + q * 4);
-        const bool a = fabsf(v.x) > thr || fabsf(v.y) > thr || fabsf(v.z) > thr || fabsf(v.w) > thr;
-        const int b = r * 8 + px;
-        if (a) { if (b < 32) lo |= 1u << b; else hi |= 1u << (b - 32); }
-      }
-    } else {
-      const int per_row = cols * C;
-      const int total = rows * per_row;
-      for (int i = lane; i < total; i += 32) {
-        const int r = i / per_row, rem = i - r * per_row;
-        const int px = rem / C, c = rem - px * C;
-        const T v = src[((int64_t)(n * H + ty * 8 + r) * W + tx * 8 + px) * ps + c];
-        bool a;
-        if (sizeof(T) == 4 && thr >= 0.0f) a = fabsf((float)v) > thr;  // float source
-        else a = v != (T)0;                                           // explicit mask source
-        const int b = r * 8 + px;
-        if (a) { if (b < 32) lo |= 1u << b; else hi |= 1u << (b - 32); }
-      }
+    const int per_row = cols * C;
+    const int total = rows * per_row;
+    for (int i = lane; i < total; i += 32) {
+      const int r = i / per_row, rem = i - r * per_row;
+      const int px = rem / C, c = rem - px * C;
+      const T v = src[((int64_t)(n * H + ty * 8 + r) * W + tx * 8 + px) * ps + c];
+      bool a;
+      if (sizeof(T) == 4 && thr >= 0.0f) a = fabsf((float)v) > thr;  // float source
+      else a = v != (T)0;                                           // explicit mask source
+      const int b = r * 8 + px;
+      if (a) { if (b < 32) lo |= 1u << b; else hi |= 1u << (b - 32); }
     }
     lo = __reduce_or_sync(0xffffffffu, lo);
     hi = __reduce_or_sync(0xffffffffu, hi);
     if (lane == 0) bits[t] = ((uint64_t)hi << 32) | lo;
+  }
+}
+
+// 16-byte pieces that lie inside one pixel each, `pieces` of them per pixel (16 bytes = 4 floats or int32, 16 mask bytes).
+// A warp takes half a tile (32 pixels): the word half is one reduction.  Bound by HBM; what the first version spent its
+// time on was two integer divisions per 16 bytes (46 MB of 32 channels: 33 us) -- here consecutive lanes take consecutive
+// pieces of a row of eight pixels, and pixel and piece follow from a division by a loop invariant reciprocal.
+template <bool FLOAT>
+__global__ void __launch_bounds__(256) mask_words_vec_kernel(const uint4 *__restrict__ src, int64_t px_bytes, int pieces, unsigned recip, int N,
+                                                             int H, int W, float thr, unsigned *__restrict__ bits32) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const int TH = (H + 7) >> 3, TW = (W + 7) >> 3;
+  const int halves = 2 * N * TH * TW;
+  const int lane = threadIdx.x & 31;
+  const int warps_per_grid = (gridDim.x * blockDim.x) >> 5;
+  const int total = 32 * pieces;
+  for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < halves; u += warps_per_grid) {
+    const int t = u >> 1;
+    const int tx = t % TW, ty = (t / TW) % TH, n = t / (TW * TH);
+    const int y0 = ty * 8 + (u & 1) * 4, x0 = tx * 8;
+    const char *base = reinterpret_cast<const char *>(src) + ((int64_t)(n * H + y0) * W + x0) * px_bytes;
+    unsigned half = 0;
+#pragma unroll 1
+    for (int i0 = lane; i0 < total; i0 += 256) {
+      uint4 v[8];
+      int px[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {      // eight independent loads in flight
+        const int i = i0 + 32 * j;
+        px[j] = pieces == 1 ? i : (int)__umulhi((unsigned)i, recip);       // i / pieces
+        v[j] = make_uint4(0u, 0u, 0u, 0u);
+        if (i < total && y0 + (px[j] >> 3) < H && x0 + (px[j] & 7) < W)
+          v[j] = *reinterpret_cast<const uint4 *>(base + ((int64_t)(px[j] >> 3) * W + (px[j] & 7)) * px_bytes + (i - px[j] * pieces) * 16);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        bool a;
+        if (FLOAT)
+          a = fabsf(__uint_as_float(v[j].x)) > thr || fabsf(__uint_as_float(v[j].y)) > thr || fabsf(__uint_as_float(v[j].z)) > thr ||
+              fabsf(__uint_as_float(v[j].w)) > thr;
+        else
+          a = (v[j].x | v[j].y | v[j].z | v[j].w) != 0u;
+        if (a) half |= 1u << px[j];
+      }
+    }
+    half = __reduce_or_sync(0xffffffffu, half);
+    if (lane == 0) bits32[u] = half;
   }
 }
 
@@ -115,6 +147,10 @@ static int mask_grid(int ntiles) {
   return blocks < cap ? (blocks > 0 ? blocks : 1) : cap;
 }
 
+// i / pieces = umulhi(i, ceil(2^32 / pieces)) for i < 32 * pieces + 256 while the error i * (pieces - 1) stays below 2^32
+constexpr int MASK_MAX_PIECES = 4096;
+static unsigned piece_reciprocal(int pieces) { return pieces == 1 ? 0u : (unsigned)(((1ull << 32) + pieces - 1) / pieces); }
+
 extern "C" int mie_mask_from_delta(const float *delta, int64_t ps, int N, int C, int H, int W, float thr,
                                    uint64_t *bits, void *stream) {
   if (!delta || !bits || N <= 0 || C <= 0 || H <= 0 || W <= 0 || ps < C || !(thr >= 0.0f)) return MIE_EINVAL;
@@ -127,8 +163,10 @@ extern "C" int mie_mask_from_delta(const float *delta, int64_t ps, int N, int C,
     launch_chained(mask_words_px_kernel<float>, dim3(blocks), dim3(256), 0, st, delta, ps, C, N, H, W, thr, reinterpret_cast<unsigned *>(bits));
     return check_launch();
   }
-  if (vec) launch_chained(mask_words_kernel<float, true>, dim3(mask_grid(ntiles)), dim3(256), 0, st, delta, ps, C, N, H, W, thr, bits);
-  else launch_chained(mask_words_kernel<float, false>, dim3(mask_grid(ntiles)), dim3(256), 0, st, delta, ps, C, N, H, W, thr, bits);
+  if (vec && C / 4 <= MASK_MAX_PIECES)
+    launch_chained(mask_words_vec_kernel<true>, dim3(mask_grid(2 * ntiles)), dim3(256), 0, st, reinterpret_cast<const uint4 *>(delta), ps * 4, C / 4,
+                   piece_reciprocal(C / 4), N, H, W, thr, reinterpret_cast<unsigned *>(bits));
+  else launch_chained(mask_words_kernel<float>, dim3(mask_grid(ntiles)), dim3(256), 0, st, delta, ps, C, N, H, W, thr, bits);
   return check_launch();
 }
 
@@ -137,12 +175,17 @@ extern "C" int mie_mask_from_mask(const void *mask, int elem_size, int64_t mps, 
   if (!mask || !bits || N <= 0 || cm <= 0 || H <= 0 || W <= 0 || mps < cm) return MIE_EINVAL;
   const int ntiles = N * divup(H, 8) * divup(W, 8);
   cudaStream_t st = (cudaStream_t)stream;
+  if (elem_size != 1 && elem_size != 4) return MIE_EUNSUPPORTED;
+  const int pieces = cm * elem_size / 16;
+  if (cm * elem_size % 16 == 0 && mps * elem_size % 16 == 0 && aligned16(mask) && pieces <= MASK_MAX_PIECES) {
+    launch_chained(mask_words_vec_kernel<false>, dim3(mask_grid(2 * ntiles)), dim3(256), 0, st, (const uint4 *)mask, mps * elem_size, pieces,
+                   piece_reciprocal(pieces), N, H, W, 0.0f, reinterpret_cast<unsigned *>(bits));
+    return check_launch();
+  }
   if (elem_size == 1)
-    launch_chained(mask_words_kernel<uint8_t, false>, dim3(mask_grid(ntiles)), dim3(256), 0, st, (const uint8_t *)mask, mps, cm, N, H, W, -1.0f, bits);
-  else if (elem_size == 4)
-    launch_chained(mask_words_kernel<int32_t, false>, dim3(mask_grid(ntiles)), dim3(256), 0, st, (const int32_t *)mask, mps, cm, N, H, W, -1.0f, bits);
+    launch_chained(mask_words_kernel<uint8_t>, dim3(mask_grid(ntiles)), dim3(256), 0, st, (const uint8_t *)mask, mps, cm, N, H, W, -1.0f, bits);
   else
-    return MIE_EUNSUPPORTED;
+    launch_chained(mask_words_kernel<int32_t>, dim3(mask_grid(ntiles)), dim3(256), 0, st, (const int32_t *)mask, mps, cm, N, H, W, -1.0f, bits);
   return check_launch();
 }
 
@@ -202,11 +245,47 @@ __global__ void __launch_bounds__(256) tiles_dilate_kernel(
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  int na, ns;
-  block_ordered_compact2([&](int i) { return (int)__ldcg(flags + i); }, ntiles, list, stale, &na, &ns);
+  // One chunk of consecutive tiles per thread: count it, scan the counts over the block, write it out.  (A sweep of the
+  // whole block over 256 tiles at a time costs three barriers and a round trip per step: 38400 tiles took 75 us.)
+  __shared__ int s_wa[8], s_wb[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int chunk = ((ntiles + 255) / 256 + 15) & ~15, lo = min((int)threadIdx.x * chunk, ntiles), hi = min(lo + chunk, ntiles);
+  const bool vec = aligned16(flags);
+  int ca = 0, cs = 0;
+  auto sweep = [&](auto &&visit) {     // visit(first tile, flag bytes of four tiles)
+    int i = lo;
+    if (vec)
+      for (; i + 16 <= hi; i += 16) {
+        const uint4 f = __ldcg(reinterpret_cast<const uint4 *>(flags + i));
+        visit(i, f.x); visit(i + 4, f.y); visit(i + 8, f.z); visit(i + 12, f.w);
+      }
+    for (; i < hi; ++i) visit(i, (unsigned)__ldcg(flags + i));
+  };
+  sweep([&](int, unsigned f) { ca += __popc(f & 0x01010101u); cs += __popc(f & 0x02020202u); });
+  int ia = ca, is = cs;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, ia, d), b = __shfl_up_sync(0xffffffffu, is, d);
+    if (lane >= d) { ia += a; is += b; }
+  }
+  if (lane == 31) { s_wa[warp] = ia; s_wb[warp] = is; }
+  __syncthreads();
+  int oa = ia - ca, os = is - cs, na = 0, ns = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    if (w < warp) { oa += s_wa[w]; os += s_wb[w]; }
+    na += s_wa[w];
+    ns += s_wb[w];
+  }
+  sweep([&](int i, unsigned f) {
+    for (int k = 0; f; ++k, f >>= 8) {
+      if (f & 1u) list[oa++] = i + k;
+      else if ((f & 2u) && stale) stale[os++] = i + k;
+    }
+  });
   if (threadIdx.x == 0) {
     counts[0] = na;
-    counts[1] = ns;
+    counts[1] = stale ? ns : 0;
     counts[2] = 0;
   }
 }

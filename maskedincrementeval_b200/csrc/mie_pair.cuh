@@ -1,0 +1,90 @@
+// What the CTA-pair convolution kernels share: taps and views of the reduction, cta_group::2 wrappers.
+#pragma once
+#include "mie_tc.cuh"
+
+namespace mie {
+namespace {
+
+// The reduction of one channel chunk: for every view of the input a halo origin (relative to the tile's first pixel, in
+// view pixels) and its taps, each an index into the filter and an offset into the halo in units of 128 bytes.
+struct PairTaps {
+  int nviews;
+  int first[5];
+  int x0[4], y0[4];
+  unsigned char tap[49], off[49];
+};
+
+// Views and taps of a k x k filter with this stride and padding; *wp: halo extent (rows and columns) of a tile in a view.
+// Stride 1: one view, the input itself.  Stride 2: four parity views (row parity * 2 + column parity).
+static inline void pair_make_taps(int k, int stride, int pad, PairTaps *t, int *wp) {
+  const int s = stride;
+  int lo[2] = {0, 0}, span = k;                 // first offset of a parity, largest number of offsets of a parity
+  if (s == 2) {
+    int cnt[2] = {0, 0};
+    for (int i = 0; i < k; ++i) {
+      const int d = i - pad, par = d & 1, off = (d - par) / 2;
+      if (!cnt[par]++) lo[par] = off;           // offsets ascend with i
+    }
+    span = cnt[0] > cnt[1] ? cnt[0] : cnt[1];
+  }
+  *wp = 8 + span - 1;
+  t->nviews = s == 2 ? 4 : 1;
+  int nt = 0;
+  for (int v = 0; v < t->nviews; ++v) {
+    const int py = v >> 1, px = v & 1;
+    t->first[v] = nt;
+    t->y0[v] = s == 2 ? lo[py] : -pad;
+    t->x0[v] = s == 2 ? lo[px] : -pad;
+    for (int ky = 0; ky < k; ++ky)
+      for (int kx = 0; kx < k; ++kx) {
+        const int dy = ky - pad, dx = kx - pad;
+        if (s == 2 && ((dy & 1) != py || (dx & 1) != px)) continue;
+        const int oy = s == 2 ? (dy - py) / 2 - lo[py] : ky, ox = s == 2 ? (dx - px) / 2 - lo[px] : kx;
+        t->tap[nt] = (unsigned char)(ky * k + kx);
+        t->off[nt] = (unsigned char)(oy * 2 * *wp + ox);
+        ++nt;
+      }
+  }
+  t->first[t->nviews] = nt;
+}
+
+__device__ __forceinline__ void tma_load_4d_pair(unsigned smem_addr, const CUtensorMap *map, unsigned bar_cluster_addr, int c0, int c1,
+                                                 int c2, int c3) {
+  // .cta_group::2: the barrier may lie in the other block of the pair
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_addr), "l"(reinterpret_cast<unsigned long long>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+
+// Up to four K-slices (8 channels = 32 bytes each) of one tap.  Called by a converged warp; the electing happens inside the
+// asm block, next to the instructions it guards, so that the predicate stays uniform for the compiler.
+__device__ __forceinline__ void pair_mma(unsigned tmem_d, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc, unsigned accumulate,
+                                         unsigned nks) {
+  asm volatile(
+      "{\n\t.reg .pred p, q, e, r1, r2, r3;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.eq.b32 q, 0, 0;\n\t"
+      "setp.gt.and.u32 r1, %5, 1, e;\n\tsetp.gt.and.u32 r2, %5, 2, e;\n\tsetp.gt.and.u32 r3, %5, 3, e;\n\t"
+      "add.u64 a1, %1, 2;\n\tadd.u64 a2, %1, 4;\n\tadd.u64 a3, %1, 6;\n\t"
+      "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t"
+      "@r1 tcgen05.mma.cta_group::2.kind::tf32 [%0], a1, b1, %3, q;\n\t"
+      "@r2 tcgen05.mma.cta_group::2.kind::tf32 [%0], a2, b2, %3, q;\n\t"
+      "@r3 tcgen05.mma.cta_group::2.kind::tf32 [%0], a3, b3, %3, q;\n\t}"
+      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(nks)
+      : "memory");
+}
+// Arrives on the barrier at the same offset in both blocks once the instructions issued so far have completed.
+__device__ __forceinline__ void pair_commit(unsigned long long *bar) {
+  asm volatile("{\n\t.reg .pred e;\n\t.reg .b16 m;\n\telect.sync _|e, 0xffffffff;\n\tmov.b16 m, 3;\n\t"
+               "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void pair_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
+}  // namespace
+}  // namespace mie

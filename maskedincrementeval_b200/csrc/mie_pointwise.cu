@@ -1147,6 +1147,46 @@ __global__ void __launch_bounds__(PW_THREADS) accumulate_kernel(float *__restric
   }
 }
 
+// 16-byte version; a block takes 32 channels of a tile, a thread four pixels of one channel quad, all its loads in flight
+// at once.  KEEP: also kept = d on the whole tile and kept_bits = its word (the delta handed to the next step), one pass
+// instead of an accumulation and two copies.  Bound by HBM (64 channels at 132x176: 40 -> 5 us).
+template <bool KEEP>
+__global__ void __launch_bounds__(128) accumulate_vec_kernel(float *__restrict__ y, int64_t y_ps, const float *__restrict__ d,
+                                                             int64_t d_ps, const uint64_t *__restrict__ d_bits, float *__restrict__ kept,
+                                                             int64_t k_ps, uint64_t *__restrict__ kept_bits, int N, int C, int H, int W) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const int ncb = (C + 31) >> 5, items = N * ((H + 7) >> 3) * ((W + 7) >> 3) * ncb;
+  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    const int t = item / ncb, cb = item - t * ncb, c = cb * 32 + 4 * (threadIdx.x & 7);
+    const uint64_t w = d_bits[t];
+    if (KEEP && cb == 0 && threadIdx.x == 0) kept_bits[t] = w;
+    if ((!KEEP && w == 0ull) || c >= C) continue;
+    const TileGeom g = tile_geom(t, H, W);
+    float4 dv[4], yv[4];
+    bool on[4], in[4];
+    int64_t pix[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int p = (int)(threadIdx.x >> 3) + 16 * j;
+      in[j] = pix_valid(g, p);
+      on[j] = in[j] && ((w >> p) & 1ull);
+      pix[j] = pix_index(g, p, H, W);
+      dv[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (on[j]) {
+        dv[j] = *reinterpret_cast<const float4 *>(d + pix[j] * d_ps + c);
+        yv[j] = *reinterpret_cast<const float4 *>(y + pix[j] * y_ps + c);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (on[j])
+        *reinterpret_cast<float4 *>(y + pix[j] * y_ps + c) = make_float4(yv[j].x + dv[j].x, yv[j].y + dv[j].y, yv[j].z + dv[j].z, yv[j].w + dv[j].w);
+      if (KEEP && in[j]) *reinterpret_cast<float4 *>(kept + pix[j] * k_ps + c) = dv[j];   // zero where the bit is clear, as d is
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // dense activation increment over n contiguous floats (the reference's native entry point)
 // ---------------------------------------------------------------------------------------------
@@ -1603,7 +1643,24 @@ extern "C" int mie_accumulate(float *y, int64_t y_ps, const float *d, int64_t d_
   if (N <= 0 || C <= 0 || H <= 0 || W <= 0 || !d_bits) return MIE_EINVAL;
   MIE_CHECK_FIELD(y, y_ps, C); MIE_CHECK_FIELD(d, d_ps, C);
   const int ntiles = N * divup(H, 8) * divup(W, 8);
+  if (C % 4 == 0 && y_ps % 4 == 0 && d_ps % 4 == 0 && aligned16(y) && aligned16(d)) {
+    launch_chained(accumulate_vec_kernel<false>, dim3(item_grid((int64_t)ntiles * divup(C, 32))), dim3(128), 0, (cudaStream_t)stream, y, y_ps, d, d_ps,
+                   d_bits, nullptr, (int64_t)0, nullptr, N, C, H, W);
+    return check_launch();
+  }
   launch_chained(accumulate_kernel, dim3(tile_grid(ntiles)), dim3(PW_THREADS), 0, (cudaStream_t)stream, y, y_ps, d, d_ps, d_bits, N, C, H, W);
+  return check_launch();
+}
+
+extern "C" int mie_accumulate_keep(float *y, int64_t y_ps, const float *d, int64_t d_ps, const uint64_t *d_bits, float *kept, int64_t k_ps,
+                                   uint64_t *kept_bits, int N, int C, int H, int W, void *stream) {
+  if (N <= 0 || C <= 0 || H <= 0 || W <= 0 || !d_bits || !kept_bits) return MIE_EINVAL;
+  MIE_CHECK_FIELD(y, y_ps, C); MIE_CHECK_FIELD(d, d_ps, C); MIE_CHECK_FIELD(kept, k_ps, C);
+  if (C % 4 || y_ps % 4 || d_ps % 4 || k_ps % 4) return MIE_EUNSUPPORTED;
+  if (!aligned16(y) || !aligned16(d) || !aligned16(kept)) return MIE_EALIGN;
+  const int ntiles = N * divup(H, 8) * divup(W, 8);
+  launch_chained(accumulate_vec_kernel<true>, dim3(item_grid((int64_t)ntiles * divup(C, 32))), dim3(128), 0, (cudaStream_t)stream, y, y_ps, d, d_ps, d_bits,
+                 kept, k_ps, kept_bits, N, C, H, W);
   return check_launch();
 }
 

@@ -44,8 +44,9 @@ class IncrConfig:
                      T = carry + dx; q = k*floor(0.5 + T/k); carry = T - q with this quantisation step k, and the
                      convolution sees q (one more kernel per convolution; what is rounded away stays pending)
     refresh          "native" (default): the networks' dense pass (forward_refresh_reservoirs) runs on this library's
-                     FP32 kernels in dense-evaluation mode -- every tile listed, bias added, state set instead of
-                     advanced; "library": it runs on PyTorch's dense operators (cuDNN), as the reference's does
+                     kernels in dense-evaluation mode -- every tile listed, bias added, state set instead of
+                     advanced, fp32 precision (on the tensor cores from two TF32 parts per operand, unless
+                     ``tensor_cores`` is "off"); "library": it runs on PyTorch's dense operators (cuDNN), as the reference's does
     tail_dilation    True: a convolution's tile dilation rides in the tail of the kernel that produces its input mask
                      (one launch less per convolution; measured slower than the separate launch when launches overlap
                      through programmatic dependent launch, so it is off by default); False: separate launch
@@ -303,16 +304,18 @@ def reset_delta_state(model) -> None:
     """Zero every persistent delta buffer and tile-word array of ``model`` (the module-owned ``Scratch`` buffers and
     the convolution plans).  Called after a dense pass that ran through the kernels: it leaves dense values where the
     incremental steps expect deltas that are exactly zero."""
+    zero = []
     for m in model.modules():
         sc = m.__dict__.get("_scratch")
         if isinstance(sc, Scratch):
-            for t in sc._b.values():
-                t.zero_()
+            zero += sc._b.values()
         for plan in getattr(m, "_plans", {}).values() if hasattr(m, "_plans") else ():
-            plan.out.zero_()
-            plan.out_bits.zero_()
-            plan.counts[:3].zero_()
-            plan.own_scratch.zero_()
+            zero += (plan.out, plan.out_bits, plan.counts[:3], plan.own_scratch)
+    by_type: Dict[torch.dtype, list] = {}
+    for t in zero:
+        by_type.setdefault(t.dtype, []).append(t)
+    for ts in by_type.values():          # a few launches for all buffers instead of one for each
+        torch._foreach_zero_(ts)
 
 
 class Scratch:
@@ -430,6 +433,19 @@ def accumulate(y, d, m: TileMask) -> None:
                                      n, c, h, w, nat.stream_ptr(d.device)), "accumulate")
 
 
+def accumulate_keep(y, d, m: TileMask, kept, kept_bits) -> None:
+    """y += d, and a copy of the delta and its words for the next step."""
+    n, c, h, w = d.shape
+    if c % 4:
+        accumulate(y, d, m)
+        kept.copy_(d)
+        kept_bits.copy_(m.bits)
+        return
+    nat.check(nat.lib.mie_accumulate_keep(y.data_ptr(), pixel_stride(y), d.data_ptr(), pixel_stride(d), m.bits.data_ptr(),
+                                          kept.data_ptr(), pixel_stride(kept), kept_bits.data_ptr(), n, c, h, w,
+                                          nat.stream_ptr(d.device)), "accumulate_keep")
+
+
 def pack_conv_weights(weight: torch.Tensor) -> Tuple[torch.Tensor, int, int]:
     """[Cout,Cin,k,k] -> device buffer laid out [k*k][cin_pad][cout_pad]; returns (buffer, cin_pad, cout_pad)."""
     cout, cin, k, k2 = weight.shape
@@ -454,6 +470,28 @@ def pack_conv_weights_tc(weight: torch.Tensor) -> torch.Tensor:
     nat.check(nat.lib.mie_pack_conv_weights_tc(w.data_ptr(), cout, cin, k, buf.data_ptr(),
                                                nat.stream_ptr(weight.device)), "pack_conv_weights_tc")
     return buf
+
+
+def pack_conv_weights_exact(weight: torch.Tensor) -> torch.Tensor:
+    """[Cout,Cin,k,k] -> device buffer for the dense pass in fp32 precision on the tensor cores (hi and lo rows)."""
+    cout, cin, k, _ = weight.shape
+    nf = C.c_int64()
+    nat.check(nat.lib.mie_conv_pack_dims_exact(cin, cout, k, C.byref(nf)), "pack_dims_exact")
+    w = weight.detach().float().contiguous()
+    buf = torch.empty(nf.value, dtype=torch.float32, device=weight.device)
+    nat.check(nat.lib.mie_pack_conv_weights_exact(w.data_ptr(), cout, cin, k, buf.data_ptr(), nat.stream_ptr(weight.device)),
+              "pack_conv_weights_exact")
+    return buf
+
+
+def split_exact(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Two new channels-last fields hi = tf32(x), lo = tf32(x - hi); channel counts rounded up to 4, the rest zero."""
+    n, c, h, w = x.shape
+    cp = (c + 3) // 4 * 4
+    both = torch.empty((2, n, h, w, cp), dtype=torch.float32, device=x.device)
+    nat.check(nat.lib.mie_split_exact(x.data_ptr(), pixel_stride(x), c, n * h * w, both[0].data_ptr(), both[1].data_ptr(), cp,
+                                      nat.stream_ptr(x.device)), "split_exact")
+    return both[0].permute(0, 3, 1, 2)[:, :c], both[1].permute(0, 3, 1, 2)[:, :c]
 
 
 # A first layer that runs in split precision asks the producer of its input delta for the split copy: the request is

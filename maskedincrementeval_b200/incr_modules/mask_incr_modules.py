@@ -279,6 +279,7 @@ class nnConvIncr(nn.Conv2d):
         self._k, self._s, self._p = _square(self.kernel_size), _square(self.stride), _square(self.padding)
         self.precision = None   # None: TF32 on the tensor cores; "split": split precision there (see _split_input)
         self._packed = {}   # cin_limit -> (version, device, buffer, cin_pad, cout_pad)
+        self._packed_exact = {}   # cin_limit -> (version, buffer): the dense pass in fp32 precision on the tensor cores
         self._plans = {}
         self._cw = None
         self._scratch = Scratch()
@@ -294,8 +295,16 @@ class nnConvIncr(nn.Conv2d):
     def load_state_dict(self, state_dict: 'OrderedDict[str, torch.Tensor]', strict: bool = True):
         r = nn.Conv2d.load_state_dict(self, state_dict, strict=strict)
         self._packed.clear()
+        self._packed_exact.clear()
         self._cw = None
         return r
+
+    def _weights_exact(self, cin: int) -> torch.Tensor:
+        ver = (self.weight._version, self.weight.device, self.weight.data_ptr())
+        hit = self._packed_exact.get(cin)
+        if hit is None or hit[0] != ver:
+            hit = self._packed_exact[cin] = (ver, fl.pack_conv_weights_exact(self.weight[:, :cin]))
+        return hit[1]
 
     def _split_input(self, cin: int) -> bool:
         """Whether this layer runs on the tensor cores in split precision: input [d, d - tf32(d), d] against the
@@ -454,6 +463,7 @@ class nnConvIncr(nn.Conv2d):
                                                plan.counts.data_ptr(), plan.flags.data_ptr(), st), "tiles_dilate")
             fl.offer_tail(job)
         a.in_, a.in_ps, a.cin = d.data_ptr(), fl.pixel_stride(d), cin
+        a.wpacked_exact, a.in_lo = None, None
         a.wpacked, a.cin_pad, a.cout, a.cout_pad = wbuf.data_ptr(), cp, self.out_channels, op
         a.wpacked_tc = wtc.data_ptr() if (wtc is not None and config.tensor_cores == "auto" and not refresh) else None
         a.refresh = 1 if refresh else 0
@@ -476,6 +486,13 @@ class nnConvIncr(nn.Conv2d):
             a.act, a.thr, a.res, a.res_ps, a.emitted, a.emitted_ps = nat.ACT_NONE, 0.0, None, 0, None, 0
         if a.thr > 0.0 or a.emitted:
             nat.set_option(nat.OPT_TC_THRESHOLDED, 1 if config.tc_thresholded else 0)
+        if refresh and config.tensor_cores == "auto" and 3 <= self._k <= 7 and self.out_channels % 4 == 0:
+            # fp32 precision on the tensor cores: the input as two TF32 fields (released after the launch)
+            hi, lo = fl.split_exact(d)
+            wx = self._weights_exact(cin)
+            a.in_, a.in_ps, a.in_lo, a.wpacked_exact = hi.data_ptr(), fl.pixel_stride(hi), lo.data_ptr(), wx.data_ptr()
+            if not nat.lib.mie_conv_is_exact(C.byref(a)):
+                a.in_, a.in_ps, a.in_lo, a.wpacked_exact = d.data_ptr(), fl.pixel_stride(d), None, None
         self.last_used_tensor_cores = bool(nat.lib.mie_conv_uses_tensor_cores(C.byref(a)))
         self.last_cluster_size = int(nat.lib.mie_conv_cluster_size(C.byref(a)))
         if split and not self.last_used_tensor_cores:

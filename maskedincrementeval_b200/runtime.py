@@ -158,12 +158,8 @@ class IncrementalRunner:
         """After an incremental step: accumulate its state deltas and keep a copy for the next step (the network's own
         buffers are overwritten by that step while it still reads them)."""
         for (h, c), (dh, bh, dc, bc), ((sh, mh), (sc, mc)) in zip(self._states, self._prev_incr, states_incr):
-            fl.accumulate(h, sh, mh)
-            fl.accumulate(c, sc, mc)
-            dh.copy_(sh)
-            bh.copy_(mh.bits)
-            dc.copy_(sc)
-            bc.copy_(mc.bits)
+            fl.accumulate_keep(h, sh, mh, dh, bh)
+            fl.accumulate_keep(c, sc, mc, dc, bc)
 
     # -- incremental pass ------------------------------------------------------------------------
     def _step_body(self):

@@ -1,0 +1,106 @@
+"""The dense pass in fp32 precision on the tensor cores, and the vectorised mask, dilation and feedback kernels, at the
+sizes where they change path."""
+import ctypes as C
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+from oracle import restatement as R  # noqa: E402
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    torch.backends.cudnn.allow_tf32 = False
+    torch.backends.cuda.matmul.allow_tf32 = False
+    return torch.device("cuda:0")
+
+
+def cl(t):
+    return t.contiguous(memory_format=torch.channels_last)
+
+
+# cin, cout, k, stride, n, h, w, addend: ragged tiles, one pair of tiles, partial chunks and slabs, both block widths
+@pytest.mark.parametrize("case", [(5, 32, 5, 1, 1, 41, 50, False), (2, 64, 3, 2, 1, 18, 26, False), (64, 40, 3, 1, 2, 8, 16, False),
+                                  (32, 64, 5, 2, 1, 67, 89, False), (256, 256, 3, 1, 1, 33, 44, True), (256, 128, 5, 1, 1, 34, 44, False),
+                                  (96, 96, 7, 1, 1, 24, 40, False), (130, 36, 3, 1, 1, 9, 9, False)])
+def test_dense_pass_against_float64(dev, case):
+    from maskedincrementeval_b200 import fields as fl, _native as nat
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    cin, cout, k, s, n, h, w, with_addend = case
+    torch.manual_seed(1)
+    layer = ConvLayerIncr(cin, cout, k, s, k // 2, activation="sigmoid").to(dev).eval()
+    g = torch.Generator(device=dev).manual_seed(2)
+    x = cl(torch.randn(n, cin, h, w, generator=g, device=dev))
+    c = layer.conv2d
+    want = F.conv2d(x.double(), c.weight.detach().double(), c.bias.detach().double(), stride=s, padding=k // 2)
+    addend = None
+    if with_addend:
+        addend = [cl(torch.randn(want.shape, generator=g, device=dev)), fl.full_mask(n, *want.shape[2:], dev)]
+        want = want + addend[0].double()
+    err = {}
+    old = fl.config.tensor_cores
+    try:
+        for mode in ("auto", "off"):
+            fl.config.tensor_cores = mode
+            with torch.no_grad():
+                y, m = NATIVE.conv(c, NATIVE.lift(x), layer.activation, addend=addend)
+            assert bool(nat.lib.mie_conv_is_exact(C.byref(c._plan(n, h, w, dev).args))) == (mode == "auto")
+            res = layer.activation.in_res.reservoir
+            err[mode] = float((res.double() - want).norm() / want.norm())
+            assert float((y.double() - torch.sigmoid(res.double())).abs().max()) <= 1e-6
+            assert bool(m.pixel_mask().all())
+    finally:
+        fl.config.tensor_cores = old
+    # no worse than the CUDA-core kernel's own rounding (3e-7 for the shortest reductions to 1.4e-6 for the longest)
+    assert err["auto"] <= max(1.2 * err["off"], 6e-7), err
+
+
+@pytest.mark.parametrize("c,dtype", [(20, torch.float32), (32, torch.float32), (132, torch.float32), (16, torch.uint8), (48, torch.uint8), (20, torch.int32)])
+def test_mask_words_vectorised(dev, c, dtype):
+    from maskedincrementeval_b200 import fields as fl
+    g = torch.Generator(device=dev).manual_seed(c)
+    n, h, w = 2, 21, 43
+    x = torch.randn(n, c, h, w, generator=g, device=dev) * (torch.rand(n, c, h, w, generator=g, device=dev) < 0.01)
+    x = cl(x if dtype == torch.float32 else (x != 0).to(dtype))
+    m = fl.mask_from_delta(x) if dtype == torch.float32 else fl.mask_from_tensor(x)
+    assert torch.equal(m.pixel_mask(), (x != 0).any(1, keepdim=True).to(torch.uint8))
+
+
+@pytest.mark.parametrize("n,h,w", [(1, 200, 168), (8, 480, 640), (3, 260, 346)])
+def test_dilation_of_large_fields(dev, n, h, w):
+    from maskedincrementeval_b200 import fields as fl, _native as nat
+    g = torch.Generator().manual_seed(n)
+    for frac in (0.0, 0.002, 1.0):
+        act = (torch.rand(n, 1, h, w, generator=g) < frac).to(torch.uint8)
+        m = fl.mask_from_tensor(act.to(dev))
+        nt = fl.n_tiles(n, h, w)
+        lst, stale = (torch.zeros(nt, dtype=torch.int32, device=dev) for _ in range(2))
+        counts, flags = torch.zeros(4, dtype=torch.int32, device=dev), torch.zeros(nt, dtype=torch.uint8, device=dev)
+        words = torch.full((nt,), 3, dtype=torch.int64, device=dev)
+        nat.check(nat.lib.mie_tiles_dilate(m.bits.data_ptr(), n, h, w, h, w, 5, 1, 2, None, words.data_ptr(), lst.data_ptr(), stale.data_ptr(),
+                                           counts.data_ptr(), flags.data_ptr(), nat.stream_ptr(dev)), "dilate")
+        want = R.tile_list(R.conv_out_mask(act, 5, 1, 2)).tolist()
+        na, ns = counts[:2].tolist()
+        assert lst[:na].tolist() == want and na + ns == nt
+        assert stale[:ns].tolist() == sorted(set(range(nt)) - set(want)) and int(words.abs().max()) == 0
+
+
+def test_accumulate_and_keep(dev):
+    from maskedincrementeval_b200 import fields as fl
+    g = torch.Generator(device=dev).manual_seed(3)
+    for c in (4, 36, 64):
+        y = cl(torch.randn(2, c, 19, 45, generator=g, device=dev))
+        kept = cl(torch.randn(2, c, 19, 45, generator=g, device=dev))
+        d = cl(torch.randn(2, c, 19, 45, generator=g, device=dev) * (torch.rand(2, 1, 19, 45, generator=g, device=dev) < 0.1))
+        m, kb = fl.mask_from_delta(d), fl.new_bits(2, 19, 45, dev)
+        want = y + d
+        z = y.clone(memory_format=torch.channels_last)
+        fl.accumulate(z, d, m)
+        fl.accumulate_keep(y, d, m, kept, kb)
+        assert torch.equal(y, want) and torch.equal(z, want) and torch.equal(kept, d) and torch.equal(kb, m.bits)

@@ -236,6 +236,11 @@ typedef struct mie_conv_args {
   const float *in_lo;
 } mie_conv_args;
 
+/* One incremental step of a layer in one call: with `mask_bits`, mie_mask_from_delta of args->in into it (pixels whose
+ * channels all lie within mask_thr are off); with `dilate`, mie_tiles_dilate as that job describes; then mie_conv_tiles. */
+int mie_conv_step(const mie_conv_args *args /* host */, uint64_t *mask_bits, float mask_thr, const mie_tail_job *dilate /* host */,
+                  void *stream);
+
 /* Host only: 1 if mie_conv_tiles would run these arguments in fp32 precision on the tensor cores, else 0. */
 int mie_conv_is_exact(const mie_conv_args *args /* host */);
 

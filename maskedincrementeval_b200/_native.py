@@ -75,6 +75,7 @@ SIGNATURES = {
     "mie_pack_conv_weights": (_i, [_vp, _i, _i, _i, _vp, _vp]),
     "mie_conv_pack_dims_tc": (_i, [_i, _i, _i, C.POINTER(_i), C.POINTER(_i), C.POINTER(_i64)]),
     "mie_pack_conv_weights_tc": (_i, [_vp, _i, _i, _i, _vp, _vp]),
+    "mie_conv_step": (_i, [C.POINTER(ConvArgs), _vp, _f, _vp, _vp]),
     "mie_conv_is_exact": (_i, [C.POINTER(ConvArgs)]),
     "mie_split_exact": (_i, [_vp, _i64, _i, _i64, _vp, _vp, _i64, _vp]),
     "mie_conv_pack_dims_exact": (_i, [_i, _i, _i, C.POINTER(_i64)]),
@@ -146,8 +147,13 @@ def check(status: int, what: str = "") -> None:
     raise MieError(f"libmie {what}: {msg}")
 
 
+option_epoch = [0]      # counts the changes of the library's options: what was decided under others is decided again
+
+
 def set_option(option: int, value: int) -> None:
     check(lib.mie_set_option(option, int(value)), "set_option")
+    if option != OPT_LAUNCH_COUNT:
+        option_epoch[0] += 1
 
 
 def get_option(option: int) -> int:
@@ -172,8 +178,14 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)    # the stream's address without a Stream object around it
+
+
 def stream_ptr(device=None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = None if device is None else device.index
+    if _raw_stream is None or index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(index)
 
 
 def require_cuda(t: torch.Tensor, name: str) -> None:

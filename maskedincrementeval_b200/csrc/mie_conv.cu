@@ -20,6 +20,7 @@ bool tc_eligible(const mie_conv_args *a);
 int launch_conv_tc(const mie_conv_args *a, cudaStream_t st);
 bool exact_takes(const mie_conv_args *a);
 int launch_conv_exact(const mie_conv_args *a, cudaStream_t st);
+int pack_exact(const float *w, int cout, int cin, int k, int ihwo, float *wpacked, cudaStream_t st);
 }  // namespace mie
 
 namespace {
@@ -640,13 +641,26 @@ extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
   return MIE_EUNSUPPORTED;
 }
 
+extern "C" int mie_conv_step(const mie_conv_args *a, uint64_t *mask_bits, float mask_thr, const mie_tail_job *dilate, void *stream) {
+  if (!a) return MIE_EINVAL;
+  int s = MIE_OK;
+  if (mask_bits) s = mie_mask_from_delta(a->in, a->in_ps, a->n, a->cin, a->hin, a->win, mask_thr, mask_bits, stream);
+  if (s == MIE_OK && dilate)
+    s = mie_tiles_dilate(dilate->in_bits, dilate->N, dilate->Hin, dilate->Win, dilate->Hout, dilate->Wout, dilate->k, dilate->stride,
+                         dilate->pad, dilate->union_bits, dilate->out_bits, dilate->list, dilate->stale, dilate->counts, dilate->flags, stream);
+  return s == MIE_OK ? mie_conv_tiles(a, stream) : s;
+}
+
 // ---------------------------------------------------------------------------------------------
 // reference-shaped entry point: conv{k}x{k}_increment_ext(x_incr, mask, filter, out_incr, stride)
 // ---------------------------------------------------------------------------------------------
 namespace {
 struct IncWs {
-  size_t bits_in, bits_out, list, stale, counts, flags, wpacked, total;
+  size_t bits_in, bits_out, counts, list, stale, flags, wpacked, wexact, hi, lo, total;
+  int cp;      // channels of the split input
 };
+// fp32 precision on the tensor cores pays off from a reduction of a few instructions on, whatever the activity
+bool inc_exact(int cin, int cout, int k) { return k >= 3 && cout % 4 == 0 && cin * k * k >= 72; }
 IncWs inc_layout(int N, int cin, int H, int W, int cout, int k, int stride) {
   const int pad = k / 2;
   const int Ho = (H + 2 * pad - k) / stride + 1, Wo = (W + 2 * pad - k) / stride + 1;
@@ -656,13 +670,22 @@ IncWs inc_layout(int N, int cin, int H, int W, int cout, int k, int stride) {
   size_t o = 0;
   w.bits_in = o; o += up(nti * 8);
   w.bits_out = o; o += up(nto * 8);
+  w.counts = o; o += 256;      // behind the output words: both are cleared together
   w.list = o; o += up(nto * 4);
   w.stale = o; o += up(nto * 4);
-  w.counts = o; o += 256;
   w.flags = o; o += up(nto);
   int cp, op; int64_t nf;
   mie_conv_pack_dims(cin, cout, k, &cp, &op, &nf);
   w.wpacked = o; o += up((size_t)nf * 4);
+  w.wexact = w.hi = w.lo = o;
+  w.cp = (cin + 3) / 4 * 4;
+  if (inc_exact(cin, cout, k)) {
+    int64_t ne;
+    mie_conv_pack_dims_exact(cin, cout, k, &ne);
+    o += up((size_t)ne * 4);
+    w.hi = o; o += up((size_t)N * H * W * w.cp * 4);
+    w.lo = o; o += up((size_t)N * H * W * w.cp * 4);
+  }
   w.total = o;
   return w;
 }
@@ -708,8 +731,7 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   float *wp = reinterpret_cast<float *>(ws + L.wpacked);
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e;
-  if ((e = cudaMemsetAsync(counts, 0, 16, st)) != cudaSuccess) { set_cuda_error(e); return MIE_ECUDA; }
-  if ((e = cudaMemsetAsync(bits_out, 0, (size_t)nto * 8, st)) != cudaSuccess) { set_cuda_error(e); return MIE_ECUDA; }
+  if ((e = cudaMemsetAsync(bits_out, 0, L.counts + 16 - L.bits_out, st)) != cudaSuccess) { set_cuda_error(e); return MIE_ECUDA; }
   // the caller hands in uninitialised memory: inactive tiles must read as zero
   if ((e = cudaMemsetAsync(out_incr, 0, (size_t)N * Ho * Wo * cout * 4, st)) != cudaSuccess) { set_cuda_error(e); return MIE_ECUDA; }
   int s;
@@ -718,7 +740,12 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   if (s != MIE_OK) return s;
   int cp, op; int64_t nf;
   mie_conv_pack_dims(cin, cout, k, &cp, &op, &nf);
-  {
+  const bool exact = inc_exact(cin, cout, k) && aligned16(out_incr);
+  float *wx = reinterpret_cast<float *>(ws + L.wexact), *hi = reinterpret_cast<float *>(ws + L.hi), *lo = reinterpret_cast<float *>(ws + L.lo);
+  if (exact) {
+    if ((s = pack_exact(filter, cout, cin, k, 1, wx, st)) != MIE_OK) return s;
+    if ((s = mie_split_exact(x_incr, cin, cin, (int64_t)N * H * W, hi, lo, L.cp, stream)) != MIE_OK) return s;
+  } else {
     int blocks = (int)((nf + 255) / 256);
     if (blocks > MIE_SM_COUNT * 8) blocks = MIE_SM_COUNT * 8;
     pack_weights_ihwo_kernel<<<blocks, 256, 0, st>>>(filter, cout, cin, k, cp, op, wp, nf);
@@ -734,5 +761,10 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   a.list = list; a.stale = nullptr; a.counts = counts; a.max_tiles = nto;
   a.out = out_incr; a.out_ps = cout; a.out_bits = bits_out;
   a.act = MIE_ACT_NONE; a.thr = 0.0f;
+  if (exact) {      // (without bias and activation a dense evaluation is the plain convolution of the listed tiles)
+    a.refresh = 1;
+    a.in = hi; a.in_lo = lo; a.in_ps = L.cp; a.wpacked_exact = wx;
+    if (!exact_takes(&a)) return MIE_EALIGN;
+  }
   return mie_conv_tiles(&a, stream);
 }

@@ -415,7 +415,9 @@ __global__ void __launch_bounds__(256) split_exact_kernel(const float *__restric
 }
 
 // [tap][chunk][hi: cout_pad rows | lo: cout_pad rows][32] <- w[cout][cin][ky][kx], zero padded
-__global__ void pack_weights_exact_kernel(const float *__restrict__ w, int cout, int cin, int k, int nch, int cout_pad, float *__restrict__ wp, int64_t total) {
+// (ihwo: the filter is stored [cin][ky][kx][cout] instead)
+__global__ void pack_weights_exact_kernel(const float *__restrict__ w, int cout, int cin, int k, int nch, int cout_pad, float *__restrict__ wp, int64_t total,
+                                          int ihwo) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int cl = (int)(i % 32);
     int64_t rest = i / 32;
@@ -423,10 +425,20 @@ __global__ void pack_weights_exact_kernel(const float *__restrict__ w, int cout,
     rest /= 2 * cout_pad;
     const int ci = (int)(rest % nch) * 32 + cl, tap = (int)(rest / nch), co = row < cout_pad ? row : row - cout_pad;
     float v = 0.0f;
-    if (co < cout && ci < cin) v = w[((int64_t)co * cin + ci) * k * k + tap];
+    if (co < cout && ci < cin) v = w[ihwo ? ((int64_t)ci * k * k + tap) * cout + co : ((int64_t)co * cin + ci) * k * k + tap];
     const float h = round_tf32(v);
     wp[i] = row < cout_pad ? h : round_tf32(v - h);
   }
+}
+
+int pack_exact(const float *w, int cout, int cin, int k, int ihwo, float *wpacked, cudaStream_t st) {
+  int64_t total;
+  const int s = mie_conv_pack_dims_exact(cin, cout, k, &total);
+  if (s != MIE_OK) return s;
+  int64_t blocks = divup64(total, 256);
+  if (blocks > MIE_SM_COUNT * 8) blocks = MIE_SM_COUNT * 8;
+  pack_weights_exact_kernel<<<(unsigned)blocks, 256, 0, st>>>(w, cout, cin, k, divup(cin, 32), divup(cout, 32) * 32, wpacked, total, ihwo);
+  return check_launch();
 }
 
 }  // namespace mie
@@ -448,12 +460,6 @@ extern "C" int mie_conv_pack_dims_exact(int cin, int cout, int k, int64_t *n_flo
 }
 
 extern "C" int mie_pack_conv_weights_exact(const float *w_oihw, int cout, int cin, int k, float *wpacked, void *stream) {
-  int64_t total;
   if (!w_oihw || !wpacked) return MIE_EINVAL;
-  const int s = mie_conv_pack_dims_exact(cin, cout, k, &total);
-  if (s != MIE_OK) return s;
-  int64_t blocks = divup64(total, 256);
-  if (blocks > MIE_SM_COUNT * 8) blocks = MIE_SM_COUNT * 8;
-  pack_weights_exact_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(w_oihw, cout, cin, k, divup(cin, 32), divup(cout, 32) * 32, wpacked, total);
-  return check_launch();
+  return pack_exact(w_oihw, cout, cin, k, 0, wpacked, (cudaStream_t)stream);
 }

@@ -54,7 +54,7 @@ def _conv_increment(k, x_incr, mask, filter, out_incr, stride):
         if tuple(mask.shape) != tuple(x_incr.shape):
             raise RuntimeError("mask must have the shape of x_incr")
         if mask.dtype == torch.bool:
-            mask = mask.to(torch.uint8)
+            mask = mask.contiguous(memory_format=cl).view(torch.uint8)
         if mask.dtype not in (torch.uint8, torch.int32):
             mask = mask.to(torch.int32)
         mask = mask.contiguous(memory_format=cl)

@@ -266,6 +266,71 @@ class _ConvPlan:
         self.accumulated = False    # ... and reports here that it did
 
 
+class _PreparedCall:
+    """An incremental call of one convolution with everything decided: what a layer that is called again with the same
+    kind of input needs is a few identity checks and one call of the library, where deciding it anew took most of the
+    40 us a small layer's step lasted.  Built at the end of a full call (``nnConvIncr.forward_fused``) and valid while
+    nothing it was decided by has changed: the library's configuration and options, the filter, the activation's state
+    buffers and threshold, the input's geometry and the address of its tile words."""
+    __slots__ = ("activation", "cin_limit", "epoch", "options", "weight", "weight_key", "reservoir", "reservoir_ptr", "emitted",
+                 "threshold", "shape", "stride", "device", "mask_bits", "mask_ptr", "geometry", "plan", "args", "args_ref", "dilate", "tc_option",
+                 "out", "input_threshold", "keep")
+
+    def __init__(self, conv, activation, cin_limit, plan, d, mask, derived, dilate, thresholded):
+        self.activation, self.cin_limit, self.plan = activation, cin_limit, plan     # (not the convolution: that would be a cycle)
+        self.epoch, self.options = config.epoch, nat.option_epoch[0]
+        self.weight = conv.weight
+        self.weight_key = (self.weight._version, self.weight.data_ptr())
+        self.reservoir = self.emitted = self.threshold = None
+        self.reservoir_ptr = 0
+        if activation is not None:
+            self.reservoir, self.emitted, self.threshold = activation.in_res.reservoir, activation.emitted, activation.threshold
+            self.reservoir_ptr = self.reservoir.data_ptr()
+        self.shape, self.stride, self.device = d.shape, d.stride(), d.device
+        self.geometry = (mask.n, mask.h, mask.w)
+        self.mask_bits = mask.bits if derived else None      # the tile words this call derives from the delta itself
+        self.mask_ptr = mask.bits.data_ptr()
+        self.args, self.args_ref = plan.args, C.byref(plan.args)
+        self.dilate = C.addressof(plan.tail.c) if dilate else None
+        self.keep = plan.tail
+        self.tc_option = (1 if config.tc_thresholded else 0) if thresholded else None
+        self.input_threshold = float(config.input_threshold)
+        self.out = (plan.out, plan.mask)
+
+    def run(self, conv, x_incr):
+        """The call's result, or None when it has to be decided anew."""
+        d, m = x_incr[0], x_incr[1]
+        w = conv._parameters["weight"]
+        plan = self.plan
+        if (self.epoch != config.epoch or self.options != nat.option_epoch[0] or d.shape != self.shape or d.stride() != self.stride
+                or d.device != self.device or d.dtype is not torch.float32 or w is not self.weight
+                or (w._version, w.data_ptr()) != self.weight_key or plan.needs_clear or plan.accum_target is not None or plan.tail is not self.keep):
+            return None
+        act = self.activation
+        if act is not None:
+            r = act.in_res.reservoir
+            if r is not self.reservoir or r.data_ptr() != self.reservoir_ptr or act.emitted is not self.emitted or act.threshold != self.threshold:
+                return None
+        ptr = d.data_ptr()
+        if m is None:
+            if self.mask_bits is None:
+                return None
+            mask_ptr = self.mask_ptr
+        elif type(m) is TileMask and self.mask_bits is None and m.bits.data_ptr() == self.mask_ptr and (m.n, m.h, m.w) == self.geometry:
+            mask_ptr = None
+        else:
+            return None
+        if ptr & 15:
+            return None
+        if self.tc_option is not None:
+            nat.lib.mie_set_option(nat.OPT_TC_THRESHOLDED, self.tc_option)
+        self.args.in_ = ptr
+        st = nat.lib.mie_conv_step(self.args_ref, mask_ptr, self.input_threshold, self.dilate, nat.stream_ptr(self.device))
+        if st:
+            nat.check(st, "conv_step")
+        return list(self.out)
+
+
 class nnConvIncr(nn.Conv2d):
     """Convolution of a masked delta (reference ``:146-196``).
 
@@ -281,6 +346,7 @@ class nnConvIncr(nn.Conv2d):
         self._packed = {}   # cin_limit -> (version, device, buffer, cin_pad, cout_pad)
         self._packed_exact = {}   # cin_limit -> (version, buffer): the dense pass in fp32 precision on the tensor cores
         self._plans = {}
+        self._prepared = None     # _PreparedCall of the last full call
         self._cw = None
         self._scratch = Scratch()
 
@@ -388,6 +454,13 @@ class nnConvIncr(nn.Conv2d):
         ``refresh=True`` is the dense evaluation of the same layer on the same kernels: the input pair carries a dense
         tensor, the bias is added, the activation's reservoir is set to conv + bias (+ addend) and the output is
         f(reservoir) -- in full fp32, whatever ``config.tensor_cores`` says."""
+        plain = addend is None and second is None and bn is None and not refresh
+        fast = self._prepared
+        if plain and fast is not None and fast.activation is activation and fast.cin_limit == cin_limit:
+            out = fast.run(self, x_incr)
+            if out is not None:
+                return out
+        self._prepared = None
         sc = self._scratch
         if refresh and bn is not None:
             raise NotImplementedError("dense evaluation with a folded batch-norm")
@@ -485,7 +558,7 @@ class nnConvIncr(nn.Conv2d):
         else:
             a.act, a.thr, a.res, a.res_ps, a.emitted, a.emitted_ps = nat.ACT_NONE, 0.0, None, 0, None, 0
         if a.thr > 0.0 or a.emitted:
-            nat.set_option(nat.OPT_TC_THRESHOLDED, 1 if config.tc_thresholded else 0)
+            nat.lib.mie_set_option(nat.OPT_TC_THRESHOLDED, 1 if config.tc_thresholded else 0)
         if refresh and config.tensor_cores == "auto" and 3 <= self._k <= 7 and self.out_channels % 4 == 0:
             # fp32 precision on the tensor cores: the input as two TF32 fields (released after the launch)
             hi, lo = fl.split_exact(d)
@@ -504,6 +577,9 @@ class nnConvIncr(nn.Conv2d):
         if tgt is not None and not refresh and self.takes_second_input() and tgt.shape == plan.out.shape:
             a.accum, a.accum_ps, plan.accumulated = tgt.data_ptr(), fl.pixel_stride(tgt), True
         nat.check(nat.lib.mie_conv_tiles(C.byref(a), st), "conv_tiles")
+        if (plain and not split and not config.kfenced_step and not config.tail_dilation and not a.accum and (x_incr[1] is None or x_incr[1] is m)
+                and d is x_incr[0] and (activation is None or type(activation).thr is nnReservedActivation.thr) and a.in_ % 16 == 0):
+            self._prepared = _PreparedCall(self, activation, cin_limit, plan, d, m, x_incr[1] is None, not a.head, a.thr > 0.0 or bool(a.emitted))
         if refresh and activation is not None and activation.emitted is not None:
             if activation.emitted.shape == plan.out.shape and activation.thr() > 0.0 and config.carry:
                 activation.emitted.copy_(plan.out)      # what has been sent so far = f(reservoir)

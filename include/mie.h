@@ -241,6 +241,11 @@ typedef struct mie_conv_args {
 int mie_conv_step(const mie_conv_args *args /* host */, uint64_t *mask_bits, float mask_thr, const mie_tail_job *dilate /* host */,
                   void *stream);
 
+/* One dense evaluation of a layer in fp32 precision on the tensor cores in one call: mie_tiles_dilate as `dilate` describes,
+ * mie_split_exact of the field x into args->in and args->in_lo, then mie_conv_tiles. */
+int mie_conv_refresh_step(const mie_conv_args *args /* host */, const float *x, int64_t x_ps, const mie_tail_job *dilate /* host */,
+                          void *stream);
+
 /* Host only: 1 if mie_conv_tiles would run these arguments in fp32 precision on the tensor cores, else 0. */
 int mie_conv_is_exact(const mie_conv_args *args /* host */);
 

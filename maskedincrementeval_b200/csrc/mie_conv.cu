@@ -484,6 +484,131 @@ __global__ void __launch_bounds__(256) conv1x1_small_kernel(const ConvParams p) 
   run_tail_job(p.tail);
 }
 
+// ---------------------------------------------------------------------------------------------
+// 3x3 convolution of one or two input channels (event-count images) in fp32: at 18 multiplications per output the layer is a
+// pass over the state, bound by HBM (per active pixel Cout * 12 bytes).  Block = (tile, 32 output channels), eight lanes per
+// pixel, so that every access of the epilogue covers whole 128-byte lines; filter and input window in shared memory.  The
+// general kernel above stages eight channels and 64 accumulators per thread for this: 2 -> 32 channels, 2 x 256x336: 55 us.
+// Sums in the general kernel's order: same result to the bit.
+// ---------------------------------------------------------------------------------------------
+template <int CIN, int S>
+__global__ void __launch_bounds__(256) conv_few_kernel(const ConvParams p) {
+  constexpr int T = 7 * S + 3;
+  __shared__ float4 s_w[9 * CIN][8];
+  __shared__ float s_in[T * T * CIN];
+  __shared__ unsigned s_bits[2];
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const bool head_ok = run_head_job(p.head, HEAD_SPIN_LIMIT);
+  if (threadIdx.x == blockDim.x - 1) count_head_job_passed(p.head);
+  const int tid = threadIdx.x, lane = tid & 31, q = tid & 7;
+  const int THo = (p.hout + 7) >> 3, TWo = (p.wout + 7) >> 3, ntiles_total = p.n * THo * TWo;
+  const int n_cblk = p.cout_pad >> 5, cb = blockIdx.x % n_cblk, co = cb * 32 + 4 * q;
+  const int first = blockIdx.x / n_cblk, step = gridDim.x / n_cblk;     // the grid is a multiple of n_cblk
+  for (int i = tid; i < 9 * CIN * 8; i += 256) {
+    const int r = i >> 3, tap = r / CIN, c = r - tap * CIN;
+    s_w[r][i & 7] = *reinterpret_cast<const float4 *>(p.w + ((int64_t)tap * p.cin_pad + c) * p.cout_pad + cb * 32 + 4 * (i & 7));
+  }
+  const int n_stale = (p.stale && head_ok) ? min(p.counts[1], p.max_tiles) : 0;
+  for (int s = blockIdx.x; s < n_stale; s += gridDim.x) {
+    const int t = p.stale[s];
+    if (t < 0 || t >= ntiles_total) { if (tid == 0) atomicOr(&p.counts[3], MIE_ERR_BAD_TILE); continue; }
+    const int tx = t % TWo, ty = (t / TWo) % THo, n = t / (TWo * THo);
+    for (int i = tid; i < 64 * p.cout; i += 256) {
+      const int px = i / p.cout, c = i - px * p.cout;
+      const int oy = ty * 8 + (px >> 3), ox = tx * 8 + (px & 7);
+      if (oy < p.hout && ox < p.wout) p.out[((int64_t)(n * p.hout + oy) * p.wout + ox) * p.out_ps + c] = 0.0f;
+    }
+  }
+  const int n_active = head_ok ? min(p.counts[0], p.max_tiles) : 0;
+  for (int li = first; li < n_active; li += step) {
+    const int t = p.list[li];
+    if (t < 0 || t >= ntiles_total) { if (tid == 0) atomicOr(&p.counts[3], MIE_ERR_BAD_TILE); continue; }
+    const int tx = t % TWo, ty = (t / TWo) % THo, n = t / (TWo * THo);
+    int64_t pix[2];
+    bool ok[2];
+    float4 x[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int px = (tid >> 3) + 32 * i, oy = ty * 8 + (px >> 3), ox = tx * 8 + (px & 7);
+      ok[i] = oy < p.hout && ox < p.wout && co < p.cout;
+      pix[i] = (int64_t)(n * p.hout + oy) * p.wout + ox;
+      x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (ok[i] && p.act != MIE_ACT_NONE && !p.refresh) x[i] = *reinterpret_cast<const float4 *>(p.res + pix[i] * p.res_ps + co);
+    }
+    __syncthreads();      // the previous tile's reads of the window and of the word are done
+    for (int i = tid; i < T * T; i += 256) {
+      const int yy = i / T, xx = i - yy * T, iy = ty * 8 * S - p.pad + yy, ix = tx * 8 * S - p.pad + xx;
+      const bool in = iy >= 0 && iy < p.hin && ix >= 0 && ix < p.win;
+      const float *src = p.in + ((int64_t)(n * p.hin + iy) * p.win + ix) * p.in_ps;
+#pragma unroll
+      for (int c = 0; c < CIN; ++c) s_in[i * CIN + c] = in ? src[c] : 0.0f;
+    }
+    if (tid < 2) s_bits[tid] = 0u;
+    __syncthreads();
+    float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap)
+#pragma unroll
+      for (int c = 0; c < CIN; ++c) {
+        const float4 w = s_w[tap * CIN + c][q];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int px = (tid >> 3) + 32 * i;
+          const float v = s_in[(((px >> 3) * S + tap / 3) * T + (px & 7) * S + tap % 3) * CIN + c];
+          acc[i].x = fmaf(v, w.x, acc[i].x); acc[i].y = fmaf(v, w.y, acc[i].y); acc[i].z = fmaf(v, w.z, acc[i].z); acc[i].w = fmaf(v, w.w, acc[i].w);
+        }
+      }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float4 d = acc[i], base = make_float4(0.f, 0.f, 0.f, 0.f);
+      bool flag = p.refresh != 0 && ok[i];
+      if (ok[i]) {
+        if (p.bias) { d.x += p.bias[co]; d.y += p.bias[co + 1]; d.z += p.bias[co + 2]; d.w += p.bias[co + 3]; }
+        if (p.addend) {
+          const float *ad = p.addend + pix[i] * p.addend_ps + co;
+          d.x += ad[0]; d.y += ad[1]; d.z += ad[2]; d.w += ad[3];
+        }
+        if (p.act != MIE_ACT_NONE && (p.refresh || p.emitted || d.x != 0.0f || d.y != 0.0f || d.z != 0.0f || d.w != 0.0f)) {
+          const float4 xn = make_float4(x[i].x + d.x, x[i].y + d.y, x[i].z + d.z, x[i].w + d.w);
+          *reinterpret_cast<float4 *>(p.res + pix[i] * p.res_ps + co) = xn;
+          if (p.emitted) base = *reinterpret_cast<const float4 *>(p.emitted + pix[i] * p.emitted_ps + co);
+          else if (!p.refresh) base = make_float4(act_apply(p.act, x[i].x), act_apply(p.act, x[i].y), act_apply(p.act, x[i].z), act_apply(p.act, x[i].w));
+          d = make_float4(act_apply(p.act, xn.x) - base.x, act_apply(p.act, xn.y) - base.y, act_apply(p.act, xn.z) - base.z, act_apply(p.act, xn.w) - base.w);
+        }
+        flag |= fabsf(d.x) > p.thr || fabsf(d.y) > p.thr || fabsf(d.z) > p.thr || fabsf(d.w) > p.thr;
+      }
+      const unsigned bal = __ballot_sync(0xffffffffu, flag);
+      if (ok[i]) {
+        const bool send = (bal >> (lane & 28)) & 0xFu;      // the four lanes of this 16-channel group
+        *reinterpret_cast<float4 *>(p.out + pix[i] * p.out_ps + co) = send ? d : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.emitted && send)
+          *reinterpret_cast<float4 *>(p.emitted + pix[i] * p.emitted_ps + co) = make_float4(base.x + d.x, base.y + d.y, base.z + d.z, base.w + d.w);
+      }
+      // four pixels per warp: px = 4 * warp .. + 3 of half tile i
+      if (lane == 0 && bal) {
+        unsigned nib = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) if ((bal >> (8 * k)) & 0xFFu) nib |= 1u << k;
+        atomicOr(&s_bits[i], nib << (4 * (tid >> 5)));
+      }
+    }
+    __syncthreads();
+    if (tid < 2 && s_bits[tid]) atomicOr(reinterpret_cast<unsigned *>(p.out_bits + t) + tid, s_bits[tid]);
+  }
+  run_tail_job(p.tail);
+}
+
+template <int CIN, int S>
+int launch_few(const ConvParams &p, cudaStream_t st) {
+  const int n_cblk = p.cout_pad / 32;
+  int groups = MIE_SM_COUNT * 6 / n_cblk;
+  if (groups > p.max_tiles) groups = p.max_tiles;
+  if (groups < 1) groups = 1;
+  launch_chained(conv_few_kernel<CIN, S>, dim3(groups * n_cblk), dim3(256), 0, st, p);
+  return check_launch();
+}
+
 template <int K, int S, int WT, int WN, int CPT = 8>
 int launch_conv(const ConvParams &p, int max_items, cudaStream_t st) {
   using G = Geo<K, S>;
@@ -625,6 +750,12 @@ extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
   }
 
   if (a->in2 || a->accum) return MIE_EUNSUPPORTED;   // only the 1x1 head kernel above takes them
+  if (a->k == 3 && a->cin <= 2 && p.io_vec && (!a->addend || a->addend_ps >= a->cout)) {
+    cudaStream_t st = (cudaStream_t)stream;
+    const int r = a->cin == 1 ? (a->stride == 1 ? launch_few<1, 1>(p, st) : launch_few<1, 2>(p, st))
+                              : (a->stride == 1 ? launch_few<2, 1>(p, st) : launch_few<2, 2>(p, st));
+    return tail_after_launch(r, a->tail, true, stream);
+  }
   // block shape: 32 channels -> 4 tiles x 1; otherwise 4 tiles x 64 channels.  (A thresholded fused activation
   // decides per 16-channel group, which both shapes hold inside one warp.)
   int wt = 4, wn = 2;
@@ -639,6 +770,15 @@ extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
   MIE_CASE(5, 1); MIE_CASE(5, 2); MIE_CASE(7, 1); MIE_CASE(7, 2);
 #undef MIE_CASE
   return MIE_EUNSUPPORTED;
+}
+
+extern "C" int mie_conv_refresh_step(const mie_conv_args *a, const float *x, int64_t x_ps, const mie_tail_job *d, void *stream) {
+  if (!a || !d || !exact_takes(a)) return MIE_EINVAL;
+  int s = mie_tiles_dilate(d->in_bits, d->N, d->Hin, d->Win, d->Hout, d->Wout, d->k, d->stride, d->pad, d->union_bits, d->out_bits, d->list,
+                           d->stale, d->counts, d->flags, stream);
+  if (s == MIE_OK)
+    s = mie_split_exact(x, x_ps, a->cin, (int64_t)a->n * a->hin * a->win, const_cast<float *>(a->in), const_cast<float *>(a->in_lo), a->in_ps, stream);
+  return s == MIE_OK ? mie_conv_tiles(a, stream) : s;
 }
 
 extern "C" int mie_conv_step(const mie_conv_args *a, uint64_t *mask_bits, float mask_thr, const mie_tail_job *dilate, void *stream) {

@@ -688,13 +688,17 @@ __global__ void __launch_bounds__(256) mul_incr_vec_kernel(
   }
 }
 
-// Channel concatenation, float4 over channels: work item = (tile, block of 64 output channels).
+// Channel concatenation in pieces of four or two floats (V): work item = (tile, block of 64 output channels).  Pieces of
+// two serve the flow decoders, whose two prediction channels put every skip at an odd multiple of 8 bytes; element by
+// element those copies took 14-24 us where they take 5-8.
+template <typename V>
 __global__ void __launch_bounds__(PW_THREADS) cat2_vec_kernel(
     const float *__restrict__ a, int64_t a_ps, const uint64_t *__restrict__ a_bits, int ca, const float *__restrict__ b,
     int64_t b_ps, const uint64_t *__restrict__ b_bits, int cb, float *__restrict__ out, int64_t out_ps,
     uint64_t *out_bits, int N, int H, int W, const mie_tail_job tail) {
   grid_dependency_wait();
   grid_dependency_trigger();
+  constexpr int E = sizeof(V) / 4, FULL = 64 / E;
   const int ntiles = N * ((H + 7) >> 3) * ((W + 7) >> 3);
   const int C = ca + cb;
   const int ncb = (C + 63) / 64;
@@ -706,21 +710,21 @@ __global__ void __launch_bounds__(PW_THREADS) cat2_vec_kernel(
     if (w == 0ull) {
       if (blk == 0 && out_bits[t] != 0ull) {   // only this block reads or writes the word
         __syncthreads();
-        zero_tile4(out, out_ps, C, g, H, W);
+        zero_tile(out, out_ps, C, g, H, W);
         if (threadIdx.x == 0) out_bits[t] = 0ull;
       }
       continue;
     }
-    const int c_lo = blk * 64, q4 = (min(C, c_lo + 64) - c_lo) >> 2;
+    const int c_lo = blk * 64, pieces = (min(C, c_lo + 64) - c_lo) / E;
 #pragma unroll 4
-    for (int e = threadIdx.x; e < 64 * q4; e += blockDim.x) {   // independent copies: four loads in flight per thread
-      const int p = e / q4, c = c_lo + (e - p * q4) * 4;
+    for (int e = threadIdx.x; e < 64 * pieces; e += blockDim.x) {   // independent copies: four loads in flight per thread
+      const int p = pieces == FULL ? e / FULL : e / pieces, c = c_lo + (e - p * pieces) * E;
       if (!pix_valid(g, p)) continue;
       const int64_t pix = pix_index(g, p, H, W);
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c < ca) { if ((wa >> p) & 1ull) v = ld4(a + pix * a_ps + c); }
-      else { if ((wb >> p) & 1ull) v = ld4(b + pix * b_ps + (c - ca)); }
-      st4(out + pix * out_ps + c, v);
+      V v = {};
+      if (c < ca) { if ((wa >> p) & 1ull) v = *reinterpret_cast<const V *>(a + pix * a_ps + c); }
+      else { if ((wb >> p) & 1ull) v = *reinterpret_cast<const V *>(b + pix * b_ps + (c - ca)); }
+      *reinterpret_cast<V *>(out + pix * out_ps + c) = v;
     }
     if (blk == 0 && threadIdx.x == 0) out_bits[t] = w;
   }
@@ -847,6 +851,18 @@ __global__ void __launch_bounds__(PW_THREADS) upsample2x_vec_kernel(
 // loaded at all) and the 64 outputs are blended from shared memory.  Same interpolation arithmetic (up_src).
 constexpr int UP_WIN = 6;
 
+// A quad of which only the first n channels (n < 4: the field's last ones) belong to the field.
+__device__ __forceinline__ float4 ld4_part(const float *p, int n) {
+  if (n >= 4) return ld4(p);
+  return make_float4(p[0], n > 1 ? p[1] : 0.0f, n > 2 ? p[2] : 0.0f, 0.0f);
+}
+__device__ __forceinline__ void st4_part(float *p, float4 v, int n) {
+  if (n >= 4) { st4(p, v); return; }
+  p[0] = v.x;
+  if (n > 1) p[1] = v.y;
+  if (n > 2) p[2] = v.z;
+}
+
 __global__ void __launch_bounds__(PW_THREADS, 8) upsample2x_tile_kernel(
     const float *__restrict__ a, int64_t a_ps, const uint64_t *__restrict__ a_bits, const float *__restrict__ b,
     int64_t b_ps, const uint64_t *__restrict__ b_bits, float *__restrict__ out, int64_t out_ps, uint64_t *out_bits, int N,
@@ -898,14 +914,15 @@ __global__ void __launch_bounds__(PW_THREADS, 8) upsample2x_tile_kernel(
     const uint64_t wout = ((uint64_t)s_out[1] << 32) | s_out[0];
     if (wout == 0ull) {
       if (cb == 0 && out_bits[t] != 0ull) {      // only this block reads or writes the word
-        zero_tile4(out, out_ps, C, g, Ho, Wo);
+        if (C & 3) zero_tile(out, out_ps, C, g, Ho, Wo);
+        else zero_tile4(out, out_ps, C, g, Ho, Wo);
         __syncthreads();
         if (tid == 0) out_bits[t] = 0ull;
       }
       continue;
     }
-    const int c_lo = cb * CB, q4 = (min(C, c_lo + CB) - c_lo) >> 2;
-    if (q4 == CB / 4) {
+    const int c_lo = cb * CB, q4 = (min(C, c_lo + CB) - c_lo + 3) >> 2;
+    if (c_lo + CB <= C) {
       // ---- whole 32-channel blocks: every index is a shift or a per-thread constant.  (The general loops below spend
       // more than 200 instructions per 16-byte store on divisions, up_src and 64-bit pixel indices, and the kernel was
       // bound by instruction issue at a third of the memory bandwidth.)
@@ -969,8 +986,8 @@ __global__ void __launch_bounds__(PW_THREADS, 8) upsample2x_tile_kernel(
       if ((on_mask >> sp) & 1ull) {
         const int sy = min(max(r0 + sp / UP_WIN, 0), H - 1), sx = min(max(c0 + sp % UP_WIN, 0), W - 1);
         const int64_t pix = (int64_t)(g.n * H + sy) * W + sx;
-        if ((mask_a >> sp) & 1ull) v = ld4(a + pix * a_ps + c_lo + q * 4);
-        if ((mask_b >> sp) & 1ull) v = f4add(v, ld4(b + pix * b_ps + c_lo + q * 4));
+        if ((mask_a >> sp) & 1ull) v = ld4_part(a + pix * a_ps + c_lo + q * 4, C - c_lo - q * 4);
+        if ((mask_b >> sp) & 1ull) v = f4add(v, ld4_part(b + pix * b_ps + c_lo + q * 4, C - c_lo - q * 4));
       }
       s_src[sp][q] = v;
     }
@@ -997,7 +1014,7 @@ __global__ void __launch_bounds__(PW_THREADS, 8) upsample2x_tile_kernel(
           v.w = ay * (ax * v00.w + wx * v01.w) + wy * (ax * v10.w + wx * v11.w);
         }
       }
-      st4(out + pix_index(g, p, Ho, Wo) * out_ps + c_lo + q * 4, v);
+      st4_part(out + pix_index(g, p, Ho, Wo) * out_ps + c_lo + q * 4, v, C - c_lo - q * 4);
     }
     if (cb == 0 && tid == 0) out_bits[t] = wout;
   }
@@ -1582,7 +1599,9 @@ extern "C" int mie_upsample(const float *a, int64_t a_ps, const uint64_t *a_bits
   MIE_CHECK_FIELD(a, a_ps, C); MIE_CHECK_FIELD(out, out_ps, C);
   if (b && (!b_bits || b_ps < C)) return MIE_EINVAL;
   const int ntiles = N * divup(scale * H, 8) * divup(scale * W, 8);
-  if (scale == 2 && C % 4 == 0 && a_ps % 4 == 0 && out_ps % 4 == 0 && aligned16(a) && aligned16(out) &&
+  // (from 32 channels on a count that is no multiple of four leaves one ragged quad behind whole blocks: 130 channels to
+  // 256x336 took the general kernel 38 us a stream, this one 12)
+  if (scale == 2 && (C % 4 == 0 || C >= CB) && a_ps % 4 == 0 && out_ps % 4 == 0 && aligned16(a) && aligned16(out) &&
       (!b || (b_ps % 4 == 0 && aligned16(b)))) {
     launch_chained(upsample2x_tile_kernel, dim3(item_grid((int64_t)ntiles * divup(C, CB))), dim3(PW_THREADS), 0, (cudaStream_t)stream,
         a, a_ps, a_bits, b, b_ps, b_bits, out, out_ps, out_bits, N, C, H, W, mode, tail_for_kernel(tail));
@@ -1629,7 +1648,13 @@ extern "C" int mie_cat2(const float *a, int64_t a_ps, const uint64_t *a_bits, in
   MIE_CHECK_FIELD(a, a_ps, ca); MIE_CHECK_FIELD(b, b_ps, cb); MIE_CHECK_FIELD(out, out_ps, ca + cb);
   const int ntiles = N * divup(H, 8) * divup(W, 8);
   if (ca % 4 == 0 && cb % 4 == 0 && a_ps % 4 == 0 && b_ps % 4 == 0 && out_ps % 4 == 0 && aligned16(a) && aligned16(b) && aligned16(out)) {
-    launch_chained(cat2_vec_kernel, dim3(item_grid((int64_t)ntiles * divup(ca + cb, 64))), dim3(PW_THREADS), 0, (cudaStream_t)stream,
+    launch_chained(cat2_vec_kernel<float4>, dim3(item_grid((int64_t)ntiles * divup(ca + cb, 64))), dim3(PW_THREADS), 0, (cudaStream_t)stream,
+                   a, a_ps, a_bits, ca, b, b_ps, b_bits, cb, out, out_ps, out_bits, N, H, W, tail_for_kernel(tail));
+    return tail_after_launch(check_launch(), tail, true, stream);
+  }
+  auto aligned8 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 7) == 0; };
+  if (ca % 2 == 0 && cb % 2 == 0 && a_ps % 2 == 0 && b_ps % 2 == 0 && out_ps % 2 == 0 && aligned8(a) && aligned8(b) && aligned8(out)) {
+    launch_chained(cat2_vec_kernel<float2>, dim3(item_grid((int64_t)ntiles * divup(ca + cb, 64))), dim3(PW_THREADS), 0, (cudaStream_t)stream,
                    a, a_ps, a_bits, ca, b, b_ps, b_bits, cb, out, out_ps, out_bits, N, H, W, tail_for_kernel(tail));
     return tail_after_launch(check_launch(), tail, true, stream);
   }

@@ -164,13 +164,15 @@ class ConvLSTMIncr(nn.Module):
         n, _, h, w = x.shape
         C, dev = self.hidden_size, x.device
         shapes = ((n, 4 * C, h, w), (n, C, h, w), (n, C, h, w))
-        bufs = []
+        bufs, kept = [], []
         for buf, shape in zip((self._g, self._cell, self._cprev), shapes):
             if buf is None or tuple(buf.shape) != shape or buf.device != dev:
                 buf = fl.new_field(*shape, dev)
             else:
-                buf.zero_()
+                kept.append(buf)
             bufs.append(buf)
+        if kept:
+            torch._foreach_zero_(kept)
         self._g, self._cell, self._cprev = bufs
         dcp = mcp = None
         if prev_state is None:

@@ -290,7 +290,8 @@ class _PreparedCall:
         self.geometry = (mask.n, mask.h, mask.w)
         self.mask_bits = mask.bits if derived else None      # the tile words this call derives from the delta itself
         self.mask_ptr = mask.bits.data_ptr()
-        self.args, self.args_ref = plan.args, C.byref(plan.args)
+        self.args = nat.ConvArgs.from_buffer_copy(plan.args)     # its own: dense passes fill the plan's
+        self.args_ref = C.byref(self.args)
         self.dilate = C.addressof(plan.tail.c) if dilate else None
         self.keep = plan.tail
         self.tc_option = (1 if config.tc_thresholded else 0) if thresholded else None
@@ -331,6 +332,53 @@ class _PreparedCall:
         return list(self.out)
 
 
+class _PreparedRefresh:
+    """The same for the dense evaluation of a layer in fp32 precision on the tensor cores (60 us of deciding per layer
+    otherwise, more than its kernels take)."""
+    __slots__ = ("activation", "cin_limit", "epoch", "options", "params", "reservoir", "reservoir_ptr", "geometry", "mask_ptr", "addend_ptrs",
+                 "plan", "args", "fields", "fields_ps", "x_ps", "job", "out")
+
+    def __init__(self, conv, activation, cin_limit, plan, d, mask, addend):
+        self.activation, self.cin_limit, self.plan = activation, cin_limit, plan
+        self.epoch, self.options = config.epoch, nat.option_epoch[0]
+        self.params = self.parameters_of(conv)
+        self.reservoir = None if activation is None else activation.in_res.reservoir
+        self.reservoir_ptr = 0 if activation is None else self.reservoir.data_ptr()
+        self.geometry, self.mask_ptr = (d.shape, d.stride(), d.device), mask.bits.data_ptr()
+        self.addend_ptrs = None if addend is None else (addend[0].data_ptr(), addend[1].bits.data_ptr())
+        n, c, h, w = d.shape
+        cp = (c + 3) // 4 * 4
+        self.fields, self.fields_ps, self.x_ps = (2, n, h, w, cp), n * h * w * cp * 4, fl.pixel_stride(d)
+        self.job, self.out = plan.tail, (plan.out, plan.mask)
+        self.args = nat.ConvArgs.from_buffer_copy(plan.args)
+
+    @staticmethod
+    def parameters_of(conv):
+        w, b = conv._parameters["weight"], conv._parameters["bias"]
+        return (id(w), w._version, w.data_ptr()) + (() if b is None else (id(b), b.data_ptr()))
+
+    def run(self, conv, x_incr, addend):
+        d, m = x_incr[0], x_incr[1]
+        plan, act = self.plan, self.activation
+        if (self.epoch != config.epoch or self.options != nat.option_epoch[0] or type(m) is not TileMask or m.bits.data_ptr() != self.mask_ptr
+                or (d.shape, d.stride(), d.device) != self.geometry or d.dtype is not torch.float32 or self.parameters_of(conv) != self.params
+                or plan.needs_clear or plan.accum_target is not None or plan.tail is not self.job):
+            return None
+        if act is not None:
+            r = act.in_res.reservoir
+            if r is not self.reservoir or r.data_ptr() != self.reservoir_ptr or act.emitted is not None:
+                return None
+        if addend is not None and (type(addend[1]) is not TileMask or (addend[0].data_ptr(), addend[1].bits.data_ptr()) != self.addend_ptrs):
+            return None
+        both = torch.empty(self.fields, dtype=torch.float32, device=d.device)     # released after the launch
+        a = self.args
+        a.in_ = both.data_ptr()
+        a.in_lo = a.in_ + self.fields_ps
+        nat.check(nat.lib.mie_conv_refresh_step(C.byref(a), d.data_ptr(), self.x_ps, C.addressof(self.job.c), nat.stream_ptr(d.device)),
+                  "conv_refresh_step")
+        return list(self.out)
+
+
 class nnConvIncr(nn.Conv2d):
     """Convolution of a masked delta (reference ``:146-196``).
 
@@ -346,7 +394,8 @@ class nnConvIncr(nn.Conv2d):
         self._packed = {}   # cin_limit -> (version, device, buffer, cin_pad, cout_pad)
         self._packed_exact = {}   # cin_limit -> (version, buffer): the dense pass in fp32 precision on the tensor cores
         self._plans = {}
-        self._prepared = None     # _PreparedCall of the last full call
+        self._prepared = None             # _PreparedCall of the last full incremental call
+        self._prepared_refresh = None     # _PreparedRefresh of the last full dense evaluation
         self._cw = None
         self._scratch = Scratch()
 
@@ -456,11 +505,20 @@ class nnConvIncr(nn.Conv2d):
         f(reservoir) -- in full fp32, whatever ``config.tensor_cores`` says."""
         plain = addend is None and second is None and bn is None and not refresh
         fast = self._prepared
-        if plain and fast is not None and fast.activation is activation and fast.cin_limit == cin_limit:
-            out = fast.run(self, x_incr)
-            if out is not None:
-                return out
-        self._prepared = None
+        if plain:
+            if fast is not None and fast.activation is activation and fast.cin_limit == cin_limit:
+                out = fast.run(self, x_incr)
+                if out is not None:
+                    return out
+            self._prepared = None
+        fast = self._prepared_refresh
+        if refresh:
+            if (fast is not None and second is None and bn is None and fast.activation is activation and fast.cin_limit == cin_limit
+                    and (addend is None) == (fast.addend_ptrs is None)):
+                out = fast.run(self, x_incr, addend)
+                if out is not None:
+                    return out
+            self._prepared_refresh = None
         sc = self._scratch
         if refresh and bn is not None:
             raise NotImplementedError("dense evaluation with a folded batch-norm")
@@ -580,6 +638,9 @@ class nnConvIncr(nn.Conv2d):
         if (plain and not split and not config.kfenced_step and not config.tail_dilation and not a.accum and (x_incr[1] is None or x_incr[1] is m)
                 and d is x_incr[0] and (activation is None or type(activation).thr is nnReservedActivation.thr) and a.in_ % 16 == 0):
             self._prepared = _PreparedCall(self, activation, cin_limit, plan, d, m, x_incr[1] is None, not a.head, a.thr > 0.0 or bool(a.emitted))
+        if (refresh and a.wpacked_exact and not a.head and not config.tail_dilation and second is None and x_incr[1] is m and x_incr[0].data_ptr() == d.data_ptr()
+                and (activation is None or activation.emitted is None) and (addend is None or type(addend[1]) is TileMask)):
+            self._prepared_refresh = _PreparedRefresh(self, activation, cin_limit, plan, d, m, addend)
         if refresh and activation is not None and activation.emitted is not None:
             if activation.emitted.shape == plan.out.shape and activation.thr() > 0.0 and config.carry:
                 activation.emitted.copy_(plan.out)      # what has been sent so far = f(reservoir)

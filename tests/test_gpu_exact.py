@@ -104,3 +104,49 @@ def test_accumulate_and_keep(dev):
         fl.accumulate(z, d, m)
         fl.accumulate_keep(y, d, m, kept, kb)
         assert torch.equal(y, want) and torch.equal(z, want) and torch.equal(kept, d) and torch.equal(kb, m.bits)
+
+
+# one or two input channels: ragged tiles, both strides, partial channel blocks, two column blocks
+@pytest.mark.parametrize("case", [(2, 32, 1, 21, 43), (2, 64, 2, 34, 50), (1, 36, 1, 8, 9), (2, 96, 1, 17, 24)])
+@pytest.mark.parametrize("thr", [0.0, 0.05])
+def test_few_input_channels_against_the_restatement(dev, case, thr):
+    from maskedincrementeval_b200 import fields as fl
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    cin, cout, s, h, w = case
+    torch.manual_seed(4)
+    layer = ConvLayerIncr(cin, cout, 3, s, 1, activation="relu").to(dev).eval()
+    layer.activation.threshold = thr
+    wt, b = layer.conv2d.weight.detach().cpu(), layer.conv2d.bias.detach().cpu()
+    g = torch.Generator().manual_seed(5)
+    x0 = torch.randn(2, cin, h, w, generator=g)
+    res, sent = R.conv_dense(x0, wt, b, s, 1), None
+    with torch.no_grad():
+        sent = layer.forward_refresh_reservoirs(cl(x0.to(dev))).clone()
+        for frac in (0.1, 0.0, 0.02, 1.0):
+            dx = torch.randn(2, cin, h, w, generator=g) * (torch.rand(2, 1, h, w, generator=g) < frac)
+            dy, m = layer([cl(dx.to(dev)), None])
+            sent += dy
+            want, _ = R.act_incr(res, R.conv_delta(dx, wt, s, 1), "relu")
+            res = layer.activation.in_res.reservoir.cpu().contiguous()
+            if thr == 0.0:
+                assert float((dy.cpu() - want).abs().max()) <= 1e-5
+            assert float((sent - torch.relu(layer.activation.in_res.reservoir)).abs().max()) <= thr + 1e-5
+            assert torch.equal(m.pixel_mask(), (dy != 0).any(1, keepdim=True).to(torch.uint8))
+
+
+@pytest.mark.parametrize("c", [32, 34, 66, 130])
+def test_upsample_and_concat_of_ragged_channel_counts(dev, c):
+    from maskedincrementeval_b200 import fields as fl
+    from maskedincrementeval_b200.fields import Scratch
+    from maskedincrementeval_b200.incr_modules._algebra import INCR
+    g = torch.Generator(device=dev).manual_seed(c)
+    sc = Scratch()
+    for frac in (0.3, 0.0, 0.02):
+        a = cl(torch.randn(1, 2, 11, 22, generator=g, device=dev) * (torch.rand(1, 1, 11, 22, generator=g, device=dev) < frac))
+        b = cl(torch.randn(1, c - 2, 11, 22, generator=g, device=dev) * (torch.rand(1, 1, 11, 22, generator=g, device=dev) < frac))
+        x, m = INCR.cat([a, fl.mask_from_delta(a)], [b, fl.mask_from_delta(b)], sc, "cat")
+        want = torch.cat([a, b], 1)
+        assert torch.equal(x, want)
+        up, mu = INCR.upsample2x([x, m], None, sc, pad4=True)
+        assert float((up - F.interpolate(want, scale_factor=2, mode="bilinear", align_corners=False)).abs().max()) <= 1e-6
+        assert float((up * (1 - mu.pixel_mask().float())).abs().max()) == 0.0

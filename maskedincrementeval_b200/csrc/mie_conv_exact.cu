@@ -6,8 +6,8 @@
 //     hi(input) x [hi(filter) | lo(filter)]  ->  N = 2 CB columns,      lo(input) x hi(filter)  ->  N = CB columns.
 // What keeps the result at fp32 level is where the sums are rounded: the tensor core truncates each time it adds to an
 // accumulator (1.7e-8 of the value per addition, always towards zero: 3e-5 after the 2400 additions of a 256-channel 5x5
-// layer).  So the first product starts from zero again with every ring stage (at most 16 additions) and the epilogue warps
-// add the partial sums to registers, rounded to nearest, while the next stage runs; the second product is 2^-12 of the first
+// layer).  So the first product starts from zero again with every segment (at most 20 additions) and the epilogue warps
+// add the partial sums to registers, rounded to nearest, while the next segments run; the second product is 2^-12 of the first
 // and stays in its accumulator for the whole work item.  Against a float64 convolution the error is that of the CUDA-core
 // FP32 kernel or below it (see tests/test_gpu_exact.py).
 // Epilogue: reservoir = conv + bias (+ addend), output = f(reservoir), every pixel of a listed tile marked.
@@ -20,6 +20,7 @@ namespace {
 
 constexpr int EXACT_THREADS = 384;
 constexpr int EXACT_MAX_STAGES = 8;
+constexpr int EXACT_SEG_TAPS = 5;      // a segment: 5 taps x 4 K-slices = 20 additions into a tensor-memory accumulator
 constexpr int EXACT_MAX_HALOS = 4;
 
 struct ExactParams {
@@ -27,24 +28,116 @@ struct ExactParams {
   const int32_t *list; int32_t *counts; int max_tiles;
   float *out; int64_t out_ps; unsigned int *out_bits32;
   int act; float *res; int64_t res_ps; const float *addend; int64_t addend_ps; const float *bias;
-  int cb, stages, halos, tps, wp;
+  int cb, stages, halos, tps, wp;   // tps: taps per ring stage
   unsigned spin_limit;
   mie_tail_job tail;
   PairTaps t;
 };
 struct ExactMaps {
-  CUtensorMap hi[4], lo[4], w;
+  CUtensorMap hi[4], lo[4], w, out, res;
 };
 
-__device__ __forceinline__ void tmem_add16(unsigned taddr, float *acc) {
-  unsigned r[16];
+// acc[i] += column i (of n = 16 or 32) at taddr, + column i at taddr2: all loads in flight before the first addition
+__device__ __forceinline__ void tmem_ld16_async(unsigned taddr, unsigned *r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
                  "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                : "r"(taddr));
+}
+template <int N>
+__device__ __forceinline__ void tmem_add(unsigned taddr, float *acc) {
+  unsigned r[N];
+#pragma unroll
+  for (int g = 0; g < N; g += 16) tmem_ld16_async(taddr + g, r + g);
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 16; ++i) acc[i] += __uint_as_float(r[i]);
+  for (int i = 0; i < N; ++i) acc[i] += __uint_as_float(r[i]);
+}
+
+// Segment accumulators (2 CB columns each) beside the two item accumulators (CB each) in 512 columns: enough that the round
+// trip of a segment to the epilogue and back does not hold up the issuer.
+__host__ __device__ constexpr unsigned exact_segs(int cb) { return cb == 64 ? 3u : 6u; }
+
+template <int CB>
+__device__ __forceinline__ void exact_issue(const ExactParams &p, int bid, int nblk, int n_items, unsigned tmem_base, unsigned a_base, unsigned b_base,
+    unsigned row_bytes, unsigned halo_bytes, unsigned tap_bytes, unsigned stage_bytes, unsigned long long *b_full, unsigned long long *b_empty,
+    unsigned long long *a_full, unsigned long long *a_empty, unsigned long long *seg_full, unsigned long long *seg_empty, unsigned long long *item_full,
+    unsigned long long *item_empty, volatile int *abort_flag) {
+  constexpr unsigned NSEG = exact_segs(CB), item_col = NSEG * 2u * CB;
+  const unsigned id0 = (make_idesc_tf32(0) & ~(31u << 24)) | (16u << 24);       // M = 256
+  const unsigned id_hi = id0 | ((unsigned)(2 * CB >> 3) << 17), id_lo = id0 | ((unsigned)(CB >> 3) << 17);
+  const unsigned long long b_tmpl = make_smem_desc(0), a_tmpl = make_smem_desc(0, row_bytes);
+  const unsigned long long b_hi = b_tmpl & 0xFFFFFFFF00000000ull, a_hi = a_tmpl & 0xFFFFFFFF00000000ull;
+  const unsigned lo_flags = (unsigned)(b_tmpl & 0xFFFF0000ull);
+  const int nv = p.t.nviews;
+  unsigned bs = 0, bpar = 0, as = 0, apar = 0, item_idx = 0, seg = 0, seg_par = 1, stage_addr = b_base;
+#pragma unroll 1
+  for (int item = bid; item < n_items; item += nblk, ++item_idx) {
+    const unsigned buf = item_idx & 1u;
+    if (item_idx >= 2 && !mbar_wait(&item_empty[buf], ((item_idx >> 1) - 1) & 1u, abort_flag, p.spin_limit)) return;
+    unsigned started = 0;
+#pragma unroll 1
+    for (int chunk = 0; chunk < p.n_chunks; ++chunk) {
+      const unsigned nks = (unsigned)min(4, (p.cin - chunk * 32 + 7) >> 3);
+#pragma unroll 1
+      for (int v = 0; v < nv; ++v) {
+        if (!mbar_wait(&a_full[as], apar, abort_flag, p.spin_limit)) return;
+        const unsigned halo = lo_flags | ((a_base + as * halo_bytes) >> 4);
+        const int end = p.t.first[v + 1];
+        int in_seg = 0;          // taps in the current segment
+#pragma unroll 1
+        for (int i = p.t.first[v]; i < end; i += p.tps) {
+          const int nt = min(p.tps, end - i);
+          unsigned b_lo = lo_flags | (stage_addr >> 4);
+          if (!mbar_wait(&b_full[bs], bpar, abort_flag, p.spin_limit)) return;
+          tc_fence_after();
+#pragma unroll 1
+          for (int k = 0; k < nt; ++k, b_lo += tap_bytes >> 4) {
+            if (!in_seg) {
+              if (!mbar_wait(&seg_empty[seg], seg_par, abort_flag, p.spin_limit)) return;
+              tc_fence_after();
+            }
+            pair_mma(tmem_base + seg * (2u * CB), a_hi | (halo + ((unsigned)p.t.off[i + k] * 8u)), b_hi | b_lo, id_hi, (unsigned)in_seg, nks);
+            if (++in_seg == EXACT_SEG_TAPS || i + k + 1 == end) {
+              pair_commit(&seg_full[seg]);
+              in_seg = 0;
+              if (++seg == NSEG) { seg = 0; seg_par ^= 1u; }
+            }
+          }
+          pair_commit(&b_empty[bs]);
+          stage_addr += stage_bytes;
+          if (++bs == (unsigned)p.stages) { bs = 0; bpar ^= 1u; stage_addr = b_base; }
+        }
+        pair_commit(&a_empty[as]);
+        if (++as == (unsigned)p.halos) { as = 0; apar ^= 1u; }
+      }
+#pragma unroll 1
+      for (int v = 0; v < nv; ++v) {
+        if (!mbar_wait(&a_full[as], apar, abort_flag, p.spin_limit)) return;
+        const unsigned halo = lo_flags | ((a_base + as * halo_bytes) >> 4);
+        const int end = p.t.first[v + 1];
+#pragma unroll 1
+        for (int i = p.t.first[v]; i < end; i += p.tps) {
+          const int nt = min(p.tps, end - i);
+          unsigned b_lo = lo_flags | (stage_addr >> 4);
+          if (!mbar_wait(&b_full[bs], bpar, abort_flag, p.spin_limit)) return;
+          tc_fence_after();
+          const unsigned d = tmem_base + item_col + buf * CB;
+#pragma unroll 1
+          for (int k = 0; k < nt; ++k, b_lo += tap_bytes >> 4) {
+            pair_mma(d, a_hi | (halo + ((unsigned)p.t.off[i + k] * 8u)), b_hi | b_lo, id_lo, started, nks);
+            started = 1u;
+          }
+          pair_commit(&b_empty[bs]);
+          stage_addr += stage_bytes;
+          if (++bs == (unsigned)p.stages) { bs = 0; bpar ^= 1u; stage_addr = b_base; }
+        }
+        pair_commit(&a_empty[as]);
+        if (++as == (unsigned)p.halos) { as = 0; apar ^= 1u; }
+      }
+    }
+    pair_commit(&item_full[buf]);
+  }
 }
 
 // HW: channels per epilogue set (CB = 2 HW channels per block)
@@ -59,7 +152,7 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
   const unsigned halo_bytes = ((unsigned)p.wp * 2u * row_bytes + 1023u) & ~1023u;
   const unsigned stage_bytes = tap_bytes * (unsigned)p.tps;
   __shared__ unsigned long long b_full[EXACT_MAX_STAGES], b_empty[EXACT_MAX_STAGES], a_full[EXACT_MAX_HALOS], a_empty[EXACT_MAX_HALOS],
-      seg_full[2], seg_empty[2], item_full[2], item_empty[2];
+      seg_full[6], seg_empty[6], item_full[2], item_empty[2];
   __shared__ unsigned s_tmem_base;
   __shared__ int s_abort;
 
@@ -68,13 +161,13 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
   const int bid = (int)(blockIdx.x >> 1), nblk = (int)(gridDim.x >> 1);
   const int THo = (p.hout + 7) >> 3, TWo = (p.wout + 7) >> 3;
   const int ntiles_total = p.n * THo * TWo;
-  // columns: two segment buffers of 2 CB (hi and lo of the filter), two item buffers of CB (lo of the input)
-  constexpr unsigned tmem_cols = CB == 64 ? 512u : 256u, item_col = 4u * CB;
+  constexpr unsigned NSEG = exact_segs(CB), item_col = NSEG * 2u * CB, tmem_cols = 512u;
 
   if (tid == 0) {
     for (int s = 0; s < p.stages; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
     for (int s = 0; s < p.halos; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&seg_full[b], 1); mbar_init(&seg_empty[b], 16); mbar_init(&item_full[b], 1); mbar_init(&item_empty[b], 16); }
+    for (unsigned b = 0; b < NSEG; ++b) { mbar_init(&seg_full[b], 1); mbar_init(&seg_empty[b], 16); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&item_full[b], 1); mbar_init(&item_empty[b], 16); }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -186,47 +279,7 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
   } else if (warp == 2) {
     // =========================== MMA issuer (first block of the pair) ===========================
     if (crank == 0u) {
-      const unsigned id0 = (make_idesc_tf32(0) & ~(31u << 24)) | (16u << 24);       // M = 256
-      const unsigned id_hi = id0 | ((unsigned)(2 * CB >> 3) << 17), id_lo = id0 | ((unsigned)(CB >> 3) << 17);
-      const unsigned long long b_tmpl = make_smem_desc(0), a_tmpl = make_smem_desc(0, row_bytes);
-      const unsigned long long b_hi = b_tmpl & 0xFFFFFFFF00000000ull, a_hi = a_tmpl & 0xFFFFFFFF00000000ull;
-      const unsigned lo_flags = (unsigned)(b_tmpl & 0xFFFF0000ull);
-      unsigned bs = 0, bpar = 0, as = 0, apar = 0, item_idx = 0, seg = 0, stage_addr = b_base;
-      bool ok = true;
-      for (int item = bid; item < n_items && ok; item += nblk, ++item_idx) {
-        const unsigned buf = item_idx & 1u;
-        if (item_idx >= 2 && !__all_sync(0xffffffffu, mbar_wait_cluster(&item_empty[buf], ((item_idx >> 1) - 1) & 1u, &s_abort, p.spin_limit))) break;
-        unsigned started = 0;          // the item accumulator holds something
-        for (int chunk = 0; chunk < p.n_chunks && ok; ++chunk) {
-          const unsigned nks = (unsigned)min(4, (p.cin - chunk * 32 + 7) >> 3);
-          for (int u = 0; u < 2 * nv && ok; ++u) {
-            const bool lo = u >= nv;
-            const int v = lo ? u - nv : u, end = p.t.first[v + 1];
-            if (!__all_sync(0xffffffffu, mbar_wait(&a_full[as], apar, &s_abort, p.spin_limit))) { ok = false; break; }
-            const unsigned halo = lo_flags | ((a_base + as * halo_bytes) >> 4);
-            for (int i = p.t.first[v]; i < end; i += p.tps) {
-              const int nt = min(p.tps, end - i);
-              if (!__all_sync(0xffffffffu, mbar_wait(&b_full[bs], bpar, &s_abort, p.spin_limit))) { ok = false; break; }
-              if (!lo && seg >= 2 && !__all_sync(0xffffffffu, mbar_wait_cluster(&seg_empty[seg & 1u], ((seg >> 1) - 1) & 1u, &s_abort, p.spin_limit))) { ok = false; break; }
-              tc_fence_after();
-              const unsigned d = tmem_base + (lo ? item_col + buf * CB : (seg & 1u) * (2u * CB));
-              unsigned b_lo = lo_flags | (stage_addr >> 4);
-              for (int k = 0; k < nt; ++k, b_lo += tap_bytes >> 4)
-                pair_mma(d, a_hi | (halo + (unsigned)p.t.off[i + k] * 8u), b_hi | b_lo, lo ? id_lo : id_hi, lo ? (started | (unsigned)k) : (unsigned)k, nks);
-              pair_commit(&b_empty[bs]);
-              if (lo) started = 1u;
-              else { pair_commit(&seg_full[seg & 1u]); ++seg; }
-              stage_addr += stage_bytes;
-              if (++bs == (unsigned)p.stages) { bs = 0; bpar ^= 1u; stage_addr = b_base; }
-            }
-            if (!ok) break;
-            pair_commit(&a_empty[as]);
-            if (++as == (unsigned)p.halos) { as = 0; apar ^= 1u; }
-          }
-        }
-        if (!ok) break;
-        pair_commit(&item_full[buf]);
-      }
+      exact_issue<CB>(p, bid, nblk, n_items, tmem_base, a_base, b_base, row_bytes, halo_bytes, tap_bytes, stage_bytes, b_full, b_empty, a_full, a_empty, seg_full, seg_empty, item_full, item_empty, &s_abort);
     }
   } else if (warp >= 4) {
     // =========================== epilogue: set `set` takes channels [set * HW, set * HW + HW) of the block ===========================
@@ -234,9 +287,16 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
     const int slot = (lane >> 3) & 1, prow = 2 * q + (lane >> 4), pcol = lane & 7;
     const unsigned lane_base = tmem_base + ((unsigned)(q * 32) << 16);
     int segs_per_chunk = 0;
-    for (int v = 0; v < nv; ++v) segs_per_chunk += (p.t.first[v + 1] - p.t.first[v] + p.tps - 1) / p.tps;
+    for (int v = 0; v < nv; ++v) segs_per_chunk += (p.t.first[v + 1] - p.t.first[v] + EXACT_SEG_TAPS - 1) / EXACT_SEG_TAPS;
     const int segs = segs_per_chunk * p.n_chunks;
-    unsigned item_idx = 0, seg = 0;
+    // slabs of this set: output, then reservoir; 128 rows of HW channels, 16-byte pieces swizzled as TMA does for rows of
+    // 128 bytes (piece ^ (row & 7)) or 64 bytes (piece ^ (row / 2 & 3))
+    constexpr unsigned SLAB = 128u * HW * 4u;
+    const int row = slot * 64 + prow * 8 + pcol, sw = HW == 32 ? row & 7 : (row >> 1) & 3;
+    const unsigned slab = a_base + (unsigned)p.halos * halo_bytes + (unsigned)set * (p.act != MIE_ACT_NONE ? 2u : 1u) * SLAB;
+    const unsigned out_row = slab + (unsigned)row * (HW * 4u), res_row = out_row + SLAB;
+    const bool chief = q == 0 && elect_one();
+    unsigned item_idx = 0, seg = 0, seg_par = 0;
     bool ok = true;
     for (int item = bid; item < n_items && ok; item += nblk, ++item_idx) {
       const int quad = item / n_cblk, cb = item - quad * n_cblk;
@@ -250,42 +310,56 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
       float acc[HW];
 #pragma unroll
       for (int i = 0; i < HW; ++i) acc[i] = 0.0f;
-      for (int s = 0; s < segs; ++s, ++seg) {
-        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&seg_full[seg & 1u], (seg >> 1) & 1u, &s_abort, p.spin_limit)))) break;
+      for (int s = 0; s < segs; ++s) {
+        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&seg_full[seg], seg_par, &s_abort, p.spin_limit)))) break;
         tc_fence_after();
-        const unsigned c = lane_base + (seg & 1u) * (2u * CB) + (unsigned)set * CB;     // [hi | lo] columns of this set's channels
-#pragma unroll
-        for (int g = 0; g < HW; g += 16) {
-          tmem_add16(c + g, acc + g);
-          tmem_add16(c + HW + g, acc + g);
-        }
+        const unsigned c = lane_base + seg * (2u * CB) + (unsigned)set * CB;     // [hi | lo] columns of this set's channels
+        tmem_add<HW>(c, acc);
+        tmem_add<HW>(c + HW, acc);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&seg_empty[seg & 1u]), 0));
+        if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&seg_empty[seg]), 0));
+        if (++seg == NSEG) { seg = 0; seg_par ^= 1u; }
       }
-      if (!ok) break;
-      if (!(ok = __all_sync(0xffffffffu, mbar_wait(&item_full[buf], (item_idx >> 1) & 1u, &s_abort, p.spin_limit)))) break;
+      // a warp whose wait gave up goes on to the barrier of its set, where the four of them leave together
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&item_full[buf], (item_idx >> 1) & 1u, &s_abort, p.spin_limit));
       tc_fence_after();
-#pragma unroll
-      for (int g = 0; g < HW; g += 16) tmem_add16(lane_base + item_col + buf * CB + (unsigned)(set * HW + g), acc + g);
+      if (ok) tmem_add<HW>(lane_base + item_col + buf * CB + (unsigned)(set * HW), acc);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&item_empty[buf]), 0));
+      if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&item_empty[buf]), 0));
       const int co = cb * CB + set * HW;
-      if (valid) {
+      // the slabs are free once the previous item's stores have read them
+      if (chief) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      __syncwarp();
+      ok = set_all(1 + set, ok);
+      if (!ok) break;
 #pragma unroll
-        for (int h = 0; h < HW / 4; ++h) {
-          const int c = co + 4 * h;
-          if (c >= p.cout) break;
-          float4 v = make_float4(acc[4 * h], acc[4 * h + 1], acc[4 * h + 2], acc[4 * h + 3]);
-          if (p.bias) v = f4add(v, make_float4(__ldg(p.bias + c), __ldg(p.bias + c + 1), __ldg(p.bias + c + 2), __ldg(p.bias + c + 3)));
-          if (p.addend) v = f4add(v, *reinterpret_cast<const float4 *>(p.addend + pix * p.addend_ps + c));
-          if (p.act != MIE_ACT_NONE) {
-            *reinterpret_cast<float4 *>(p.res + pix * p.res_ps + c) = v;
-            v = make_float4(act_apply(p.act, v.x), act_apply(p.act, v.y), act_apply(p.act, v.z), act_apply(p.act, v.w));
-          }
-          *reinterpret_cast<float4 *>(p.out + pix * p.out_ps + c) = v;
+      for (int h = 0; h < HW / 4; ++h) {
+        const int c = co + 4 * h;
+        float4 v = make_float4(acc[4 * h], acc[4 * h + 1], acc[4 * h + 2], acc[4 * h + 3]);
+        if (p.bias && c < p.cout) v = f4add(v, make_float4(__ldg(p.bias + c), __ldg(p.bias + c + 1), __ldg(p.bias + c + 2), __ldg(p.bias + c + 3)));
+        if (p.addend && valid && c < p.cout) v = f4add(v, *reinterpret_cast<const float4 *>(p.addend + pix * p.addend_ps + c));
+        const unsigned at = (unsigned)(h ^ sw) << 4;
+        if (p.act != MIE_ACT_NONE) {
+          sts4(res_row + at, v);
+          v = p.act == MIE_ACT_RELU ? make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f))
+                                    : make_float4(tc_act_call(p.act, v.x), tc_act_call(p.act, v.y), tc_act_call(p.act, v.z), tc_act_call(p.act, v.w));
         }
+        sts4(out_row + at, v);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");
+      if (chief && co < p.cout) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          const int es = 4 * quad + 2 * (int)crank + s, ts = es < n_active ? p.list[es] : -1;
+          if (ts < 0 || ts >= ntiles_total) continue;
+          const int x = (ts % TWo) * 8, y = ((ts / TWo) % THo) * 8, ns = ts / (TWo * THo);
+          tma_store_slab(slab + s * (SLAB / 2), &maps.out, co, x, y, ns);
+          if (p.act != MIE_ACT_NONE) tma_store_slab(slab + SLAB + s * (SLAB / 2), &maps.res, co, x, y, ns);
+        }
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
       // every pixel written is marked; ballot bytes: [tile 0 row 2q][tile 1 row 2q][tile 0 row 2q+1][tile 1 row 2q+1]
       const unsigned bal = __ballot_sync(0xffffffffu, valid);
@@ -294,6 +368,7 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
         if (rows) atomicOr(p.out_bits32 + 2 * (size_t)t + (q >> 1), rows << ((q & 1) * 16));
       }
     }
+    if (chief) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
   // ---- teardown ----
@@ -339,15 +414,17 @@ int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
   if (a->cout_pad % 64 == 0 &&
       (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 107 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 82)
     p.cb = 64;
-  const int halo_bytes = (p.wp * 2 * p.wp * 128 + 1023) & ~1023, budget = 222 * 1024;
-  p.tps = 4;                       // additions into one segment accumulator: 4 taps x 4 K-slices
-  const int stage_bytes = p.tps * p.cb * 128;
+  // fat stages: what the issuer and the producers spend per stage does not depend on its size
+  const int halo_bytes = (p.wp * 2 * p.wp * 128 + 1023) & ~1023, slab_bytes = 2 * (a->act != MIE_ACT_NONE ? 2 : 1) * 128 * (p.cb / 2) * 4;
+  const int budget = 222 * 1024 - slab_bytes;
+  p.tps = p.cb == 32 ? 9 : 5;
+  const int stage_bytes = p.tps * p.cb * 128, want = p.cb == 32 ? 3 : 3;
   p.halos = EXACT_MAX_HALOS;
-  while (p.halos > 2 && budget - p.halos * halo_bytes < 3 * stage_bytes) --p.halos;
+  while (p.halos > 2 && budget - p.halos * halo_bytes < want * stage_bytes) --p.halos;
   p.stages = (budget - p.halos * halo_bytes) / stage_bytes;
   if (p.stages > EXACT_MAX_STAGES) p.stages = EXACT_MAX_STAGES;
   if (p.stages < 2) return MIE_EUNSUPPORTED;
-  const size_t smem = (size_t)((p.stages * stage_bytes + 1023) & ~1023) + (size_t)p.halos * halo_bytes + 1024;
+  const size_t smem = (size_t)((p.stages * stage_bytes + 1023) & ~1023) + (size_t)p.halos * halo_bytes + slab_bytes + 1024;
 
   ExactMaps maps;
   memset(&maps, 0, sizeof(maps));
@@ -369,6 +446,17 @@ int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
     const cuuint64_t str[3] = {128, rows * 128, nch * rows * 128};
     const cuuint32_t box_w[4] = {32, (cuuint32_t)(p.cb / 2), 1, 1};
     if (!tc_encode(&maps.w, 4, a->wpacked_exact, dims, str, box_w, CU_TENSOR_MAP_SWIZZLE_128B)) return MIE_EINVAL;
+  }
+  {
+    // epilogue slabs: half a block's channels of one tile
+    const cuuint32_t box[4] = {(cuuint32_t)(p.cb / 2), 8, 8, 1};
+    const CUtensorMapSwizzle sw = p.cb == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+    auto slab_map = [&](CUtensorMap *m, const float *base, int64_t ps) {
+      const cuuint64_t dims[4] = {(cuuint64_t)a->cout, (cuuint64_t)a->wout, (cuuint64_t)a->hout, (cuuint64_t)a->n};
+      const cuuint64_t str[3] = {(cuuint64_t)ps * 4, (cuuint64_t)a->wout * ps * 4, (cuuint64_t)a->hout * a->wout * ps * 4};
+      return tc_encode(m, 4, base, dims, str, box, sw);
+    };
+    if (!slab_map(&maps.out, a->out, a->out_ps) || (a->act != MIE_ACT_NONE && !slab_map(&maps.res, a->res, a->res_ps))) return MIE_EINVAL;
   }
   const int64_t items = (int64_t)quads * (a->cout_pad / p.cb);
   const int clusters = (int)(items < clusters_max ? items : clusters_max);

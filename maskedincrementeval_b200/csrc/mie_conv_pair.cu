@@ -72,33 +72,9 @@ __device__ __forceinline__ void tmem_ld16_pair(unsigned taddr, unsigned taddr2, 
 __device__ __forceinline__ void tma_load_slab(unsigned smem_addr, const CUtensorMap *map, unsigned bar, int c0, int x, int y, int n) {
   tma_load_4d_raw(smem_addr, map, bar, c0, x, y, n);
 }
-__device__ __forceinline__ void tma_store_slab(unsigned smem_addr, const CUtensorMap *map, int c0, int x, int y, int n) {
-  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-               ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_addr), "r"(c0), "r"(x), "r"(y), "r"(n) : "memory");
-}
 __device__ __forceinline__ void tma_add_slab(unsigned smem_addr, const CUtensorMap *map, int c0, int x, int y, int n) {
   asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
                ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_addr), "r"(c0), "r"(x), "r"(y), "r"(n) : "memory");
-}
-
-// Barrier of the 128 threads of an epilogue set: whether all of them bring `ok`.
-__device__ __forceinline__ bool set_all(int id, bool ok) {
-  int r;
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %2, 0;\n\tbarrier.cta.red.and.pred q, %1, 128, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
-               : "=r"(r) : "r"(id), "r"((int)ok) : "memory");
-  return r != 0;
-}
-
-// Shared-memory accesses by explicit address.  Through generic pointers (float4 * into the dynamic shared memory) the whole
-// kernel was compiled such that an MMA took 85-117 clocks to issue instead of 40-65, even where the accesses never ran:
-// decoder 0 / 2 of 8 streams 260x346 went from 184 / 416 us to 112 / 197 us with these two functions.
-__device__ __forceinline__ float4 lds4(unsigned addr) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ void sts4(unsigned addr, float4 v) {
-  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
 // One pixel, 16 channels (quads h0 .. h0 + 3 of a slab): v, the accumulator values; xs / es / os, shared addresses of the pixel's rows of the
@@ -160,7 +136,7 @@ __device__ __forceinline__ void pair_issue(const PairIssue a, const PairTapTable
   unsigned bs = 0, bpar = 0, as = 0, apar = 0, item_idx = 0, stage_addr = a.b_base;
   for (int item = a.item0; item < a.n_items; item += a.item_step, ++item_idx) {
     const unsigned buf = item_idx & 1u;
-    if (item_idx >= 2 && !mbar_wait_cluster(&acc_empty[buf], ((item_idx >> 1) - 1) & 1u, abort_flag, a.limit)) return;
+    if (item_idx >= 2 && !mbar_wait(&acc_empty[buf], ((item_idx >> 1) - 1) & 1u, abort_flag, a.limit)) return;
     tc_fence_after();
     const unsigned tmem_d = a.tmem_base + buf * a.nacc * (unsigned)a.NB;
     unsigned ntap = 0;
@@ -447,7 +423,7 @@ conv_pair_kernel(const PairParams P, const __grid_constant__ PairMaps maps) {
             if (h0 == 4 && sl + ds >= n_slabs) {     // last read of this warp: hand the accumulator back
               tc_fence_before();
               __syncwarp();
-              if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[buf]), 0));
+              if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&acc_empty[buf]), 0));
             }
             const bool f = thresholded ? pair_group_act<true>(p, v, xs, es, os, pcol, h0, ad, nq) : pair_group_act<false>(p, v, xs, es, os, pcol, h0, ad, nq);
             sent |= valid && f && co < p.cout;

@@ -82,8 +82,39 @@ __device__ __forceinline__ void pair_commit(unsigned long long *bar) {
                "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(smem_u32(bar))
                : "memory");
 }
+// "This warp has read the accumulator": an arrival on a barrier of the other (or this) block of the pair.  What it orders is
+// tensor memory (tcgen05.wait::ld and tcgen05.fence before it), no shared or global data; with release.cluster semantics the
+// arrival first waits for every store of the warp to drain, about 1000 clocks per segment of conv_exact_kernel.
+__device__ __forceinline__ void mbar_arrive_remote(unsigned cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 __device__ __forceinline__ void pair_cluster_sync() {
   asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tma_store_slab(unsigned smem_addr, const CUtensorMap *map, int c0, int x, int y, int n) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+               ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_addr), "r"(c0), "r"(x), "r"(y), "r"(n) : "memory");
+}
+
+// Barrier of the 128 threads of an epilogue set: whether all of them bring `ok`.
+__device__ __forceinline__ bool set_all(int id, bool ok) {
+  int r;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %2, 0;\n\tbarrier.cta.red.and.pred q, %1, 128, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+               : "=r"(r) : "r"(id), "r"((int)ok) : "memory");
+  return r != 0;
+}
+
+// Shared-memory accesses by explicit address.  Through generic pointers (float4 * into the dynamic shared memory) the whole
+// kernel was compiled such that an MMA took 85-117 clocks to issue instead of 40-65, even where the accesses never ran:
+// decoder 0 / 2 of 8 streams 260x346 went from 184 / 416 us to 112 / 197 us with these two functions.
+__device__ __forceinline__ float4 lds4(unsigned addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts4(unsigned addr, float4 v) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
 }  // namespace

@@ -527,12 +527,12 @@ int launch_conv_pair(const mie_conv_args *a, cudaStream_t st) {
   while (P.halos > 2 && budget - P.halos * halo_bytes < 64 * 1024) --P.halos;
   int stage_bytes = 0;
   for (;; p.nb >>= 1) {      // (large halos beside three slabs per set leave little for the ring: narrower blocks then)
-    P.tps = p.nb == 256 ? 1 : p.nb == 128 ? 2 : p.nb == 64 ? 4 : 7;
+    P.tps = p.nb == 256 ? 1 : p.nb == 128 ? 3 : p.nb == 64 ? 5 : 9;
     while (P.tps > 1 && 3 * P.tps * p.nb * 64 > budget - P.halos * halo_bytes) --P.tps;
     stage_bytes = P.tps * p.nb * 64;
     p.stages = (budget - P.halos * halo_bytes) / stage_bytes;
     if (p.stages > PAIR_MAX_STAGES) p.stages = PAIR_MAX_STAGES;
-    if (p.stages >= 3) break;
+    if (p.stages >= 2) break;
     if (p.nb == 32) return MIE_EUNSUPPORTED;
   }
   const size_t smem = (size_t)((p.stages * stage_bytes + 1023) & ~1023) + (size_t)P.halos * halo_bytes + 2 * P.slab_bufs * PAIR_SLAB_BYTES + 1024;

@@ -1303,6 +1303,64 @@ __global__ void __launch_bounds__(256) delta_mask_kernel(const float *__restrict
   run_tail_job(tail);
 }
 
+// Up to eight channels: both frames are read once into registers, all loads of a pixel in flight together, and the split
+// copy is written as whole 16-byte pieces (its padding channels are zero and stay zero).  Same results as the kernel above.
+template <int C>
+__global__ void __launch_bounds__(256) delta_mask_few_kernel(const float *__restrict__ x, int64_t x_ps, float *__restrict__ xp,
+                                                             int64_t xp_ps, float *__restrict__ dx, int64_t dx_ps,
+                                                             unsigned *__restrict__ bits32, int N, int H, int W, float thr,
+                                                             float *__restrict__ split, int64_t split_ps,
+                                                             unsigned *__restrict__ split_bits32, const mie_tail_job tail) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const int TH = (H + 7) >> 3, TW = (W + 7) >> 3;
+  const int ntiles = N * TH * TW;
+  const int lane = threadIdx.x & 31;
+  for (int t = blockIdx.x * 4 + (threadIdx.x >> 6); t < ntiles; t += gridDim.x * 4) {
+    const int p = threadIdx.x & 63;
+    const int tx = t % TW, ty = (t / TW) % TH, n = t / (TW * TH);
+    const int y = ty * 8 + (p >> 3), xx = tx * 8 + (p & 7);
+    const bool inside = y < H && xx < W;
+    const int64_t pix = inside ? (int64_t)(n * H + y) * W + xx : 0;
+    const size_t wi = 2 * (size_t)t + ((p >> 5) & 1);
+    const unsigned old = split ? split_bits32[wi] : 0u;
+    float v[C], d[8];
+    bool a = false;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) d[c] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < C; ++c) { v[c] = x[pix * x_ps + c]; d[c] = xp[pix * xp_ps + c]; }
+#pragma unroll
+    for (int c = 0; c < C; ++c) { d[c] = v[c] - d[c]; a |= fabsf(d[c]) > thr; }
+    a = a && inside;
+    const unsigned half = __ballot_sync(0xffffffffu, a);
+    if (inside) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        if (!a) d[c] = 0.0f;
+        dx[pix * dx_ps + c] = d[c];
+        if (a) xp[pix * xp_ps + c] = v[c];
+      }
+      if (split && (half | old) != 0u) {
+        float4 *o = reinterpret_cast<float4 *>(split + pix * split_ps);
+        float l[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) l[c] = d[c] - __uint_as_float(__float_as_uint(d[c]) & 0xFFFFE000u);
+        const float4 d0 = make_float4(d[0], d[1], d[2], d[3]), d1 = make_float4(d[4], d[5], d[6], d[7]);
+        o[0] = d0; o[1] = d1;
+        o[2] = make_float4(l[0], l[1], l[2], l[3]); o[3] = make_float4(l[4], l[5], l[6], l[7]);
+        o[4] = d0; o[5] = d1;
+      }
+    }
+    __syncwarp();      // every lane has read the copy's old word before lane 0 replaces it
+    if (lane == 0) {
+      bits32[wi] = half;
+      if (split) split_bits32[wi] = half;
+    }
+  }
+  run_tail_job(tail);
+}
+
 __global__ void __launch_bounds__(256) events_to_voxel_kernel(const float *__restrict__ ev, int n_events, int bins, int sh,
                                                               int sw, float *__restrict__ vox, int64_t ps, int H, int W,
                                                               int pl, int pt) {
@@ -1700,6 +1758,15 @@ extern "C" int mie_delta_mask(const float *x, int64_t x_ps, float *x_prev, int64
   const int ntiles = N * divup(H, 8) * divup(W, 8);
   int blocks = divup(ntiles, 4);
   if (blocks > MIE_SM_COUNT * 8) blocks = MIE_SM_COUNT * 8;
+  if ((C == 2 || C == 5) && (!split || (split_ps % 4 == 0 && aligned16(split)))) {      // count images, five voxel bins
+    auto launch = [&](auto kernel) {
+      launch_chained(kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, x, x_ps, x_prev, xp_ps, dx, dx_ps, reinterpret_cast<unsigned *>(bits),
+                     N, H, W, thr, split, split_ps, reinterpret_cast<unsigned *>(split_bits), tail_for_kernel(tail));
+    };
+    if (C == 2) launch(delta_mask_few_kernel<2>);
+    else launch(delta_mask_few_kernel<5>);
+    return tail_after_launch(check_launch(), tail, true, stream);
+  }
   launch_chained(delta_mask_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, x, x_ps, x_prev, xp_ps, dx, dx_ps,
                                                               reinterpret_cast<unsigned *>(bits), N, C, H, W, thr, split, split_ps,
                                                               shalf, reinterpret_cast<unsigned *>(split_bits), tail_for_kernel(tail));

@@ -484,114 +484,6 @@ __global__ void __launch_bounds__(256) conv1x1_small_kernel(const ConvParams p) 
   run_tail_job(p.tail);
 }
 
-// The same with whole channel quads: eight lanes per pixel, a quad each (further ones in turn), so that a warp's loads cover
-// whole 128-byte lines; the sums meet in a butterfly and lane j finishes output channel j.  Bound by HBM (Cin * 4 bytes per
-// pixel and input).  With a thread per pixel every load of a warp touched 32 lines.
-__global__ void __launch_bounds__(256) conv1x1_quads_kernel(const ConvParams p) {
-  grid_dependency_wait();
-  grid_dependency_trigger();
-  extern __shared__ float s_w[];  // [cin][SMALL_COUT]
-  __shared__ unsigned s_bits[2];
-  const int tid = threadIdx.x, lane = tid & 31, q = tid & 7;
-  for (int i = tid; i < p.cin * SMALL_COUT; i += blockDim.x) {
-    const int ci = i / SMALL_COUT, co = i - ci * SMALL_COUT;
-    s_w[i] = (co < p.cout) ? p.w[(int64_t)ci * p.cout_pad + co] : 0.0f;
-  }
-  __syncthreads();
-  const int THo = (p.hout + 7) >> 3, TWo = (p.wout + 7) >> 3;
-  const int ntiles_total = p.n * THo * TWo;
-  const bool head_ok = run_head_job(p.head, HEAD_SPIN_LIMIT);
-  if (threadIdx.x == blockDim.x - 1) count_head_job_passed(p.head);
-  const int n_stale = (p.stale && head_ok) ? min(p.counts[1], p.max_tiles) : 0;
-  for (int s = blockIdx.x; s < n_stale; s += gridDim.x) {
-    const int t = p.stale[s];
-    if (t < 0 || t >= ntiles_total) { if (tid == 0) atomicOr(&p.counts[3], MIE_ERR_BAD_TILE); continue; }
-    const int tx = t % TWo, ty = (t / TWo) % THo, n = t / (TWo * THo);
-    const int oy = ty * 8 + ((tid & 63) >> 3), ox = tx * 8 + (tid & 7), c = tid >> 6;     // 64 pixels x 4 channels
-    if (oy < p.hout && ox < p.wout && c < p.cout) p.out[((int64_t)(n * p.hout + oy) * p.wout + ox) * p.out_ps + c] = 0.0f;
-  }
-  const int n_active = head_ok ? min(p.counts[0], p.max_tiles) : 0;
-  for (int li = blockIdx.x; li < n_active; li += gridDim.x) {
-    const int t = p.list[li];
-    if (t < 0 || t >= ntiles_total) { if (tid == 0) atomicOr(&p.counts[3], MIE_ERR_BAD_TILE); continue; }
-    const int tx = t % TWo, ty = (t / TWo) % THo, n = t / (TWo * THo);
-    __syncthreads();      // the previous tile's word has been stored
-    if (tid < 2) s_bits[tid] = 0u;
-    __syncthreads();
-    float acc[2][SMALL_COUT] = {};
-    int64_t pix[2];
-    bool valid[2];
-    float x[2] = {0.0f, 0.0f};
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int px = (tid >> 3) + 32 * i, oy = ty * 8 + (px >> 3), ox = tx * 8 + (px & 7);
-      valid[i] = oy < p.hout && ox < p.wout;
-      pix[i] = (int64_t)(n * p.hout + oy) * p.wout + ox;      // 1x1, stride 1: input pixel == output pixel
-      if (valid[i] && q < p.cout && p.act != MIE_ACT_NONE && !p.refresh) x[i] = p.res[pix[i] * p.res_ps + q];
-    }
-#pragma unroll 2
-    for (int c = 4 * q; c < p.cin; c += 32)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        if (!valid[i]) continue;
-        float4 v = *reinterpret_cast<const float4 *>(p.in + pix[i] * p.in_ps + c);
-        if (p.in2) {
-          const float4 u = *reinterpret_cast<const float4 *>(p.in2 + pix[i] * p.in2_ps + c);
-          v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
-        }
-        const float *w = s_w + c * SMALL_COUT;
-#pragma unroll
-        for (int j = 0; j < SMALL_COUT; ++j)
-          acc[i][j] += v.x * w[j] + v.y * w[SMALL_COUT + j] + v.z * w[2 * SMALL_COUT + j] + v.w * w[3 * SMALL_COUT + j];
-      }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      float d = 0.0f;
-      bool any_d = p.refresh != 0;
-#pragma unroll
-      for (int j = 0; j < SMALL_COUT; ++j) {
-        float a = acc[i][j];
-        a += __shfl_xor_sync(0xffffffffu, a, 4);
-        a += __shfl_xor_sync(0xffffffffu, a, 2);
-        a += __shfl_xor_sync(0xffffffffu, a, 1);
-        if (j == q) d = a;
-      }
-      const bool mine = valid[i] && q < p.cout;
-      if (mine) {
-        if (p.bias) d += p.bias[q];
-        if (p.addend) d += p.addend[pix[i] * p.addend_ps + q];
-      }
-      // "does this pixel carry any change", over its output channels
-      any_d |= ((__ballot_sync(0xffffffffu, mine && d != 0.0f) >> (lane & 24)) & 0xFFu) != 0u;
-      float dy = mine ? d : 0.0f;
-      if (mine && p.act != MIE_ACT_NONE) {
-        if (any_d || p.emitted) {
-          const float xn = x[i] + d;
-          if (any_d) p.res[pix[i] * p.res_ps + q] = xn;
-          const float base = p.refresh ? 0.0f : (p.emitted ? p.emitted[pix[i] * p.emitted_ps + q] : act_apply(p.act, x[i]));
-          dy = act_apply(p.act, xn) - base;
-        } else {
-          dy = 0.0f;
-        }
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, mine && fabsf(dy) > p.thr);
-      const bool flag = valid[i] && (((bal >> (lane & 24)) & 0xFFu) != 0u || p.refresh != 0);
-      if (mine) {
-        const float v = flag ? dy : 0.0f;
-        p.out[pix[i] * p.out_ps + q] = v;
-        if (p.emitted && flag) p.emitted[pix[i] * p.emitted_ps + q] += v;
-        if (p.accum && flag) p.accum[pix[i] * p.accum_ps + q] += v;
-      }
-      const unsigned px4 = __ballot_sync(0xffffffffu, flag && q == 0);     // pixels 4 * warp .. + 3 of half tile i
-      if (lane == 0 && px4)
-        atomicOr(&s_bits[i], ((px4 & 1u) | ((px4 >> 7) & 2u) | ((px4 >> 14) & 4u) | ((px4 >> 21) & 8u)) << (4 * (tid >> 5)));
-    }
-    __syncthreads();
-    if (tid < 2 && s_bits[tid]) reinterpret_cast<unsigned *>(p.out_bits)[2 * (size_t)t + tid] = s_bits[tid];
-  }
-  run_tail_job(p.tail);
-}
-
 // ---------------------------------------------------------------------------------------------
 // 3x3 convolution of one or two input channels (event-count images) in fp32: at 18 multiplications per output the layer is a
 // pass over the state, bound by HBM (per active pixel Cout * 12 bytes).  Block = (tile, 32 output channels), eight lanes per
@@ -853,11 +745,6 @@ extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
     if (blocks > MIE_SM_COUNT * 8) blocks = MIE_SM_COUNT * 8;
     p.in_vec = p.in_vec && (a->cin % 4 == 0 || a->in_ps >= (a->cin + 3) / 4 * 4) &&
                (!a->in2 || (a->in2_ps % 4 == 0 && aligned16(a->in2) && a->in2_ps >= (a->cin + 3) / 4 * 4));
-    if (p.in_vec && a->cin % 4 == 0) {
-      blocks = a->max_tiles < MIE_SM_COUNT * 8 ? a->max_tiles : MIE_SM_COUNT * 8;
-      launch_chained(conv1x1_quads_kernel, dim3(blocks), dim3(256), (size_t)a->cin * SMALL_COUT * sizeof(float), (cudaStream_t)stream, p);
-      return tail_after_launch(check_launch(), a->tail, true, stream);
-    }
     launch_chained(conv1x1_small_kernel, dim3(blocks), dim3(256), (size_t)a->cin * SMALL_COUT * sizeof(float), (cudaStream_t)stream, p);
     return tail_after_launch(check_launch(), a->tail, true, stream);
   }

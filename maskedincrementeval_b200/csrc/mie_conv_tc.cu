@@ -17,6 +17,9 @@
 //   Roles (192 threads): warp 0 = TMA producer (one lane), warp 1 = MMA issuer (one lane) and owner of the
 //   tensor-memory allocation, warps 2..5 = epilogue.  Takes stride 2, k = 1 and blocks of 256 channels.
 //
+// (Layers with k >= 3 run on the CTA-pair kernel of mie_conv_pair.cu; of the kernels here the per-tap one takes k = 1, and
+// both take the cluster form behind MIE_OPT_TC_KSPLIT.)
+//
 // conv_tc_halo_kernel (halo-resident): stride 1, k in {3,5,7}.  The input halo of both tiles stays in shared
 // memory for a whole channel chunk, a filter tap is an address shift of the operand descriptor, and only filter
 // slices stream through the ring -- several taps per stage, two MMA-issuing warps.  See the comment at the kernel.
@@ -1130,11 +1133,9 @@ int launch_conv_tc(const mie_conv_args *a, cudaStream_t st) {
   while (acc_cols < nb) acc_cols <<= 1;
   const int64_t max_items = (int64_t)((a->max_tiles + 1) / 2) * (a->cout_pad / nb);
 
-  // ---- halo-resident kernel: stride 1, k in {3,5,7} ----
-  // Two shapes stay on the per-tap kernel: blocks of 256 channels with more work items than SMs (bound by the
-  // tensor core itself, not by instruction issue: per-tap measured 15 % faster), and layers of a single channel
-  // chunk with a 3x3 filter (the halo is used for 9 taps only once: per-tap measured 8 % faster on 32 -> 32 channels).
-  if (a->stride == 1 && a->k >= 3 && a->k <= 7 && !(nb == 256 && max_items > MIE_SM_COUNT) && (p.cin_pad > 32 || a->k >= 5) && halo_enabled()) {
+  // ---- halo-resident kernel, as clusters: stride 1, k in {3,5,7} (everything else with k >= 3 is the pair kernel's) ----
+  // Layers of a single channel chunk with a 3x3 filter stay on the per-tap kernel (the halo is used for 9 taps only once).
+  if (ksplit > 1 && a->stride == 1 && (p.cin_pad > 32 || a->k >= 5) && halo_enabled()) {
     const int Wh = 8 + a->k - 1;
     const int a_bytes = 2 * (Wh * 2 * 8 * Wh * 16);          // two buffers of [Hh][2 tiles][8 groups][Wh][16 B]
     // A stage holds `tps` consecutive taps of one channel chunk (one TMA): the issuing thread pays its wait /
@@ -1154,11 +1155,6 @@ int launch_conv_tc(const mie_conv_args *a, cudaStream_t st) {
     if (stages >= 2) {
       p.stages = stages;
       const size_t smem = (size_t)stages * b_bytes + a_bytes + part_bytes + 1024;
-      int blocks_per_sm = (int)((220 * 1024) / (smem + 2048));
-      const int by_tmem = 512 / (2 * p.issuers * acc_cols);
-      if (blocks_per_sm > by_tmem) blocks_per_sm = by_tmem;
-      if (blocks_per_sm > 1) blocks_per_sm = 1;   // registers: 384 threads x ~112
-      if (blocks_per_sm < 1) blocks_per_sm = 1;
       CUtensorMap map_in, map_w;
       const cuuint64_t dims[5] = {4, (cuuint64_t)a->win, (cuuint64_t)((a->cin + 3) / 4), (cuuint64_t)a->hin, (cuuint64_t)a->n};
       const cuuint64_t str[4] = {(cuuint64_t)a->in_ps * 4, 16, (cuuint64_t)a->win * a->in_ps * 4, (cuuint64_t)a->hin * a->win * a->in_ps * 4};
@@ -1168,13 +1164,9 @@ int launch_conv_tc(const mie_conv_args *a, cudaStream_t st) {
       const cuuint64_t wstr[3] = {128, (cuuint64_t)a->cout_pad * 128, nch * a->cout_pad * 128};
       const cuuint32_t box_w[4] = {32, (cuuint32_t)nb, 1, (cuuint32_t)p.tps};
       if (tc_encode(&map_in, 5, a->in, dims, str, box, CU_TENSOR_MAP_SWIZZLE_NONE) && tc_encode(&map_w, 4, a->wpacked_tc, wdims, wstr, box_w, CU_TENSOR_MAP_SWIZZLE_128B)) {
-        const int64_t cap = (int64_t)MIE_SM_COUNT * blocks_per_sm;
-        int grid = max_items < cap ? (int)max_items : (int)cap;
-        if (grid < 1) grid = 1;
-        grid = (int)own_grid(ksplit > 1 ? max_items : grid, ksplit > 1 ? 8 : 4);   // clusters: one per possible item, as below
+        own_grid(max_items, 8);   // clusters: one per possible item
         if (own_status != MIE_OK) return own_status;
-        static int halo_smem_set[MAX_DEVICES] = {0};
-        if (ksplit > 1) {
+        {
           static int halo_ks_smem_set[MAX_DEVICES] = {0};
           static int halo_ks_own_smem_set[MAX_DEVICES] = {0};
           p.ksplit = ksplit;
@@ -1189,15 +1181,6 @@ int launch_conv_tc(const mie_conv_args *a, cudaStream_t st) {
                                  (unsigned)ksplit, p, map_in, map_w);
           return check_launch();
         }
-        if (p.own) {
-          static int halo_own_smem_set[MAX_DEVICES] = {0};
-          { const int s_ = ensure_dynamic_smem(conv_tc_halo_kernel<false, true>, halo_own_smem_set, smem); if (s_ != MIE_OK) return s_; }
-          launch_chained(conv_tc_halo_kernel<false, true>, dim3(grid), dim3(HALO_THREADS), smem, st, p, map_in, map_w);
-          return check_launch();
-        }
-        { const int s_ = ensure_dynamic_smem(conv_tc_halo_kernel<false, false>, halo_smem_set, smem); if (s_ != MIE_OK) return s_; }
-        launch_chained(conv_tc_halo_kernel<false, false>, dim3(grid), dim3(HALO_THREADS), smem, st, p, map_in, map_w);
-        return check_launch();
       }
       // a tensor map the driver refuses (unusual strides): the per-tap kernel below takes the layer
     }

@@ -390,14 +390,47 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
 
 }  // namespace
 
+// How a launch divides its columns and its shared memory; `stages` < 2: no split of it fits.
+struct ExactShape {
+  PairTaps t;
+  int wp, cb, tps, stages, halos;
+  size_t smem;
+};
+static ExactShape exact_shape(const mie_conv_args *a) {
+  ExactShape h;
+  pair_make_taps(a->k, a->stride, a->pad, &h.t, &h.wp);
+  const int quads = divup(a->max_tiles, 4), clusters_max = MIE_SM_COUNT / 2;
+  // 64 channels per block (107 clocks per K-slice and tap) unless blocks of 32 (82) take fewer clocks over all rounds
+  h.cb = 32;
+  if (a->cout_pad % 64 == 0 &&
+      (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 107 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 82)
+    h.cb = 64;
+  const int halo_bytes = (h.wp * 2 * h.wp * 128 + 1023) & ~1023, slab_bytes = 2 * (a->act != MIE_ACT_NONE ? 2 : 1) * 128 * (h.cb / 2) * 4;
+  const int budget = 222 * 1024 - slab_bytes;
+  // Fat stages: what the issuer and the producers spend per stage does not depend on its size.  Three of them where
+  // halo buffers can be spared for that, else two; a 7x7 filter's halos beside the slabs of a wide block leave room for
+  // two stages of three taps (still ahead of blocks of 32 channels with nine: 64 -> 64 on 2 x 256x336 366 against 436 us,
+  // on 104x104 46 against 56).
+  h.tps = h.cb == 32 ? 9 : 5;
+  h.halos = EXACT_MAX_HALOS;
+  while (h.halos > 2 && budget - h.halos * halo_bytes < 3 * h.tps * h.cb * 128) --h.halos;
+  while (h.tps > 1 && budget - h.halos * halo_bytes < 2 * h.tps * h.cb * 128) --h.tps;
+  const int stage_bytes = h.tps * h.cb * 128;
+  h.stages = (budget - h.halos * halo_bytes) / stage_bytes;
+  if (h.stages > EXACT_MAX_STAGES) h.stages = EXACT_MAX_STAGES;
+  h.smem = (size_t)((h.stages * stage_bytes + 1023) & ~1023) + (size_t)h.halos * halo_bytes + slab_bytes + 1024;
+  return h;
+}
+
 bool exact_takes(const mie_conv_args *a) {
   return a->refresh && !a->head && a->wpacked_exact && a->in_lo && a->k >= 3 && a->k <= 7 && (a->stride == 1 || a->stride == 2) && !a->in2 && !a->accum &&
          a->in_ps % 4 == 0 && aligned16(a->in) && aligned16(a->in_lo) && aligned16(a->wpacked_exact) && a->cout % 4 == 0 && a->out_ps % 4 == 0 &&
          aligned16(a->out) && (!a->res || (a->res_ps % 4 == 0 && aligned16(a->res))) && (!a->addend || (a->addend_ps % 4 == 0 && aligned16(a->addend))) &&
-         a->cout_pad % 32 == 0;
+         a->cout_pad % 32 == 0 && exact_shape(a).stages >= 2;
 }
 
 int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
+  const ExactShape h = exact_shape(a);
   ExactParams p;
   memset(&p, 0, sizeof(p));
   p.spin_limit = g_opt_spin_limit;
@@ -407,24 +440,9 @@ int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
   p.out = a->out; p.out_ps = a->out_ps; p.out_bits32 = reinterpret_cast<unsigned int *>(a->out_bits);
   p.act = a->act; p.res = a->res; p.res_ps = a->res_ps; p.addend = a->addend; p.addend_ps = a->addend_ps; p.bias = a->bias;
   p.tail = tail_for_kernel(a->tail);
-  pair_make_taps(a->k, a->stride, a->pad, &p.t, &p.wp);
+  p.t = h.t; p.wp = h.wp; p.cb = h.cb; p.tps = h.tps; p.stages = h.stages; p.halos = h.halos;
+  const size_t smem = h.smem;
   const int quads = divup(a->max_tiles, 4), clusters_max = MIE_SM_COUNT / 2;
-  // 64 channels per block (107 clocks per K-slice and tap) unless blocks of 32 (82) take fewer clocks over all rounds
-  p.cb = 32;
-  if (a->cout_pad % 64 == 0 &&
-      (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 107 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 82)
-    p.cb = 64;
-  // fat stages: what the issuer and the producers spend per stage does not depend on its size
-  const int halo_bytes = (p.wp * 2 * p.wp * 128 + 1023) & ~1023, slab_bytes = 2 * (a->act != MIE_ACT_NONE ? 2 : 1) * 128 * (p.cb / 2) * 4;
-  const int budget = 222 * 1024 - slab_bytes;
-  p.tps = p.cb == 32 ? 9 : 5;
-  const int stage_bytes = p.tps * p.cb * 128, want = p.cb == 32 ? 3 : 3;
-  p.halos = EXACT_MAX_HALOS;
-  while (p.halos > 2 && budget - p.halos * halo_bytes < want * stage_bytes) --p.halos;
-  p.stages = (budget - p.halos * halo_bytes) / stage_bytes;
-  if (p.stages > EXACT_MAX_STAGES) p.stages = EXACT_MAX_STAGES;
-  if (p.stages < 2) return MIE_EUNSUPPORTED;
-  const size_t smem = (size_t)((p.stages * stage_bytes + 1023) & ~1023) + (size_t)p.halos * halo_bytes + slab_bytes + 1024;
 
   ExactMaps maps;
   memset(&maps, 0, sizeof(maps));

@@ -24,10 +24,12 @@ def cl(t):
     return t.contiguous(memory_format=torch.channels_last)
 
 
-# cin, cout, k, stride, n, h, w, addend: ragged tiles, one pair of tiles, partial chunks and slabs, both block widths
+# cin, cout, k, stride, n, h, w, addend: ragged tiles, one pair of tiles, partial chunks and slabs, both block widths for
+# every filter size (7x7 in blocks of 64 channels: the halos leave the least room for the filter ring)
 @pytest.mark.parametrize("case", [(5, 32, 5, 1, 1, 41, 50, False), (2, 64, 3, 2, 1, 18, 26, False), (64, 40, 3, 1, 2, 8, 16, False),
                                   (32, 64, 5, 2, 1, 67, 89, False), (256, 256, 3, 1, 1, 33, 44, True), (256, 128, 5, 1, 1, 34, 44, False),
-                                  (96, 96, 7, 1, 1, 24, 40, False), (130, 36, 3, 1, 1, 9, 9, False)])
+                                  (96, 96, 7, 1, 1, 24, 40, False), (130, 36, 3, 1, 1, 9, 9, False),
+                                  (64, 64, 7, 1, 1, 104, 104, False), (64, 64, 7, 2, 1, 205, 208, False), (32, 64, 5, 1, 1, 104, 100, False)])
 def test_dense_pass_against_float64(dev, case):
     from maskedincrementeval_b200 import fields as fl, _native as nat
     from maskedincrementeval_b200.incr_modules._algebra import NATIVE

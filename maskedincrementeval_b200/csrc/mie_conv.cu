@@ -880,8 +880,19 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   if (s != MIE_OK) return s;
   int cp, op; int64_t nf;
   mie_conv_pack_dims(cin, cout, k, &cp, &op, &nf);
-  const bool exact = inc_exact(cin, cout, k) && aligned16(out_incr);
+  mie_conv_args a;
+  memset(&a, 0, sizeof(a));
+  a.in = x_incr; a.in_ps = cin; a.cin = cin; a.hin = H; a.win = W;
+  a.wpacked = wp; a.cin_pad = cp; a.cout = cout; a.cout_pad = op;
+  a.n = N; a.hout = Ho; a.wout = Wo; a.k = k; a.stride = stride; a.pad = pad;
+  a.list = list; a.stale = nullptr; a.counts = counts; a.max_tiles = nto;
+  a.out = out_incr; a.out_ps = cout; a.out_bits = bits_out;
+  a.act = MIE_ACT_NONE; a.thr = 0.0f;
+  mie_conv_args x = a;       // without bias and activation a dense evaluation is the plain convolution of the listed tiles
   float *wx = reinterpret_cast<float *>(ws + L.wexact), *hi = reinterpret_cast<float *>(ws + L.hi), *lo = reinterpret_cast<float *>(ws + L.lo);
+  x.refresh = 1;
+  x.in = hi; x.in_lo = lo; x.in_ps = L.cp; x.wpacked_exact = wx;
+  const bool exact = inc_exact(cin, cout, k) && exact_takes(&x);
   if (exact) {
     if ((s = pack_exact(filter, cout, cin, k, 1, wx, st)) != MIE_OK) return s;
     if ((s = mie_split_exact(x_incr, cin, cin, (int64_t)N * H * W, hi, lo, L.cp, stream)) != MIE_OK) return s;
@@ -893,18 +904,5 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   }
   s = mie_tiles_dilate(bits_in, N, H, W, Ho, Wo, k, stride, pad, nullptr, nullptr, list, nullptr, counts, flags, stream);
   if (s != MIE_OK) return s;
-  mie_conv_args a;
-  memset(&a, 0, sizeof(a));
-  a.in = x_incr; a.in_ps = cin; a.cin = cin; a.hin = H; a.win = W;
-  a.wpacked = wp; a.cin_pad = cp; a.cout = cout; a.cout_pad = op;
-  a.n = N; a.hout = Ho; a.wout = Wo; a.k = k; a.stride = stride; a.pad = pad;
-  a.list = list; a.stale = nullptr; a.counts = counts; a.max_tiles = nto;
-  a.out = out_incr; a.out_ps = cout; a.out_bits = bits_out;
-  a.act = MIE_ACT_NONE; a.thr = 0.0f;
-  if (exact) {      // (without bias and activation a dense evaluation is the plain convolution of the listed tiles)
-    a.refresh = 1;
-    a.in = hi; a.in_lo = lo; a.in_ps = L.cp; a.wpacked_exact = wx;
-    if (!exact_takes(&a)) return MIE_EALIGN;
-  }
-  return mie_conv_tiles(&a, stream);
+  return mie_conv_tiles(exact ? &x : &a, stream);
 }

@@ -63,6 +63,27 @@ def test_dense_pass_against_float64(dev, case):
     assert err["auto"] <= max(1.2 * err["off"], 6e-7), err
 
 
+# stride 2 on fields one pixel wide or high, which have no odd columns or rows
+@pytest.mark.parametrize("h,w", [(17, 1), (1, 22), (1, 1), (2, 9)])
+@pytest.mark.parametrize("k", [3, 5])
+def test_stride_two_on_one_pixel_fields(dev, h, w, k):
+    from maskedincrementeval_b200.ext.pointops import pointops_functional as pf
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    torch.manual_seed(6)
+    layer = ConvLayerIncr(32, 64, k, 2, k // 2, activation="relu").to(dev).eval()
+    c = layer.conv2d
+    x = cl(torch.randn(2, 32, h, w, device=dev))
+    want = F.conv2d(x.double(), c.weight.detach().double(), c.bias.detach().double(), stride=2, padding=k // 2)
+    with torch.no_grad():
+        NATIVE.conv(c, NATIVE.lift(x), layer.activation)
+        got = layer.activation.in_res.reservoir
+        y, _ = pf.functional_conv_module(x, c.conv2d_weights, mask=None, stride=(2, 2), padding=(k // 2, k // 2))
+    assert float((got.double() - want).norm() / want.norm()) <= 2e-6      # fp32 sums of 32 * k * k products
+    want = want - c.bias.detach().double().view(1, -1, 1, 1)
+    assert float((y.double() - want).norm() / want.norm()) <= 2e-6
+
+
 @pytest.mark.parametrize("c,dtype", [(20, torch.float32), (32, torch.float32), (132, torch.float32), (16, torch.uint8), (48, torch.uint8), (20, torch.int32)])
 def test_mask_words_vectorised(dev, c, dtype):
     from maskedincrementeval_b200 import fields as fl

@@ -426,7 +426,7 @@ bool exact_takes(const mie_conv_args *a) {
   // a field one pixel wide or high has no odd columns or rows: that parity view of stride 2 would be empty, and a tensor map
   // cannot say so
   if (a->stride == 2 && (a->hin == 1 || a->win == 1)) return false;
-  return a->refresh && !a->head && a->wpacked_exact && a->in_lo && a->k >= 3 && a->k <= 7 && (a->stride == 1 || a->stride == 2) && !a->in2 && !a->accum &&
+  return a->refresh && !a->head && a->wpacked_exact && a->in_lo && a->k >= 3 && a->k <= 7 && (a->k & 1) && (a->stride == 1 || a->stride == 2) && !a->in2 && !a->accum &&
          a->in_ps % 4 == 0 && aligned16(a->in) && aligned16(a->in_lo) && aligned16(a->wpacked_exact) && a->cout % 4 == 0 && a->out_ps % 4 == 0 &&
          aligned16(a->out) && (!a->res || (a->res_ps % 4 == 0 && aligned16(a->res))) && (!a->addend || (a->addend_ps % 4 == 0 && aligned16(a->addend))) &&
          a->cout_pad % 32 == 0 && exact_shape(a).stages >= 2;

@@ -45,6 +45,17 @@ def test_host_side_argument_checks_need_no_gpu():
     assert nat.lib.mie_conv_increment_workspace_bytes(1, 32, 260, 346, 32, 3, 1) > 0
 
 
+def test_dense_evaluation_takes_the_filter_sizes_that_a_step_takes():
+    import ctypes as C
+    for k in range(1, 9):
+        a = nat.ConvArgs()
+        a.in_ = a.in_lo = a.wpacked_exact = a.out = a.res = 1 << 20      # never dereferenced: the question is the host's
+        a.cin, a.in_ps, a.cout, a.cout_pad, a.out_ps, a.res_ps = 64, 64, 64, 64, 64, 64
+        a.n, a.hin, a.win, a.hout, a.wout, a.max_tiles = 1, 64, 64, 64, 64, 64
+        a.k, a.stride, a.pad, a.refresh, a.act = k, 1, k // 2, 1, nat.ACT_RELU
+        assert nat.lib.mie_conv_is_exact(C.byref(a)) == (k in (3, 5, 7)), k
+
+
 def test_geometry_helpers():
     assert fl.n_tiles(1, 260, 346) == 33 * 44
     assert fl.conv_out_hw(264, 352, 5, 2, 2) == (132, 176)

@@ -270,15 +270,16 @@ class _PreparedCall:
     """An incremental call of one convolution with everything decided: what a layer that is called again with the same
     kind of input needs is a few identity checks and one call of the library, where deciding it anew took most of the
     40 us a small layer's step lasted.  Built at the end of a full call (``nnConvIncr.forward_fused``) and valid while
-    nothing it was decided by has changed: the library's configuration and options, the filter, the activation's state
-    buffers and threshold, the input's geometry and the address of its tile words."""
-    __slots__ = ("activation", "cin_limit", "epoch", "options", "weight", "weight_key", "reservoir", "reservoir_ptr", "emitted",
+    nothing it was decided by has changed: the library's configuration and options, the filter and the layer's precision,
+    the activation's function, state buffers and threshold, the input's geometry and the address of its tile words."""
+    __slots__ = ("activation", "cin_limit", "epoch", "options", "precision", "op", "weight", "weight_key", "reservoir", "reservoir_ptr", "emitted",
                  "threshold", "shape", "stride", "device", "mask_bits", "mask_ptr", "geometry", "plan", "args", "args_ref", "dilate", "tc_option",
                  "out", "input_threshold", "keep")
 
     def __init__(self, conv, activation, cin_limit, plan, d, mask, derived, dilate, thresholded):
         self.activation, self.cin_limit, self.plan = activation, cin_limit, plan     # (not the convolution: that would be a cycle)
         self.epoch, self.options = config.epoch, nat.option_epoch[0]
+        self.precision, self.op = conv.precision, None if activation is None else activation.op
         self.weight = conv.weight
         self.weight_key = (self.weight._version, self.weight.data_ptr())
         self.reservoir = self.emitted = self.threshold = None
@@ -304,13 +305,14 @@ class _PreparedCall:
         w = conv._parameters["weight"]
         plan = self.plan
         if (self.epoch != config.epoch or self.options != nat.option_epoch[0] or d.shape != self.shape or d.stride() != self.stride
-                or d.device != self.device or d.dtype is not torch.float32 or w is not self.weight
+                or d.device != self.device or d.dtype is not torch.float32 or w is not self.weight or conv.precision != self.precision
                 or (w._version, w.data_ptr()) != self.weight_key or plan.needs_clear or plan.accum_target is not None or plan.tail is not self.keep):
             return None
         act = self.activation
         if act is not None:
             r = act.in_res.reservoir
-            if r is not self.reservoir or r.data_ptr() != self.reservoir_ptr or act.emitted is not self.emitted or act.threshold != self.threshold:
+            if (r is not self.reservoir or r.data_ptr() != self.reservoir_ptr or act.emitted is not self.emitted or act.threshold != self.threshold
+                    or act.op is not self.op):
                 return None
         ptr = d.data_ptr()
         if m is None:
@@ -335,12 +337,13 @@ class _PreparedCall:
 class _PreparedRefresh:
     """The same for the dense evaluation of a layer in fp32 precision on the tensor cores (60 us of deciding per layer
     otherwise, more than its kernels take)."""
-    __slots__ = ("activation", "cin_limit", "epoch", "options", "params", "reservoir", "reservoir_ptr", "geometry", "mask_ptr", "addend_ptrs",
+    __slots__ = ("activation", "cin_limit", "epoch", "options", "op", "params", "reservoir", "reservoir_ptr", "geometry", "mask_ptr", "addend_ptrs",
                  "plan", "args", "fields", "fields_ps", "x_ps", "job", "out")
 
     def __init__(self, conv, activation, cin_limit, plan, d, mask, addend):
         self.activation, self.cin_limit, self.plan = activation, cin_limit, plan
         self.epoch, self.options = config.epoch, nat.option_epoch[0]
+        self.op = None if activation is None else activation.op
         self.params = self.parameters_of(conv)
         self.reservoir = None if activation is None else activation.in_res.reservoir
         self.reservoir_ptr = 0 if activation is None else self.reservoir.data_ptr()
@@ -366,7 +369,7 @@ class _PreparedRefresh:
             return None
         if act is not None:
             r = act.in_res.reservoir
-            if r is not self.reservoir or r.data_ptr() != self.reservoir_ptr or act.emitted is not None:
+            if r is not self.reservoir or r.data_ptr() != self.reservoir_ptr or act.emitted is not None or act.op is not self.op:
                 return None
         if addend is not None and (type(addend[1]) is not TileMask or (addend[0].data_ptr(), addend[1].bits.data_ptr()) != self.addend_ptrs):
             return None

@@ -1,0 +1,222 @@
+"""A layer that is called again with the same kind of input takes a prepared call.  Whatever that call was decided by may
+change between two calls: the prepared call has to be given up then, and the result has to be the one that a layer which
+decides every call anew gives, to the bit."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+N, C, H, W = 1, 32, 40, 56
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch.device("cuda:0")
+
+
+@pytest.fixture(autouse=True)
+def restore_config():
+    from maskedincrementeval_b200 import _native as nat, fields as fl
+    names = ("threshold", "carry", "tensor_cores", "tc_thresholded", "own_tiles", "kfenced_step", "input_threshold", "head_dilation", "tail_dilation")
+    saved, own = {k: getattr(fl.config, k) for k in names}, nat.get_option(nat.OPT_TC_OWN_KERNELS)
+    yield
+    for k, v in saved.items():
+        setattr(fl.config, k, v)
+    nat.set_option(nat.OPT_TC_OWN_KERNELS, own)
+    fl.forget_tails()
+
+
+@pytest.fixture
+def prepared(monkeypatch):
+    """The outcomes of the prepared calls and refreshes of the test so far: True where one was taken."""
+    from maskedincrementeval_b200.incr_modules import mask_incr_modules as mim
+    taken = []
+
+    def watch(cls):
+        run = cls.run
+        monkeypatch.setattr(cls, "run", lambda self, *a: (lambda out: (taken.append(out is not None), out)[1])(run(self, *a)))
+
+    watch(mim._PreparedCall)
+    watch(mim._PreparedRefresh)
+    return taken
+
+
+def cl(t):
+    return t.contiguous(memory_format=torch.channels_last)
+
+
+def _layer(dev):
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    torch.manual_seed(0)
+    return ConvLayerIncr(C, C, 3, 1, 1, activation="relu").to(dev).eval()
+
+
+def _sparse(g, dev, std=0.5):
+    return cl(torch.randn(N, C, H, W, generator=g, device=dev) * std * (torch.rand(N, 1, H, W, generator=g, device=dev) < 0.2))
+
+
+def _decide_anew(layer):
+    layer.conv2d._prepared = layer.conv2d._prepared_refresh = None
+
+
+def _set(obj, **kw):
+    for k, v in kw.items():
+        setattr(obj, k, v)
+
+
+def _config(**kw):
+    def change(layer):
+        from maskedincrementeval_b200 import fields as fl
+        _set(fl.config, **kw)
+    return change
+
+
+def _scaled(layer):
+    with torch.no_grad():
+        layer.conv2d.weight.mul_(1.5)
+
+
+def _replaced(layer):
+    layer.conv2d.weight = torch.nn.Parameter(layer.conv2d.weight.detach().clone() * -1.0)
+
+
+def _moved(layer):
+    layer.conv2d.weight.data = layer.conv2d.weight.detach().clone() * 0.5
+
+
+def _state_replaced(layer):
+    layer.activation.in_res.reservoir = cl(layer.activation.in_res.reservoir.clone() + 0.25)
+
+
+def _option(layer):
+    from maskedincrementeval_b200 import _native as nat
+    nat.set_option(nat.OPT_TC_OWN_KERNELS, 0)
+
+
+CHANGES = {
+    "weight in place": _scaled, "weight replaced": _replaced, "weight moved": _moved,
+    "precision": lambda l: _set(l.conv2d, precision="split"), "function": lambda l: _set(l.activation, op=torch.tanh),
+    "threshold of the layer": lambda l: _set(l.activation, threshold=0.05), "threshold": _config(threshold=0.05), "state replaced": _state_replaced,
+    "input threshold": _config(input_threshold=0.3), "tensor cores off": _config(tensor_cores="off"), "own tiles off": _config(own_tiles=False),
+    "quantiser": _config(kfenced_step=0.25), "dilation at the head": _config(head_dilation=2048), "dilation in the tail": _config(tail_dilation=True),
+    "option": _option,
+}
+
+
+@pytest.mark.parametrize("what", CHANGES)
+@pytest.mark.parametrize("given", [False, True], ids=["mask derived", "mask given"])
+def test_a_change_gives_the_prepared_call_up(dev, prepared, what, given):
+    from maskedincrementeval_b200 import fields as fl
+    a, b = _layer(dev), _layer(dev)
+    g = torch.Generator(device=dev).manual_seed(1)
+    x0, deltas = cl(torch.randn(N, C, H, W, generator=g, device=dev)), [_sparse(g, dev) for _ in range(4)]
+    bits = fl.new_bits(N, H, W, dev)
+    with torch.no_grad():
+        for l in (a, b):
+            l.forward_refresh_reservoirs(x0)
+        for i, d in enumerate(deltas):
+            if i == 2:
+                for l in (a, b):
+                    CHANGES[what](l)
+            mask = fl.mask_from_delta(d, 0.0, bits) if given else None
+            del prepared[:]
+            ya, ma = a([d, mask])
+            if i < 3:       # the call after the change may be prepared again, under the new conditions
+                assert (True in prepared) == (i == 1), (i, prepared)
+            _decide_anew(b)
+            yb, mb = b([d, mask])
+            assert torch.equal(ya, yb) and torch.equal(ma.bits, mb.bits), (what, i)
+            assert torch.equal(a.activation.in_res.reservoir, b.activation.in_res.reservoir), (what, i)
+
+
+def test_a_change_of_precision_reaches_the_result(dev):
+    """set_precision after the first call: the next step is the fp32 convolution (2e-5), not the TF32 one (2^-11)."""
+    from maskedincrementeval_b200.incr_modules.mask_incr_modules import set_precision
+    from oracle import restatement as R
+    l = _layer(dev)
+    g = torch.Generator(device=dev).manual_seed(1)
+    with torch.no_grad():
+        l.forward_refresh_reservoirs(cl(torch.randn(N, C, H, W, generator=g, device=dev)))
+        for _ in range(2):
+            l([_sparse(g, dev), None])
+        set_precision(l, "split")
+        res, d = l.activation.in_res.reservoir.cpu().contiguous(), _sparse(g, dev)
+        y, _ = l([d, None])
+    want, _ = R.act_incr(res, R.conv_delta(d.cpu().contiguous(), l.conv2d.weight.detach().cpu(), 1, 1), "relu")
+    assert float((y.cpu() - want).abs().max()) <= 2e-5 * max(float(want.abs().max()), 1.0)
+
+
+INPUTS = {
+    "another buffer": lambda d: (cl(d.clone()), True),
+    "a slice of a wider field": lambda d: (cl(torch.cat([d, d], 1))[:, :C], False),
+    "not channels-last": lambda d: (d.contiguous(), False),
+    "another geometry": lambda d: (cl(d[:, :, :24, :48]), False),
+}
+
+
+@pytest.mark.parametrize("what", INPUTS)
+def test_another_kind_of_input_gives_the_prepared_call_up(dev, prepared, what):
+    a, b = _layer(dev), _layer(dev)
+    g = torch.Generator(device=dev).manual_seed(2)
+    x0 = cl(torch.randn(N, C, H, W, generator=g, device=dev))
+    d, taken = INPUTS[what](_sparse(g, dev))
+    with torch.no_grad():
+        for l in (a, b):
+            l.forward_refresh_reservoirs(x0)
+        for _ in range(2):
+            e = _sparse(g, dev)
+            a([e, None])
+            _decide_anew(b)
+            b([e, None])
+        for l in (a, b):
+            if d.shape != x0.shape:
+                l.forward_refresh_reservoirs(cl(x0[:, :, :24, :48]))
+        del prepared[:]
+        ya, ma = a([d, None])
+        assert (True in prepared) == taken
+        _decide_anew(b)
+        yb, mb = b([d, None])
+        assert torch.equal(ya, yb) and torch.equal(ma.bits, mb.bits)
+        assert torch.equal(a.activation.in_res.reservoir, b.activation.in_res.reservoir)
+
+
+def _bias_replaced(layer):
+    layer.conv2d.bias = torch.nn.Parameter(layer.conv2d.bias.detach() + 1.0)
+
+
+def _bias_in_place(layer):
+    with torch.no_grad():
+        layer.conv2d.bias.add_(1.0)
+
+
+REFRESH_CHANGES = {
+    "weight in place": (_scaled, False), "weight replaced": (_replaced, False), "weight moved": (_moved, False), "bias replaced": (_bias_replaced, False),
+    "bias in place": (_bias_in_place, True),      # the kernel reads it where it is
+    "function": (lambda l: _set(l.activation, op=torch.tanh), False), "state replaced": (_state_replaced, False),
+    "tensor cores off": (_config(tensor_cores="off"), False),
+}
+
+
+@pytest.mark.parametrize("what", REFRESH_CHANGES)
+@pytest.mark.parametrize("with_addend", [False, True])
+def test_a_change_gives_the_prepared_refresh_up(dev, prepared, what, with_addend):
+    from maskedincrementeval_b200 import fields as fl
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    a, b = _layer(dev), _layer(dev)
+    g = torch.Generator(device=dev).manual_seed(3)
+    xs = [cl(torch.randn(N, C, H, W, generator=g, device=dev)) for _ in range(3)]
+    addend = [cl(torch.randn(N, C, H, W, generator=g, device=dev)), fl.full_mask(N, H, W, dev)] if with_addend else None
+    change, taken = REFRESH_CHANGES[what]
+    with torch.no_grad():
+        for i, x in enumerate(xs):
+            if i == 2:
+                for l in (a, b):
+                    change(l)
+            del prepared[:]
+            ya, _ = NATIVE.conv(a.conv2d, NATIVE.lift(x), a.activation, addend=addend)
+            assert (True in prepared) == (i == 1 or (i == 2 and taken)), (i, prepared)
+            _decide_anew(b)
+            yb, _ = NATIVE.conv(b.conv2d, NATIVE.lift(x), b.activation, addend=addend)
+            assert torch.equal(ya, yb) and torch.equal(a.activation.in_res.reservoir, b.activation.in_res.reservoir), (what, i)

@@ -337,14 +337,15 @@ class _PreparedCall:
 class _PreparedRefresh:
     """The same for the dense evaluation of a layer in fp32 precision on the tensor cores (60 us of deciding per layer
     otherwise, more than its kernels take)."""
-    __slots__ = ("activation", "cin_limit", "epoch", "options", "op", "params", "reservoir", "reservoir_ptr", "geometry", "mask_ptr", "addend_ptrs",
+    __slots__ = ("activation", "cin_limit", "epoch", "options", "op", "weight", "bias", "params_key", "reservoir", "reservoir_ptr", "geometry", "mask_ptr", "addend_ptrs",
                  "plan", "args", "fields", "fields_ps", "x_ps", "job", "out")
 
     def __init__(self, conv, activation, cin_limit, plan, d, mask, addend):
         self.activation, self.cin_limit, self.plan = activation, cin_limit, plan
         self.epoch, self.options = config.epoch, nat.option_epoch[0]
         self.op = None if activation is None else activation.op
-        self.params = self.parameters_of(conv)
+        self.weight, self.bias = conv._parameters["weight"], conv._parameters["bias"]
+        self.params_key = self.key_of(self.weight, self.bias)
         self.reservoir = None if activation is None else activation.in_res.reservoir
         self.reservoir_ptr = 0 if activation is None else self.reservoir.data_ptr()
         self.geometry, self.mask_ptr = (d.shape, d.stride(), d.device), mask.bits.data_ptr()
@@ -356,16 +357,16 @@ class _PreparedRefresh:
         self.args = nat.ConvArgs.from_buffer_copy(plan.args)
 
     @staticmethod
-    def parameters_of(conv):
-        w, b = conv._parameters["weight"], conv._parameters["bias"]
-        return (id(w), w._version, w.data_ptr()) + (() if b is None else (id(b), b.data_ptr()))
+    def key_of(w, b):
+        return w._version, w.data_ptr(), 0 if b is None else b.data_ptr()       # the bias is read where it is, in every call
 
     def run(self, conv, x_incr, addend):
         d, m = x_incr[0], x_incr[1]
+        w, b = conv._parameters["weight"], conv._parameters["bias"]
         plan, act = self.plan, self.activation
         if (self.epoch != config.epoch or self.options != nat.option_epoch[0] or type(m) is not TileMask or m.bits.data_ptr() != self.mask_ptr
-                or (d.shape, d.stride(), d.device) != self.geometry or d.dtype is not torch.float32 or self.parameters_of(conv) != self.params
-                or plan.needs_clear or plan.accum_target is not None or plan.tail is not self.job):
+                or (d.shape, d.stride(), d.device) != self.geometry or d.dtype is not torch.float32
+                or w is not self.weight or b is not self.bias or self.key_of(w, b) != self.params_key or plan.needs_clear or plan.accum_target is not None or plan.tail is not self.job):
             return None
         if act is not None:
             r = act.in_res.reservoir
@@ -394,8 +395,10 @@ class nnConvIncr(nn.Conv2d):
         self.kf = KFencedMaskModule(0.3)
         self._k, self._s, self._p = _square(self.kernel_size), _square(self.stride), _square(self.padding)
         self.precision = None   # None: TF32 on the tensor cores; "split": split precision there (see _split_input)
-        self._packed = {}   # cin_limit -> (version, device, buffer, cin_pad, cout_pad)
-        self._packed_exact = {}   # cin_limit -> (version, buffer): the dense pass in fp32 precision on the tensor cores
+        # Packed filters hold the parameter (and batch-norm) they were made from: while they do, no other can stand at its
+        # address, so that identity, version and address together tell whether it is still the one.
+        self._packed = {}   # cin_limit -> ((parameter, batch-norm), version key, buffer, cin_pad, cout_pad, tensor-core copy)
+        self._packed_exact = {}   # cin_limit -> (parameter, version key, buffer): the dense pass in fp32 precision on the tensor cores
         self._plans = {}
         self._prepared = None             # _PreparedCall of the last full incremental call
         self._prepared_refresh = None     # _PreparedRefresh of the last full dense evaluation
@@ -405,10 +408,10 @@ class nnConvIncr(nn.Conv2d):
     # The reference keeps a [Cin,kH,kW,Cout] copy of the filter in this attribute (``:156``).
     @property
     def conv2d_weights(self):
-        v = (self.weight._version, self.weight.device)
-        if self._cw is None or self._cw[0] != v:
-            self._cw = (v, torch.permute(self.weight.detach(), (1, 2, 3, 0)).contiguous())
-        return self._cw[1]
+        v = (self.weight._version, self.weight.device, self.weight.data_ptr())
+        if self._cw is None or self._cw[0] is not self.weight or self._cw[1] != v:
+            self._cw = (self.weight, v, torch.permute(self.weight.detach(), (1, 2, 3, 0)).contiguous())
+        return self._cw[2]
 
     def load_state_dict(self, state_dict: 'OrderedDict[str, torch.Tensor]', strict: bool = True):
         r = nn.Conv2d.load_state_dict(self, state_dict, strict=strict)
@@ -420,9 +423,9 @@ class nnConvIncr(nn.Conv2d):
     def _weights_exact(self, cin: int) -> torch.Tensor:
         ver = (self.weight._version, self.weight.device, self.weight.data_ptr())
         hit = self._packed_exact.get(cin)
-        if hit is None or hit[0] != ver:
-            hit = self._packed_exact[cin] = (ver, fl.pack_conv_weights_exact(self.weight[:, :cin]))
-        return hit[1]
+        if hit is None or hit[0] is not self.weight or hit[1] != ver:
+            hit = self._packed_exact[cin] = (self.weight, ver, fl.pack_conv_weights_exact(self.weight[:, :cin]))
+        return hit[2]
 
     def _split_input(self, cin: int) -> bool:
         """Whether this layer runs on the tensor cores in split precision: input [d, d - tf32(d), d] against the
@@ -448,13 +451,13 @@ class nnConvIncr(nn.Conv2d):
         key = cin_limit or self.in_channels
         ver = (self.weight._version, self.weight.device, self.weight.data_ptr())
         if bn is not None:
-            ver = ver + (id(bn), bn.running_var._version, bn.running_var.data_ptr(), bn.eps,
+            ver = ver + (bn.running_var._version, bn.running_var.data_ptr(), bn.eps,
                          None if bn.weight is None else (bn.weight._version, bn.weight.data_ptr()))
             key = ("bn", id(bn), key)
         if split:
             key = ("split", key)
         hit = self._packed.get(key)
-        if hit is None or hit[0] != ver:
+        if hit is None or hit[0][0] is not self.weight or hit[0][1] is not bn or hit[1] != ver:
             w = self.weight.detach()
             if bn is not None:
                 scale = (bn.weight.detach() if bn.weight is not None else 1.0) / torch.sqrt(bn.running_var + bn.eps)
@@ -479,9 +482,9 @@ class nnConvIncr(nn.Conv2d):
             # the library decides per call whether the tensor-core copy is used; it never is below this depth
             if key_depth * self._k * self._k >= 256 and self.out_channels % 4 == 0:
                 tc = fl.pack_conv_weights_tc(w.float())
-            hit = (ver, buf, cp, op, tc)
+            hit = ((self.weight, bn), ver, buf, cp, op, tc)
             self._packed[key] = hit
-        return hit[1], hit[2], hit[3], hit[4]
+        return hit[2:]
 
     def _plan(self, n, hin, win, device) -> _ConvPlan:
         if self.dilation != (1, 1) or self.groups != 1 or self.padding_mode != "zeros":

@@ -220,3 +220,27 @@ def test_a_change_gives_the_prepared_refresh_up(dev, prepared, what, with_addend
             _decide_anew(b)
             yb, _ = NATIVE.conv(b.conv2d, NATIVE.lift(x), b.activation, addend=addend)
             assert torch.equal(ya, yb) and torch.equal(a.activation.in_res.reservoir, b.activation.in_res.reservoir), (what, i)
+
+
+@pytest.mark.parametrize("refresh", [False, True])
+def test_a_new_parameter_at_the_old_address(dev, refresh):
+    """A parameter that is taken off a layer may be followed by one at the same address with the same version: its values count."""
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    a, b = _layer(dev), _layer(dev)
+    g = torch.Generator(device=dev).manual_seed(4)
+    x0, d = cl(torch.randn(N, C, H, W, generator=g, device=dev)), _sparse(g, dev)
+    w = [torch.randn(C, C, 3, 3, generator=g, device=dev) * 0.06 for _ in range(2)]
+    with torch.no_grad():
+        for v in w:
+            a.conv2d.weight = None
+            a.conv2d.weight = torch.nn.Parameter(v.clone())
+            NATIVE.conv(a.conv2d, NATIVE.lift(x0), a.activation)
+            if not refresh:
+                ya, _ = a([d, None])
+        b.conv2d.weight = torch.nn.Parameter(w[1].clone())
+        NATIVE.conv(b.conv2d, NATIVE.lift(x0), b.activation)
+        if not refresh:
+            yb, _ = b([d, None])
+            assert torch.equal(ya, yb)
+        assert torch.equal(a.activation.in_res.reservoir, b.activation.in_res.reservoir)
+        assert torch.equal(a.conv2d.conv2d_weights, b.conv2d.conv2d_weights)

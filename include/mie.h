@@ -264,7 +264,9 @@ int mie_conv_cluster_size(const mie_conv_args *args /* host */);
 int mie_conv_pack_dims(int cin, int cout, int k, int *cin_pad, int *cout_pad, int64_t *n_floats);
 
 /* Fp32 precision on the tensor cores: hi = v rounded to TF32, lo = v - hi rounded to TF32 (together v to 2^-24), for a dense
- * field of `pixels` pixels, and for a filter as [tap][32-channel chunk][hi rows | lo rows][32]. */
+ * field of `pixels` pixels, and for a filter as [tap][32-channel chunk][hi rows | lo rows][32].  An infinite or NaN value
+ * becomes lo with hi = 0, so that the three products (hi*hi, hi*lo, lo*hi) give what fp32 gives; only where an infinite input
+ * meets an infinite filter entry is the result NaN. */
 int mie_split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, void *stream);
 int mie_conv_pack_dims_exact(int cin, int cout, int k, int64_t *n_floats /* host */);
 int mie_pack_conv_weights_exact(const float *w_oihw, int cout, int cin, int k, float *wpacked, void *stream);

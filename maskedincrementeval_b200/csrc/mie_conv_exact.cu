@@ -491,11 +491,24 @@ int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
   return p.cb == 64 ? launch(conv_exact_kernel<32>, 1) : launch(conv_exact_kernel<16>, 0);
 }
 
-// Round to nearest TF32 (10 mantissa bits); NaN and infinity pass through.
+// Round to nearest TF32 (10 mantissa bits).
 __device__ __forceinline__ float round_tf32(float v) {
   unsigned r;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
   return __uint_as_float(r);
+}
+// v as two TF32 numbers.  A finite v that would round up to infinity is truncated instead.  Infinity and NaN have no low part
+// (inf - inf), and infinity times the low part of the other operand has any sign: they become the low part themselves, which
+// meets nothing but the high part of the other operand, and give what fp32 gives.
+__device__ __forceinline__ void split_two_tf32(float v, float &hi, float &lo) {
+  if (!isfinite(v)) {
+    hi = 0.0f;
+    lo = isnan(v) ? __uint_as_float(0x7FC00000u) : v;     // (a NaN whose payload is in the bits that TF32 drops would read as infinity)
+    return;
+  }
+  hi = round_tf32(v);
+  if (isinf(hi)) hi = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
+  lo = round_tf32(v - hi);
 }
 
 // hi = round(v), lo = round(v - hi): one pass over a dense field, a thread per four channels of a pixel.  HBM bound.
@@ -517,7 +530,7 @@ __global__ void __launch_bounds__(256) split_exact_kernel(const float *__restric
     }
     float h[4], l[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { h[j] = round_tf32(v[j]); l[j] = round_tf32(v[j] - h[j]); }
+    for (int j = 0; j < 4; ++j) split_two_tf32(v[j], h[j], l[j]);
     *reinterpret_cast<float4 *>(hi + px * out_ps + c) = make_float4(h[0], h[1], h[2], h[3]);
     *reinterpret_cast<float4 *>(lo + px * out_ps + c) = make_float4(l[0], l[1], l[2], l[3]);
   }
@@ -535,8 +548,9 @@ __global__ void pack_weights_exact_kernel(const float *__restrict__ w, int cout,
     const int ci = (int)(rest % nch) * 32 + cl, tap = (int)(rest / nch), co = row < cout_pad ? row : row - cout_pad;
     float v = 0.0f;
     if (co < cout && ci < cin) v = w[ihwo ? ((int64_t)ci * k * k + tap) * cout + co : ((int64_t)co * cin + ci) * k * k + tap];
-    const float h = round_tf32(v);
-    wp[i] = row < cout_pad ? h : round_tf32(v - h);
+    float h, l;
+    split_two_tf32(v, h, l);
+    wp[i] = row < cout_pad ? h : l;
   }
 }
 

@@ -63,6 +63,47 @@ def test_dense_pass_against_float64(dev, case):
     assert err["auto"] <= max(1.2 * err["off"], 6e-7), err
 
 
+# infinities, NaN and values that round up to infinity in TF32, in the input or in the filter: what the fp32 kernel gives
+@pytest.mark.parametrize("where", ["input", "filter"])
+@pytest.mark.parametrize("case", [(32, 64, 3, 1, 1, 41, 50), (5, 32, 5, 2, 2, 33, 40)])
+def test_dense_pass_on_non_finite_values(dev, case, where):
+    from maskedincrementeval_b200 import fields as fl
+    from maskedincrementeval_b200.ext.pointops import pointops_functional as pf
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    cin, cout, k, s, n, h, w = case
+    torch.manual_seed(8)
+    layer = ConvLayerIncr(cin, cout, k, s, k // 2, activation="relu").to(dev).eval()
+    c = layer.conv2d
+    x = cl(torch.randn(n, cin, h, w, device=dev) * 0.2)      # (below 1: no product with the largest number lies at the edge of overflow)
+    odd = [float("inf"), -float("inf"), float("nan"), torch.finfo(torch.float32).max, -torch.finfo(torch.float32).max]
+    with torch.no_grad():
+        for i, v in enumerate(odd):
+            if where == "input":
+                x[i % n, (3 * i) % cin, 6 * i + 3, 7 * i + 2] = v
+            else:
+                c.weight[4 * i, (3 * i) % cin, i % k, 0] = v
+        x[0, 0, h - 1, w - 1] = torch.finfo(torch.float32).max * 0.9999      # and a finite one that stays finite, next to zeros
+        states = {}
+        old = fl.config.tensor_cores
+        try:
+            for mode in ("auto", "off"):
+                fl.config.tensor_cores = mode
+                NATIVE.conv(c, NATIVE.lift(x), layer.activation)
+                states[mode] = layer.activation.in_res.reservoir.clone()
+        finally:
+            fl.config.tensor_cores = old
+        ext, _ = pf.functional_conv_module(x, c.conv2d_weights, mask=torch.ones_like(x, dtype=torch.bool), stride=(s, s), padding=(k // 2, k // 2))
+    for got, want in ((states["auto"], states["off"]), (ext, states["off"] - c.bias.detach().view(1, -1, 1, 1))):
+        assert not bool(want.isfinite().all())
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+        # relative to the products that a value is the sum of: fp32 sums of cin * k * k terms
+        fine = want.isfinite() & (want.abs() < 1e30)
+        assert float((got[fine] - want[fine]).abs().max()) <= 1e-5
+        big = want.isfinite() & ~fine
+        assert float(((got[big] - want[big]) / want[big]).abs().max()) <= 1e-5 if bool(big.any()) else True
+
+
 # stride 2 on fields one pixel wide or high, which have no odd columns or rows
 @pytest.mark.parametrize("h,w", [(17, 1), (1, 22), (1, 1), (2, 9)])
 @pytest.mark.parametrize("k", [3, 5])

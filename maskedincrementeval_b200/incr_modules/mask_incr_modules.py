@@ -272,12 +272,12 @@ class _PreparedCall:
     40 us a small layer's step lasted.  Built at the end of a full call (``nnConvIncr.forward_fused``) and valid while
     nothing it was decided by has changed: the library's configuration and options, the filter and the layer's precision,
     the activation's function, state buffers and threshold, the input's geometry and the address of its tile words."""
-    __slots__ = ("activation", "cin_limit", "epoch", "options", "precision", "op", "weight", "weight_key", "reservoir", "reservoir_ptr", "emitted",
+    __slots__ = ("activation", "epoch", "options", "precision", "op", "weight", "weight_key", "reservoir", "reservoir_ptr", "emitted",
                  "threshold", "shape", "stride", "device", "mask_bits", "mask_ptr", "geometry", "plan", "args", "args_ref", "dilate", "tc_option",
                  "out", "input_threshold", "keep")
 
-    def __init__(self, conv, activation, cin_limit, plan, d, mask, derived, dilate, thresholded):
-        self.activation, self.cin_limit, self.plan = activation, cin_limit, plan     # (not the convolution: that would be a cycle)
+    def __init__(self, conv, activation, plan, d, mask, derived, dilate, thresholded):
+        self.activation, self.plan = activation, plan     # (not the convolution: that would be a cycle)
         self.epoch, self.options = config.epoch, nat.option_epoch[0]
         self.precision, self.op = conv.precision, None if activation is None else activation.op
         self.weight = conv.weight
@@ -337,11 +337,11 @@ class _PreparedCall:
 class _PreparedRefresh:
     """The same for the dense evaluation of a layer in fp32 precision on the tensor cores (60 us of deciding per layer
     otherwise, more than its kernels take)."""
-    __slots__ = ("activation", "cin_limit", "epoch", "options", "op", "weight", "bias", "params_key", "reservoir", "reservoir_ptr", "geometry", "mask_ptr", "addend_ptrs",
+    __slots__ = ("activation", "epoch", "options", "op", "weight", "bias", "params_key", "reservoir", "reservoir_ptr", "geometry", "mask_ptr", "addend_ptrs",
                  "plan", "args", "fields", "fields_ps", "x_ps", "job", "out")
 
-    def __init__(self, conv, activation, cin_limit, plan, d, mask, addend):
-        self.activation, self.cin_limit, self.plan = activation, cin_limit, plan
+    def __init__(self, conv, activation, plan, d, mask, addend):
+        self.activation, self.plan = activation, plan
         self.epoch, self.options = config.epoch, nat.option_epoch[0]
         self.op = None if activation is None else activation.op
         self.weight, self.bias = conv._parameters["weight"], conv._parameters["bias"]
@@ -400,8 +400,9 @@ class nnConvIncr(nn.Conv2d):
         self._packed = {}   # cin_limit -> ((parameter, batch-norm), version key, buffer, cin_pad, cout_pad, tensor-core copy)
         self._packed_exact = {}   # cin_limit -> (parameter, version key, buffer): the dense pass in fp32 precision on the tensor cores
         self._plans = {}
-        self._prepared = None             # _PreparedCall of the last full incremental call
-        self._prepared_refresh = None     # _PreparedRefresh of the last full dense evaluation
+        # (input shape, cin_limit) -> _PreparedCall / _PreparedRefresh of the last full call of that kind; as many as there are plans
+        self._prepared = {}
+        self._prepared_refresh = {}
         self._cw = None
         self._scratch = Scratch()
 
@@ -510,21 +511,23 @@ class nnConvIncr(nn.Conv2d):
         tensor, the bias is added, the activation's reservoir is set to conv + bias (+ addend) and the output is
         f(reservoir) -- in full fp32, whatever ``config.tensor_cores`` says."""
         plain = addend is None and second is None and bn is None and not refresh
-        fast = self._prepared
+        kind = (x_incr[0].shape, cin_limit)
         if plain:
-            if fast is not None and fast.activation is activation and fast.cin_limit == cin_limit:
-                out = fast.run(self, x_incr)
+            fast = self._prepared.get(kind)
+            if fast is not None:
+                out = fast.run(self, x_incr) if fast.activation is activation else None
                 if out is not None:
                     return out
-            self._prepared = None
-        fast = self._prepared_refresh
-        if refresh:
-            if (fast is not None and second is None and bn is None and fast.activation is activation and fast.cin_limit == cin_limit
-                    and (addend is None) == (fast.addend_ptrs is None)):
-                out = fast.run(self, x_incr, addend)
+                del self._prepared[kind]
+        elif refresh:
+            fast = self._prepared_refresh.get(kind)
+            if fast is not None:
+                out = None
+                if second is None and bn is None and fast.activation is activation and (addend is None) == (fast.addend_ptrs is None):
+                    out = fast.run(self, x_incr, addend)
                 if out is not None:
                     return out
-            self._prepared_refresh = None
+                del self._prepared_refresh[kind]
         sc = self._scratch
         if refresh and bn is not None:
             raise NotImplementedError("dense evaluation with a folded batch-norm")
@@ -643,10 +646,10 @@ class nnConvIncr(nn.Conv2d):
         nat.check(nat.lib.mie_conv_tiles(C.byref(a), st), "conv_tiles")
         if (plain and not split and not config.kfenced_step and not config.tail_dilation and not a.accum and (x_incr[1] is None or x_incr[1] is m)
                 and d is x_incr[0] and (activation is None or type(activation).thr is nnReservedActivation.thr) and a.in_ % 16 == 0):
-            self._prepared = _PreparedCall(self, activation, cin_limit, plan, d, m, x_incr[1] is None, not a.head, a.thr > 0.0 or bool(a.emitted))
+            self._prepared[kind] = _PreparedCall(self, activation, plan, d, m, x_incr[1] is None, not a.head, a.thr > 0.0 or bool(a.emitted))
         if (refresh and a.wpacked_exact and not a.head and not config.tail_dilation and second is None and x_incr[1] is m and x_incr[0].data_ptr() == d.data_ptr()
                 and (activation is None or activation.emitted is None) and (addend is None or type(addend[1]) is TileMask)):
-            self._prepared_refresh = _PreparedRefresh(self, activation, cin_limit, plan, d, m, addend)
+            self._prepared_refresh[kind] = _PreparedRefresh(self, activation, plan, d, m, addend)
         if refresh and activation is not None and activation.emitted is not None:
             if activation.emitted.shape == plan.out.shape and activation.thr() > 0.0 and config.carry:
                 activation.emitted.copy_(plan.out)      # what has been sent so far = f(reservoir)

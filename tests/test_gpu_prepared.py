@@ -58,7 +58,8 @@ def _sparse(g, dev, std=0.5):
 
 
 def _decide_anew(layer):
-    layer.conv2d._prepared = layer.conv2d._prepared_refresh = None
+    layer.conv2d._prepared.clear()
+    layer.conv2d._prepared_refresh.clear()
 
 
 def _set(obj, **kw):
@@ -244,3 +245,19 @@ def test_a_new_parameter_at_the_old_address(dev, refresh):
             assert torch.equal(ya, yb)
         assert torch.equal(a.activation.in_res.reservoir, b.activation.in_res.reservoir)
         assert torch.equal(a.conv2d.conv2d_weights, b.conv2d.conv2d_weights)
+
+
+def test_geometries_in_turn_keep_their_prepared_calls(dev, prepared):
+    """A convolution that is called at two geometries in turn decides each of them once."""
+    a, b = _layer(dev).conv2d, _layer(dev).conv2d
+    g = torch.Generator(device=dev).manual_seed(5)
+    with torch.no_grad():
+        for i in range(3):
+            for h, w in ((H, W), (24, 48)):
+                d = cl(_sparse(g, dev)[:, :, :h, :w])
+                del prepared[:]
+                ya, ma = a([d, None])
+                assert prepared == ([True] if i else [])
+                b._prepared.clear()
+                yb, mb = b([d, None])
+                assert torch.equal(ya, yb) and torch.equal(ma.bits, mb.bits)

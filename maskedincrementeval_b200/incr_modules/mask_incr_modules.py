@@ -271,12 +271,13 @@ class _PreparedCall:
     kind of input needs is a few identity checks and one call of the library, where deciding it anew took most of the
     40 us a small layer's step lasted.  Built at the end of a full call (``nnConvIncr.forward_fused``) and valid while
     nothing it was decided by has changed: the library's configuration and options, the filter and the layer's precision,
-    the activation's function, state buffers and threshold, the input's geometry and the address of its tile words."""
+    the activation's function, state buffers and threshold, the input's geometry and the address of its tile words.  It holds
+    every buffer that its argument block points to, but for the input."""
     __slots__ = ("activation", "epoch", "options", "precision", "op", "weight", "weight_key", "reservoir", "reservoir_ptr", "emitted",
                  "threshold", "shape", "stride", "device", "mask_bits", "mask_ptr", "geometry", "plan", "args", "args_ref", "dilate", "tc_option",
-                 "out", "input_threshold", "keep")
+                 "out", "input_threshold", "job", "packed")
 
-    def __init__(self, conv, activation, plan, d, mask, derived, dilate, thresholded):
+    def __init__(self, conv, activation, plan, d, mask, derived, dilate, thresholded, packed):
         self.activation, self.plan = activation, plan     # (not the convolution: that would be a cycle)
         self.epoch, self.options = config.epoch, nat.option_epoch[0]
         self.precision, self.op = conv.precision, None if activation is None else activation.op
@@ -294,7 +295,7 @@ class _PreparedCall:
         self.args = nat.ConvArgs.from_buffer_copy(plan.args)     # its own: dense passes fill the plan's
         self.args_ref = C.byref(self.args)
         self.dilate = C.addressof(plan.tail.c) if dilate else None
-        self.keep = plan.tail
+        self.job, self.packed = plan.tail, packed
         self.tc_option = (1 if config.tc_thresholded else 0) if thresholded else None
         self.input_threshold = float(config.input_threshold)
         self.out = (plan.out, plan.mask)
@@ -306,7 +307,7 @@ class _PreparedCall:
         plan = self.plan
         if (self.epoch != config.epoch or self.options != nat.option_epoch[0] or d.shape != self.shape or d.stride() != self.stride
                 or d.device != self.device or d.dtype is not torch.float32 or w is not self.weight or conv.precision != self.precision
-                or (w._version, w.data_ptr()) != self.weight_key or plan.needs_clear or plan.accum_target is not None or plan.tail is not self.keep):
+                or (w._version, w.data_ptr()) != self.weight_key or plan.needs_clear or plan.accum_target is not None or plan.tail is not self.job):
             return None
         act = self.activation
         if act is not None:
@@ -337,10 +338,10 @@ class _PreparedCall:
 class _PreparedRefresh:
     """The same for the dense evaluation of a layer in fp32 precision on the tensor cores (60 us of deciding per layer
     otherwise, more than its kernels take)."""
-    __slots__ = ("activation", "epoch", "options", "op", "weight", "bias", "params_key", "reservoir", "reservoir_ptr", "geometry", "mask_ptr", "addend_ptrs",
-                 "plan", "args", "fields", "fields_ps", "x_ps", "job", "out")
+    __slots__ = ("activation", "epoch", "options", "op", "weight", "bias", "params_key", "reservoir", "reservoir_ptr", "geometry", "mask_key", "addend_key",
+                 "plan", "args", "fields", "fields_ps", "x_ps", "job", "out", "packed")
 
-    def __init__(self, conv, activation, plan, d, mask, addend):
+    def __init__(self, conv, activation, plan, d, mask, addend, packed):
         self.activation, self.plan = activation, plan
         self.epoch, self.options = config.epoch, nat.option_epoch[0]
         self.op = None if activation is None else activation.op
@@ -348,23 +349,31 @@ class _PreparedRefresh:
         self.params_key = self.key_of(self.weight, self.bias)
         self.reservoir = None if activation is None else activation.in_res.reservoir
         self.reservoir_ptr = 0 if activation is None else self.reservoir.data_ptr()
-        self.geometry, self.mask_ptr = (d.shape, d.stride(), d.device), mask.bits.data_ptr()
-        self.addend_ptrs = None if addend is None else (addend[0].data_ptr(), addend[1].bits.data_ptr())
+        self.geometry, self.mask_key = (d.shape, d.stride(), d.device), self.key_of_mask(mask)
+        self.addend_key = None if addend is None else self.key_of_addend(addend)
         n, c, h, w = d.shape
         cp = (c + 3) // 4 * 4
         self.fields, self.fields_ps, self.x_ps = (2, n, h, w, cp), n * h * w * cp * 4, fl.pixel_stride(d)
-        self.job, self.out = plan.tail, (plan.out, plan.mask)
+        self.job, self.out, self.packed = plan.tail, (plan.out, plan.mask), packed
         self.args = nat.ConvArgs.from_buffer_copy(plan.args)
 
     @staticmethod
     def key_of(w, b):
         return w._version, w.data_ptr(), 0 if b is None else b.data_ptr()       # the bias is read where it is, in every call
 
+    @staticmethod
+    def key_of_mask(m):
+        return m.bits.data_ptr(), m.n, m.h, m.w
+
+    @classmethod
+    def key_of_addend(cls, addend):
+        return addend[0].data_ptr(), addend[0].shape, addend[0].stride(), addend[0].dtype, cls.key_of_mask(addend[1])
+
     def run(self, conv, x_incr, addend):
         d, m = x_incr[0], x_incr[1]
         w, b = conv._parameters["weight"], conv._parameters["bias"]
         plan, act = self.plan, self.activation
-        if (self.epoch != config.epoch or self.options != nat.option_epoch[0] or type(m) is not TileMask or m.bits.data_ptr() != self.mask_ptr
+        if (self.epoch != config.epoch or self.options != nat.option_epoch[0] or type(m) is not TileMask or self.key_of_mask(m) != self.mask_key
                 or (d.shape, d.stride(), d.device) != self.geometry or d.dtype is not torch.float32
                 or w is not self.weight or b is not self.bias or self.key_of(w, b) != self.params_key or plan.needs_clear or plan.accum_target is not None or plan.tail is not self.job):
             return None
@@ -372,7 +381,7 @@ class _PreparedRefresh:
             r = act.in_res.reservoir
             if r is not self.reservoir or r.data_ptr() != self.reservoir_ptr or act.emitted is not None or act.op is not self.op:
                 return None
-        if addend is not None and (type(addend[1]) is not TileMask or (addend[0].data_ptr(), addend[1].bits.data_ptr()) != self.addend_ptrs):
+        if addend is not None and (type(addend[1]) is not TileMask or self.key_of_addend(addend) != self.addend_key):
             return None
         both = torch.empty(self.fields, dtype=torch.float32, device=d.device)     # released after the launch
         a = self.args
@@ -523,7 +532,7 @@ class nnConvIncr(nn.Conv2d):
             fast = self._prepared_refresh.get(kind)
             if fast is not None:
                 out = None
-                if second is None and bn is None and fast.activation is activation and (addend is None) == (fast.addend_ptrs is None):
+                if second is None and bn is None and fast.activation is activation and (addend is None) == (fast.addend_key is None):
                     out = fast.run(self, x_incr, addend)
                 if out is not None:
                     return out
@@ -646,10 +655,11 @@ class nnConvIncr(nn.Conv2d):
         nat.check(nat.lib.mie_conv_tiles(C.byref(a), st), "conv_tiles")
         if (plain and not split and not config.kfenced_step and not config.tail_dilation and not a.accum and (x_incr[1] is None or x_incr[1] is m)
                 and d is x_incr[0] and (activation is None or type(activation).thr is nnReservedActivation.thr) and a.in_ % 16 == 0):
-            self._prepared[kind] = _PreparedCall(self, activation, plan, d, m, x_incr[1] is None, not a.head, a.thr > 0.0 or bool(a.emitted))
+            self._prepared[kind] = _PreparedCall(self, activation, plan, d, m, x_incr[1] is None, not a.head, a.thr > 0.0 or bool(a.emitted),
+                                                 (wbuf, wtc))
         if (refresh and a.wpacked_exact and not a.head and not config.tail_dilation and second is None and x_incr[1] is m and x_incr[0].data_ptr() == d.data_ptr()
                 and (activation is None or activation.emitted is None) and (addend is None or type(addend[1]) is TileMask)):
-            self._prepared_refresh[kind] = _PreparedRefresh(self, activation, plan, d, m, addend)
+            self._prepared_refresh[kind] = _PreparedRefresh(self, activation, plan, d, m, addend, (wbuf, wx))
         if refresh and activation is not None and activation.emitted is not None:
             if activation.emitted.shape == plan.out.shape and activation.thr() > 0.0 and config.carry:
                 activation.emitted.copy_(plan.out)      # what has been sent so far = f(reservoir)

@@ -261,3 +261,30 @@ def test_geometries_in_turn_keep_their_prepared_calls(dev, prepared):
                 b._prepared.clear()
                 yb, mb = b([d, None])
                 assert torch.equal(ya, yb) and torch.equal(ma.bits, mb.bits)
+
+
+@pytest.mark.parametrize("refresh", [False, True])
+def test_prepared_calls_hold_the_packed_filter(dev, prepared, refresh):
+    """load_state_dict drops the packed filters; where it leaves the parameter as it was, the prepared call still holds its own."""
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    a, b = _layer(dev), _layer(dev)
+    g = torch.Generator(device=dev).manual_seed(6)
+    x0 = cl(torch.randn(N, C, H, W, generator=g, device=dev))
+    with torch.no_grad():
+        for i in range(3):
+            d = _sparse(g, dev)
+            if i == 2:
+                a.conv2d.load_state_dict({}, strict=False)
+                taken = [torch.full((s,), float("nan"), device=dev) for s in (9 * 32 * 32, 2 * 9 * 32 * 32, 9 * 32 * 32) for _ in range(8)]
+            for l in (a, b):
+                del prepared[:]
+                if refresh:
+                    NATIVE.conv(l.conv2d, NATIVE.lift(x0), l.activation)
+                else:
+                    if i == 0:
+                        l.forward_refresh_reservoirs(x0)
+                    l([d, None])
+                assert prepared == ([True] if i else [])
+            assert torch.equal(a.activation.in_res.reservoir, b.activation.in_res.reservoir)
+            assert bool(a.activation.in_res.reservoir.isfinite().all())
+    del taken

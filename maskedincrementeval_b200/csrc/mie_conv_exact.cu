@@ -30,6 +30,7 @@ struct ExactParams {
   int act; float *res; int64_t res_ps; const float *addend; int64_t addend_ps; const float *bias;
   int cb, stages, halos, tps, wp;   // tps: taps per ring stage
   unsigned spin_limit;
+  int withhold_loads;      // self-test: the producers issue nothing, so the first wait runs out (MIE_OPT_TC_WITHHOLD_LOADS)
   mie_tail_job tail;
   PairTaps t;
 };
@@ -188,94 +189,25 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
   const unsigned b_base = smem_u32(smem), a_base = b_base + (((unsigned)p.stages * stage_bytes + 1023u) & ~1023u);
   const int nv = p.t.nviews;
 
+  // units of a chunk: the high parts of the views, then the low parts
+  const PairWork work = {bid, nblk, n_items, n_cblk, p.n_chunks, 2 * nv, crank, p.spin_limit, p.withhold_loads};
   if (warp == 0) {
-    // =========================== halo producer: hi views, then lo views of a chunk ===========================
-    const unsigned leader = elect_one();
-    unsigned s = 0, parity = 0;
-    bool first_lap = true, ok = true;
-    for (int item = bid; item < n_items && ok; item += nblk) {
-      const int e = 4 * (item / n_cblk) + 2 * (int)crank;
-      int tx8[2], ty8[2], tn[2];
-      bool have[2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        int t = __shfl_sync(0xffffffffu, e + i < n_active ? p.list[e + i] : -1, 0);
-        have[i] = e + i < n_active;
-        if (have[i] && (t < 0 || t >= ntiles_total)) {      // reported, skipped by the epilogue; tile 0 stands in for it here
-          if (leader) atomicOr(&p.counts[3], MIE_ERR_BAD_TILE);
-          t = 0;
-        }
-        tx8[i] = have[i] ? (t % TWo) * 8 : 0; ty8[i] = have[i] ? ((t / TWo) % THo) * 8 : 0; tn[i] = have[i] ? t / (TWo * THo) : 0;
-      }
-      const unsigned tx_bytes = (unsigned)min(4, n_active - 4 * (item / n_cblk)) * (unsigned)p.wp * row_bytes;
-      for (int chunk = 0; chunk < p.n_chunks && ok; ++chunk)
-        for (int u = 0; u < 2 * nv; ++u) {
-          if (!first_lap) ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[s], parity, &s_abort, p.spin_limit));
-          if (!ok) break;
-          const int v = u < nv ? u : u - nv;
-          const unsigned bar = mapa_shared(smem_u32(&a_full[s]), 0);
-          if (leader) {
-            if (crank == 0u)
-              asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&a_full[s])), "r"(tx_bytes) : "memory");
-            const CUtensorMap *map = u < nv ? &maps.hi[v] : &maps.lo[v];
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-              if (have[i]) {
-                unsigned dst = a_base + s * halo_bytes + (unsigned)i * row_bytes;
-                for (int r = 0; r < p.wp; ++r, dst += 2u * row_bytes) tma_load_4d_pair(dst, map, bar, chunk * 32, tx8[i] + p.t.x0[v], ty8[i] + p.t.y0[v] + r, tn[i]);
-              }
-          }
-          __syncwarp();
-          if (++s == (unsigned)p.halos) { s = 0; if (!first_lap) parity ^= 1u; first_lap = false; }
-        }
-    }
-    for (int i = 0; i < p.halos && ok; ++i) {       // nothing may signal this block's barriers after it has left
-      if (first_lap && (unsigned)i >= s) break;
-      if (first_lap) ok = mbar_wait(&a_empty[i], 0u, &s_abort, p.spin_limit);
-      else {
-        ok = mbar_wait(&a_empty[s], parity, &s_abort, p.spin_limit);
-        if (++s == (unsigned)p.halos) { s = 0; parity ^= 1u; }
-      }
-    }
+    // =========================== halo producer ===========================
+    const PairRing ring = {a_full, a_empty, a_base, halo_bytes, (unsigned)p.halos};
+    pair_produce_halos(work, ring, p.t, p.wp, row_bytes, p.list, n_active, ntiles_total, TWo, THo, p.counts, &s_abort, [&](int u, int &v) {
+      v = u < nv ? u : u - nv;
+      return u < nv ? &maps.hi[v] : &maps.lo[v];
+    });
   } else if (warp == 1) {
-    // =========================== filter producer ===========================
-    const unsigned leader = elect_one();
-    unsigned s = 0, parity = 0, stage_addr = b_base;
-    bool first_lap = true, ok = true;
-    for (int item = bid; item < n_items && ok; item += nblk) {
-      const int row = (item % n_cblk) * CB + (int)crank * HW;
-      for (int chunk = 0; chunk < p.n_chunks && ok; ++chunk)
-        for (int u = 0; u < 2 * nv && ok; ++u) {
-          const int v = u < nv ? u : u - nv;
-          for (int i = p.t.first[v]; i < p.t.first[v + 1]; i += p.tps) {
-            if (!first_lap) ok = __all_sync(0xffffffffu, mbar_wait(&b_empty[s], parity, &s_abort, p.spin_limit));
-            if (!ok) break;
-            const int nt = min(p.tps, p.t.first[v + 1] - i);
-            if (leader) {
-              if (crank == 0u)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&b_full[s])),
-                             "r"((unsigned)nt * 2u * (u < nv ? tap_bytes : half_bytes)) : "memory");
-              const unsigned bar = mapa_shared(smem_u32(&b_full[s]), 0);
-              for (int k = 0; k < nt; ++k) {
-                const unsigned dst = stage_addr + (unsigned)k * tap_bytes;
-                tma_load_4d_pair(dst, &maps.w, bar, 0, row, chunk, (int)p.t.tap[i + k]);
-                if (u < nv) tma_load_4d_pair(dst + half_bytes, &maps.w, bar, 0, p.cout_pad + row, chunk, (int)p.t.tap[i + k]);
-              }
-            }
-            __syncwarp();
-            stage_addr += stage_bytes;
-            if (++s == (unsigned)p.stages) { s = 0; stage_addr = b_base; if (!first_lap) parity ^= 1u; first_lap = false; }
-          }
-        }
-    }
-    for (int i = 0; i < p.stages && ok; ++i) {
-      if (first_lap && (unsigned)i >= s) break;
-      if (first_lap) ok = mbar_wait(&b_empty[i], 0u, &s_abort, p.spin_limit);
-      else {
-        ok = mbar_wait(&b_empty[s], parity, &s_abort, p.spin_limit);
-        if (++s == (unsigned)p.stages) { s = 0; parity ^= 1u; }
-      }
-    }
+    // =========================== filter producer: hi and lo rows beside the high part of the input, hi rows beside the low part ===========================
+    const PairRing ring = {b_full, b_empty, b_base, stage_bytes, (unsigned)p.stages};
+    pair_produce_filter(work, ring, p.t, p.tps, tap_bytes, &s_abort, [&](int u) { return u < nv ? u : u - nv; },
+                        [&](int u) { return 2u * (u < nv ? tap_bytes : half_bytes); },
+                        [&](int u, int tap, unsigned dst, unsigned bar, int cb, int chunk) {
+                          const int row = cb * CB + (int)crank * HW;
+                          tma_load_4d_pair(dst, &maps.w, bar, 0, row, chunk, tap);
+                          if (u < nv) tma_load_4d_pair(dst + half_bytes, &maps.w, bar, 0, p.cout_pad + row, chunk, tap);
+                        });
   } else if (warp == 2) {
     // =========================== MMA issuer (first block of the pair) ===========================
     if (crank == 0u) {
@@ -437,6 +369,7 @@ int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
   ExactParams p;
   memset(&p, 0, sizeof(p));
   p.spin_limit = g_opt_spin_limit;
+  p.withhold_loads = g_opt_withhold_loads;
   p.cin = a->cin; p.cout = a->cout; p.cout_pad = a->cout_pad; p.n_chunks = divup(a->cin, 32);
   p.n = a->n; p.hout = a->hout; p.wout = a->wout;
   p.list = a->list; p.counts = a->counts; p.max_tiles = a->max_tiles;

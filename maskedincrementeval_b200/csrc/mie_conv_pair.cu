@@ -263,90 +263,19 @@ conv_pair_kernel(const PairParams P, const __grid_constant__ PairMaps maps) {
   const unsigned a_base = b_base + (((unsigned)p.stages * stage_bytes + 1023u) & ~1023u);
   unsigned char *epi = smem + (a_base - b_base) + (size_t)P.halos * halo_bytes;   // slabs of the epilogue sets
 
+  const PairWork work = {item0, item_step, n_items, n_cblk, n_chunks, P.t.nviews, crank, p.spin_limit, p.withhold_loads};
   if (warp == 0) {
     // =========================== halo producer ===========================
-    // One copy per halo row and tile, issued by one elected lane of the converged warp: with a row per lane the copies
-    // are issued one by one all the same, at several times the cost (no uniform registers), and paced every layer.
-    const unsigned leader = elect_one();
-    unsigned s = 0, parity = 0;
-    bool first_lap = true, ok = true;
-    for (int item = item0; item < n_items && ok && !p.withhold_loads; item += item_step) {
-      const int e = 4 * (item / n_cblk) + 2 * (int)crank;
-      int tx8[2], ty8[2], tn[2];
-      bool have[2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        int t = __shfl_sync(0xffffffffu, e + i < n_active ? lst[e + i] : -1, 0);
-        have[i] = e + i < n_active;
-        // an entry outside the field is reported and skipped by the epilogue; here tile 0 stands in for it
-        if (have[i] && (t < 0 || t >= ntiles_total)) {
-          if (leader) atomicOr(&p.counts[3], MIE_ERR_BAD_TILE);
-          t = 0;
-        }
-        tx8[i] = have[i] ? (t % TWo) * 8 : 0; ty8[i] = have[i] ? ((t / TWo) % THo) * 8 : 0; tn[i] = have[i] ? t / (TWo * THo) : 0;
-      }
-      const unsigned tx_bytes = (unsigned)min(4, n_active - 4 * (item / n_cblk)) * (unsigned)P.hp * row_bytes;   // both blocks
-      for (int chunk = 0; chunk < n_chunks && ok; ++chunk)
-        for (int v = 0; v < P.t.nviews; ++v) {
-          if (!first_lap) ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[s], parity, &s_abort, p.spin_limit));
-          if (!ok) break;
-          const unsigned bar = mapa_shared(smem_u32(&a_full[s]), 0);
-          if (leader) {
-            if (crank == 0u)
-              asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&a_full[s])), "r"(tx_bytes) : "memory");
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-              if (have[i]) {
-                unsigned dst = a_base + s * halo_bytes + (unsigned)i * row_bytes;
-                const int x = tx8[i] + P.t.x0[v], y = ty8[i] + P.t.y0[v];
-                for (int r = 0; r < P.hp; ++r, dst += 2u * row_bytes) tma_load_4d_pair(dst, &maps.in[v], bar, chunk * 32, x, y + r, tn[i]);
-              }
-          }
-          __syncwarp();
-          if (++s == (unsigned)P.halos) { s = 0; if (!first_lap) parity ^= 1u; first_lap = false; }
-        }
-    }
-    // wait until the last uses of the buffers are over: nothing may signal this block's barriers after it has left
-    for (int i = 0; i < P.halos && ok && !s_abort && !p.withhold_loads; ++i) {
-      if (first_lap && (unsigned)i >= s) break;
-      if (first_lap) ok = mbar_wait(&a_empty[i], 0u, &s_abort, p.spin_limit);
-      else {
-        ok = mbar_wait(&a_empty[s], parity, &s_abort, p.spin_limit);
-        if (++s == (unsigned)P.halos) { s = 0; parity ^= 1u; }
-      }
-    }
+    const PairRing ring = {a_full, a_empty, a_base, halo_bytes, (unsigned)P.halos};
+    pair_produce_halos(work, ring, P.t, P.hp, row_bytes, lst, n_active, ntiles_total, TWo, THo, p.counts, &s_abort,
+                       [&](int u, int &v) { v = u; return &maps.in[u]; });
   } else if (warp == 1) {
     // =========================== filter producer ===========================
-    const unsigned leader = elect_one();
-    unsigned s = 0, parity = 0, stage_addr = b_base;
-    bool first_lap = true, ok = true;
-    for (int item = item0; item < n_items && ok && !s_abort && !p.withhold_loads; item += item_step) {
-      const int row = (item % n_cblk) * NB + (int)crank * (NB >> 1);
-      for (int chunk = 0; chunk < n_chunks && ok; ++chunk)
-        for (int v = 0; v < P.t.nviews && ok; ++v)
-          for (int i = P.t.first[v]; i < P.t.first[v + 1]; i += P.tps) {
-            if (!first_lap && !mbar_wait(&b_empty[s], parity, &s_abort, p.spin_limit)) { ok = false; break; }
-            const int nt = min(P.tps, P.t.first[v + 1] - i);
-            if (leader) {
-              if (crank == 0u)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&b_full[s])), "r"((unsigned)nt * 2u * tap_bytes) : "memory");
-              const unsigned bar = mapa_shared(smem_u32(&b_full[s]), 0);
-              for (int k = 0; k < nt; ++k)
-                tma_load_4d_pair(stage_addr + (unsigned)k * tap_bytes, &maps.w, bar, 0, row, chunk, (int)P.t.tap[i + k]);
-            }
-            __syncwarp();
-            stage_addr += stage_bytes;
-            if (++s == (unsigned)p.stages) { s = 0; stage_addr = b_base; if (!first_lap) parity ^= 1u; first_lap = false; }
-          }
-    }
-    for (int i = 0; i < p.stages && ok && !s_abort && !p.withhold_loads; ++i) {
-      if (first_lap && (unsigned)i >= s) break;
-      if (first_lap) ok = mbar_wait(&b_empty[i], 0u, &s_abort, p.spin_limit);
-      else {
-        ok = mbar_wait(&b_empty[s], parity, &s_abort, p.spin_limit);
-        if (++s == (unsigned)p.stages) { s = 0; parity ^= 1u; }
-      }
-    }
+    const PairRing ring = {b_full, b_empty, b_base, stage_bytes, (unsigned)p.stages};
+    pair_produce_filter(work, ring, P.t, P.tps, tap_bytes, &s_abort, [](int u) { return u; }, [&](int) { return 2u * tap_bytes; },
+                        [&](int, int tap, unsigned dst, unsigned bar, int cb, int chunk) {
+                          tma_load_4d_pair(dst, &maps.w, bar, 0, cb * NB + (int)crank * (NB >> 1), chunk, tap);
+                        });
   } else if (warp == 2) {
     if (crank == 0u) {
       PairIssue a;

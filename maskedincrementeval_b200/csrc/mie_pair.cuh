@@ -97,6 +97,114 @@ __device__ __forceinline__ void tma_store_slab(unsigned smem_addr, const CUtenso
                ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_addr), "r"(c0), "r"(x), "r"(y), "r"(n) : "memory");
 }
 
+// What the two producer warps of a pair kernel walk through: items of four listed tiles and a column block, channel chunks, and
+// per chunk `units` halos (the views of the input, in two parts where the kernel splits its operands).
+struct PairWork {
+  int item0, item_step, n_items, n_cblk, n_chunks, units;
+  unsigned crank, limit;
+  int withhold;      // self-test: load nothing
+};
+struct PairRing {
+  unsigned long long *full, *empty;      // "operands are there" in the first block, "free" in each
+  unsigned base, bytes, count;           // of a buffer
+};
+
+// Waits until the last uses of a ring's buffers are over: nothing may signal this block's barriers after it has left.  s and
+// parity: the next buffer and the parity of its next release; first_lap: no buffer has been waited for yet.
+__device__ __forceinline__ void pair_drain(const PairRing &r, unsigned s, unsigned parity, bool first_lap, bool ok, volatile int *abort_flag, unsigned limit) {
+  for (int i = 0; i < (int)r.count && ok && !*abort_flag; ++i) {
+    if (first_lap && (unsigned)i >= s) break;
+    if (first_lap) ok = mbar_wait(&r.empty[i], 0u, abort_flag, limit);
+    else {
+      ok = mbar_wait(&r.empty[s], parity, abort_flag, limit);
+      if (++s == r.count) { s = 0; parity ^= 1u; }
+    }
+  }
+}
+
+// Halo producer, one converged warp: one copy per halo row and tile, issued by one elected lane.  (With a row per lane the copies
+// are issued one by one all the same, at several times the cost -- no uniform registers --, and paced every layer.)
+// source(unit, view): the tensor map of a unit, and which view it is.
+template <typename Source>
+__device__ __forceinline__ void pair_produce_halos(const PairWork &w, const PairRing &r, const PairTaps &t, int hp, unsigned row_bytes, const int32_t *lst,
+                                                   int n_active, int ntiles_total, int TWo, int THo, int32_t *counts, volatile int *abort_flag,
+                                                   Source source) {
+  const unsigned leader = elect_one();
+  unsigned s = 0, parity = 0;
+  bool first_lap = true, ok = true;
+  for (int item = w.item0; item < w.n_items && ok && !w.withhold; item += w.item_step) {
+    const int e = 4 * (item / w.n_cblk) + 2 * (int)w.crank;
+    int tx8[2], ty8[2], tn[2];
+    bool have[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      int tile = __shfl_sync(0xffffffffu, e + i < n_active ? lst[e + i] : -1, 0);
+      have[i] = e + i < n_active;
+      // an entry outside the field is reported and skipped by the epilogue; here tile 0 stands in for it
+      if (have[i] && (tile < 0 || tile >= ntiles_total)) {
+        if (leader) atomicOr(&counts[3], MIE_ERR_BAD_TILE);
+        tile = 0;
+      }
+      tx8[i] = have[i] ? (tile % TWo) * 8 : 0; ty8[i] = have[i] ? ((tile / TWo) % THo) * 8 : 0; tn[i] = have[i] ? tile / (TWo * THo) : 0;
+    }
+    const unsigned tx_bytes = (unsigned)min(4, n_active - 4 * (item / w.n_cblk)) * (unsigned)hp * row_bytes;   // both blocks
+    for (int chunk = 0; chunk < w.n_chunks && ok; ++chunk)
+      for (int u = 0; u < w.units; ++u) {
+        if (!first_lap) ok = __all_sync(0xffffffffu, mbar_wait(&r.empty[s], parity, abort_flag, w.limit));
+        if (!ok) break;
+        const unsigned bar = mapa_shared(smem_u32(&r.full[s]), 0);
+        if (leader) {
+          if (w.crank == 0u)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&r.full[s])), "r"(tx_bytes) : "memory");
+          int v;
+          const CUtensorMap *map = source(u, v);
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (have[i]) {
+              unsigned dst = r.base + s * r.bytes + (unsigned)i * row_bytes;
+              const int x = tx8[i] + t.x0[v], y = ty8[i] + t.y0[v];
+              for (int row = 0; row < hp; ++row, dst += 2u * row_bytes) tma_load_4d_pair(dst, map, bar, chunk * 32, x, y + row, tn[i]);
+            }
+        }
+        __syncwarp();
+        if (++s == r.count) { s = 0; if (!first_lap) parity ^= 1u; first_lap = false; }
+      }
+  }
+  if (!w.withhold) pair_drain(r, s, parity, first_lap, ok, abort_flag, w.limit);
+}
+
+// Filter producer, one converged warp: stages of `tps` taps.  view(unit): whose taps these are; bytes(unit): what a tap brings to
+// both blocks; load(unit, tap, dst, bar, column block, chunk): issues the copies of this block's part of a tap.
+template <typename View, typename Bytes, typename Load>
+__device__ __forceinline__ void pair_produce_filter(const PairWork &w, const PairRing &r, const PairTaps &t, int tps, unsigned tap_bytes,
+                                                    volatile int *abort_flag, View view, Bytes bytes, Load load) {
+  const unsigned leader = elect_one();
+  unsigned s = 0, parity = 0, stage_addr = r.base;
+  bool first_lap = true, ok = true;
+  for (int item = w.item0; item < w.n_items && ok && !*abort_flag && !w.withhold; item += w.item_step) {
+    const int cb = item % w.n_cblk;
+    for (int chunk = 0; chunk < w.n_chunks && ok; ++chunk)
+      for (int u = 0; u < w.units && ok; ++u) {
+        const int v = view(u), end = t.first[v + 1];
+        for (int i = t.first[v]; i < end; i += tps) {
+          if (!first_lap) ok = __all_sync(0xffffffffu, mbar_wait(&r.empty[s], parity, abort_flag, w.limit));   // (the warp leaves as one)
+          if (!ok) break;
+          const int nt = min(tps, end - i);
+          if (leader) {
+            if (w.crank == 0u)
+              asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&r.full[s])), "r"((unsigned)nt * bytes(u)) : "memory");
+            const unsigned bar = mapa_shared(smem_u32(&r.full[s]), 0);
+            for (int k = 0; k < nt; ++k) load(u, (int)t.tap[i + k], stage_addr + (unsigned)k * tap_bytes, bar, cb, chunk);
+          }
+          __syncwarp();
+          stage_addr += r.bytes;
+          if (++s == r.count) { s = 0; stage_addr = r.base; if (!first_lap) parity ^= 1u; first_lap = false; }
+        }
+      }
+  }
+  if (!w.withhold) pair_drain(r, s, parity, first_lap, ok, abort_flag, w.limit);
+}
+
 // Barrier of the 128 threads of an epilogue set: whether all of them bring `ok`.
 __device__ __forceinline__ bool set_all(int id, bool ok) {
   int r;

@@ -148,6 +148,41 @@ def test_bounded_wait_expires_cleanly(dev, cfg, own):
         check_device_errors(layer)
 
 
+@pytest.mark.parametrize("cfg", [(32, 32, 3, 1, 40, 56), (64, 64, 3, 1, 104, 104), (32, 64, 5, 2, 40, 56)])
+def test_bounded_wait_of_the_dense_pass_expires_cleanly(dev, cfg):
+    """The same for the dense evaluation on the tensor cores, in blocks of 32 and of 64 channels."""
+    import torch.nn.functional as F
+    from maskedincrementeval_b200 import _native as nat
+    from maskedincrementeval_b200 import fields as fl
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.mask_incr_modules import check_device_errors
+    cin, cout, k, s, h, w = cfg
+    fl.config.tensor_cores = "auto"
+    layer = _layer(dev, cin, cout, k, s, "relu")
+    conv = layer.conv2d
+    x = cl(torch.randn(1, cin, h, w, generator=torch.Generator().manual_seed(5)), dev)
+    want = F.conv2d(x.double(), conv.weight.detach().double(), conv.bias.detach().double(), stride=s, padding=k // 2)
+    with torch.no_grad():
+        layer.activation.in_res.update_reservoir(cl(torch.full(want.shape, 7.0), dev))
+        nat.set_option(nat.OPT_TC_SPIN_LIMIT, 300)
+        nat.set_option(nat.OPT_TC_WITHHOLD_LOADS, 1)
+        NATIVE.conv(conv, NATIVE.lift(x), layer.activation)
+        torch.cuda.synchronize()
+        plan = conv._plan(1, h, w, dev)
+        assert nat.lib.mie_conv_is_exact(C.byref(plan.args))
+        assert int(plan.counts[3]) == nat.ERR_WAIT_EXPIRED
+        assert bool((layer.activation.in_res.reservoir == 7.0).all())      # nothing was written
+        with pytest.raises(nat.MieError, match="wait ran out"):
+            check_device_errors(layer)
+        nat.set_option(nat.OPT_TC_SPIN_LIMIT, 0)
+        nat.set_option(nat.OPT_TC_WITHHOLD_LOADS, 0)
+        NATIVE.conv(conv, NATIVE.lift(x), layer.activation)
+        torch.cuda.synchronize()
+    got = layer.activation.in_res.reservoir
+    assert float((got.double() - want).norm() / want.norm()) <= 2e-6
+    check_device_errors(layer)
+
+
 def test_runner_check_names_the_layer(dev):
     from maskedincrementeval_b200 import _native as nat
     from maskedincrementeval_b200.incr_modules.fireflownet_incr import FireFlowNetIncr

@@ -21,6 +21,7 @@ int launch_conv_tc(const mie_conv_args *a, cudaStream_t st);
 bool exact_takes(const mie_conv_args *a);
 int launch_conv_exact(const mie_conv_args *a, cudaStream_t st);
 int pack_exact(const float *w, int cout, int cin, int k, int ihwo, float *wpacked, cudaStream_t st);
+int split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, const int32_t *counts, cudaStream_t st);
 }  // namespace mie
 
 namespace {
@@ -799,7 +800,10 @@ struct IncWs {
   size_t bits_in, bits_out, counts, list, stale, flags, wpacked, wexact, hi, lo, total;
   int cp;      // channels of the split input
 };
-// fp32 precision on the tensor cores pays off from a reduction of a few instructions on, whatever the activity
+// fp32 precision on the tensor cores pays off from a reduction of 72 on, from a single active blob to full activity, although
+// the split is a pass over the whole field.  Device time against the FP32 kernel, blobs of 16x16 pixels: one blob / 0.5 % / 30 %
+// active: 8 -> 8 channels 3x3 at 264x352 33 / 33 / 42 us against 36 / 36 / 41; 16 -> 8: 29 / 30 / 39 against 41 / 41 / 49;
+// 64 -> 64 at 480x640 87 / 88 / 167 against 140 / 142 / 575.  A silent step makes no parts (split_exact): 40 us against 37 there.
 bool inc_exact(int cin, int cout, int k) { return k >= 3 && cout % 4 == 0 && cin * k * k >= 72; }
 IncWs inc_layout(int N, int cin, int H, int W, int cout, int k, int stride) {
   const int pad = k / 2;
@@ -895,7 +899,6 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   const bool exact = inc_exact(cin, cout, k) && exact_takes(&x);
   if (exact) {
     if ((s = pack_exact(filter, cout, cin, k, 1, wx, st)) != MIE_OK) return s;
-    if ((s = mie_split_exact(x_incr, cin, cin, (int64_t)N * H * W, hi, lo, L.cp, stream)) != MIE_OK) return s;
   } else {
     int blocks = (int)((nf + 255) / 256);
     if (blocks > MIE_SM_COUNT * 8) blocks = MIE_SM_COUNT * 8;
@@ -904,5 +907,6 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   }
   s = mie_tiles_dilate(bits_in, N, H, W, Ho, Wo, k, stride, pad, nullptr, nullptr, list, nullptr, counts, flags, stream);
   if (s != MIE_OK) return s;
+  if (exact && (s = split_exact(x_incr, cin, cin, (int64_t)N * H * W, hi, lo, L.cp, counts, st)) != MIE_OK) return s;
   return mie_conv_tiles(exact ? &x : &a, stream);
 }

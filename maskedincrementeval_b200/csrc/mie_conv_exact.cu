@@ -445,10 +445,12 @@ __device__ __forceinline__ void split_two_tf32(float v, float &hi, float &lo) {
 }
 
 // hi = round(v), lo = round(v - hi): one pass over a dense field, a thread per four channels of a pixel.  HBM bound.
+// counts (may be null): the work list of the convolution that reads the parts; none are made where it lists no tile.
 __global__ void __launch_bounds__(256) split_exact_kernel(const float *__restrict__ in, int64_t in_ps, int C, int64_t pixels, float *__restrict__ hi,
-                                                          float *__restrict__ lo, int64_t out_ps, int quads, int vec) {
+                                                          float *__restrict__ lo, int64_t out_ps, int quads, int vec, const int32_t *counts) {
   grid_dependency_wait();
   grid_dependency_trigger();
+  if (counts && counts[0] == 0) return;
   const int64_t total = pixels * quads;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t px = i / quads;
@@ -497,16 +499,20 @@ int pack_exact(const float *w, int cout, int cin, int k, int ihwo, float *wpacke
   return check_launch();
 }
 
-}  // namespace mie
-
-extern "C" int mie_split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, void *stream) {
+int split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, const int32_t *counts, cudaStream_t st) {
   if (!in || !hi || !lo || C <= 0 || pixels <= 0 || in_ps < C || out_ps < (C + 3) / 4 * 4 || out_ps % 4) return MIE_EINVAL;
   if (!aligned16(hi) || !aligned16(lo)) return MIE_EALIGN;
   const int quads = divup(C, 4), vec = C % 4 == 0 && in_ps % 4 == 0 && aligned16(in);
   int64_t blocks = divup64(pixels * quads, 256);
   if (blocks > MIE_SM_COUNT * 16) blocks = MIE_SM_COUNT * 16;
-  launch_chained(split_exact_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, in, in_ps, C, pixels, hi, lo, out_ps, quads, vec);
+  launch_chained(split_exact_kernel, dim3((unsigned)blocks), dim3(256), 0, st, in, in_ps, C, pixels, hi, lo, out_ps, quads, vec, counts);
   return check_launch();
+}
+
+}  // namespace mie
+
+extern "C" int mie_split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, void *stream) {
+  return split_exact(in, in_ps, C, pixels, hi, lo, out_ps, nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int mie_conv_pack_dims_exact(int cin, int cout, int k, int64_t *n_floats) {

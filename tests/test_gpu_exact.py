@@ -104,6 +104,22 @@ def test_dense_pass_on_non_finite_values(dev, case, where):
         assert float(((got[big] - want[big]) / want[big]).abs().max()) <= 1e-5 if bool(big.any()) else True
 
 
+def test_extension_on_a_silent_step(dev):
+    """A delta without an active pixel: zeros, also behind a call that left the workspace full, and before one that needs it again."""
+    from maskedincrementeval_b200.ext.pointops import pointops_functional as pf
+    g = torch.Generator(device=dev).manual_seed(9)
+    w = torch.randn(32, 3, 3, 64, generator=g, device=dev) * 0.06
+    x = cl(torch.randn(1, 32, 40, 56, generator=g, device=dev))
+    want = F.conv2d(x.double(), w.permute(3, 0, 1, 2).double(), padding=1)
+    for silent in (False, True, False, True):
+        mask = torch.zeros_like(x, dtype=torch.bool) if silent else None
+        y, _ = pf.functional_conv_module(x, w, mask=mask, stride=(1, 1), padding=(1, 1))
+        if silent:
+            assert bool((y == 0).all())
+        else:
+            assert float((y.double() - want).norm() / want.norm()) <= 2e-6
+
+
 # stride 2 on fields one pixel wide or high, which have no odd columns or rows
 @pytest.mark.parametrize("h,w", [(17, 1), (1, 22), (1, 1), (2, 9)])
 @pytest.mark.parametrize("k", [3, 5])

@@ -152,6 +152,38 @@ def test_mask_words_vectorised(dev, c, dtype):
     assert torch.equal(m.pixel_mask(), (x != 0).any(1, keepdim=True).to(torch.uint8))
 
 
+@pytest.mark.parametrize("c", [1, 2, 3, 4, 5, 6, 7, 8, 9])
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("thr", [0.0, 0.4])
+def test_input_delta_of_any_channel_count(dev, c, split, thr):
+    """Channel counts on both sides of the register kernel's limit, ragged tiles, padded pixels; every result to the bit."""
+    from maskedincrementeval_b200 import fields as fl
+    g = torch.Generator(device=dev).manual_seed(c)
+    n, h, w, cp, half = 2, 13, 21, (c + 3) // 4 * 4, (c + 7) // 8 * 8
+    new = lambda k: torch.zeros(n, h, w, k, device=dev).permute(0, 3, 1, 2)
+    xp, dx, bits = cl(torch.randn(n, c, h, w, generator=g, device=dev)), new(cp)[:, :c], fl.new_bits(n, h, w, dev)
+    copy, copy_bits = new(3 * half), fl.new_bits(n, h, w, dev)
+    try:
+        if split:
+            fl.request_split(dx, copy, copy_bits)
+        for frac in (0.2, 0.0, 1.0, 0.01):
+            x = cl(xp + torch.randn(n, c, h, w, generator=g, device=dev) * (torch.rand(n, 1, h, w, generator=g, device=dev) < frac))
+            d = x - xp
+            on = (d.abs() > thr).any(1, keepdim=True)
+            d = torch.where(on, d, torch.zeros_like(d))
+            kept = torch.where(on, x, xp)
+            m = fl.delta_mask(x, xp, dx, bits, thr)
+            assert torch.equal(dx, d) and torch.equal(xp, kept) and torch.equal(m.pixel_mask(), on.to(torch.uint8))
+            if split:
+                assert fl.split_made(dx, copy) and torch.equal(copy_bits, bits)
+                want = torch.zeros_like(copy)
+                want[:, :c] = want[:, 2 * half:2 * half + c] = d
+                want[:, half:half + c] = d - (d.contiguous().view(torch.int32) & ~0x1FFF).view(torch.float32)
+                assert torch.equal(copy, want)
+    finally:
+        fl.forget_tails()
+
+
 @pytest.mark.parametrize("n,h,w", [(1, 200, 168), (8, 480, 640), (3, 260, 346)])
 def test_dilation_of_large_fields(dev, n, h, w):
     from maskedincrementeval_b200 import fields as fl, _native as nat

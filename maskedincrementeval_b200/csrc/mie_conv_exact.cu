@@ -332,10 +332,11 @@ static ExactShape exact_shape(const mie_conv_args *a) {
   ExactShape h;
   pair_make_taps(a->k, a->stride, a->pad, &h.t, &h.wp);
   const int quads = divup(a->max_tiles, 4), clusters_max = MIE_SM_COUNT / 2;
-  // 64 channels per block (107 clocks per K-slice and tap) unless blocks of 32 (82) take fewer clocks over all rounds
+  // 64 channels per block (144 clocks per K-slice and tap, both instructions) unless blocks of 32 (103) take fewer clocks over all
+  // rounds: 256 -> 64 and 32 channels, the slope from four to eight rounds at 1965 MHz for k = 5 (k = 3: 159 and 113; k = 7: 178 and 105)
   h.cb = 32;
   if (a->cout_pad % 64 == 0 &&
-      (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 107 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 82)
+      (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 144 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 103)
     h.cb = 64;
   const int halo_bytes = (h.wp * 2 * h.wp * 128 + 1023) & ~1023, slab_bytes = 2 * (a->act != MIE_ACT_NONE ? 2 : 1) * 128 * (h.cb / 2) * 4;
   const int budget = 222 * 1024 - slab_bytes;
@@ -444,7 +445,8 @@ __device__ __forceinline__ void split_two_tf32(float v, float &hi, float &lo) {
   lo = round_tf32(v - hi);
 }
 
-// hi = round(v), lo = round(v - hi): one pass over a dense field, a thread per four channels of a pixel.  HBM bound.
+// hi = round(v), lo = round(v - hi): one pass over a dense field, a thread per four channels of a pixel.  HBM bound: one read
+// and two writes at 5.6 to 6.0 TB/s on fields beyond the L2 (8 x 32 x 480x640: 167 us), 0.86 to 0.91 of a measured copy.
 // counts (may be null): the work list of the convolution that reads the parts; none are made where it lists no tile.
 __global__ void __launch_bounds__(256) split_exact_kernel(const float *__restrict__ in, int64_t in_ps, int C, int64_t pixels, float *__restrict__ hi,
                                                           float *__restrict__ lo, int64_t out_ps, int quads, int vec, const int32_t *counts) {

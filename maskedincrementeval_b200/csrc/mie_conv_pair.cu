@@ -20,8 +20,9 @@
 //
 // What bounds it: an instruction reads 4 KB of A and NB / 2 rows of B from each block's shared memory at 128 bytes per
 // clock, so it takes 39 / 43 / 64 / 128 clocks for N = 32 / 64 / 128 / 256 (measured with resident operands) where the
-// tensor core itself needs 16 / 32 / 64 / 128.  The filter taps written by TMA share that port: 20.5 / 24.6 / 32.8 / 49 KB
-// per tap and chunk in all.
+// tensor core itself needs 16 / 32 / 64 / 128: 156 / 172 / 256 / 512 clocks per tap and chunk of four K-slices.  The filter taps
+// written by TMA share that port (20.5 / 24.6 / 32.8 / 49 KB per tap and chunk in all).  What a tap and chunk takes in the
+// kernel is at pair_block_width().
 #include "mie_pair.cuh"
 
 using namespace mie;
@@ -407,8 +408,12 @@ conv_pair_kernel(const PairParams P, const __grid_constant__ PairMaps maps) {
 }  // namespace
 
 // Output channels per pair: the width whose rounds of work items over the 74 clusters cost least.  Wide blocks are cheaper
-// per column -- KB through the shared-memory port per tap and chunk, see the head of this file --, small layers need the
-// narrow ones to occupy the machine.
+// per column, small layers need the narrow ones to occupy the machine.  The costs are relative ones per tap and chunk, chosen
+// on whole networks.  Measured by themselves (256 -> NB channels, every tile active, from a list, the slope from four to eight
+// rounds, 1965 MHz), k = 3 / 5 / 7: 32 channels 212 / 187 / 178 clocks, 64 250 / 203 / 201, 128 398 / 329 / 349, 256 721 / 660 /
+// 825.  Against the best width of each of 338 shapes (k 3 to 7, 64 and 256 -> 64 to 512 channels, 8 to 700 quads, from a list) the
+// table's choice takes 1.02 times as long on average and 1.3 times at worst (one round of 256 channels at 45 quads, where 64 channels
+// take three).  That sweep leaves out what one block per layer saves: its blocks find their own tiles without a dilation launch.
 static int pair_block_width(const mie_conv_args *a) {
   static const struct { int nb, cost; } width[4] = {{256, 512}, {128, 270}, {64, 200}, {32, 164}};
   const int64_t quads = ((int64_t)a->max_tiles + 3) / 4, clusters = MIE_SM_COUNT / 2;

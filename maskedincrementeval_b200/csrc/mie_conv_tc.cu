@@ -15,12 +15,13 @@
 //      Stride-2 layers read from four parity views of the input (one tensor map per row/column parity).
 //   B: box [1 tap][NB output channels][32 input channels] of the filter, stored [tap][cout][cin].
 //   Roles (192 threads): warp 0 = TMA producer (one lane), warp 1 = MMA issuer (one lane) and owner of the
-//   tensor-memory allocation, warps 2..5 = epilogue.  Takes stride 2, k = 1 and blocks of 256 channels.
+//   tensor-memory allocation, warps 2..5 = epilogue.
 //
-// (Layers with k >= 3 run on the CTA-pair kernel of mie_conv_pair.cu; of the kernels here the per-tap one takes k = 1, and
-// both take the cluster form behind MIE_OPT_TC_KSPLIT.)
+// (Layers with k >= 3 run on the CTA-pair kernel of mie_conv_pair.cu.  Of the kernels here the per-tap one takes k = 1.  With
+// MIE_OPT_TC_KSPLIT, off by default, small layers take the cluster forms: the halo kernel stride 1, the per-tap kernel stride 2
+// and 3x3 layers of a single channel chunk.)
 //
-// conv_tc_halo_kernel (halo-resident): stride 1, k in {3,5,7}.  The input halo of both tiles stays in shared
+// conv_tc_halo_kernel (halo-resident, as clusters only): stride 1, k in {3,5,7}.  The input halo of both tiles stays in shared
 // memory for a whole channel chunk, a filter tap is an address shift of the operand descriptor, and only filter
 // slices stream through the ring -- several taps per stage, two MMA-issuing warps.  See the comment at the kernel.
 //
@@ -990,22 +991,8 @@ int g_opt_own_kernels = 7;                  // MIE_OPT_TC_OWN_KERNELS
 
 namespace {
 
-// Shared memory the halo kernel's operands may take (KB) and the largest filter ring (slots); MIE_TC_RING_KB /
-// MIE_TC_RING_CAP in the environment override them for A/B measurements.
-int halo_ring_kb() {
-  static const int v = []() { const char *e = getenv("MIE_TC_RING_KB"); const int x = e ? atoi(e) : 0; return (x >= 128 && x <= 224) ? x : 200; }();
-  return v;
-}
-int halo_ring_cap() {
-  static const int v = []() { const char *e = getenv("MIE_TC_RING_CAP"); const int x = e ? atoi(e) : 0; return (x >= 2 && x <= HALO_MAX_STAGES) ? x : 4; }();
-  return v;
-}
-
-// MIE_TC_HALO=0 in the environment keeps every layer on the per-tap kernel (for A/B measurements).
-bool halo_enabled() {
-  static const bool on = []() { const char *e = getenv("MIE_TC_HALO"); return !(e && e[0] == '0'); }();
-  return on;
-}
+constexpr int HALO_RING_KB = 200;     // shared memory of the halo kernel's operands
+constexpr int HALO_RING_CAP = 4;      // its largest filter ring (slots)
 
 }  // namespace
 
@@ -1013,7 +1000,7 @@ bool halo_enabled() {
 bool tc_eligible(const mie_conv_args *a) {
   if (a->in2 || a->accum) return false;   // the 1x1 head kernel's extras
   if (!a->wpacked_tc) return false;
-  if (a->refresh || a->bias) return false;   // dense evaluation (full fp32, bias, reservoir set) is the FP32 kernel's
+  if (a->refresh || a->bias) return false;   // dense evaluation needs fp32 precision: conv_exact_kernel or the FP32 kernel
   if (!(a->stride == 1 || a->stride == 2)) return false;
   if (a->k != 1 && a->k != 3 && a->k != 5 && a->k != 7) return false;
   if (a->in_ps % 4 || !aligned16(a->in)) return false;                           // TMA: 16-byte strides and base
@@ -1036,7 +1023,9 @@ bool tc_eligible(const mie_conv_args *a) {
   // FP32 path, but it sees the raw input delta: truncating O(1) values to TF32 every step random-walks in the
   // first reservoir and measured 1.1e-3 of the output range against 1.3e-5 with the head in FP32.)
   if ((int64_t)a->cin * a->k * a->k < 256) return false;
-  if (a->stride == 2 && ((a->hin & 1) || (a->win & 1))) return false;            // parity views need even extents
+  // Odd extents at stride 2 stay on the FP32 kernel.  The parity views would take them, but the layers that have them give fp32
+  // results today, and TF32 inputs would lose 2^-11 of each product.
+  if (a->stride == 2 && ((a->hin & 1) || (a->win & 1))) return false;
   return true;
 }
 
@@ -1047,9 +1036,7 @@ static void tc_block_shape(const mie_conv_args *a, int *nb_out, int *ksplit_out)
   // could not keep about half of the SMs busy even at full activity -- the small-image layers of a UNet have
   // a few dozen tiles but thousands of reduction steps.  Measured on B200: a pipeline stage costs about
   // 0.6 us whatever its width, so narrowing pays only until the work items cover the machine once.
-  // MIE_TC_NB_MAX in the environment caps the block width (A/B measurements)
-  static const int nb_max = []() { const char *e = getenv("MIE_TC_NB_MAX"); const int x = e ? atoi(e) : 0; return (x == 32 || x == 64 || x == 128) ? x : 256; }();
-  int nb = nb_max;
+  int nb = 256;
   while (nb > 16 && a->cout_pad % nb) nb >>= 1;
   const int64_t pairs = (a->max_tiles + 1) / 2;
   while (nb > 32 && a->cout_pad % (nb / 2) == 0 && pairs * (a->cout_pad / nb) < 64) nb >>= 1;
@@ -1064,7 +1051,7 @@ static void tc_block_shape(const mie_conv_args *a, int *nb_out, int *ksplit_out)
     while (nbw > 32 && a->cout_pad % nbw) nbw >>= 1;
     const int n_chunks = cin_pad32 / 32;
     const int64_t items_w = pairs * (a->cout_pad / nbw);
-    const bool halo = a->stride == 1 && (cin_pad32 > 32 || a->k >= 5) && halo_enabled();   // which kernel takes the layer
+    const bool halo = a->stride == 1 && (cin_pad32 > 32 || a->k >= 5);   // which kernel takes the layer
     const int Wh = 8 + a->k - 1;
     const int a_bytes = 2 * (Wh * 2 * 8 * Wh * 16);
     for (int cs = 4; cs >= 2 && ksplit == 1; cs >>= 1) {
@@ -1135,7 +1122,7 @@ int launch_conv_tc(const mie_conv_args *a, cudaStream_t st) {
 
   // ---- halo-resident kernel, as clusters: stride 1, k in {3,5,7} (everything else with k >= 3 is the pair kernel's) ----
   // Layers of a single channel chunk with a 3x3 filter stay on the per-tap kernel (the halo is used for 9 taps only once).
-  if (ksplit > 1 && a->stride == 1 && (p.cin_pad > 32 || a->k >= 5) && halo_enabled()) {
+  if (ksplit > 1 && a->stride == 1 && (p.cin_pad > 32 || a->k >= 5)) {
     const int Wh = 8 + a->k - 1;
     const int a_bytes = 2 * (Wh * 2 * 8 * Wh * 16);          // two buffers of [Hh][2 tiles][8 groups][Wh][16 B]
     // A stage holds `tps` consecutive taps of one channel chunk (one TMA): the issuing thread pays its wait /
@@ -1143,11 +1130,11 @@ int launch_conv_tc(const mie_conv_args *a, cudaStream_t st) {
     // taps), else one filter row (k taps), else a single tap -- even if only two ring slots remain (measured:
     // 5-tap stages x 2 slots beat 1-tap stages x 4 slots by 25 % on a 5x5 256->128 layer).
     const int part_bytes = ksplit > 1 ? (ksplit - 1) * (nb / ksplit) * 512 : 0;   // partial sums received from the cluster
-    const int budget = halo_ring_kb() * 1024 - a_bytes - part_bytes;
+    const int budget = HALO_RING_KB * 1024 - a_bytes - part_bytes;
     int tps = 0, stages = 0;
     const int cand[3] = {a->k * a->k, a->k, 1};
     for (int i = 0; i < 3 && !tps; ++i)
-      if (2 * cand[i] * nb * 128 <= budget) { tps = cand[i]; stages = budget / (cand[i] * nb * 128); if (stages > halo_ring_cap()) stages = halo_ring_cap(); }
+      if (2 * cand[i] * nb * 128 <= budget) { tps = cand[i]; stages = budget / (cand[i] * nb * 128); if (stages > HALO_RING_CAP) stages = HALO_RING_CAP; }
     p.tps = tps ? tps : 1;
     const int b_bytes = p.tps * nb * 128;
     p.issuers = (2 * 2 * acc_cols <= 512 && (p.cin_pad / 32 / ksplit) * (a->k * a->k / p.tps) >= 2) ? 2 : 1;   // stages per CTA
@@ -1201,10 +1188,6 @@ int launch_conv_tc(const mie_conv_args *a, cudaStream_t st) {
   if (nb <= 128 && stages > 3) {
     const int deep = ((220 * 1024) / 3 - 3072 - epi_bytes) / stage_bytes;
     stages = deep > 3 ? (deep < stages ? deep : stages) : 3;
-  }
-  { // MIE_TC_TAP_STAGES in the environment forces the per-tap ring depth (A/B measurements)
-    static const int forced = []() { const char *e = getenv("MIE_TC_TAP_STAGES"); const int x = e ? atoi(e) : 0; return (x >= 2 && x <= 8) ? x : 0; }();
-    if (forced && forced * stage_bytes <= 200 * 1024) stages = forced;
   }
   const int part_bytes = ksplit > 1 ? (ksplit - 1) * (nb / ksplit) * 512 : 0;   // partial sums received from the cluster
   if (ksplit > 1) {

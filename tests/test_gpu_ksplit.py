@@ -24,10 +24,11 @@ def restore_config():
     from maskedincrementeval_b200 import _native as nat
     from maskedincrementeval_b200 import fields as fl
     saved = {k: getattr(fl.config, k) for k in ("threshold", "carry", "tensor_cores", "tc_thresholded", "compat")}
+    ksplit = nat.get_option(nat.OPT_TC_KSPLIT)
     yield
     for k, v in saved.items():
         setattr(fl.config, k, v)
-    nat.set_option(nat.OPT_TC_KSPLIT, 1)
+    nat.set_option(nat.OPT_TC_KSPLIT, ksplit)
 
 
 def cl(t, dev):

@@ -6,10 +6,13 @@
 //     hi(input) x [hi(filter) | lo(filter)]  ->  N = 2 CB columns,      lo(input) x hi(filter)  ->  N = CB columns.
 // What keeps the result at fp32 level is where the sums are rounded: the tensor core truncates each time it adds to an
 // accumulator (1.7e-8 of the value per addition, always towards zero: 3e-5 after the 2400 additions of a 256-channel 5x5
-// layer).  So the first product starts from zero again with every segment (at most 20 additions) and the epilogue warps
-// add the partial sums to registers, rounded to nearest, while the next segments run; the second product is 2^-12 of the first
-// and stays in its accumulator for the whole work item.  Against a float64 convolution the error is that of the CUDA-core
-// FP32 kernel or below it (see tests/test_gpu_exact.py).
+// layer).  So the first product starts from zero again with every segment of two to five taps (exact_shape()) and the epilogue
+// warps add the partial sums to registers, rounded to nearest, while the next segments run, low parts apart from high parts; the
+// second product is 2^-12 of the first and stays in its accumulator for the whole work item.
+// Error against a float64 convolution over that of the CUDA-core FP32 kernel: 0.68 to 0.95 for the first layers of the networks
+// on their event inputs, 0.3 to 0.9 for normal and for rectified inputs from a reduction (cin * k * k) of 72 on.  It is larger only
+// where few products meet, since the two parts leave 1e-7 of a value however short its sum: 1.2 to 1.6 for a reduction of 18, 1.1
+// to 2.2 where isolated pixels are active and cin is below 48; and up to 1.4 where every product is positive.
 // Epilogue: reservoir = conv + bias (+ addend), output = f(reservoir), every pixel of a listed tile marked.
 #include "mie_pair.cuh"
 
@@ -20,7 +23,6 @@ namespace {
 
 constexpr int EXACT_THREADS = 384;
 constexpr int EXACT_MAX_STAGES = 8;
-constexpr int EXACT_SEG_TAPS = 5;      // a segment: 5 taps x 4 K-slices = 20 additions into a tensor-memory accumulator
 constexpr int EXACT_MAX_HALOS = 4;
 
 struct ExactParams {
@@ -29,6 +31,7 @@ struct ExactParams {
   float *out; int64_t out_ps; unsigned int *out_bits32;
   int act; float *res; int64_t res_ps; const float *addend; int64_t addend_ps; const float *bias;
   int cb, stages, halos, tps, wp;   // tps: taps per ring stage
+  int seg;     // taps per segment of the first product's sum
   unsigned spin_limit;
   int withhold_loads;      // self-test: the producers issue nothing, so the first wait runs out (MIE_OPT_TC_WITHHOLD_LOADS)
   mie_tail_job tail;
@@ -99,7 +102,7 @@ __device__ __forceinline__ void exact_issue(const ExactParams &p, int bid, int n
               tc_fence_after();
             }
             pair_mma(tmem_base + seg * (2u * CB), a_hi | (halo + ((unsigned)p.t.off[i + k] * 8u)), b_hi | b_lo, id_hi, (unsigned)in_seg, nks);
-            if (++in_seg == EXACT_SEG_TAPS || i + k + 1 == end) {
+            if (++in_seg == p.seg || i + k + 1 == end) {
               pair_commit(&seg_full[seg]);
               in_seg = 0;
               if (++seg == NSEG) { seg = 0; seg_par ^= 1u; }
@@ -219,7 +222,7 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
     const int slot = (lane >> 3) & 1, prow = 2 * q + (lane >> 4), pcol = lane & 7;
     const unsigned lane_base = tmem_base + ((unsigned)(q * 32) << 16);
     int segs_per_chunk = 0;
-    for (int v = 0; v < nv; ++v) segs_per_chunk += (p.t.first[v + 1] - p.t.first[v] + EXACT_SEG_TAPS - 1) / EXACT_SEG_TAPS;
+    for (int v = 0; v < nv; ++v) segs_per_chunk += (p.t.first[v + 1] - p.t.first[v] + p.seg - 1) / p.seg;
     const int segs = segs_per_chunk * p.n_chunks;
     // slabs of this set: output, then reservoir; 128 rows of HW channels, 16-byte pieces swizzled as TMA does for rows of
     // 128 bytes (piece ^ (row & 7)) or 64 bytes (piece ^ (row / 2 & 3))
@@ -239,15 +242,15 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
       const int tx = (t >= 0) ? (t % TWo) * 8 : 0, ty = (t >= 0) ? ((t / TWo) % THo) * 8 : 0, n = (t >= 0) ? t / (TWo * THo) : 0;
       const bool valid = t >= 0 && ty + prow < p.hout && tx + pcol < p.wout;
       const int64_t pix = valid ? (int64_t)(n * p.hout + ty + prow) * p.wout + tx + pcol : 0;
-      float acc[HW];
+      float acc[HW], low[HW];       // the low products are summed apart, so that the large sum is rounded once a segment
 #pragma unroll
-      for (int i = 0; i < HW; ++i) acc[i] = 0.0f;
+      for (int i = 0; i < HW; ++i) acc[i] = low[i] = 0.0f;
       for (int s = 0; s < segs; ++s) {
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&seg_full[seg], seg_par, &s_abort, p.spin_limit)))) break;
         tc_fence_after();
         const unsigned c = lane_base + seg * (2u * CB) + (unsigned)set * CB;     // [hi | lo] columns of this set's channels
         tmem_add<HW>(c, acc);
-        tmem_add<HW>(c + HW, acc);
+        tmem_add<HW>(c + HW, low);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&seg_empty[seg]), 0));
@@ -256,7 +259,9 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
       // a warp whose wait gave up goes on to the barrier of its set, where the four of them leave together
       if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&item_full[buf], (item_idx >> 1) & 1u, &s_abort, p.spin_limit));
       tc_fence_after();
-      if (ok) tmem_add<HW>(lane_base + item_col + buf * CB + (unsigned)(set * HW), acc);
+      if (ok) tmem_add<HW>(lane_base + item_col + buf * CB + (unsigned)(set * HW), low);
+#pragma unroll
+      for (int i = 0; i < HW; ++i) acc[i] += low[i];
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&item_empty[buf]), 0));
@@ -325,7 +330,7 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
 // How a launch divides its columns and its shared memory; `stages` < 2: no split of it fits.
 struct ExactShape {
   PairTaps t;
-  int wp, cb, tps, stages, halos;
+  int wp, cb, tps, stages, halos, seg;
   size_t smem;
 };
 static ExactShape exact_shape(const mie_conv_args *a) {
@@ -351,6 +356,12 @@ static ExactShape exact_shape(const mie_conv_args *a) {
   const int stage_bytes = h.tps * h.cb * 128;
   h.stages = (budget - h.halos * halo_bytes) / stage_bytes;
   if (h.stages > EXACT_MAX_STAGES) h.stages = EXACT_MAX_STAGES;
+  // A segment's truncation grows with its length, the FP32 kernel's rounding with the whole reduction: the longest segments that
+  // keep the error below that kernel's for rectified inputs (segments of 2 / 3 / 5 taps: 288 products 0.83 / 1.13 / 1.62 of its
+  // error, 576 0.63 / 0.85 / 1.21, 800 0.55 / 0.70 / 1.09, 1152 0.44 / 0.58 / 0.83).  Shorter ones cost time: a refresh of eight
+  // E2Depth streams 480x640 takes 14.3 / 13.6 / 13.4 ms with one length for all layers.
+  const int depth = a->cin * a->k * a->k;
+  h.seg = depth < 400 ? 2 : depth < 1152 ? 3 : 5;
   h.smem = (size_t)((h.stages * stage_bytes + 1023) & ~1023) + (size_t)h.halos * halo_bytes + slab_bytes + 1024;
   return h;
 }
@@ -377,7 +388,7 @@ int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
   p.out = a->out; p.out_ps = a->out_ps; p.out_bits32 = reinterpret_cast<unsigned int *>(a->out_bits);
   p.act = a->act; p.res = a->res; p.res_ps = a->res_ps; p.addend = a->addend; p.addend_ps = a->addend_ps; p.bias = a->bias;
   p.tail = tail_for_kernel(a->tail);
-  p.t = h.t; p.wp = h.wp; p.cb = h.cb; p.tps = h.tps; p.stages = h.stages; p.halos = h.halos;
+  p.t = h.t; p.wp = h.wp; p.cb = h.cb; p.tps = h.tps; p.stages = h.stages; p.halos = h.halos; p.seg = h.seg;
   const size_t smem = h.smem;
   const int quads = divup(a->max_tiles, 4), clusters_max = MIE_SM_COUNT / 2;
 

@@ -59,13 +59,44 @@ def test_dense_pass_against_float64(dev, case):
             assert bool(m.pixel_mask().all())
     finally:
         fl.config.tensor_cores = old
-    # no worse than the CUDA-core kernel's own rounding (3e-7 for the shortest reductions to 1.4e-6 for the longest)
-    assert err["auto"] <= max(1.2 * err["off"], 6e-7), err
+    # no worse than the CUDA-core kernel's own rounding, or what two TF32 parts leave of a value (2^-24 of either operand, and the
+    # rounding of the result)
+    assert err["auto"] <= max(err["off"], 1.5e-7), err
+
+
+# reductions on both sides of the rule that sets the length of a segment
+@pytest.mark.parametrize("cin,k", [(8, 3), (5, 5), (16, 3), (32, 3), (44, 3), (45, 3), (64, 3), (32, 5), (127, 3), (128, 3), (64, 5), (256, 3)])
+@pytest.mark.parametrize("kind", ["normal", "rectified", "isolated"])
+def test_dense_pass_is_no_less_precise_than_fp32(dev, cin, k, kind):
+    from maskedincrementeval_b200 import fields as fl
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    torch.manual_seed(3)
+    layer = ConvLayerIncr(cin, 64, k, 1, k // 2, activation="relu").to(dev).eval()
+    c = layer.conv2d
+    g = torch.Generator(device=dev).manual_seed(4)
+    x = torch.randn(1, cin, 64, 72, generator=g, device=dev)
+    if kind == "rectified":
+        x = torch.relu(x)
+    if kind == "isolated":
+        x = x * (torch.rand(1, 1, 64, 72, generator=g, device=dev) < 0.05)
+    want = F.conv2d(x.double(), c.weight.detach().double(), c.bias.detach().double(), padding=k // 2)
+    err = {}
+    old = fl.config.tensor_cores
+    try:
+        for mode in ("auto", "off"):
+            fl.config.tensor_cores = mode
+            with torch.no_grad():
+                NATIVE.conv(c, NATIVE.lift(cl(x)), layer.activation)
+            err[mode] = float((layer.activation.in_res.reservoir.double() - want).norm() / want.norm())
+    finally:
+        fl.config.tensor_cores = old
+    assert err["auto"] <= max(err["off"], 1.5e-7), err
 
 
 # infinities, NaN and values that round up to infinity in TF32, in the input or in the filter: what the fp32 kernel gives
 @pytest.mark.parametrize("where", ["input", "filter"])
-@pytest.mark.parametrize("case", [(32, 64, 3, 1, 1, 41, 50), (5, 32, 5, 2, 2, 33, 40)])
+@pytest.mark.parametrize("case", [(64, 64, 3, 1, 1, 41, 50), (5, 32, 5, 2, 2, 33, 40)])
 def test_dense_pass_on_non_finite_values(dev, case, where):
     from maskedincrementeval_b200 import fields as fl
     from maskedincrementeval_b200.ext.pointops import pointops_functional as pf
@@ -94,7 +125,10 @@ def test_dense_pass_on_non_finite_values(dev, case, where):
         finally:
             fl.config.tensor_cores = old
         ext, _ = pf.functional_conv_module(x, c.conv2d_weights, mask=torch.ones_like(x, dtype=torch.bool), stride=(s, s), padding=(k // 2, k // 2))
-    for got, want in ((states["auto"], states["off"]), (ext, states["off"] - c.bias.detach().view(1, -1, 1, 1))):
+    pairs = [(states["auto"], states["off"])]
+    if cin >= 48:      # (the extension runs narrower layers on the FP32 kernel, which sends no NaN)
+        pairs.append((ext, states["off"] - c.bias.detach().view(1, -1, 1, 1)))
+    for got, want in pairs:
         assert not bool(want.isfinite().all())
         assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
         # relative to the products that a value is the sum of: fp32 sums of cin * k * k terms
@@ -108,8 +142,8 @@ def test_extension_on_a_silent_step(dev):
     """A delta without an active pixel: zeros, also behind a call that left the workspace full, and before one that needs it again."""
     from maskedincrementeval_b200.ext.pointops import pointops_functional as pf
     g = torch.Generator(device=dev).manual_seed(9)
-    w = torch.randn(32, 3, 3, 64, generator=g, device=dev) * 0.06
-    x = cl(torch.randn(1, 32, 40, 56, generator=g, device=dev))
+    w = torch.randn(64, 3, 3, 64, generator=g, device=dev) * 0.04
+    x = cl(torch.randn(1, 64, 40, 56, generator=g, device=dev))
     want = F.conv2d(x.double(), w.permute(3, 0, 1, 2).double(), padding=1)
     for silent in (False, True, False, True):
         mask = torch.zeros_like(x, dtype=torch.bool) if silent else None
@@ -128,15 +162,15 @@ def test_stride_two_on_one_pixel_fields(dev, h, w, k):
     from maskedincrementeval_b200.incr_modules._algebra import NATIVE
     from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
     torch.manual_seed(6)
-    layer = ConvLayerIncr(32, 64, k, 2, k // 2, activation="relu").to(dev).eval()
+    layer = ConvLayerIncr(64, 64, k, 2, k // 2, activation="relu").to(dev).eval()
     c = layer.conv2d
-    x = cl(torch.randn(2, 32, h, w, device=dev))
+    x = cl(torch.randn(2, 64, h, w, device=dev))
     want = F.conv2d(x.double(), c.weight.detach().double(), c.bias.detach().double(), stride=2, padding=k // 2)
     with torch.no_grad():
         NATIVE.conv(c, NATIVE.lift(x), layer.activation)
         got = layer.activation.in_res.reservoir
         y, _ = pf.functional_conv_module(x, c.conv2d_weights, mask=None, stride=(2, 2), padding=(k // 2, k // 2))
-    assert float((got.double() - want).norm() / want.norm()) <= 2e-6      # fp32 sums of 32 * k * k products
+    assert float((got.double() - want).norm() / want.norm()) <= 2e-6      # fp32 sums of 64 * k * k products
     want = want - c.bias.detach().double().view(1, -1, 1, 1)
     assert float((y.double() - want).norm() / want.norm()) <= 2e-6
 

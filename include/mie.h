@@ -295,7 +295,7 @@ int mie_activation_increment(float *X, const float *in_incr, float *out_incr, in
  * (0 = no mask given: derive it from x_incr != 0); filter [Cin,k,k,Cout] contiguous
  * (pointops_functional.py:13-14); out_incr [N,Cout,Hout,Wout] channels-last, every element is
  * written (the reference hands in torch.empty, pointops_functional.py:29).  pad = k/2.
- * Layers with Cin * k * k >= 72, k >= 3 and Cout a multiple of 4 run in fp32 precision on the tensor cores, the others on the
+ * Layers with Cin >= 48, k >= 3 and Cout a multiple of 4 run in fp32 precision on the tensor cores, the others on the
  * FP32 kernels (also where a pointer is not 16-byte aligned, and stride 2 on fields one pixel wide or high).
  * workspace: device scratch of mie_conv_increment_workspace_bytes(...) bytes, 256-byte aligned; for the layers named it holds the
  * packed filter and two copies of the input. */

@@ -800,11 +800,13 @@ struct IncWs {
   size_t bits_in, bits_out, counts, list, stale, flags, wpacked, wexact, hi, lo, total;
   int cp;      // channels of the split input
 };
-// fp32 precision on the tensor cores pays off from a reduction of 72 on, from a single active blob to full activity, although
-// the split is a pass over the whole field.  Device time against the FP32 kernel, blobs of 16x16 pixels: one blob / 0.5 % / 30 %
-// active: 8 -> 8 channels 3x3 at 264x352 33 / 33 / 42 us against 36 / 36 / 41; 16 -> 8: 29 / 30 / 39 against 41 / 41 / 49;
-// 64 -> 64 at 480x640 87 / 88 / 167 against 140 / 142 / 575.  A silent step makes no parts (split_exact): 40 us against 37 there.
-bool inc_exact(int cin, int cout, int k) { return k >= 3 && cout % 4 == 0 && cin * k * k >= 72; }
+// fp32 precision on the tensor cores, for deltas of 48 channels or more: with fewer, the few products that meet at an isolated
+// active pixel leave the FP32 kernel the smaller error (5 channels 9e-8 against 5e-8, 16 1.0e-7 / 8e-8, 32 1.3e-7 / 1.1e-7; 48
+// 1.24e-7 / 1.26e-7, 64 1.3e-7 / 1.5e-7, and at 5 % activity 64 1.4e-7 / 2.0e-7).  It is faster from a single active blob to full
+// activity, although the split is a pass over the whole field: 64 -> 64 channels at 480x640, blobs of 16x16 pixels, one blob / 0.5 % /
+// 30 % / all active 87 / 88 / 167 / 193 us against 140 / 142 / 575 / 729.  A silent step makes no parts (split_exact): 40 us
+// against 37.
+bool inc_exact(int cin, int cout, int k) { return k >= 3 && cout % 4 == 0 && cin >= 48; }
 IncWs inc_layout(int N, int cin, int H, int W, int cout, int k, int stride) {
   const int pad = k / 2;
   const int Ho = (H + 2 * pad - k) / stride + 1, Wo = (W + 2 * pad - k) / stride + 1;

@@ -94,6 +94,19 @@ def test_dense_pass_is_no_less_precise_than_fp32(dev, cin, k, kind):
     assert err["auto"] <= max(err["off"], 1.5e-7), err
 
 
+def test_extension_is_no_less_precise_than_fp32(dev):
+    """conv*_increment_ext on isolated active pixels: layers below 48 channels keep to the FP32 kernel."""
+    from maskedincrementeval_b200.ext.pointops import pointops_functional as pf
+    g = torch.Generator(device=dev).manual_seed(10)
+    for cin, bound in ((5, 7e-8), (16, 1e-7), (32, 1.2e-7), (47, 1.4e-7), (48, 1.4e-7), (64, 1.5e-7)):      # the FP32 kernel's: sums of cin products
+        w = torch.randn(cin, 3, 3, 32, generator=g, device=dev) / (9 * cin) ** 0.5
+        x = torch.zeros(2, cin, 60, 80, device=dev)
+        x[:, :, ::9, ::9] = torch.randn(2, cin, 7, 9, generator=g, device=dev)
+        y, _ = pf.functional_conv_module(cl(x), w, mask=None, stride=(1, 1), padding=(1, 1))
+        want = F.conv2d(x.double(), w.permute(3, 0, 1, 2).double(), padding=1)
+        assert float((y.double() - want).norm() / want.norm()) <= bound, cin
+
+
 # infinities, NaN and values that round up to infinity in TF32, in the input or in the filter: what the fp32 kernel gives
 @pytest.mark.parametrize("where", ["input", "filter"])
 @pytest.mark.parametrize("case", [(64, 64, 3, 1, 1, 41, 50), (5, 32, 5, 2, 2, 33, 40)])

@@ -86,6 +86,10 @@ class IncrConfig:
 
 config = IncrConfig()
 
+# Counts the packed filters that were replaced or dropped because their parameter changed: a captured step that was recorded
+# under another count may read one that is gone.
+filter_epoch = [0]
+
 
 def pixel_stride(x: torch.Tensor) -> int:
     """Pixel stride (floats) of a [N,C,H,W] tensor stored channels-last, possibly a channel slice."""

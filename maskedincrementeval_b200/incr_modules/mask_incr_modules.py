@@ -425,6 +425,8 @@ class nnConvIncr(nn.Conv2d):
 
     def load_state_dict(self, state_dict: 'OrderedDict[str, torch.Tensor]', strict: bool = True):
         r = nn.Conv2d.load_state_dict(self, state_dict, strict=strict)
+        if self._packed:
+            fl.filter_epoch[0] += 1
         self._packed.clear()
         self._packed_exact.clear()
         self._cw = None
@@ -454,20 +456,27 @@ class nnConvIncr(nn.Conv2d):
         return (getattr(self, "precision", None) == "split" and cin * self._k * self._k >= 256
                 and self._k in (1, 3, 5, 7) and self._s in (1, 2))
 
+    def _filter_version(self, bn: "Optional[nn.BatchNorm2d]"):
+        ver = (self.weight._version, self.weight.device, self.weight.data_ptr())
+        if bn is not None:
+            ver = ver + (bn.running_var._version, bn.running_var.data_ptr(), bn.eps,
+                         None if bn.weight is None else (bn.weight._version, bn.weight.data_ptr()))
+        return ver
+
     def _weights(self, cin_limit: Optional[int] = None, split: bool = False, bn: "Optional[nn.BatchNorm2d]" = None):
         """Packed filter for the kernels, repacked whenever the parameter changed or moved.  ``bn``: an eval
         batch-norm that follows the convolution; on a delta it is a per-channel scale (``bn2d_from_module``), which
         is folded into the packed filter."""
         key = cin_limit or self.in_channels
-        ver = (self.weight._version, self.weight.device, self.weight.data_ptr())
+        ver = self._filter_version(bn)
         if bn is not None:
-            ver = ver + (bn.running_var._version, bn.running_var.data_ptr(), bn.eps,
-                         None if bn.weight is None else (bn.weight._version, bn.weight.data_ptr()))
             key = ("bn", id(bn), key)
         if split:
             key = ("split", key)
         hit = self._packed.get(key)
         if hit is None or hit[0][0] is not self.weight or hit[0][1] is not bn or hit[1] != ver:
+            if hit is not None:
+                fl.filter_epoch[0] += 1
             w = self.weight.detach()
             if bn is not None:
                 scale = (bn.weight.detach() if bn.weight is not None else 1.0) / torch.sqrt(bn.running_var + bn.eps)
@@ -698,6 +707,10 @@ class nnConvIncr(nn.Conv2d):
         # switched on (config.kfenced_step) its carry is cleared instead.
         if config.kfenced_step and self.kf.delta.reservoir is not None:
             self.kf.delta.reservoir.zero_()
+        for key, hit in list(self._packed.items()):      # filters that the steps after this pass may not use any more
+            if hit[0][0] is not self.weight or hit[1] != self._filter_version(hit[0][1]):
+                del self._packed[key]
+                fl.filter_epoch[0] += 1
         return nn.Conv2d.forward(self, x)
 
 

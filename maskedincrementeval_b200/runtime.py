@@ -50,7 +50,9 @@ class IncrementalRunner:
 
     model          E2VIDRecurrentIncr, FireFlowNetIncr or MultiResUNetRecurrentIncr (takes ``prev_states`` iff
                    it is the first)
-    use_graph      replay the incremental step as a CUDA graph (captured on the second incremental step)
+    use_graph      replay the incremental step as a CUDA graph (captured on the second incremental step).  The configuration and
+                   the layers' options hold as they were then; after a change of parameters, which needs a refresh, the
+                   step is recorded again
     refresh_every  dense refresh period in frames (None: only when ``refresh`` is called)
     feedback       feed the recurrent state back (E2Depth only).  The reference's drivers pass ``prev_states=None``
                    to every incremental step (``run_e2depth_continuous_dataset.py:70``), so as driven the network
@@ -78,6 +80,7 @@ class IncrementalRunner:
         self._x_prev = self._x_in = self._dx = None
         self._y: List[torch.Tensor] = []
         self._graph = None
+        self._graph_filters = 0    # fields.filter_epoch at the capture
         self._pipe = None
         self._eager_steps = 0
         self._frame = 0
@@ -218,6 +221,8 @@ class IncrementalRunner:
 
     def _advance(self):
         """One incremental step on the frame that sits in the input buffer."""
+        if self._graph is not None and self._graph_filters != fl.filter_epoch[0]:
+            self._graph, self._eager_steps = None, 0      # a filter was packed anew since the capture: record the step again
         with torch.no_grad():
             if self._graph is not None:
                 self._graph.replay()
@@ -228,7 +233,7 @@ class IncrementalRunner:
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g):
                     self._step_body()
-                self._graph = g
+                self._graph, self._graph_filters = g, fl.filter_epoch[0]
                 g.replay()
                 self.graph_replays += 1
             else:

@@ -288,3 +288,50 @@ def test_prepared_calls_hold_the_packed_filter(dev, prepared, refresh):
             assert torch.equal(a.activation.in_res.reservoir, b.activation.in_res.reservoir)
             assert bool(a.activation.in_res.reservoir.isfinite().all())
     del taken
+
+
+@pytest.mark.parametrize("refresh", ["native", "library"])
+@pytest.mark.parametrize("how", ["in place", "replaced"])
+def test_a_captured_step_follows_new_parameters(dev, refresh, how):
+    """Parameters change while a step is captured: the packed filters that it reads are dropped, so it has to be recorded again."""
+    from maskedincrementeval_b200 import fields as fl
+    from maskedincrementeval_b200.incr_modules.fireflownet_incr import FireFlowNetIncr
+    from maskedincrementeval_b200.runtime import IncrementalRunner
+
+    def runner():
+        torch.manual_seed(7)
+        net = FireFlowNetIncr(dict(base_num_channels=32, kernel_size=3, mask_output=False), 2, compat="exact").to(dev).eval()
+        return net, IncrementalRunner(net)
+
+    def change(net):
+        with torch.no_grad():
+            for i, p in enumerate(net.parameters()):
+                if how == "in place":
+                    p.mul_(1.0 + 0.1 * (i % 3))
+            if how == "replaced":
+                for m in net.modules():
+                    if isinstance(m, torch.nn.Conv2d):
+                        m.weight = torch.nn.Parameter(m.weight.detach() * 1.25)
+
+    old = fl.config.refresh
+    fl.config.refresh = refresh
+    torch.backends.cudnn.allow_tf32 = False
+    try:
+        g = torch.Generator(device=dev).manual_seed(8)
+        xs = [cl(torch.randn(1, 2, 40, 56, generator=g, device=dev)) for _ in range(5)]
+        (net, run), (twin, fresh) = runner(), runner()
+        run.refresh(xs[0])
+        for x in xs[1:4]:
+            run.step(x)
+        replays = run.graph_replays
+        assert replays == 2
+        change(net), change(twin)
+        run.refresh(xs[0]), fresh.refresh(xs[0])
+        taken = [torch.full((n,), float("nan"), device=dev) for n in (9 * 32 * 32, 9 * 96 * 32, 9 * 8 * 32) for _ in range(16)]
+        for i, x in enumerate(xs[1:]):
+            assert torch.equal(run.step(x), fresh.step(x)), i
+        assert run.graph_replays == replays + 3      # one eager step, then captured again
+        run.check()
+        del taken
+    finally:
+        fl.config.refresh = old

@@ -196,8 +196,9 @@ typedef struct mie_conv_args {
   /* Dense evaluation (the refresh pass, nnConvIncr.forward_refresh_reservoirs + the activation's,
    * incr_modules/mask_incr_modules.py:182-196, 253-256): with `refresh` non-zero the input is a dense tensor, not a
    * delta: d = conv + bias (+ addend); *res = d (set, not advanced); out = f(d) (act == NONE: out = d); every pixel of
-   * every listed tile is written and marked in the tile words.  Needs thr == 0 and no carry buffer; always runs on the
-   * FP32 kernel.  `bias` (cout floats, may be null) is only read in this mode or when given. */
+   * every listed tile is written and marked in the tile words.  Needs thr == 0 and no carry buffer; runs on the FP32
+   * kernel, or in fp32 precision on the tensor cores (`wpacked_exact`, `in_lo` below).  `bias` (cout floats, may be
+   * null) is only read in this mode or when given. */
   const float *bias;
   int refresh;
   /* optional tile dilation of the next convolution, run in this kernel's tail (in_bits == out_bits of this call) */
@@ -230,8 +231,9 @@ typedef struct mie_conv_args {
   void *own_scratch;
   /* Dense evaluation (`refresh`) in fp32 precision on the tensor cores, both or neither: the filter packed by
    * mie_pack_conv_weights_exact, and the second field of mie_split_exact (`in` is then its first one, same pixel stride).
-   * Taken for k in {3, 5, 7} without a second input when the fields are 16-byte aligned; else, and with either null, the
-   * FP32 kernel runs (on `in` as given: pass the unsplit field there).  Every output tile has to be listed. */
+   * Taken for k in {3, 5, 7} without a second input when the fields are 16-byte aligned, but for stride 2 on a field one
+   * pixel wide or high (mie_conv_is_exact tells); else, and with either null, the FP32 kernel runs (on `in` as given: pass
+   * the unsplit field there).  Every output tile has to be listed. */
   const float *wpacked_exact;
   const float *in_lo;
 } mie_conv_args;

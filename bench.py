@@ -327,15 +327,15 @@ def roofline_conv3x3(dev, peak_gbs, peak_kind, repeats=3, args_tc=True):
     flops = [t * 64 * 32 * 9 * 32 * 2 for t in tiles]
     achieved = sum(byts) / tot_t / 1e9
     traffic = None  # DRAM bytes per launch of this kernel from the committed ncu capture of this same command
-    tp = os.path.join(ROOT, "profiles", "conv_tc_c1_conv3x3_260x346.md")
+    tp = os.path.join(ROOT, "profiles", "conv_pair_c1_conv3x3_260x346.md")
     if os.path.exists(tp):
         for ln in open(tp):
             if ln.startswith("dram_bytes_per_launch:"):
                 traffic = float(ln.split(":")[1])
     return {"bound": "hbm", "achieved": achieved, "peak": peak_gbs, "unit": "GB/s", "frac": achieved / peak_gbs,
             "traffic": traffic, "traffic_source": "recorded: dram__bytes_read.sum + dram__bytes_write.sum per launch from the "
-            "committed ncu capture of this kernel (profiles/conv_tc_c1_conv3x3_260x346.md), not measured in this run",
-            "peak_kind": f"of {peak_kind}", "kernel": ("conv_tc_kernel" if conv.last_used_tensor_cores else "conv_tiles_kernel<3,1,4,1>") + " (conv3x3 32->32 + ReLU, 260x346)",
+            "committed ncu capture of this kernel (profiles/conv_pair_c1_conv3x3_260x346.md), not measured in this run",
+            "peak_kind": f"of {peak_kind}", "kernel": ("conv_pair_kernel" if conv.last_used_tensor_cores else "conv_tiles_kernel<3,1,4,1>") + " (conv3x3 32->32 + ReLU, 260x346)",
             "bytes_per_launch": sum(byts) / len(byts), "us_per_launch": 1e6 * tot_t / len(times),
             "active_tiles_mean": sum(tiles) / len(tiles), "tiles_total": fl.n_tiles(1, H, W),
             "active_pixel_frac": sum(px) / len(px), "fp32_tflops": sum(flops) / tot_t / 1e12, "launches": len(times),
@@ -776,8 +776,10 @@ def run_ours(args):
                              "note": "forward_refresh_reservoirs every step on PyTorch's dense operators (cuDNN), same "
                                      "frames; context only",
                              "refresh_native_ms": time_native_refresh(),
-                             "refresh_native_note": "the same dense pass on this library's FP32 kernels (what a refresh "
-                                                    "costs in IncrementalRunner), eager launches"}
+                             "refresh_native_note": "the same dense pass on this library's kernels, in fp32 precision on the "
+                                                    "tensor cores.  Eager launches, one pass per event pair with the L2 "
+                                                    "flushed before it: the device waits for the host, which enqueues some "
+                                                    "fifty short kernels (passes back to back: 1.0 ms)"}
             line["activity"] = activity_table(net, run, frames_dev[2 + Wm + K], dev)
             # the same frames with activation / ConvLSTM thresholds and carry: the sparsest setting of the threshold
             # study that stays inside the 2e-3 tolerance with these weights

@@ -459,21 +459,21 @@ def roofline_other_kernels(dev, peak_gbs, peak_kind):
     def dm_set():
         full = torch.zeros(n2, 8, h2, w2, device=dev).contiguous(memory_format=torch.channels_last)
         return dict(x=field(n2, 5, h2, w2, 1.0), xp=field(n2, 5, h2, w2, 1.0), dx=full[:, :5], bits=fl.new_bits(n2, h2, w2, dev))
-    measure("delta_mask_kernel", f"input delta, previous-frame update and mask, 5 bins, {h2}x{w2}", px2 * 5 * 4 * 4, dm_set,
+    measure("delta_mask_few_kernel", f"input delta, previous-frame update and mask, 5 bins, {h2}x{w2}", px2 * 5 * 4 * 4, dm_set,
             lambda s_: fl.delta_mask(s_["x"], s_["xp"], s_["dx"], s_["bits"], 0.0),
             "frame read, previous frame read + written, delta written")
 
     # mask words of a 32-channel field
     def mw_set():
         return dict(d=field(n2, c2, h2, w2), bits=fl.new_bits(n2, h2, w2, dev))
-    measure("mask_words_kernel", f"tile words of a {c2}-channel field, {h2}x{w2}", px2 * c2 * 4 + fl.n_tiles(n2, h2, w2) * 8, mw_set,
+    measure("mask_words_vec_kernel", f"tile words of a {c2}-channel field, {h2}x{w2}", px2 * c2 * 4 + fl.n_tiles(n2, h2, w2) * 8, mw_set,
             lambda s_: fl.mask_from_delta(s_["d"], 1e-3, s_["bits"]))
 
     # split-precision copy of a 32-channel field (the pass in front of a split-precision convolution)
     def sp_set():
         return dict(d=field(n2, c2, h2, w2), m=full_bits(n2, h2, w2), out=fl.new_field(n2, 3 * c2, h2, w2, dev),
                     ob=fl.new_bits(n2, h2, w2, dev))
-    measure("split_tf32_kernel", f"split-precision copy, {c2} ch, {h2}x{w2}", px2 * c2 * 4 * 4, sp_set,
+    measure("split_tf32_vec_kernel", f"split-precision copy, {c2} ch, {h2}x{w2}", px2 * c2 * 4 * 4, sp_set,
             lambda s_: fl.split_tf32(s_["d"], s_["m"], s_["out"], s_["ob"]), "field read, three copies written")
 
     # tile dilation of a full 33x44-tile mask for a 3x3 convolution: a latency-bound single-block kernel

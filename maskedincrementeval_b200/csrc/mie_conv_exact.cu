@@ -204,10 +204,9 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
   } else if (warp == 1) {
     // =========================== filter producer: hi and lo rows beside the high part of the input, hi rows beside the low part ===========================
     const PairRing ring = {b_full, b_empty, b_base, stage_bytes, (unsigned)p.stages};
-    pair_produce_filter(work, ring, p.t, p.tps, tap_bytes, &s_abort, [&](int u) { return u < nv ? u : u - nv; },
+    pair_produce_filter(work, ring, p.t, p.tps, tap_bytes, (int)crank * HW, CB, &s_abort, [&](int u) { return u < nv ? u : u - nv; },
                         [&](int u) { return 2u * (u < nv ? tap_bytes : half_bytes); },
-                        [&](int u, int tap, unsigned dst, unsigned bar, int cb, int chunk) {
-                          const int row = cb * CB + (int)crank * HW;
+                        [&](int u, int tap, unsigned dst, unsigned bar, int row, int chunk) {
                           tma_load_4d_pair(dst, &maps.w, bar, 0, row, chunk, tap);
                           if (u < nv) tma_load_4d_pair(dst + half_bytes, &maps.w, bar, 0, p.cout_pad + row, chunk, tap);
                         });

@@ -273,10 +273,9 @@ conv_pair_kernel(const PairParams P, const __grid_constant__ PairMaps maps) {
   } else if (warp == 1) {
     // =========================== filter producer ===========================
     const PairRing ring = {b_full, b_empty, b_base, stage_bytes, (unsigned)p.stages};
-    pair_produce_filter(work, ring, P.t, P.tps, tap_bytes, &s_abort, [](int u) { return u; }, [&](int) { return 2u * tap_bytes; },
-                        [&](int, int tap, unsigned dst, unsigned bar, int cb, int chunk) {
-                          tma_load_4d_pair(dst, &maps.w, bar, 0, cb * NB + (int)crank * (NB >> 1), chunk, tap);
-                        });
+    pair_produce_filter(work, ring, P.t, P.tps, tap_bytes, (int)crank * (NB >> 1), NB, &s_abort, [](int u) { return u; },
+                        [&](int) { return 2u * tap_bytes; },
+                        [&](int, int tap, unsigned dst, unsigned bar, int row, int chunk) { tma_load_4d_pair(dst, &maps.w, bar, 0, row, chunk, tap); });
   } else if (warp == 2) {
     if (crank == 0u) {
       PairIssue a;

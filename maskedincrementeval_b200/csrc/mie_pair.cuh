@@ -174,33 +174,36 @@ __device__ __forceinline__ void pair_produce_halos(const PairWork &w, const Pair
 }
 
 // Filter producer, one converged warp: stages of `tps` taps.  view(unit): whose taps these are; bytes(unit): what a tap brings to
-// both blocks; load(unit, tap, dst, bar, column block, chunk): issues the copies of this block's part of a tap.
+// both blocks; load(unit, tap, dst, bar, row, chunk): issues the copies of this block's part of a tap; row: of its column block's
+// first filter row, row0 + column block * row_step.  A lane whose wait gave up stays with its warp until the end of the chunk,
+// where they leave together: a vote for every stage took 0.5 % of an eight-stream step.
 template <typename View, typename Bytes, typename Load>
-__device__ __forceinline__ void pair_produce_filter(const PairWork &w, const PairRing &r, const PairTaps &t, int tps, unsigned tap_bytes,
-                                                    volatile int *abort_flag, View view, Bytes bytes, Load load) {
+__device__ __forceinline__ void pair_produce_filter(const PairWork &w, const PairRing &r, const PairTaps &t, int tps, unsigned tap_bytes, int row0,
+                                                    int row_step, volatile int *abort_flag, View view, Bytes bytes, Load load) {
   const unsigned leader = elect_one();
   unsigned s = 0, parity = 0, stage_addr = r.base;
   bool first_lap = true, ok = true;
-  for (int item = w.item0; item < w.n_items && ok && !*abort_flag && !w.withhold; item += w.item_step) {
-    const int cb = item % w.n_cblk;
-    for (int chunk = 0; chunk < w.n_chunks && ok; ++chunk)
-      for (int u = 0; u < w.units && ok; ++u) {
+  for (int item = w.item0; item < w.n_items && ok && !w.withhold; item += w.item_step) {
+    const int row = row0 + (item % w.n_cblk) * row_step;
+    for (int chunk = 0; chunk < w.n_chunks && ok; ++chunk) {
+      for (int u = 0; u < w.units; ++u) {
         const int v = view(u), end = t.first[v + 1];
         for (int i = t.first[v]; i < end; i += tps) {
-          if (!first_lap) ok = __all_sync(0xffffffffu, mbar_wait(&r.empty[s], parity, abort_flag, w.limit));   // (the warp leaves as one)
-          if (!ok) break;
+          if (!first_lap && ok) ok = mbar_wait(&r.empty[s], parity, abort_flag, w.limit);
           const int nt = min(tps, end - i);
-          if (leader) {
+          if (leader && ok) {
             if (w.crank == 0u)
               asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&r.full[s])), "r"((unsigned)nt * bytes(u)) : "memory");
             const unsigned bar = mapa_shared(smem_u32(&r.full[s]), 0);
-            for (int k = 0; k < nt; ++k) load(u, (int)t.tap[i + k], stage_addr + (unsigned)k * tap_bytes, bar, cb, chunk);
+            for (int k = 0; k < nt; ++k) load(u, (int)t.tap[i + k], stage_addr + (unsigned)k * tap_bytes, bar, row, chunk);
           }
           __syncwarp();
           stage_addr += r.bytes;
           if (++s == r.count) { s = 0; stage_addr = r.base; if (!first_lap) parity ^= 1u; first_lap = false; }
         }
       }
+      ok = __all_sync(0xffffffffu, ok);
+    }
   }
   if (!w.withhold) pair_drain(r, s, parity, first_lap, ok, abort_flag, w.limit);
 }

@@ -4,13 +4,15 @@
 // and a product is hi*hi + hi*lo + lo*hi; the dropped lo*lo is 2^-24 of it.  The input comes as two fields (mie_split_exact),
 // the filter as two arrays of rows.  Per filter tap two instructions per K-slice:
 //     hi(input) x [hi(filter) | lo(filter)]  ->  N = 2 CB columns,      lo(input) x hi(filter)  ->  N = CB columns.
+// (The split of an operand is that of Markidis et al., 2018; sums kept outside the tensor core because it truncates, that of
+// Ootomo and Yokota, 2022.)
 // What keeps the result at fp32 level is where the sums are rounded: the tensor core truncates each time it adds to an
 // accumulator (1.7e-8 of the value per addition, always towards zero: 3e-5 after the 2400 additions of a 256-channel 5x5
 // layer).  So the first product starts from zero again with every segment of two to five taps (exact_shape()) and the epilogue
 // warps add the partial sums to registers, rounded to nearest, while the next segments run, low parts apart from high parts; the
 // second product is 2^-12 of the first and stays in its accumulator for the whole work item.
 // Error against a float64 convolution over that of the CUDA-core FP32 kernel: 0.68 to 0.95 for the first layers of the networks
-// on their event inputs, 0.3 to 0.9 for normal and for rectified inputs from a reduction (cin * k * k) of 72 on.  It is larger only
+// on their event inputs, 0.3 to 1.0 for normal and for rectified inputs from a reduction (cin * k * k) of 72 on.  It is larger only
 // where few products meet, since the two parts leave 1e-7 of a value however short its sum: 1.2 to 1.6 for a reduction of 18, 1.1
 // to 2.2 where isolated pixels are active and cin is below 48; and up to 1.4 where every product is positive.
 // Epilogue: reservoir = conv + bias (+ addend), output = f(reservoir), every pixel of a listed tile marked.

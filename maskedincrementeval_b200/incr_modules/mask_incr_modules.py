@@ -274,7 +274,7 @@ class _PreparedCall:
     the activation's function, state buffers and threshold, the input's geometry and the address of its tile words.  It holds
     every buffer that its argument block points to, but for the input."""
     __slots__ = ("activation", "epoch", "options", "precision", "op", "weight", "weight_key", "reservoir", "reservoir_ptr", "emitted",
-                 "threshold", "shape", "stride", "device", "mask_bits", "mask_ptr", "geometry", "plan", "args", "args_ref", "dilate", "tc_option",
+                 "threshold", "stride", "device", "mask_bits", "mask_ptr", "geometry", "plan", "args", "args_ref", "dilate", "tc_option",
                  "out", "input_threshold", "job", "packed")
 
     def __init__(self, conv, activation, plan, d, mask, derived, dilate, thresholded, packed):
@@ -288,7 +288,7 @@ class _PreparedCall:
         if activation is not None:
             self.reservoir, self.emitted, self.threshold = activation.in_res.reservoir, activation.emitted, activation.threshold
             self.reservoir_ptr = self.reservoir.data_ptr()
-        self.shape, self.stride, self.device = d.shape, d.stride(), d.device
+        self.stride, self.device = d.stride(), d.device
         self.geometry = (mask.n, mask.h, mask.w)
         self.mask_bits = mask.bits if derived else None      # the tile words this call derives from the delta itself
         self.mask_ptr = mask.bits.data_ptr()
@@ -301,11 +301,11 @@ class _PreparedCall:
         self.out = (plan.out, plan.mask)
 
     def run(self, conv, x_incr):
-        """The call's result, or None when it has to be decided anew."""
+        """The call's result, or None when it has to be decided anew.  (The record was found under the input's shape.)"""
         d, m = x_incr[0], x_incr[1]
         w = conv._parameters["weight"]
         plan = self.plan
-        if (self.epoch != config.epoch or self.options != nat.option_epoch[0] or d.shape != self.shape or d.stride() != self.stride
+        if (self.epoch != config.epoch or self.options != nat.option_epoch[0] or d.stride() != self.stride
                 or d.device != self.device or d.dtype is not torch.float32 or w is not self.weight or conv.precision != self.precision
                 or (w._version, w.data_ptr()) != self.weight_key or plan.needs_clear or plan.accum_target is not None or plan.tail is not self.job):
             return None

@@ -197,7 +197,7 @@ typedef struct mie_conv_args {
    * incr_modules/mask_incr_modules.py:182-196, 253-256): with `refresh` non-zero the input is a dense tensor, not a
    * delta: d = conv + bias (+ addend); *res = d (set, not advanced); out = f(d) (act == NONE: out = d); every pixel of
    * every listed tile is written and marked in the tile words.  Needs thr == 0 and no carry buffer; runs on the FP32
-   * kernel, or in fp32 precision on the tensor cores (`wpacked_exact`, `in_lo` below).  `bias` (cout floats, may be
+   * kernel, or in fp32 precision on the tensor cores (`wpacked_exact` below).  `bias` (cout floats, may be
    * null) is only read in this mode or when given. */
   const float *bias;
   int refresh;
@@ -229,11 +229,11 @@ typedef struct mie_conv_args {
    * mie_tiles_dilate launch from the entry point instead. */
   int own_tiles;
   void *own_scratch;
-  /* Dense evaluation (`refresh`) in fp32 precision on the tensor cores, both or neither: the filter packed by
-   * mie_pack_conv_weights_exact, and the second field of mie_split_exact (`in` is then its first one, same pixel stride).
+  /* Dense evaluation (`refresh`) in fp32 precision on the tensor cores: the filter packed by mie_pack_conv_weights_exact.
    * Taken for k in {3, 5, 7} without a second input when the fields are 16-byte aligned, but for stride 2 on a field one
-   * pixel wide or high (mie_conv_is_exact tells); else, and with either null, the FP32 kernel runs (on `in` as given: pass
-   * the unsplit field there).  Every output tile has to be listed. */
+   * pixel wide or high (mie_conv_is_exact tells); else, and with null, the FP32 kernel runs.  Every output tile has to be
+   * listed.  `in_lo` is no longer read (the kernel makes the parts of the input itself); `in` may be either the field or the
+   * first field of mie_split_exact. */
   const float *wpacked_exact;
   const float *in_lo;
 } mie_conv_args;
@@ -244,7 +244,8 @@ int mie_conv_step(const mie_conv_args *args /* host */, uint64_t *mask_bits, flo
                   void *stream);
 
 /* One dense evaluation of a layer in fp32 precision on the tensor cores in one call: mie_tiles_dilate as `dilate` describes,
- * mie_split_exact of the field x into args->in and args->in_lo, then mie_conv_tiles. */
+ * then mie_conv_tiles on the field x; where x or its pixel stride is not 16-byte aligned, on a copy of it (mie_pad_field) that
+ * is made in args->in with pixel stride args->in_ps. */
 int mie_conv_refresh_step(const mie_conv_args *args /* host */, const float *x, int64_t x_ps, const mie_tail_job *dilate /* host */,
                           void *stream);
 
@@ -265,10 +266,13 @@ int mie_conv_cluster_size(const mie_conv_args *args /* host */);
  * the padded extents the kernels assume. */
 int mie_conv_pack_dims(int cin, int cout, int k, int *cin_pad, int *cout_pad, int64_t *n_floats);
 
-/* Fp32 precision on the tensor cores: hi = v rounded to TF32, lo = v - hi rounded to TF32 (together v to 2^-24), for a dense
- * field of `pixels` pixels, and for a filter as [tap][32-channel chunk][hi rows | lo rows][32].  An infinite or NaN value
- * becomes lo with hi = 0, so that the three products (hi*hi, hi*lo, lo*hi) give what fp32 gives; only where an infinite input
- * meets an infinite filter entry is the result NaN. */
+/* Fp32 precision on the tensor cores.
+ * mie_pack_conv_weights_exact: the filter as two FP16 numbers per entry, scaled per output channel (to 2^-24 of the entry), with
+ * the inverse scales behind them; n_floats floats, 16-byte aligned.
+ * mie_pad_field: a dense field of `pixels` pixels with a pixel stride that the tensor cores' loads can follow (out_ps a
+ * multiple of 4, >= C rounded up to 4, out 16-byte aligned; channels up to the next multiple of 4 are zero).
+ * mie_split_exact: the same into hi, and zeros into lo (the form in which callers of earlier versions pass the input). */
+int mie_pad_field(const float *in, int64_t in_ps, int C, int64_t pixels, float *out, int64_t out_ps, void *stream);
 int mie_split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, void *stream);
 int mie_conv_pack_dims_exact(int cin, int cout, int k, int64_t *n_floats /* host */);
 int mie_pack_conv_weights_exact(const float *w_oihw, int cout, int cin, int k, float *wpacked, void *stream);

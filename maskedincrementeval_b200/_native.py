@@ -78,6 +78,7 @@ SIGNATURES = {
     "mie_conv_refresh_step": (_i, [C.POINTER(ConvArgs), _vp, _i64, _vp, _vp]),
     "mie_conv_step": (_i, [C.POINTER(ConvArgs), _vp, _f, _vp, _vp]),
     "mie_conv_is_exact": (_i, [C.POINTER(ConvArgs)]),
+    "mie_pad_field": (_i, [_vp, _i64, _i, _i64, _vp, _i64, _vp]),
     "mie_split_exact": (_i, [_vp, _i64, _i, _i64, _vp, _vp, _i64, _vp]),
     "mie_conv_pack_dims_exact": (_i, [_i, _i, _i, C.POINTER(_i64)]),
     "mie_pack_conv_weights_exact": (_i, [_vp, _i, _i, _i, _vp, _vp]),

@@ -19,9 +19,9 @@ namespace mie {
 bool tc_eligible(const mie_conv_args *a);
 int launch_conv_tc(const mie_conv_args *a, cudaStream_t st);
 bool exact_takes(const mie_conv_args *a);
-int launch_conv_exact(const mie_conv_args *a, cudaStream_t st);
+int launch_conv_exact(const mie_conv_args *a, const float *fw, int64_t fw_tap, int64_t fw_ci, cudaStream_t st);
 int pack_exact(const float *w, int cout, int cin, int k, int ihwo, float *wpacked, cudaStream_t st);
-int split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, const int32_t *counts, cudaStream_t st);
+int pad_field(const float *in, int64_t in_ps, int C, int64_t pixels, float *out, float *zero, int64_t out_ps, const int32_t *counts, cudaStream_t st);
 }  // namespace mie
 
 namespace {
@@ -716,7 +716,8 @@ extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
     b.own_tiles = 0;
     return mie_conv_tiles(&b, stream);
   }
-  if (exact_takes(a)) return tail_after_launch(launch_conv_exact(a, (cudaStream_t)stream), a->tail, true, stream);
+  if (exact_takes(a)) 
+    return tail_after_launch(launch_conv_exact(a, a->wpacked, (int64_t)a->cin_pad * a->cout_pad, a->cout_pad, (cudaStream_t)stream), a->tail, true, stream);
   if (tc_eligible(a)) return tail_after_launch(launch_conv_tc(a, (cudaStream_t)stream), a->tail, true, stream);
 
   ConvParams p;
@@ -774,12 +775,17 @@ extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
 }
 
 extern "C" int mie_conv_refresh_step(const mie_conv_args *a, const float *x, int64_t x_ps, const mie_tail_job *d, void *stream) {
-  if (!a || !d || !exact_takes(a)) return MIE_EINVAL;
+  if (!a || !d || !x) return MIE_EINVAL;
+  // a field that TMA can read is read where it lies
+  const bool direct = x_ps % 4 == 0 && aligned16(x);
+  mie_conv_args b = *a;
+  if (direct) { b.in = x; b.in_ps = x_ps; }
+  if (!b.in || !exact_takes(&b)) return MIE_EINVAL;
   int s = mie_tiles_dilate(d->in_bits, d->N, d->Hin, d->Win, d->Hout, d->Wout, d->k, d->stride, d->pad, d->union_bits, d->out_bits, d->list,
                            d->stale, d->counts, d->flags, stream);
-  if (s == MIE_OK)
-    s = mie_split_exact(x, x_ps, a->cin, (int64_t)a->n * a->hin * a->win, const_cast<float *>(a->in), const_cast<float *>(a->in_lo), a->in_ps, stream);
-  return s == MIE_OK ? mie_conv_tiles(a, stream) : s;
+  if (s == MIE_OK && !direct)
+    s = pad_field(x, x_ps, a->cin, (int64_t)a->n * a->hin * a->win, const_cast<float *>(b.in), nullptr, b.in_ps, nullptr, (cudaStream_t)stream);
+  return s == MIE_OK ? mie_conv_tiles(&b, stream) : s;
 }
 
 extern "C" int mie_conv_step(const mie_conv_args *a, uint64_t *mask_bits, float mask_thr, const mie_tail_job *dilate, void *stream) {
@@ -797,15 +803,14 @@ extern "C" int mie_conv_step(const mie_conv_args *a, uint64_t *mask_bits, float 
 // ---------------------------------------------------------------------------------------------
 namespace {
 struct IncWs {
-  size_t bits_in, bits_out, counts, list, stale, flags, wpacked, wexact, hi, lo, total;
-  int cp;      // channels of the split input
+  size_t bits_in, bits_out, counts, list, stale, flags, wpacked, wexact, copy, total;
+  int cp;      // channels of the input's copy, where it needs one
 };
 // fp32 precision on the tensor cores, for deltas of 48 channels or more: with fewer, the few products that meet at an isolated
 // active pixel leave the FP32 kernel the smaller error (5 channels 9e-8 against 5e-8, 16 1.0e-7 / 8e-8, 32 1.3e-7 / 1.1e-7; 48
 // 1.24e-7 / 1.26e-7, 64 1.3e-7 / 1.5e-7, and at 5 % activity 64 1.4e-7 / 2.0e-7).  It is faster from a single active blob to full
-// activity, although the split is a pass over the whole field: 64 -> 64 channels at 480x640, blobs of 16x16 pixels, one blob / 0.5 % /
-// 30 % / all active 87 / 88 / 167 / 193 us against 140 / 142 / 575 / 729.  A silent step makes no parts (split_exact): 40 us
-// against 37.
+// activity: 64 -> 64 channels at 480x640, blobs of 16x16 pixels, one blob / 0.5 % / 30 % / all active 87 / 88 / 167 / 193 us against
+// 140 / 142 / 575 / 729 when the input was still split by a pass of its own.
 bool inc_exact(int cin, int cout, int k) { return k >= 3 && cout % 4 == 0 && cin >= 48; }
 IncWs inc_layout(int N, int cin, int H, int W, int cout, int k, int stride) {
   const int pad = k / 2;
@@ -823,14 +828,14 @@ IncWs inc_layout(int N, int cin, int H, int W, int cout, int k, int stride) {
   int cp, op; int64_t nf;
   mie_conv_pack_dims(cin, cout, k, &cp, &op, &nf);
   w.wpacked = o; o += up((size_t)nf * 4);
-  w.wexact = w.hi = w.lo = o;
+  w.wexact = w.copy = o;
   w.cp = (cin + 3) / 4 * 4;
   if (inc_exact(cin, cout, k)) {
     int64_t ne;
     mie_conv_pack_dims_exact(cin, cout, k, &ne);
     o += up((size_t)ne * 4);
-    w.hi = o; o += up((size_t)N * H * W * w.cp * 4);
-    w.lo = o; o += up((size_t)N * H * W * w.cp * 4);
+    w.copy = o;
+    if (cin % 4) o += up((size_t)N * H * W * w.cp * 4);
   }
   w.total = o;
   return w;
@@ -895,9 +900,10 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   a.out = out_incr; a.out_ps = cout; a.out_bits = bits_out;
   a.act = MIE_ACT_NONE; a.thr = 0.0f;
   mie_conv_args x = a;       // without bias and activation a dense evaluation is the plain convolution of the listed tiles
-  float *wx = reinterpret_cast<float *>(ws + L.wexact), *hi = reinterpret_cast<float *>(ws + L.hi), *lo = reinterpret_cast<float *>(ws + L.lo);
+  float *wx = reinterpret_cast<float *>(ws + L.wexact), *copy = reinterpret_cast<float *>(ws + L.copy);
   x.refresh = 1;
-  x.in = hi; x.in_lo = lo; x.in_ps = L.cp; x.wpacked_exact = wx;
+  x.wpacked_exact = wx;
+  if (cin % 4) { x.in = copy; x.in_ps = L.cp; }
   const bool exact = inc_exact(cin, cout, k) && exact_takes(&x);
   if (exact) {
     if ((s = pack_exact(filter, cout, cin, k, 1, wx, st)) != MIE_OK) return s;
@@ -909,6 +915,7 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   }
   s = mie_tiles_dilate(bits_in, N, H, W, Ho, Wo, k, stride, pad, nullptr, nullptr, list, nullptr, counts, flags, stream);
   if (s != MIE_OK) return s;
-  if (exact && (s = split_exact(x_incr, cin, cin, (int64_t)N * H * W, hi, lo, L.cp, counts, st)) != MIE_OK) return s;
-  return mie_conv_tiles(exact ? &x : &a, stream);
+  if (!exact) return mie_conv_tiles(&a, stream);
+  if (cin % 4 && (s = pad_field(x_incr, cin, cin, (int64_t)N * H * W, copy, nullptr, L.cp, counts, st)) != MIE_OK) return s;
+  return launch_conv_exact(&x, filter, cout, (int64_t)k * k * cout, st);
 }

@@ -1,21 +1,26 @@
 // Dense evaluation (the refresh pass) in fp32 precision on the tensor cores, on CTA pairs like mie_conv_pair.cu.
 //
-// Every operand is two TF32 numbers, hi = round(v) and lo = round(v - hi) (round to nearest: together they hold v to 2^-24),
-// and a product is hi*hi + hi*lo + lo*hi; the dropped lo*lo is 2^-24 of it.  The input comes as two fields (mie_split_exact),
-// the filter as two arrays of rows.  Per filter tap two instructions per K-slice:
+// Every operand is two FP16 numbers with a common power-of-two scale (mie_pair.cuh), together the fp32 value to 2^-24, and a
+// product is hi*hi + hi*lo + lo*hi; the dropped lo*lo is 2^-24 of it.  The halo arrives as fp32 and is split in shared memory by
+// eight warps of its block, in place; the filter is packed as two arrays of rows.  Per filter tap two instructions per
+// K-slice of 16 channels:
 //     hi(input) x [hi(filter) | lo(filter)]  ->  N = 2 CB columns,      lo(input) x hi(filter)  ->  N = CB columns.
-// (The split of an operand is that of Markidis et al., 2018; sums kept outside the tensor core because it truncates, that of
+// With two TF32 numbers per operand, which is what stood here before, an instruction takes 8 channels from the same 32 bytes,
+// the input had to be split by a pass of its own (one read and two writes of every layer's input through HBM) and twice the operand
+// bytes crossed L2: eight E2Depth streams 480x640 13.5 ms, now 9.2.
+// (Splitting an operand: Markidis et al., 2018; scaled FP16 parts, and sums kept outside the tensor core because it truncates:
 // Ootomo and Yokota, 2022.)
 // What keeps the result at fp32 level is where the sums are rounded: the tensor core truncates each time it adds to an
-// accumulator (1.7e-8 of the value per addition, always towards zero: 3e-5 after the 2400 additions of a 256-channel 5x5
-// layer).  So the first product starts from zero again with every segment of two to five taps (exact_shape()) and the epilogue
-// warps add the partial sums to registers, rounded to nearest, while the next segments run, low parts apart from high parts; the
-// second product is 2^-12 of the first and stays in its accumulator for the whole work item.
-// Error against a float64 convolution over that of the CUDA-core FP32 kernel: 0.68 to 0.95 for the first layers of the networks
-// on their event inputs, 0.3 to 1.0 for normal and for rectified inputs from a reduction (cin * k * k) of 72 on.  It is larger only
-// where few products meet, since the two parts leave 1e-7 of a value however short its sum: 1.2 to 1.6 for a reduction of 18, 1.1
-// to 2.2 where isolated pixels are active and cin is below 48; and up to 1.4 where every product is positive.
+// accumulator.  So the sums start from zero again with every segment of taps, which is a stage of the filter ring, and the epilogue
+// warps add the segments to registers, rounded to nearest, while the next ones run.  Error against a float64 convolution over
+// that of the CUDA-core FP32 kernel: 0.3 to 1.0 for normal and rectified inputs from a reduction (cin * k * k) of 72 on; larger only
+// where few products meet, since the two parts leave 1e-7 of a value however short its sum: 1.2 to 1.5 for a reduction of 18, 1.0
+// to 2.2 at isolated active pixels with cin below 32.
+// What bounds it: operand reads and everything else that goes through shared memory (per tap and 32 channels, blocks of 64: 172 clocks
+// of its port for the instructions, which take 214 in the tensor core, 32 for the filter arriving, 35 to 70 for the
+// halo arriving and being split), then the epilogue's slabs on layers of few units (a chunk of a view) per item.
 // Epilogue: reservoir = conv + bias (+ addend), output = f(reservoir), every pixel of a listed tile marked.
+#include <algorithm>
 #include "mie_pair.cuh"
 
 using namespace mie;
@@ -23,142 +28,152 @@ using namespace mie;
 namespace mie {
 namespace {
 
-constexpr int EXACT_THREADS = 384;
+constexpr int EXACT_THREADS = 384 + 32 * SPLIT_WARPS;
 constexpr int EXACT_MAX_STAGES = 8;
 constexpr int EXACT_MAX_HALOS = 4;
 
 struct ExactParams {
+  const float *in; int64_t in_ps; int hin, win, k, stride, pad;      // read by the FP32 fallback only, like the filter below
+  const float *fw; int64_t fw_tap, fw_ci; int fw_vec;                // filter entry (tap, ci, co) at fw[tap * fw_tap + ci * fw_ci + co]
+  const float *winv;                                                 // inverse scale of every output channel's filter; NaN: fallback
   int cin, cout, cout_pad, n_chunks, n, hout, wout;
   const int32_t *list; int32_t *counts; int max_tiles;
   float *out; int64_t out_ps; unsigned int *out_bits32;
   int act; float *res; int64_t res_ps; const float *addend; int64_t addend_ps; const float *bias;
-  int cb, stages, halos, tps, wp;   // tps: taps per ring stage
-  int seg;     // taps per segment of the first product's sum
+  int cb, stages, halos, wp;
+  int tps;     // taps per ring stage, which is a segment of the sums
+  int segs;    // segment accumulators
   unsigned spin_limit;
   int withhold_loads;      // self-test: the producers issue nothing, so the first wait runs out (MIE_OPT_TC_WITHHOLD_LOADS)
   mie_tail_job tail;
   PairTaps t;
 };
 struct ExactMaps {
-  CUtensorMap hi[4], lo[4], w, out, res;
+  CUtensorMap in[4], w, out, res;
 };
 
-// acc[i] += column i (of n = 16 or 32) at taddr, + column i at taddr2: all loads in flight before the first addition
 __device__ __forceinline__ void tmem_ld16_async(unsigned taddr, unsigned *r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
                  "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                : "r"(taddr));
 }
+// acc[i] += inv * (hi[i] + 2^-11 (mid[i] + low[i])): the columns of a segment's three products, 16 at a time
 template <int N>
-__device__ __forceinline__ void tmem_add(unsigned taddr, float *acc) {
-  unsigned r[N];
+__device__ __forceinline__ void tmem_add_split(unsigned hi, unsigned mid, unsigned low, float inv, float *acc) {
 #pragma unroll
-  for (int g = 0; g < N; g += 16) tmem_ld16_async(taddr + g, r + g);
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  for (int g = 0; g < N; g += 16) {
+    unsigned a[16], b[16], c[16];
+    tmem_ld16_async(hi + g, a);
+    tmem_ld16_async(mid + g, b);
+    tmem_ld16_async(low + g, c);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < N; ++i) acc[i] += __uint_as_float(r[i]);
+    for (int i = 0; i < 16; ++i)
+      acc[g + i] = fmaf(fmaf(__uint_as_float(b[i]) + __uint_as_float(c[i]), SPLIT_LO, __uint_as_float(a[i])), inv, acc[g + i]);
+  }
 }
 
-// Segment accumulators (2 CB columns each) beside the two item accumulators (CB each) in 512 columns: enough that the round
-// trip of a segment to the epilogue and back does not hold up the issuer.
-__host__ __device__ constexpr unsigned exact_segs(int cb) { return cb == 64 ? 3u : 6u; }
+// Segment accumulators in 512 columns, 3 CB each: [hi x hi | hi x lo] per epilogue set, then lo x hi.
+__host__ __device__ constexpr unsigned exact_segs(int cb) { return cb == 64 ? 2u : 5u; }
 
+// The MMA issuer.  A ring stage of the filter is a segment: one wait for its operands, its accumulator and (first stage) the
+// halo together, one commit for both the filter producer and the epilogue.  The issuing warp is what paces the kernel: the
+// instructions of a 3x3 chunk of 64 channels take 1930 clocks, a wait about 130 and a commit about 80 beside them.
+struct ExactIssue {
+  int bid, nblk, n_items, n_chunks, cin, tps, nviews;
+  unsigned tmem_base, a_base, b_base, row_bytes, halo_bytes, stage_bytes, stages, halos, segs, limit;
+};
 template <int CB>
-__device__ __forceinline__ void exact_issue(const ExactParams &p, int bid, int nblk, int n_items, unsigned tmem_base, unsigned a_base, unsigned b_base,
-    unsigned row_bytes, unsigned halo_bytes, unsigned tap_bytes, unsigned stage_bytes, unsigned long long *b_full, unsigned long long *b_empty,
-    unsigned long long *a_full, unsigned long long *a_empty, unsigned long long *seg_full, unsigned long long *seg_empty, unsigned long long *item_full,
-    unsigned long long *item_empty, volatile int *abort_flag) {
-  constexpr unsigned NSEG = exact_segs(CB), item_col = NSEG * 2u * CB;
-  const unsigned id0 = (make_idesc_tf32(0) & ~(31u << 24)) | (16u << 24);       // M = 256
-  const unsigned id_hi = id0 | ((unsigned)(2 * CB >> 3) << 17), id_lo = id0 | ((unsigned)(CB >> 3) << 17);
-  const unsigned long long b_tmpl = make_smem_desc(0), a_tmpl = make_smem_desc(0, row_bytes);
+__device__ __forceinline__ void exact_issue(const ExactIssue a, const PairTapTable &t, unsigned long long *b_full, unsigned long long *done,
+    unsigned long long *a_ready, unsigned long long *a_empty, unsigned long long *seg_empty, volatile int *abort_flag) {
+  constexpr unsigned tap_units = CB * 64 >> 4;
+  const unsigned id_hi = make_idesc_f16_pair(2 * CB), id_lo = make_idesc_f16_pair(CB);
+  const unsigned long long b_tmpl = make_smem_desc_64(0), a_tmpl = make_smem_desc(0, a.row_bytes);
   const unsigned long long b_hi = b_tmpl & 0xFFFFFFFF00000000ull, a_hi = a_tmpl & 0xFFFFFFFF00000000ull;
   const unsigned lo_flags = (unsigned)(b_tmpl & 0xFFFF0000ull);
-  const int nv = p.t.nviews;
-  unsigned bs = 0, bpar = 0, as = 0, apar = 0, item_idx = 0, seg = 0, seg_par = 1, stage_addr = b_base;
+  unsigned bs = 0, bpar = 0, as = 0, apar = 0, seg = 0, seg_par = 1, stage_addr = a.b_base;
 #pragma unroll 1
-  for (int item = bid; item < n_items; item += nblk, ++item_idx) {
-    const unsigned buf = item_idx & 1u;
-    if (item_idx >= 2 && !mbar_wait(&item_empty[buf], ((item_idx >> 1) - 1) & 1u, abort_flag, p.spin_limit)) return;
-    unsigned started = 0;
+  for (int item = a.bid; item < a.n_items; item += a.nblk) {
 #pragma unroll 1
-    for (int chunk = 0; chunk < p.n_chunks; ++chunk) {
-      const unsigned nks = (unsigned)min(4, (p.cin - chunk * 32 + 7) >> 3);
+    for (int chunk = 0; chunk < a.n_chunks; ++chunk) {
+      const unsigned nks = (unsigned)min(2, (a.cin - chunk * 32 + 15) >> 4);
 #pragma unroll 1
-      for (int v = 0; v < nv; ++v) {
-        if (!mbar_wait(&a_full[as], apar, abort_flag, p.spin_limit)) return;
-        const unsigned halo = lo_flags | ((a_base + as * halo_bytes) >> 4);
-        const int end = p.t.first[v + 1];
-        int in_seg = 0;          // taps in the current segment
+      for (int v = 0; v < a.nviews; ++v) {
+        const unsigned halo = lo_flags | ((a.a_base + as * a.halo_bytes) >> 4);
+        const int end = t.first[v + 1];
+        unsigned abar = smem_u32(&a_ready[as]), ap = apar;
 #pragma unroll 1
-        for (int i = p.t.first[v]; i < end; i += p.tps) {
-          const int nt = min(p.tps, end - i);
-          unsigned b_lo = lo_flags | (stage_addr >> 4);
-          if (!mbar_wait(&b_full[bs], bpar, abort_flag, p.spin_limit)) return;
+        for (int i = t.first[v]; i < end; i += a.tps) {
+          const int nt = min(a.tps, end - i);
+          unsigned b_lo = lo_flags | (stage_addr >> 4), off = (unsigned)t.off[i];
+          const unsigned d = a.tmem_base + seg * (3u * CB);
+          const unsigned bbar = smem_u32(&b_full[bs]);
+          if (!mbar_wait3(abar, ap, bbar, bpar, smem_u32(&seg_empty[seg]), seg_par, abort_flag, a.limit)) return;
           tc_fence_after();
-#pragma unroll 1
-          for (int k = 0; k < nt; ++k, b_lo += tap_bytes >> 4) {
-            if (!in_seg) {
-              if (!mbar_wait(&seg_empty[seg], seg_par, abort_flag, p.spin_limit)) return;
-              tc_fence_after();
-            }
-            pair_mma(tmem_base + seg * (2u * CB), a_hi | (halo + ((unsigned)p.t.off[i + k] * 8u)), b_hi | b_lo, id_hi, (unsigned)in_seg, nks);
-            if (++in_seg == p.seg || i + k + 1 == end) {
-              pair_commit(&seg_full[seg]);
-              in_seg = 0;
-              if (++seg == NSEG) { seg = 0; seg_par ^= 1u; }
-            }
+          for (int k = 0; k < nt; ++k, b_lo += tap_units) {
+            const unsigned a_lo = halo + off;
+            off = (unsigned)t.off[i + k + 1];     // the next tap's, while this one is issued (the table has a spare entry)
+            pair_mma_split(d, d + 2u * CB, a_hi | a_lo, b_hi | b_lo, id_hi, id_lo, (unsigned)k, nks);
           }
-          pair_commit(&b_empty[bs]);
-          stage_addr += stage_bytes;
-          if (++bs == (unsigned)p.stages) { bs = 0; bpar ^= 1u; stage_addr = b_base; }
+          pair_commit(&done[bs]);
+          if (++seg == a.segs) { seg = 0; seg_par ^= 1u; }
+          stage_addr += a.stage_bytes;
+          if (++bs == a.stages) { bs = 0; bpar ^= 1u; stage_addr = a.b_base; }
+          abar = smem_u32(&b_full[bs]); ap = bpar;      // further stages of the unit: the halo is there
         }
         pair_commit(&a_empty[as]);
-        if (++as == (unsigned)p.halos) { as = 0; apar ^= 1u; }
-      }
-#pragma unroll 1
-      for (int v = 0; v < nv; ++v) {
-        if (!mbar_wait(&a_full[as], apar, abort_flag, p.spin_limit)) return;
-        const unsigned halo = lo_flags | ((a_base + as * halo_bytes) >> 4);
-        const int end = p.t.first[v + 1];
-#pragma unroll 1
-        for (int i = p.t.first[v]; i < end; i += p.tps) {
-          const int nt = min(p.tps, end - i);
-          unsigned b_lo = lo_flags | (stage_addr >> 4);
-          if (!mbar_wait(&b_full[bs], bpar, abort_flag, p.spin_limit)) return;
-          tc_fence_after();
-          const unsigned d = tmem_base + item_col + buf * CB;
-#pragma unroll 1
-          for (int k = 0; k < nt; ++k, b_lo += tap_bytes >> 4) {
-            pair_mma(d, a_hi | (halo + ((unsigned)p.t.off[i + k] * 8u)), b_hi | b_lo, id_lo, started, nks);
-            started = 1u;
-          }
-          pair_commit(&b_empty[bs]);
-          stage_addr += stage_bytes;
-          if (++bs == (unsigned)p.stages) { bs = 0; bpar ^= 1u; stage_addr = b_base; }
-        }
-        pair_commit(&a_empty[as]);
-        if (++as == (unsigned)p.halos) { as = 0; apar ^= 1u; }
+        if (++as == a.halos) { as = 0; apar ^= 1u; }
       }
     }
-    pair_commit(&item_full[buf]);
+  }
+}
+
+// One pixel's channels [co, co + HW) with FP32 instructions, for what two FP16 parts cannot hold (SplitShared, `winv`): the same sums as
+// the FP32 kernel's, padding multiplied as zeros like there.  Bounded by its loads (about 0.5 ms for an item of 256 channels and 5x5
+// taps), which no finite field of ordinary values comes to.
+template <int HW>
+__device__ __noinline__ void exact_fp32_quad(const ExactParams &p, int n, int oy, int ox, int c, float4 &out) {
+  out = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+  for (int tap = 0; tap < p.k * p.k; ++tap) {
+    const int iy = oy * p.stride - p.pad + tap / p.k, ix = ox * p.stride - p.pad + tap % p.k;
+    const bool in = iy >= 0 && iy < p.hin && ix >= 0 && ix < p.win;
+    const float *x = p.in + (in ? ((int64_t)(n * p.hin + iy) * p.win + ix) * p.in_ps : 0), *w = p.fw + tap * p.fw_tap + c;
+#pragma unroll 4
+    for (int ci = 0; ci < p.cin; ++ci, w += p.fw_ci) {
+      const float xv = in ? __ldg(x + ci) : 0.0f;
+      const float4 f = p.fw_vec ? __ldg(reinterpret_cast<const float4 *>(w)) : make_float4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+      out.x = fmaf(xv, f.x, out.x); out.y = fmaf(xv, f.y, out.y); out.z = fmaf(xv, f.z, out.z); out.w = fmaf(xv, f.w, out.w);
+    }
+  }
+}
+template <int HW>
+__device__ __forceinline__ void exact_fp32(const ExactParams &p, int n, int oy, int ox, bool valid, int co, float *acc) {
+#pragma unroll
+  for (int h = 0; h < HW / 4; ++h) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (valid && co + 4 * h < p.cout) exact_fp32_quad<HW>(p, n, oy, ox, co + 4 * h, v);
+    acc[4 * h] = v.x; acc[4 * h + 1] = v.y; acc[4 * h + 2] = v.z; acc[4 * h + 3] = v.w;
   }
 }
 
 // HW: channels per epilogue set (CB = 2 HW channels per block)
 template <int HW>
 __global__ void __launch_bounds__(EXACT_THREADS, 1)
-conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
+conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__ ExactMaps maps) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int CB = 2 * HW;
-  constexpr unsigned half_bytes = HW * 128u, tap_bytes = 2u * half_bytes;   // this block's rows of one tap: [hi | lo] of its half of the channels
+  constexpr unsigned half_bytes = HW * 64u, tap_bytes = 2u * half_bytes;   // this block's rows of one tap: [hi | lo] of its half of the channels
   const unsigned row_bytes = (unsigned)p.wp * 128u;
   const unsigned halo_bytes = ((unsigned)p.wp * 2u * row_bytes + 1023u) & ~1023u;
   const unsigned stage_bytes = tap_bytes * (unsigned)p.tps;
-  __shared__ unsigned long long b_full[EXACT_MAX_STAGES], b_empty[EXACT_MAX_STAGES], a_full[EXACT_MAX_HALOS], a_empty[EXACT_MAX_HALOS],
-      seg_full[6], seg_empty[6], item_full[2], item_empty[2];
+  __shared__ unsigned long long b_full[EXACT_MAX_STAGES], done[EXACT_MAX_STAGES], a_full[EXACT_MAX_HALOS], a_ready[EXACT_MAX_HALOS],
+      a_empty[EXACT_MAX_HALOS], seg_empty[5];
+  __shared__ SplitShared s_split;
+  __shared__ PairTapTable s_tap;
+  __shared__ float4 s_col[2][2][HW / 4];      // per epilogue set: inverse scales and biases of its channels
   __shared__ unsigned s_tmem_base;
   __shared__ int s_abort;
 
@@ -167,15 +182,19 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
   const int bid = (int)(blockIdx.x >> 1), nblk = (int)(gridDim.x >> 1);
   const int THo = (p.hout + 7) >> 3, TWo = (p.wout + 7) >> 3;
   const int ntiles_total = p.n * THo * TWo;
-  constexpr unsigned NSEG = exact_segs(CB), item_col = NSEG * 2u * CB, tmem_cols = 512u;
+  constexpr unsigned tmem_cols = 512u;
 
   if (tid == 0) {
-    for (int s = 0; s < p.stages; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
-    for (int s = 0; s < p.halos; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_empty[s], 1); }
-    for (unsigned b = 0; b < NSEG; ++b) { mbar_init(&seg_full[b], 1); mbar_init(&seg_empty[b], 16); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&item_full[b], 1); mbar_init(&item_empty[b], 16); }
+    for (int s = 0; s < p.stages; ++s) { mbar_init(&b_full[s], 1); mbar_init(&done[s], 1); }
+    for (int s = 0; s < p.halos; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_ready[s], 2 * SPLIT_WARPS); mbar_init(&a_empty[s], 1); }
+    for (int b = 0; b < p.segs; ++b) mbar_init(&seg_empty[b], 16);
+    for (unsigned u = 0; u < SPLIT_RING; ++u) mbar_init(&s_split.inv_full[u], 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 3) {
+    for (int i = lane; i < 50; i += 32) s_tap.off[i] = i < 49 ? (int)p.t.off[i] * 8 : 0;
+    if (lane < 5) s_tap.first[lane] = p.t.first[lane];
   }
   if (warp == 2) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(tmem_cols) : "memory");
@@ -194,37 +213,35 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
   const unsigned b_base = smem_u32(smem), a_base = b_base + (((unsigned)p.stages * stage_bytes + 1023u) & ~1023u);
   const int nv = p.t.nviews;
 
-  // units of a chunk: the high parts of the views, then the low parts
-  const PairWork work = {bid, nblk, n_items, n_cblk, p.n_chunks, 2 * nv, crank, p.spin_limit, p.withhold_loads};
+  const PairWork work = {bid, nblk, n_items, n_cblk, p.n_chunks, nv, crank, p.spin_limit, p.withhold_loads};
+  const PairRing halos = {a_full, a_empty, a_base, halo_bytes, (unsigned)p.halos};
   if (warp == 0) {
     // =========================== halo producer ===========================
-    const PairRing ring = {a_full, a_empty, a_base, halo_bytes, (unsigned)p.halos};
-    pair_produce_halos(work, ring, p.t, p.wp, row_bytes, p.list, n_active, ntiles_total, TWo, THo, p.counts, &s_abort, [&](int u, int &v) {
-      v = u < nv ? u : u - nv;
-      return u < nv ? &maps.hi[v] : &maps.lo[v];
-    });
+    pair_produce_halos<true>(work, halos, p.t, p.wp, row_bytes, p.list, n_active, ntiles_total, TWo, THo, p.counts, &s_abort,
+                             [&](int u, int &v) { v = u; return &maps.in[u]; });
   } else if (warp == 1) {
-    // =========================== filter producer: hi and lo rows beside the high part of the input, hi rows beside the low part ===========================
-    const PairRing ring = {b_full, b_empty, b_base, stage_bytes, (unsigned)p.stages};
-    pair_produce_filter(work, ring, p.t, p.tps, tap_bytes, (int)crank * HW, CB, &s_abort, [&](int u) { return u < nv ? u : u - nv; },
-                        [&](int u) { return 2u * (u < nv ? tap_bytes : half_bytes); },
-                        [&](int u, int tap, unsigned dst, unsigned bar, int row, int chunk) {
+    // =========================== filter producer: hi and lo rows of a tap ===========================
+    const PairRing ring = {b_full, done, b_base, stage_bytes, (unsigned)p.stages};
+    pair_produce_filter(work, ring, p.t, p.tps, tap_bytes, (int)crank * HW, CB, &s_abort, [](int u) { return u; }, [&](int) { return 2u * tap_bytes; },
+                        [&](int, int tap, unsigned dst, unsigned bar, int row, int chunk) {
                           tma_load_4d_pair(dst, &maps.w, bar, 0, row, chunk, tap);
-                          if (u < nv) tma_load_4d_pair(dst + half_bytes, &maps.w, bar, 0, p.cout_pad + row, chunk, tap);
+                          tma_load_4d_pair(dst + half_bytes, &maps.w, bar, 0, p.cout_pad + row, chunk, tap);
                         });
   } else if (warp == 2) {
     // =========================== MMA issuer (first block of the pair) ===========================
     if (crank == 0u) {
-      exact_issue<CB>(p, bid, nblk, n_items, tmem_base, a_base, b_base, row_bytes, halo_bytes, tap_bytes, stage_bytes, b_full, b_empty, a_full, a_empty, seg_full, seg_empty, item_full, item_empty, &s_abort);
+      const ExactIssue a = {bid, nblk, n_items, p.n_chunks, p.cin, p.tps, nv, tmem_base, a_base, b_base, row_bytes, halo_bytes, stage_bytes, (unsigned)p.stages,
+                            (unsigned)p.halos, (unsigned)p.segs, p.spin_limit};
+      exact_issue<CB>(a, s_tap, b_full, done, a_ready, a_empty, seg_empty, &s_abort);
     }
+  } else if (warp >= 12) {
+    // =========================== halos as two FP16 parts ===========================
+    pair_split_halos(work, halos, a_ready, 2 * p.wp * p.wp, p.wp, n_active, tid - 384, s_split, &s_abort);
   } else if (warp >= 4) {
     // =========================== epilogue: set `set` takes channels [set * HW, set * HW + HW) of the block ===========================
     const int q = warp & 3, set = (warp - 4) >> 2;
     const int slot = (lane >> 3) & 1, prow = 2 * q + (lane >> 4), pcol = lane & 7;
     const unsigned lane_base = tmem_base + ((unsigned)(q * 32) << 16);
-    int segs_per_chunk = 0;
-    for (int v = 0; v < nv; ++v) segs_per_chunk += (p.t.first[v + 1] - p.t.first[v] + p.seg - 1) / p.seg;
-    const int segs = segs_per_chunk * p.n_chunks;
     // slabs of this set: output, then reservoir; 128 rows of HW channels, 16-byte pieces swizzled as TMA does for rows of
     // 128 bytes (piece ^ (row & 7)) or 64 bytes (piece ^ (row / 2 & 3))
     constexpr unsigned SLAB = 128u * HW * 4u;
@@ -232,41 +249,43 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
     const unsigned slab = a_base + (unsigned)p.halos * halo_bytes + (unsigned)set * (p.act != MIE_ACT_NONE ? 2u : 1u) * SLAB;
     const unsigned out_row = slab + (unsigned)row * (HW * 4u), res_row = out_row + SLAB;
     const bool chief = q == 0 && elect_one();
-    unsigned item_idx = 0, seg = 0, seg_par = 0;
+    unsigned seg = 0, stage = 0, stage_par = 0, unit = 0;
     bool ok = true;
-    for (int item = bid; item < n_items && ok; item += nblk, ++item_idx) {
-      const int quad = item / n_cblk, cb = item - quad * n_cblk;
-      const unsigned buf = item_idx & 1u;
-      const int e = 4 * quad + 2 * (int)crank + slot;
-      int t = e < n_active ? p.list[e] : -1;
-      if (t >= ntiles_total) t = -1;
+    for (int item = bid; item < n_items && ok; item += nblk) {
+      // What the end of the item needs from global memory is asked for here and first looked at behind the segments: with a chain of
+      // loads at the end (list, scales, biases, list again) it took 5000 clocks, in which no segment is taken and the issuer stands
+      // still.
+      const int quad = item / n_cblk, cb = item - quad * n_cblk, co = cb * CB + set * HW;
+      const int e = 4 * quad + 2 * (int)crank + slot, at_col = q * 32 + lane;
+      const int listed = e < n_active ? p.list[e] : -1;
+      const float col = at_col < HW ? __ldg(p.winv + co + at_col) : (at_col < 2 * HW && p.bias && co + at_col - HW < p.cout) ? __ldg(p.bias + co + at_col - HW) : 0.0f;
+      float acc[HW];
+      bool wide = false;
+#pragma unroll
+      for (int i = 0; i < HW; ++i) acc[i] = 0.0f;
+      for (int cu = 0; cu < p.n_chunks * nv && ok; ++cu, ++unit) {
+        const int v = nv == 1 ? 0 : cu % nv;
+        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&s_split.inv_full[unit % SPLIT_RING], (unit / SPLIT_RING) & 1u, &s_abort, p.spin_limit)))) break;
+        const float inv = s_split.inv[unit % SPLIT_RING];
+        for (int left = p.t.first[v + 1] - p.t.first[v]; left > 0; left -= p.tps) {
+          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&done[stage], stage_par, &s_abort, p.spin_limit)))) break;
+          tc_fence_after();
+          const unsigned c = lane_base + seg * (3u * CB), own = c + (unsigned)set * CB;      // [hi | mid] columns of this set's channels
+          tmem_add_split<HW>(own, own + HW, c + 2u * CB + (unsigned)set * HW, inv, acc);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&seg_empty[seg]), 0));
+          if (++seg == (unsigned)p.segs) seg = 0;
+          if (++stage == (unsigned)p.stages) { stage = 0; stage_par ^= 1u; }
+        }
+        wide |= inv != inv;
+      }
+      const int t = listed < ntiles_total ? listed : -1;
       const int tx = (t >= 0) ? (t % TWo) * 8 : 0, ty = (t >= 0) ? ((t / TWo) % THo) * 8 : 0, n = (t >= 0) ? t / (TWo * THo) : 0;
       const bool valid = t >= 0 && ty + prow < p.hout && tx + pcol < p.wout;
       const int64_t pix = valid ? (int64_t)(n * p.hout + ty + prow) * p.wout + tx + pcol : 0;
-      float acc[HW], low[HW];       // the low products are summed apart, so that the large sum is rounded once a segment
-#pragma unroll
-      for (int i = 0; i < HW; ++i) acc[i] = low[i] = 0.0f;
-      for (int s = 0; s < segs; ++s) {
-        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&seg_full[seg], seg_par, &s_abort, p.spin_limit)))) break;
-        tc_fence_after();
-        const unsigned c = lane_base + seg * (2u * CB) + (unsigned)set * CB;     // [hi | lo] columns of this set's channels
-        tmem_add<HW>(c, acc);
-        tmem_add<HW>(c + HW, low);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&seg_empty[seg]), 0));
-        if (++seg == NSEG) { seg = 0; seg_par ^= 1u; }
-      }
-      // a warp whose wait gave up goes on to the barrier of its set, where the four of them leave together
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&item_full[buf], (item_idx >> 1) & 1u, &s_abort, p.spin_limit));
-      tc_fence_after();
-      if (ok) tmem_add<HW>(lane_base + item_col + buf * CB + (unsigned)(set * HW), low);
-#pragma unroll
-      for (int i = 0; i < HW; ++i) acc[i] += low[i];
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&item_empty[buf]), 0));
-      const int co = cb * CB + set * HW;
+      if (at_col < 2 * HW) reinterpret_cast<float *>(s_col[set][at_col / HW])[at_col % HW] = col;
+      // a warp whose wait gave up goes on to the barrier of its set, where the four of them leave together;
       // the slabs are free once the previous item's stores have read them
       if (chief) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
       __syncwarp();
@@ -274,9 +293,16 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
       if (!ok) break;
 #pragma unroll
       for (int h = 0; h < HW / 4; ++h) {
+        const float4 f = lds4(smem_u32(&s_col[set][0][h]));
+        acc[4 * h] *= f.x; acc[4 * h + 1] *= f.y; acc[4 * h + 2] *= f.z; acc[4 * h + 3] *= f.w;
+        wide |= f.x != f.x || f.y != f.y || f.z != f.z || f.w != f.w;
+      }
+      if (wide) exact_fp32<HW>(p, n, ty + prow, tx + pcol, valid, co, acc);
+#pragma unroll
+      for (int h = 0; h < HW / 4; ++h) {
         const int c = co + 4 * h;
         float4 v = make_float4(acc[4 * h], acc[4 * h + 1], acc[4 * h + 2], acc[4 * h + 3]);
-        if (p.bias && c < p.cout) v = f4add(v, make_float4(__ldg(p.bias + c), __ldg(p.bias + c + 1), __ldg(p.bias + c + 2), __ldg(p.bias + c + 3)));
+        if (p.bias) v = f4add(v, lds4(smem_u32(&s_col[set][1][h])));
         if (p.addend && valid && c < p.cout) v = f4add(v, *reinterpret_cast<const float4 *>(p.addend + pix * p.addend_ps + c));
         const unsigned at = (unsigned)(h ^ sw) << 4;
         if (p.act != MIE_ACT_NONE) {
@@ -288,14 +314,17 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");
+      // the tiles of both slots lie in every warp (lanes 0 and 8)
+      const int t0 = __shfl_sync(0xffffffffu, t, 0), t1 = __shfl_sync(0xffffffffu, t, 8), x0 = __shfl_sync(0xffffffffu, tx, 0), x1 = __shfl_sync(0xffffffffu, tx, 8),
+                y0 = __shfl_sync(0xffffffffu, ty, 0), y1 = __shfl_sync(0xffffffffu, ty, 8), n0 = __shfl_sync(0xffffffffu, n, 0), n1 = __shfl_sync(0xffffffffu, n, 8);
       if (chief && co < p.cout) {
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const int es = 4 * quad + 2 * (int)crank + s, ts = es < n_active ? p.list[es] : -1;
-          if (ts < 0 || ts >= ntiles_total) continue;
-          const int x = (ts % TWo) * 8, y = ((ts / TWo) % THo) * 8, ns = ts / (TWo * THo);
-          tma_store_slab(slab + s * (SLAB / 2), &maps.out, co, x, y, ns);
-          if (p.act != MIE_ACT_NONE) tma_store_slab(slab + SLAB + s * (SLAB / 2), &maps.res, co, x, y, ns);
+        if (t0 >= 0) {
+          tma_store_slab(slab, &maps.out, co, x0, y0, n0);
+          if (p.act != MIE_ACT_NONE) tma_store_slab(slab + SLAB, &maps.res, co, x0, y0, n0);
+        }
+        if (t1 >= 0) {
+          tma_store_slab(slab + SLAB / 2, &maps.out, co, x1, y1, n1);
+          if (p.act != MIE_ACT_NONE) tma_store_slab(slab + SLAB + SLAB / 2, &maps.res, co, x1, y1, n1);
         }
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
@@ -328,41 +357,45 @@ conv_exact_kernel(const ExactParams p, const __grid_constant__ ExactMaps maps) {
 
 }  // namespace
 
+// Floats of a packed filter in front of its inverse scales.
+static inline int64_t exact_scales_at(int cin, int cout_pad, int k) { return (int64_t)k * k * divup(cin, 32) * 2 * cout_pad * 16; }
+
 // How a launch divides its columns and its shared memory; `stages` < 2: no split of it fits.
 struct ExactShape {
   PairTaps t;
-  int wp, cb, tps, stages, halos, seg;
+  int wp, cb, tps, stages, halos, segs;
   size_t smem;
 };
 static ExactShape exact_shape(const mie_conv_args *a) {
   ExactShape h;
   pair_make_taps(a->k, a->stride, a->pad, &h.t, &h.wp);
   const int quads = divup(a->max_tiles, 4), clusters_max = MIE_SM_COUNT / 2;
-  // 64 channels per block (144 clocks per K-slice and tap, both instructions) unless blocks of 32 (103) take fewer clocks over all
-  // rounds: 256 -> 64 and 32 channels, the slope from four to eight rounds at 1965 MHz for k = 5 (k = 3: 159 and 113; k = 7: 178 and 105)
+  // 64 channels per block unless blocks of 32, which take 0.75 of its time, need fewer rounds for it (5x5: 305 and 245 clocks per tap and
+  // 32 channels, 3x3 430 and 300)
   h.cb = 32;
   if (a->cout_pad % 64 == 0 &&
-      (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 144 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 103)
+      (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 100 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 75)
     h.cb = 64;
   const int halo_bytes = (h.wp * 2 * h.wp * 128 + 1023) & ~1023, slab_bytes = 2 * (a->act != MIE_ACT_NONE ? 2 : 1) * 128 * (h.cb / 2) * 4;
   const int budget = 222 * 1024 - slab_bytes;
-  // Fat stages: what the issuer and the producers spend per stage does not depend on its size.  Three of them where
-  // halo buffers can be spared for that, else two; a 7x7 filter's halos beside the slabs of a wide block leave room for
-  // two stages of three taps (still ahead of blocks of 32 channels with nine: 64 -> 64 on 2 x 256x336 366 against 436 us,
-  // on 104x104 46 against 56).
-  h.tps = h.cb == 32 ? 9 : 5;
+  // Taps of a segment: its truncation grows with its additions, one per 16 channels and tap, the FP32 kernel's rounding with the whole
+  // reduction.  The longest whose error is not above the FP32 kernel's, nor above that of the two TF32 parts that stood here, for
+  // rectified inputs (segments of 3 / 5 / 9 taps over the FP32 kernel's error: 125 products 0.84 / 0.91 / 1.16, 288 0.75 / 0.99 / 1.68, 576
+  // 0.53 / 0.70 / 1.22, 1152 0.40 / 0.52 / 0.88, 1600 0.36 / 0.47 / 0.71, 2304 0.29 / 0.36 / 0.60).
+  const int depth = a->cin * a->k * a->k, most = depth < 100 ? 2 : depth < 400 ? (a->cin > 16 ? 3 : 5) : depth < 1600 ? 5 : 9;
+  int taps = 0;
+  for (int v = 0; v < h.t.nviews; ++v) taps = std::max(taps, h.t.first[v + 1] - h.t.first[v]);
+  h.tps = divup(taps, divup(taps, most));
+  // Units of a single stage (3x3) need halo buffers more than stages: load, split and instructions of a unit are three links of a chain
+  // (res 256 -> 256: three halos and two stages 144 us, two and three 157).  Longer ones need the filter ahead (64 -> 32 5x5: 787 us with
+  // three halos and four stages, 939 with four and two).
+  const int ring = h.tps == taps ? 2 : 3;
   h.halos = EXACT_MAX_HALOS;
-  while (h.halos > 2 && budget - h.halos * halo_bytes < 3 * h.tps * h.cb * 128) --h.halos;
-  while (h.tps > 1 && budget - h.halos * halo_bytes < 2 * h.tps * h.cb * 128) --h.tps;
-  const int stage_bytes = h.tps * h.cb * 128;
-  h.stages = (budget - h.halos * halo_bytes) / stage_bytes;
-  if (h.stages > EXACT_MAX_STAGES) h.stages = EXACT_MAX_STAGES;
-  // A segment's truncation grows with its length, the FP32 kernel's rounding with the whole reduction: the longest segments that
-  // keep the error below that kernel's for rectified inputs (segments of 2 / 3 / 5 taps: 288 products 0.83 / 1.13 / 1.62 of its
-  // error, 576 0.63 / 0.85 / 1.21, 800 0.55 / 0.70 / 1.09, 1152 0.44 / 0.58 / 0.83).  Shorter ones cost time: a refresh of eight
-  // E2Depth streams 480x640 takes 14.3 / 13.6 / 13.4 ms with one length for all layers.
-  const int depth = a->cin * a->k * a->k;
-  h.seg = depth < 400 ? 2 : depth < 1152 ? 3 : 5;
+  while (h.halos > 2 && budget - h.halos * halo_bytes < ring * h.tps * h.cb * 64) --h.halos;
+  while (h.tps > 1 && budget - h.halos * halo_bytes < 2 * h.tps * h.cb * 64) --h.tps;
+  const int stage_bytes = h.tps * h.cb * 64;
+  h.stages = std::min((budget - h.halos * halo_bytes) / stage_bytes, EXACT_MAX_STAGES);
+  h.segs = std::min(h.stages, (int)exact_segs(h.cb));      // the epilogue learns of a segment from its stage's barrier
   h.smem = (size_t)((h.stages * stage_bytes + 1023) & ~1023) + (size_t)h.halos * halo_bytes + slab_bytes + 1024;
   return h;
 }
@@ -371,25 +404,29 @@ bool exact_takes(const mie_conv_args *a) {
   // a field one pixel wide or high has no odd columns or rows: that parity view of stride 2 would be empty, and a tensor map
   // cannot say so
   if (a->stride == 2 && (a->hin == 1 || a->win == 1)) return false;
-  return a->refresh && !a->head && a->wpacked_exact && a->in_lo && a->k >= 3 && a->k <= 7 && (a->k & 1) && (a->stride == 1 || a->stride == 2) && !a->in2 && !a->accum &&
-         a->in_ps % 4 == 0 && aligned16(a->in) && aligned16(a->in_lo) && aligned16(a->wpacked_exact) && a->cout % 4 == 0 && a->out_ps % 4 == 0 &&
+  return a->refresh && !a->head && a->wpacked_exact && a->k >= 3 && a->k <= 7 && (a->k & 1) && (a->stride == 1 || a->stride == 2) && !a->in2 && !a->accum &&
+         a->in_ps % 4 == 0 && aligned16(a->in) && aligned16(a->wpacked_exact) && a->cout % 4 == 0 && a->out_ps % 4 == 0 &&
          aligned16(a->out) && (!a->res || (a->res_ps % 4 == 0 && aligned16(a->res))) && (!a->addend || (a->addend_ps % 4 == 0 && aligned16(a->addend))) &&
          a->cout_pad % 32 == 0 && exact_shape(a).stages >= 2;
 }
 
-int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
+// fw: the filter in fp32, entry (tap, ci, co) at fw[tap * fw_tap + ci * fw_ci + co]
+int launch_conv_exact(const mie_conv_args *a, const float *fw, int64_t fw_tap, int64_t fw_ci, cudaStream_t st) {
   const ExactShape h = exact_shape(a);
   ExactParams p;
   memset(&p, 0, sizeof(p));
   p.spin_limit = g_opt_spin_limit;
   p.withhold_loads = g_opt_withhold_loads;
+  p.in = a->in; p.in_ps = a->in_ps; p.hin = a->hin; p.win = a->win; p.k = a->k; p.stride = a->stride; p.pad = a->pad;
+  p.fw = fw; p.fw_tap = fw_tap; p.fw_ci = fw_ci; p.fw_vec = aligned16(fw) && fw_tap % 4 == 0 && fw_ci % 4 == 0;
   p.cin = a->cin; p.cout = a->cout; p.cout_pad = a->cout_pad; p.n_chunks = divup(a->cin, 32);
+  p.winv = a->wpacked_exact + exact_scales_at(a->cin, a->cout_pad, a->k);
   p.n = a->n; p.hout = a->hout; p.wout = a->wout;
   p.list = a->list; p.counts = a->counts; p.max_tiles = a->max_tiles;
   p.out = a->out; p.out_ps = a->out_ps; p.out_bits32 = reinterpret_cast<unsigned int *>(a->out_bits);
   p.act = a->act; p.res = a->res; p.res_ps = a->res_ps; p.addend = a->addend; p.addend_ps = a->addend_ps; p.bias = a->bias;
   p.tail = tail_for_kernel(a->tail);
-  p.t = h.t; p.wp = h.wp; p.cb = h.cb; p.tps = h.tps; p.stages = h.stages; p.halos = h.halos; p.seg = h.seg;
+  p.t = h.t; p.wp = h.wp; p.cb = h.cb; p.tps = h.tps; p.stages = h.stages; p.halos = h.halos; p.segs = h.segs;
   const size_t smem = h.smem;
   const int quads = divup(a->max_tiles, 4), clusters_max = MIE_SM_COUNT / 2;
 
@@ -401,18 +438,15 @@ int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
     const int py = s == 2 ? v >> 1 : 0, px = s == 2 ? v & 1 : 0;
     const cuuint64_t dims[4] = {(cuuint64_t)a->cin, (cuuint64_t)((a->win - px + s - 1) / s), (cuuint64_t)((a->hin - py + s - 1) / s), (cuuint64_t)a->n};
     const cuuint64_t str[3] = {(cuuint64_t)a->in_ps * 4 * s, (cuuint64_t)a->win * a->in_ps * 4 * s, (cuuint64_t)a->hin * a->win * a->in_ps * 4};
-    const int64_t off = ((int64_t)py * a->win + px) * a->in_ps;
-    if (!tc_encode(&maps.hi[v], 4, a->in + off, dims, str, box_in, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !tc_encode(&maps.lo[v], 4, a->in_lo + off, dims, str, box_in, CU_TENSOR_MAP_SWIZZLE_128B))
-      return MIE_EINVAL;
+    if (!tc_encode(&maps.in[v], 4, a->in + ((int64_t)py * a->win + px) * a->in_ps, dims, str, box_in, CU_TENSOR_MAP_SWIZZLE_128B)) return MIE_EINVAL;
   }
   {
-    // [tap][chunk][hi rows | lo rows][32]
+    // [tap][chunk][hi rows | lo rows][32 FP16 = 16 floats]
     const cuuint64_t rows = 2 * (cuuint64_t)a->cout_pad, nch = (cuuint64_t)p.n_chunks;
-    const cuuint64_t dims[4] = {32, rows, nch, (cuuint64_t)(a->k * a->k)};
-    const cuuint64_t str[3] = {128, rows * 128, nch * rows * 128};
-    const cuuint32_t box_w[4] = {32, (cuuint32_t)(p.cb / 2), 1, 1};
-    if (!tc_encode(&maps.w, 4, a->wpacked_exact, dims, str, box_w, CU_TENSOR_MAP_SWIZZLE_128B)) return MIE_EINVAL;
+    const cuuint64_t dims[4] = {16, rows, nch, (cuuint64_t)(a->k * a->k)};
+    const cuuint64_t str[3] = {64, rows * 64, nch * rows * 64};
+    const cuuint32_t box_w[4] = {16, (cuuint32_t)(p.cb / 2), 1, 1};
+    if (!tc_encode(&maps.w, 4, a->wpacked_exact, dims, str, box_w, CU_TENSOR_MAP_SWIZZLE_64B)) return MIE_EINVAL;
   }
   {
     // epilogue slabs: half a block's channels of one tile
@@ -437,31 +471,11 @@ int launch_conv_exact(const mie_conv_args *a, cudaStream_t st) {
   return p.cb == 64 ? launch(conv_exact_kernel<32>, 1) : launch(conv_exact_kernel<16>, 0);
 }
 
-// Round to nearest TF32 (10 mantissa bits).
-__device__ __forceinline__ float round_tf32(float v) {
-  unsigned r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
-  return __uint_as_float(r);
-}
-// v as two TF32 numbers.  A finite v that would round up to infinity is truncated instead.  Infinity and NaN have no low part
-// (inf - inf), and infinity times the low part of the other operand has any sign: they become the low part themselves, which
-// meets nothing but the high part of the other operand, and give what fp32 gives.
-__device__ __forceinline__ void split_two_tf32(float v, float &hi, float &lo) {
-  if (!isfinite(v)) {
-    hi = 0.0f;
-    lo = isnan(v) ? __uint_as_float(0x7FC00000u) : v;     // (a NaN whose payload is in the bits that TF32 drops would read as infinity)
-    return;
-  }
-  hi = round_tf32(v);
-  if (isinf(hi)) hi = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
-  lo = round_tf32(v - hi);
-}
-
-// hi = round(v), lo = round(v - hi): one pass over a dense field, a thread per four channels of a pixel.  HBM bound: one read
-// and two writes at 5.6 to 6.0 TB/s on fields beyond the L2 (8 x 32 x 480x640: 167 us), 0.86 to 0.91 of a measured copy.
-// counts (may be null): the work list of the convolution that reads the parts; none are made where it lists no tile.
-__global__ void __launch_bounds__(256) split_exact_kernel(const float *__restrict__ in, int64_t in_ps, int C, int64_t pixels, float *__restrict__ hi,
-                                                          float *__restrict__ lo, int64_t out_ps, int quads, int vec, const int32_t *counts) {
+// A field with a pixel stride or an address that TMA cannot read (5 bins of a voxel grid) as one it can: one read and one write.
+// A thread per four channels of a pixel; counts (may be null): the work list of the convolution that reads the copy, nothing is
+// copied where it lists no tile.  zero (may be null): a second field of that layout, cleared.
+__global__ void __launch_bounds__(256) pad_field_kernel(const float *__restrict__ in, int64_t in_ps, int C, int64_t pixels, float *__restrict__ out,
+                                                        float *__restrict__ zero, int64_t out_ps, int quads, int vec, const int32_t *counts) {
   grid_dependency_wait();
   grid_dependency_trigger();
   if (counts && counts[0] == 0) return;
@@ -469,37 +483,61 @@ __global__ void __launch_bounds__(256) split_exact_kernel(const float *__restric
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t px = i / quads;
     const int c = (int)(i - px * quads) * 4;
-    float v[4];
+    float4 v;
     if (vec) {
-      const float4 x = *reinterpret_cast<const float4 *>(in + px * in_ps + c);
-      v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+      v = *reinterpret_cast<const float4 *>(in + px * in_ps + c);
     } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = c + j < C ? in[px * in_ps + c + j] : 0.0f;
+      const float *x = in + px * in_ps + c;
+      v = make_float4(x[0], c + 1 < C ? x[1] : 0.0f, c + 2 < C ? x[2] : 0.0f, c + 3 < C ? x[3] : 0.0f);
     }
-    float h[4], l[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) split_two_tf32(v[j], h[j], l[j]);
-    *reinterpret_cast<float4 *>(hi + px * out_ps + c) = make_float4(h[0], h[1], h[2], h[3]);
-    *reinterpret_cast<float4 *>(lo + px * out_ps + c) = make_float4(l[0], l[1], l[2], l[3]);
+    *reinterpret_cast<float4 *>(out + px * out_ps + c) = v;
+    if (zero) *reinterpret_cast<float4 *>(zero + px * out_ps + c) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
-// [tap][chunk][hi: cout_pad rows | lo: cout_pad rows][32] <- w[cout][cin][ky][kx], zero padded
-// (ihwo: the filter is stored [cin][ky][kx][cout] instead)
-__global__ void pack_weights_exact_kernel(const float *__restrict__ w, int cout, int cin, int k, int nch, int cout_pad, float *__restrict__ wp, int64_t total,
-                                          int ihwo) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int cl = (int)(i % 32);
-    int64_t rest = i / 32;
-    const int row = (int)(rest % (2 * cout_pad));
-    rest /= 2 * cout_pad;
-    const int ci = (int)(rest % nch) * 32 + cl, tap = (int)(rest / nch), co = row < cout_pad ? row : row - cout_pad;
-    float v = 0.0f;
-    if (co < cout && ci < cin) v = w[ihwo ? ((int64_t)ci * k * k + tap) * cout + co : ((int64_t)co * cin + ci) * k * k + tap];
-    float h, l;
-    split_two_tf32(v, h, l);
-    wp[i] = row < cout_pad ? h : l;
+// [tap][chunk][hi: cout_pad rows | lo: cout_pad rows][32 FP16] <- w[cout][cin][ky][kx] (ihwo: stored [cin][ky][kx][cout]), zero padded, then
+// cout_pad inverse scales.  A channel's scale puts its largest entry into [2^14, 2^15).  NaN for a channel whose entries two FP16 numbers
+// cannot hold: infinities, NaN, or entries above 2^10 (2^100 in any case) beside entries 2^-36 of them; its outputs are computed
+// with FP32 instructions.  (Below 2^10 what falls off is at most 2^-40 of an input.)  A block per NC channels, which it reads twice, the second time from the caches.
+template <int NC>
+__global__ void __launch_bounds__(512) pack_weights_exact_kernel(const float *__restrict__ w, int cout, int cin, int k, int nch, int cout_pad, float *__restrict__ wp,
+                                                                 int64_t scales_at, int ihwo) {
+  __shared__ unsigned s_max[NC], s_min[NC];
+  const int kk = k * k, co0 = blockIdx.x * NC, n = cin * kk;
+  if (threadIdx.x < NC) { s_max[threadIdx.x] = 0u; s_min[threadIdx.x] = 0x7FFFFFFFu; }
+  __syncthreads();
+  // neighbouring threads read neighbouring addresses: channels first where they are stored together
+  const int c = ihwo ? (int)threadIdx.x % NC : 0, step = ihwo ? (int)blockDim.x / NC : (int)blockDim.x, first = ihwo ? (int)threadIdx.x / NC : (int)threadIdx.x;
+  auto entry = [&](int i, int co) { return ihwo ? w[(int64_t)i * cout + co] : w[(int64_t)co * n + i]; };      // i = ci * kk + tap
+  for (int cc = ihwo ? c : 0; cc < (ihwo ? c + 1 : NC); ++cc) {
+    unsigned m = 0u, least = 0x7FFFFFFFu;
+    if (co0 + cc < cout)
+      for (int i = first; i < n; i += step) {
+        const unsigned u = __float_as_uint(entry(i, co0 + cc)) & 0x7FFFFFFFu;
+        m = max(m, u);
+        if (u) least = min(least, u);
+      }
+    atomicMax(&s_max[cc], m);
+    atomicMin(&s_min[cc], least);
+  }
+  __syncthreads();
+  __half *out = reinterpret_cast<__half *>(wp);
+  for (int cc = ihwo ? c : 0; cc < (ihwo ? c + 1 : NC); ++cc) {
+    const unsigned m = s_max[cc], e = min(max(m >> 23, 15u), 254u);
+    const float scale = __uint_as_float((268u - e) << 23);
+    const int co = co0 + cc;
+    if (first == 0 && co < cout_pad) {
+      const bool wide = m > 0x71800000u || (m > 0x44800000u && (m >> 23) - (s_min[cc] >> 23) > 36u);
+      wp[scales_at + co] = wide ? __uint_as_float(0x7FC00000u) : __uint_as_float((e - 14u) << 23);
+    }
+    for (int i = first; i < nch * 32 * kk; i += step) {
+      const int ci = i / kk, tap = i - ci * kk;
+      const float v = co < cout && ci < cin ? entry(i, co) * scale : 0.0f;
+      const __half h = __float2half_rn(v);
+      const int64_t at = (((int64_t)tap * nch + (ci >> 5)) * 2 * cout_pad + co) * 32 + (ci & 31);
+      out[at] = h;
+      out[at + (int64_t)cout_pad * 32] = __float2half_rn((v - __half2float(h)) * 2048.0f);
+    }
   }
 }
 
@@ -507,31 +545,38 @@ int pack_exact(const float *w, int cout, int cin, int k, int ihwo, float *wpacke
   int64_t total;
   const int s = mie_conv_pack_dims_exact(cin, cout, k, &total);
   if (s != MIE_OK) return s;
-  int64_t blocks = divup64(total, 256);
-  if (blocks > MIE_SM_COUNT * 8) blocks = MIE_SM_COUNT * 8;
-  pack_weights_exact_kernel<<<(unsigned)blocks, 256, 0, st>>>(w, cout, cin, k, divup(cin, 32), divup(cout, 32) * 32, wpacked, total, ihwo);
+  const int cout_pad = divup(cout, 32) * 32, nch = divup(cin, 32);
+  const int64_t at = exact_scales_at(cin, cout_pad, k);
+  if (ihwo) pack_weights_exact_kernel<4><<<cout_pad / 4, 512, 0, st>>>(w, cout, cin, k, nch, cout_pad, wpacked, at, 1);
+  else pack_weights_exact_kernel<1><<<cout_pad, 512, 0, st>>>(w, cout, cin, k, nch, cout_pad, wpacked, at, 0);
   return check_launch();
 }
 
-int split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, const int32_t *counts, cudaStream_t st) {
-  if (!in || !hi || !lo || C <= 0 || pixels <= 0 || in_ps < C || out_ps < (C + 3) / 4 * 4 || out_ps % 4) return MIE_EINVAL;
-  if (!aligned16(hi) || !aligned16(lo)) return MIE_EALIGN;
+int pad_field(const float *in, int64_t in_ps, int C, int64_t pixels, float *out, float *zero, int64_t out_ps, const int32_t *counts, cudaStream_t st) {
+  if (!in || !out || C <= 0 || pixels <= 0 || in_ps < C || out_ps < (C + 3) / 4 * 4 || out_ps % 4) return MIE_EINVAL;
+  if (!aligned16(out) || !aligned16(zero)) return MIE_EALIGN;
   const int quads = divup(C, 4), vec = C % 4 == 0 && in_ps % 4 == 0 && aligned16(in);
   int64_t blocks = divup64(pixels * quads, 256);
   if (blocks > MIE_SM_COUNT * 16) blocks = MIE_SM_COUNT * 16;
-  launch_chained(split_exact_kernel, dim3((unsigned)blocks), dim3(256), 0, st, in, in_ps, C, pixels, hi, lo, out_ps, quads, vec, counts);
+  launch_chained(pad_field_kernel, dim3((unsigned)blocks), dim3(256), 0, st, in, in_ps, C, pixels, out, zero, out_ps, quads, vec, counts);
   return check_launch();
 }
 
 }  // namespace mie
 
 extern "C" int mie_split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, void *stream) {
-  return split_exact(in, in_ps, C, pixels, hi, lo, out_ps, nullptr, (cudaStream_t)stream);
+  if (!lo) return MIE_EINVAL;
+  return pad_field(in, in_ps, C, pixels, hi, lo, out_ps, nullptr, (cudaStream_t)stream);
+}
+
+extern "C" int mie_pad_field(const float *in, int64_t in_ps, int C, int64_t pixels, float *out, int64_t out_ps, void *stream) {
+  return pad_field(in, in_ps, C, pixels, out, nullptr, out_ps, nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int mie_conv_pack_dims_exact(int cin, int cout, int k, int64_t *n_floats) {
   if (cin <= 0 || cout <= 0 || k <= 0 || !n_floats) return MIE_EINVAL;
-  *n_floats = (int64_t)k * k * divup(cin, 32) * 2 * (divup(cout, 32) * 32) * 32;
+  const int cout_pad = divup(cout, 32) * 32;
+  *n_floats = exact_scales_at(cin, cout_pad, k) + cout_pad;
   return MIE_OK;
 }
 

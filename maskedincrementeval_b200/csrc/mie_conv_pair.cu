@@ -122,10 +122,6 @@ struct PairIssue {
   int item0, item_step, n_items, n_chunks, cin, NB, tps, nviews;
   unsigned nacc, tmem_base, a_base, b_base, row_bytes, halo_bytes, tap_bytes, stage_bytes, stages, halos, limit;
 };
-struct PairTapTable {
-  int first[5];
-  int off[50];       // offset of the tap in the halo, in descriptor units
-};
 __device__ __forceinline__ void pair_issue(const PairIssue a, const PairTapTable &t, unsigned long long *b_full, unsigned long long *b_empty,
                                         unsigned long long *a_full, unsigned long long *a_empty, unsigned long long *acc_full,
                                         unsigned long long *acc_empty, volatile int *abort_flag) {
@@ -268,7 +264,7 @@ conv_pair_kernel(const PairParams P, const __grid_constant__ PairMaps maps) {
   if (warp == 0) {
     // =========================== halo producer ===========================
     const PairRing ring = {a_full, a_empty, a_base, halo_bytes, (unsigned)P.halos};
-    pair_produce_halos(work, ring, P.t, P.hp, row_bytes, lst, n_active, ntiles_total, TWo, THo, p.counts, &s_abort,
+    pair_produce_halos<false>(work, ring, P.t, P.hp, row_bytes, lst, n_active, ntiles_total, TWo, THo, p.counts, &s_abort,
                        [&](int u, int &v) { v = u; return &maps.in[u]; });
   } else if (warp == 1) {
     // =========================== filter producer ===========================

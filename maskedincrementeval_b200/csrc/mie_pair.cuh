@@ -1,5 +1,6 @@
 // What the CTA-pair convolution kernels share: taps and views of the reduction, cta_group::2 wrappers.
 #pragma once
+#include <cuda_fp16.h>
 #include "mie_tc.cuh"
 
 namespace mie {
@@ -97,6 +98,33 @@ __device__ __forceinline__ void tma_store_slab(unsigned smem_addr, const CUtenso
                ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_addr), "r"(c0), "r"(x), "r"(y), "r"(n) : "memory");
 }
 
+// Waits for three barriers at once (a barrier may be named twice): one round of their latency where three waits take three.
+__device__ __forceinline__ bool mbar_wait3(unsigned b0, unsigned p0, unsigned b1, unsigned p1, unsigned b2, unsigned p2, volatile int *abort_flag, unsigned limit) {
+  for (unsigned it = 0; it < limit; ++it) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p, q, r;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 r, [%5], %6;\n\t"
+        "and.pred p, p, q;\n\tand.pred p, p, r;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(b0), "r"(p0), "r"(b1), "r"(p1), "r"(b2), "r"(p2)
+        : "memory");
+    if (done) return true;
+    if ((it & 1023u) == 1023u && *abort_flag) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+
+// Taps of a reduction as the issuing warps read them.
+struct PairTapTable {
+  int first[5];
+  int off[50];       // offset of the tap in the halo, in descriptor units
+};
+
 // What the two producer warps of a pair kernel walk through: items of four listed tiles and a column block, channel chunks, and
 // per chunk `units` halos (the views of the input, in two parts where the kernel splits its operands).
 struct PairWork {
@@ -124,8 +152,9 @@ __device__ __forceinline__ void pair_drain(const PairRing &r, unsigned s, unsign
 
 // Halo producer, one converged warp: one copy per halo row and tile, issued by one elected lane.  (With a row per lane the copies
 // are issued one by one all the same, at several times the cost -- no uniform registers --, and paced every layer.)
-// source(unit, view): the tensor map of a unit, and which view it is.
-template <typename Source>
+// source(unit, view): the tensor map of a unit, and which view it is.  LOCAL: each block's own barrier counts its own bytes (the
+// block works on the halo before the instructions read it); else the first block's barrier counts those of both.
+template <bool LOCAL, typename Source>
 __device__ __forceinline__ void pair_produce_halos(const PairWork &w, const PairRing &r, const PairTaps &t, int hp, unsigned row_bytes, const int32_t *lst,
                                                    int n_active, int ntiles_total, int TWo, int THo, int32_t *counts, volatile int *abort_flag,
                                                    Source source) {
@@ -147,14 +176,14 @@ __device__ __forceinline__ void pair_produce_halos(const PairWork &w, const Pair
       }
       tx8[i] = have[i] ? (tile % TWo) * 8 : 0; ty8[i] = have[i] ? ((tile / TWo) % THo) * 8 : 0; tn[i] = have[i] ? tile / (TWo * THo) : 0;
     }
-    const unsigned tx_bytes = (unsigned)min(4, n_active - 4 * (item / w.n_cblk)) * (unsigned)hp * row_bytes;   // both blocks
+    const unsigned tx_bytes = (LOCAL ? (unsigned)have[0] + (unsigned)have[1] : (unsigned)min(4, n_active - 4 * (item / w.n_cblk))) * (unsigned)hp * row_bytes;
     for (int chunk = 0; chunk < w.n_chunks && ok; ++chunk)
       for (int u = 0; u < w.units; ++u) {
         if (!first_lap) ok = __all_sync(0xffffffffu, mbar_wait(&r.empty[s], parity, abort_flag, w.limit));
         if (!ok) break;
-        const unsigned bar = mapa_shared(smem_u32(&r.full[s]), 0);
+        const unsigned bar = LOCAL ? smem_u32(&r.full[s]) : mapa_shared(smem_u32(&r.full[s]), 0);
         if (leader) {
-          if (w.crank == 0u)
+          if (LOCAL || w.crank == 0u)
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&r.full[s])), "r"(tx_bytes) : "memory");
           int v;
           const CUtensorMap *map = source(u, v);
@@ -163,7 +192,10 @@ __device__ __forceinline__ void pair_produce_halos(const PairWork &w, const Pair
             if (have[i]) {
               unsigned dst = r.base + s * r.bytes + (unsigned)i * row_bytes;
               const int x = tx8[i] + t.x0[v], y = ty8[i] + t.y0[v];
-              for (int row = 0; row < hp; ++row, dst += 2u * row_bytes) tma_load_4d_pair(dst, map, bar, chunk * 32, x, y + row, tn[i]);
+              for (int row = 0; row < hp; ++row, dst += 2u * row_bytes) {
+                if (LOCAL) tma_load_4d_raw(dst, map, bar, chunk * 32, x, y + row, tn[i]);
+                else tma_load_4d_pair(dst, map, bar, chunk * 32, x, y + row, tn[i]);
+              }
             }
         }
         __syncwarp();
@@ -208,11 +240,12 @@ __device__ __forceinline__ void pair_produce_filter(const PairWork &w, const Pai
   if (!w.withhold) pair_drain(r, s, parity, first_lap, ok, abort_flag, w.limit);
 }
 
-// Barrier of the 128 threads of an epilogue set: whether all of them bring `ok`.
+// Barrier of the threads of an epilogue set (or of the splitting warps): whether all of them bring `ok`.
+template <int THREADS = 128>
 __device__ __forceinline__ bool set_all(int id, bool ok) {
   int r;
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %2, 0;\n\tbarrier.cta.red.and.pred q, %1, 128, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
-               : "=r"(r) : "r"(id), "r"((int)ok) : "memory");
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %2, 0;\n\tbarrier.cta.red.and.pred q, %1, %3, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+               : "=r"(r) : "r"(id), "r"((int)ok), "n"(THREADS) : "memory");
   return r != 0;
 }
 
@@ -226,6 +259,180 @@ __device__ __forceinline__ float4 lds4(unsigned addr) {
 }
 __device__ __forceinline__ void sts4(unsigned addr, float4 v) {
   asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+
+// ---------------------------------------------------------------------------------------------------------------
+// fp32 operands as two FP16 numbers each.  An operand v, scaled by a power of two s, is hi = fp16(s v) and lo = fp16(2^11 (s v - hi)),
+// rounded to nearest: together they hold v to 2^-24, as two TF32 numbers do, but an instruction takes 16 of them where it takes 8
+// TF32 numbers.  (A scaled FP16 split: Ootomo and Yokota, 2022.)  The input's scale is chosen for every halo in
+// shared memory, so that its largest value lies in [2^14, 2^15): a value keeps its 24 bits down to 2^-28 of that, and an absolute
+// step of 2^-49 of it below.  Halos for which that would not do -- an infinity, a NaN, values above 2^100, or above 2^14 beside
+// values 2^-36 of it -- are marked (inverse scale NaN), and the epilogue computes their pixels with FP32 instructions.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr unsigned SPLIT_RING = 16;      // inverse scales kept: more than halo buffers and segment accumulators in flight
+constexpr float SPLIT_LO = 1.0f / 2048.0f;
+
+// [D1] += A hi x [B hi | B lo], [D2] += A lo x B hi for up to two K-slices (16 channels = 32 bytes each).  A: rows of 128 bytes, 32 hi then
+// 32 lo; B: rows of 64 bytes.  Called by a converged warp.
+__device__ __forceinline__ void pair_mma_split(unsigned d1, unsigned d2, unsigned long long a_desc, unsigned long long b_desc, unsigned id1, unsigned id2,
+                                               unsigned accumulate, unsigned nks) {
+  asm volatile(
+      "{\n\t.reg .pred p, q, e, r1;\n\t.reg .b64 a1, a2, a3, b1;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "setp.eq.b32 q, 0, 0;\n\t"
+      "setp.gt.and.u32 r1, %7, 1, e;\n\t"
+      "add.u64 a1, %2, 2;\n\tadd.u64 a2, %2, 4;\n\tadd.u64 a3, %2, 6;\n\tadd.u64 b1, %3, 2;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %2, %3, %4, p;\n\t"
+      "@r1 tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %4, q;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], a2, %3, %5, p;\n\t"
+      "@r1 tcgen05.mma.cta_group::2.kind::f16 [%1], a3, b1, %5, q;\n\t}"
+      ::"r"(d1), "r"(d2), "l"(a_desc), "l"(b_desc), "r"(id1), "r"(id2), "r"(accumulate), "r"(nks)
+      : "memory");
+}
+// Instruction descriptor: FP16 operands, both K-major, FP32 accumulator, M = 256.
+__device__ __forceinline__ unsigned make_idesc_f16_pair(int n) { return (1u << 4) | ((unsigned)(n >> 3) << 17) | (16u << 24); }
+// Rows of 64 bytes, 64-byte swizzle, 8-row groups 512 bytes apart.
+__device__ __forceinline__ unsigned long long make_smem_desc_64(unsigned smem_addr) {
+  return (unsigned long long)((smem_addr & 0x3FFFFu) >> 4) | (unsigned long long)1 << 16 | (unsigned long long)(512 >> 4) << 32 |
+         (unsigned long long)1 << 46 | (unsigned long long)4 << 61;
+}
+
+__device__ __forceinline__ void split_fp16(const float *v, float scale, float4 &hi, float4 &lo) {      // eight channels
+  unsigned h[4], l[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float a = v[2 * j] * scale, b = v[2 * j + 1] * scale;
+    const __half2 t = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(t);
+    const __half2 u = __floats2half2_rn((a - f.x) * 2048.0f, (b - f.y) * 2048.0f);
+    h[j] = *reinterpret_cast<const unsigned *>(&t);
+    l[j] = *reinterpret_cast<const unsigned *>(&u);
+  }
+  hi = make_float4(__uint_as_float(h[0]), __uint_as_float(h[1]), __uint_as_float(h[2]), __uint_as_float(h[3]));
+  lo = make_float4(__uint_as_float(l[0]), __uint_as_float(l[1]), __uint_as_float(l[2]), __uint_as_float(l[3]));
+}
+
+// The splitting warps (t: thread among theirs).  A halo lies in shared memory as `rows` rows of 128 bytes (32 fp32 channels of a
+// pixel, 128-byte swizzle; [halo row][tile][halo column]) and is replaced in place by 64 bytes of hi and 64 bytes of lo.  A thread
+// takes eight channels: it reads pieces 2 c and 2 c + 1 of a row and writes pieces c and 4 + c; the eight rows of a warp are dealt such that
+// neighbouring lanes hold rows whose swizzles differ in bits 0 and 2, so that neither reads nor writes meet in a bank.
+// What it costs: one read and one write of the halo through shared memory (400 clocks of its port for a 3x3 layer's 25 KB), and a
+// chain of about 2200 clocks a unit (read 600, largest value of all warps 400, split and write 1100), beside the instructions of
+// the unit before.
+constexpr int SPLIT_WARPS = 8, SPLIT_PASS = 8 * SPLIT_WARPS;      // rows of a pass
+constexpr int SPLIT_REGS = 288 / SPLIT_PASS + (288 % SPLIT_PASS != 0);      // passes held in registers: halos up to 12 x 12; larger ones (7x7) read the rest twice
+struct SplitShared {
+  float red[2][SPLIT_WARPS];
+  unsigned least[SPLIT_WARPS];
+  float inv[SPLIT_RING];                       // inverse scale of a unit's halo (NaN: marked) ...
+  unsigned long long inv_full[SPLIT_RING];     // ... and that it is there
+};
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {      // of magnitudes; a NaN stays
+  float d;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// Predicated accesses (no branch: the passes of a halo are one stretch of code that the compiler can interleave)
+__device__ __forceinline__ float4 lds4_if(unsigned addr, bool on) {
+  float4 v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+               "@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"((unsigned)on) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts4_if(unsigned addr, float4 v, bool on) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n\t}"
+               ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"((unsigned)on) : "memory");
+}
+__device__ __forceinline__ void pair_split_halos(const PairWork &w, const PairRing &r, unsigned long long *ready, int rows, int wp, int n_active, int t,
+                                                 SplitShared &sh, volatile int *abort_flag) {
+  const int lane = t & 31, cw = t >> 5, c = lane & 3;
+  const int row0 = cw * 8 + (int)((0x63724150u >> (4 * (lane >> 2))) & 7u);
+  const int sw = row0 & 7, passes = (rows + SPLIT_PASS - 1) / SPLIT_PASS;
+  const unsigned at = (unsigned)row0 * 128u, rd0 = at + (unsigned)((2 * c) ^ sw) * 16u, rd1 = at + (unsigned)((2 * c + 1) ^ sw) * 16u,
+                 wr0 = at + (unsigned)(c ^ sw) * 16u, wr1 = at + (unsigned)((4 + c) ^ sw) * 16u;
+  // which of the thread's rows hold input: of two tiles, or of the first alone (what lies in an absent tile's rows is none)
+  unsigned both = 0, one = 0;
+  for (int it = 0; it < passes; ++it)
+    if (row0 + SPLIT_PASS * it < rows) { both |= 1u << it; if (!(((row0 + SPLIT_PASS * it) / wp) & 1)) one |= 1u << it; }
+  unsigned s = 0, parity = 0, unit = 0;
+  for (int item = w.item0; item < w.n_items; item += w.item_step) {
+    const int tiles = n_active - 4 * (item / w.n_cblk) - 2 * (int)w.crank;
+    const unsigned live = tiles >= 2 ? both : tiles == 1 ? one : 0u;
+    for (int cu = 0; cu < w.n_chunks * w.units; ++cu, ++unit) {
+      const bool ok = mbar_wait(&r.full[s], parity, abort_flag, w.limit);
+      const unsigned base = r.base + s * r.bytes;
+      auto read = [&](int it, float *v) {
+        const float4 a = lds4_if(base + rd0 + (unsigned)(it * SPLIT_PASS * 128), live >> it & 1u), b = lds4_if(base + rd1 + (unsigned)(it * SPLIT_PASS * 128), live >> it & 1u);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+      };
+      auto largest = [](const float *v, float m) { return max3_abs(max3_abs(max3_abs(max3_abs(m, v[0], v[1]), v[2], v[3]), v[4], v[5]), v[6], v[7]); };
+      float v[SPLIT_REGS][8], m = 0.0f;
+#pragma unroll
+      for (int it = 0; it < SPLIT_REGS; ++it) read(it, v[it]);
+#pragma unroll
+      for (int it = 0; it < SPLIT_REGS; ++it) m = largest(v[it], m);
+#pragma unroll 1
+      for (int it = SPLIT_REGS; it < passes; ++it) {
+        float x[8];
+        read(it, x);
+        m = largest(x, m);
+      }
+      m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));      // (of non-negative floats, NaN above all)
+      if (lane == 0) sh.red[unit & 1u][cw] = m;
+      if (!set_all<32 * SPLIT_WARPS>(3, ok)) return;
+      m = 0.0f;
+#pragma unroll
+      for (int i = 0; i < SPLIT_WARPS; i += 2) m = max3_abs(m, sh.red[unit & 1u][i], sh.red[unit & 1u][i + 1]);
+      const unsigned mb = __float_as_uint(m);
+      bool wide = false;
+      if (mb >= 0x46800000u) {      // 2^14 or more: is it too much for what lies beside it?
+        unsigned least = 0x7FFFFFFFu;
+        auto scan = [&](const float *x) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) { const unsigned u = __float_as_uint(x[j]) & 0x7FFFFFFFu; if (u) least = min(least, u); }
+        };
+#pragma unroll
+        for (int it = 0; it < SPLIT_REGS; ++it) scan(v[it]);
+#pragma unroll 1
+        for (int it = SPLIT_REGS; it < passes; ++it) { float x[8]; read(it, x); scan(x); }
+        least = __reduce_min_sync(0xffffffffu, least);
+        if (lane == 0) sh.least[cw] = least;
+        set_all<32 * SPLIT_WARPS>(3, true);
+#pragma unroll
+        for (int i = 0; i < SPLIT_WARPS; ++i) least = min(least, sh.least[i]);
+        wide = mb > 0x71800000u || (mb >> 23) - (least >> 23) > 36u;
+      }
+      const unsigned e = min(max(mb >> 23, 15u), 254u);
+      const float scale = __uint_as_float((268u - e) << 23);
+      if (t == 0) {
+        sh.inv[unit % SPLIT_RING] = wide ? __uint_as_float(0x7FC00000u) : __uint_as_float((e - 14u) << 23);
+        mbar_arrive(&sh.inv_full[unit % SPLIT_RING]);
+      }
+      auto write = [&](int it, const float *x) {
+        float4 hi, lo;
+        split_fp16(x, scale, hi, lo);
+        sts4_if(base + wr0 + (unsigned)(it * SPLIT_PASS * 128), hi, live >> it & 1u);
+        sts4_if(base + wr1 + (unsigned)(it * SPLIT_PASS * 128), lo, live >> it & 1u);
+      };
+#pragma unroll
+      for (int it = 0; it < SPLIT_REGS; ++it) write(it, v[it]);
+#pragma unroll 1
+      for (int it = SPLIT_REGS; it < passes; ++it) {
+        float x[8];
+        read(it, x);
+        __syncwarp();      // in place: the lanes of a row read before one of them writes
+        write(it, x);
+      }
+      // The instructions read it through the asynchronous proxy.  What the arrival orders is this block's shared memory alone, so the
+      // default (block) scope of its release is enough; with release.cluster it took 1300 clocks, as long as the splitting.
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&ready[s]), 0));
+      if (++s == r.count) { s = 0; parity ^= 1u; }
+    }
+  }
 }
 
 }  // namespace

@@ -45,7 +45,7 @@ class IncrConfig:
                      convolution sees q (one more kernel per convolution; what is rounded away stays pending)
     refresh          "native" (default): the networks' dense pass (forward_refresh_reservoirs) runs on this library's
                      kernels in dense-evaluation mode -- every tile listed, bias added, state set instead of
-                     advanced, fp32 precision (on the tensor cores from two TF32 parts per operand, unless
+                     advanced, fp32 precision (on the tensor cores from two FP16 parts per operand, unless
                      ``tensor_cores`` is "off"); "library": it runs on PyTorch's dense operators (cuDNN), as the reference's does
     tail_dilation    True: a convolution's tile dilation rides in the tail of the kernel that produces its input mask
                      (one launch less per convolution; measured slower than the separate launch when launches overlap
@@ -495,14 +495,15 @@ def pack_conv_weights_exact(weight: torch.Tensor) -> torch.Tensor:
     return buf
 
 
-def split_exact(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
-    """Two new channels-last fields hi = tf32(x), lo = tf32(x - hi); channel counts rounded up to 4, the rest zero."""
+def tma_field(x: torch.Tensor) -> torch.Tensor:
+    """``x``, or where its address or pixel stride is no multiple of 16 bytes a copy with channels rounded up to 4."""
+    if x.data_ptr() % 16 == 0 and pixel_stride(x) % 4 == 0:
+        return x
     n, c, h, w = x.shape
     cp = (c + 3) // 4 * 4
-    both = torch.empty((2, n, h, w, cp), dtype=torch.float32, device=x.device)
-    nat.check(nat.lib.mie_split_exact(x.data_ptr(), pixel_stride(x), c, n * h * w, both[0].data_ptr(), both[1].data_ptr(), cp,
-                                      nat.stream_ptr(x.device)), "split_exact")
-    return both[0].permute(0, 3, 1, 2)[:, :c], both[1].permute(0, 3, 1, 2)[:, :c]
+    copy = torch.empty((n, h, w, cp), dtype=torch.float32, device=x.device)
+    nat.check(nat.lib.mie_pad_field(x.data_ptr(), pixel_stride(x), c, n * h * w, copy.data_ptr(), cp, nat.stream_ptr(x.device)), "pad_field")
+    return copy.permute(0, 3, 1, 2)[:, :c]
 
 
 # A first layer that runs in split precision asks the producer of its input delta for the split copy: the request is

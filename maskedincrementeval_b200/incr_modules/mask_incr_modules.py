@@ -339,7 +339,7 @@ class _PreparedRefresh:
     """The same for the dense evaluation of a layer in fp32 precision on the tensor cores (60 us of deciding per layer
     otherwise, more than its kernels take)."""
     __slots__ = ("activation", "epoch", "options", "op", "weight", "bias", "params_key", "reservoir", "reservoir_ptr", "geometry", "mask_key", "addend_key",
-                 "plan", "args", "fields", "fields_ps", "x_ps", "job", "out", "packed")
+                 "plan", "args", "field", "x_ps", "job", "out", "packed")
 
     def __init__(self, conv, activation, plan, d, mask, addend, packed):
         self.activation, self.plan = activation, plan
@@ -352,8 +352,7 @@ class _PreparedRefresh:
         self.geometry, self.mask_key = (d.shape, d.stride(), d.device), self.key_of_mask(mask)
         self.addend_key = None if addend is None else self.key_of_addend(addend)
         n, c, h, w = d.shape
-        cp = (c + 3) // 4 * 4
-        self.fields, self.fields_ps, self.x_ps = (2, n, h, w, cp), n * h * w * cp * 4, fl.pixel_stride(d)
+        self.field, self.x_ps = (n, h, w, (c + 3) // 4 * 4), fl.pixel_stride(d)
         self.job, self.out, self.packed = plan.tail, (plan.out, plan.mask), packed
         self.args = nat.ConvArgs.from_buffer_copy(plan.args)
 
@@ -383,11 +382,11 @@ class _PreparedRefresh:
                 return None
         if addend is not None and (type(addend[1]) is not TileMask or self.key_of_addend(addend) != self.addend_key):
             return None
-        both = torch.empty(self.fields, dtype=torch.float32, device=d.device)     # released after the launch
-        a = self.args
-        a.in_ = both.data_ptr()
-        a.in_lo = a.in_ + self.fields_ps
-        nat.check(nat.lib.mie_conv_refresh_step(C.byref(a), d.data_ptr(), self.x_ps, C.addressof(self.job.c), nat.stream_ptr(d.device)),
+        a, ptr, copy = self.args, d.data_ptr(), None
+        if ptr % 16 or self.x_ps % 4:      # room for a copy that TMA can read, released after the launch
+            copy = torch.empty(self.field, dtype=torch.float32, device=d.device)
+            a.in_, a.in_ps = copy.data_ptr(), self.field[3]
+        nat.check(nat.lib.mie_conv_refresh_step(C.byref(a), ptr, self.x_ps, C.addressof(self.job.c), nat.stream_ptr(d.device)),
                   "conv_refresh_step")
         return list(self.out)
 
@@ -645,12 +644,12 @@ class nnConvIncr(nn.Conv2d):
         if a.thr > 0.0 or a.emitted:
             nat.lib.mie_set_option(nat.OPT_TC_THRESHOLDED, 1 if config.tc_thresholded else 0)
         if refresh and config.tensor_cores == "auto" and 3 <= self._k <= 7 and self.out_channels % 4 == 0:
-            # fp32 precision on the tensor cores: the input as two TF32 fields (released after the launch)
-            hi, lo = fl.split_exact(d)
+            # fp32 precision on the tensor cores (a copy of the input, where it needs one, is released after the launch)
+            aligned = fl.tma_field(d)
             wx = self._weights_exact(cin)
-            a.in_, a.in_ps, a.in_lo, a.wpacked_exact = hi.data_ptr(), fl.pixel_stride(hi), lo.data_ptr(), wx.data_ptr()
+            a.in_, a.in_ps, a.wpacked_exact = aligned.data_ptr(), fl.pixel_stride(aligned), wx.data_ptr()
             if not nat.lib.mie_conv_is_exact(C.byref(a)):
-                a.in_, a.in_ps, a.in_lo, a.wpacked_exact = d.data_ptr(), fl.pixel_stride(d), None, None
+                a.in_, a.in_ps, a.wpacked_exact = d.data_ptr(), fl.pixel_stride(d), None
         self.last_used_tensor_cores = bool(nat.lib.mie_conv_uses_tensor_cores(C.byref(a)))
         self.last_cluster_size = int(nat.lib.mie_conv_cluster_size(C.byref(a)))
         if split and not self.last_used_tensor_cores:

@@ -151,6 +151,54 @@ def test_dense_pass_on_non_finite_values(dev, case, where):
         assert float(((got[big] - want[big]) / want[big]).abs().max()) <= 1e-5 if bool(big.any()) else True
 
 
+# Values that lie far apart in one halo: what two FP16 numbers with a common scale hold is computed on the tensor cores, the rest with FP32
+# instructions.  Every output against the sum of its products' magnitudes: fp32 sums of cin * k * k terms, or (below 2^17) a step
+# of 2^-49 of the largest value times the filter's entries (below 0.05).  (At 40000 some halos lie below 2^14.)
+@pytest.mark.parametrize("case", [(48, 32, 3, 1, 24, 40), (64, 64, 7, 1, 17, 23), (5, 32, 5, 2, 33, 40)])
+@pytest.mark.parametrize("big,small", [(1.0, 1e-3), (1e-30, 1e-33), (16383.0, 1e-6), (40000.0, 1e-6), (1e6, 1e-9), (1e20, 1.0), (1e31, 1e30), (1e36, 0.2)])
+def test_dense_pass_on_values_far_apart(dev, case, big, small):
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    cin, cout, k, s, h, w = case
+    torch.manual_seed(12)
+    layer = ConvLayerIncr(cin, cout, k, s, k // 2, activation="relu").to(dev).eval()
+    c = layer.conv2d
+    with torch.no_grad():
+        c.weight.mul_(0.05 / c.weight.abs().max())
+        c.bias.zero_()
+    x = cl(torch.randn(1, cin, h, w, device=dev).clamp_(-3, 3) * (small / 3))
+    x[0, :, 3::11, 5::13] *= big / small
+    want = F.conv2d(x.double(), c.weight.detach().double(), stride=s, padding=k // 2)
+    size = F.conv2d(x.double().abs(), c.weight.detach().double().abs(), stride=s, padding=k // 2)
+    with torch.no_grad():
+        NATIVE.conv(c, NATIVE.lift(x), layer.activation)
+    got = layer.activation.in_res.reservoir.double()
+    step = big * 2.0 ** -49 * 0.05 * cin * k * k if big < 2 ** 17 else 0.0
+    assert bool(got.isfinite().all())
+    assert float(((got - want).abs() - 2e-6 * size).max()) <= step
+
+
+# the same for a filter whose entries lie far apart, and for one of tiny entries
+@pytest.mark.parametrize("big,small", [(1e6, 1e-6), (1e30, 1e-3), (1e-20, 1e-22), (900.0, 1e-3)])
+def test_dense_pass_on_filters_far_apart(dev, big, small):
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    torch.manual_seed(13)
+    layer = ConvLayerIncr(48, 64, 3, 1, 1, activation="relu").to(dev).eval()
+    c = layer.conv2d
+    with torch.no_grad():
+        c.weight.normal_().clamp_(-3, 3).mul_(small / 3)
+        c.weight[::5, :, 0, 0] *= big / small
+        c.bias.zero_()
+    x = cl(torch.randn(1, 48, 21, 30, device=dev))
+    want = F.conv2d(x.double(), c.weight.detach().double(), padding=1)
+    size = F.conv2d(x.double().abs(), c.weight.detach().double().abs(), padding=1)
+    with torch.no_grad():
+        NATIVE.conv(c, NATIVE.lift(x), layer.activation)
+    got = layer.activation.in_res.reservoir.double()
+    assert float(((got - want).abs() / size).max()) <= 2e-6
+
+
 def test_extension_on_a_silent_step(dev):
     """A delta without an active pixel: zeros, also behind a call that left the workspace full, and before one that needs it again."""
     from maskedincrementeval_b200.ext.pointops import pointops_functional as pf

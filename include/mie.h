@@ -229,11 +229,12 @@ typedef struct mie_conv_args {
    * mie_tiles_dilate launch from the entry point instead. */
   int own_tiles;
   void *own_scratch;
-  /* Dense evaluation (`refresh`) in fp32 precision on the tensor cores: the filter packed by mie_pack_conv_weights_exact.
-   * Taken for k in {3, 5, 7} without a second input when the fields are 16-byte aligned, but for stride 2 on a field one
-   * pixel wide or high (mie_conv_is_exact tells); else, and with null, the FP32 kernel runs.  Every output tile has to be
-   * listed.  `in_lo` is no longer read (the kernel makes the parts of the input itself); `in` may be either the field or the
-   * first field of mie_split_exact. */
+  /* Fp32 precision on the tensor cores, for a dense evaluation (`refresh`) or a step: the filter packed by
+   * mie_pack_conv_weights_exact.  Taken for k in {3, 5, 7} without a second input when the fields are 16-byte aligned, but for
+   * stride 2 on a field one pixel wide or high (mie_conv_is_exact tells); else, and with null, the other kernels run (a dense
+   * evaluation: the FP32 kernel).  In a dense evaluation every output tile has to be listed; a step honours `head`,
+   * `own_tiles`, threshold and carry.  `wpacked` is read where FP16 parts cannot hold a value.  `in_lo` is no longer read
+   * (the kernel makes the parts of the input itself); `in` may be either the field or the first field of mie_split_exact. */
   const float *wpacked_exact;
   const float *in_lo;
 } mie_conv_args;
@@ -249,7 +250,7 @@ int mie_conv_step(const mie_conv_args *args /* host */, uint64_t *mask_bits, flo
 int mie_conv_refresh_step(const mie_conv_args *args /* host */, const float *x, int64_t x_ps, const mie_tail_job *dilate /* host */,
                           void *stream);
 
-/* Host only: 1 if mie_conv_tiles would run these arguments in fp32 precision on the tensor cores, else 0. */
+/* Host only: 1 if mie_conv_tiles would run these arguments in fp32 precision on the tensor cores (`wpacked_exact`), else 0. */
 int mie_conv_is_exact(const mie_conv_args *args /* host */);
 
 int mie_conv_tiles(const mie_conv_args *args /* host */, void *stream);

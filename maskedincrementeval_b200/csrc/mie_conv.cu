@@ -686,7 +686,9 @@ extern "C" int mie_pack_conv_weights(const float *w_oihw, int cout, int cin, int
 
 extern "C" int mie_conv_is_exact(const mie_conv_args *a) { return (a && exact_takes(a)) ? 1 : 0; }
 
-extern "C" int mie_conv_uses_tensor_cores(const mie_conv_args *a) { return (a && tc_eligible(a)) ? 1 : 0; }
+extern "C" int mie_conv_uses_tensor_cores(const mie_conv_args *a) {
+  return (a && (tc_eligible(a) || (!a->refresh && exact_takes(a)))) ? 1 : 0;
+}
 
 extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
   if (!a || !a->in || !a->wpacked || !a->list || !a->counts || !a->out || !a->out_bits) return MIE_EINVAL;
@@ -706,7 +708,8 @@ extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
   // launch, then a plain convolution.
   if (a->own_tiles && (!a->head || !a->own_scratch || (reinterpret_cast<uintptr_t>(a->own_scratch) & 7))) return MIE_EINVAL;
   // own-tiles mode exists in the tensor-core kernels only; elsewhere it is the separate launch and a plain convolution
-  if (a->head && (a->own_tiles ? !tc_eligible(a) : (!tail_fits(a->head) || mie_conv_cluster_size(a) > 1))) {
+  const bool exact = exact_takes(a);
+  if (a->head && !exact && (a->own_tiles ? !tc_eligible(a) : (!tail_fits(a->head) || mie_conv_cluster_size(a) > 1))) {
     const mie_tail_job *h = a->head;
     const int s = mie_tiles_dilate(h->in_bits, h->N, h->Hin, h->Win, h->Hout, h->Wout, h->k, h->stride, h->pad, h->union_bits,
                                    h->out_bits, h->list, h->stale, h->counts, h->flags, stream);
@@ -716,7 +719,7 @@ extern "C" int mie_conv_tiles(const mie_conv_args *a, void *stream) {
     b.own_tiles = 0;
     return mie_conv_tiles(&b, stream);
   }
-  if (exact_takes(a)) 
+  if (exact)
     return tail_after_launch(launch_conv_exact(a, a->wpacked, (int64_t)a->cin_pad * a->cout_pad, a->cout_pad, (cudaStream_t)stream), a->tail, true, stream);
   if (tc_eligible(a)) return tail_after_launch(launch_conv_tc(a, (cudaStream_t)stream), a->tail, true, stream);
 
@@ -780,7 +783,7 @@ extern "C" int mie_conv_refresh_step(const mie_conv_args *a, const float *x, int
   const bool direct = x_ps % 4 == 0 && aligned16(x);
   mie_conv_args b = *a;
   if (direct) { b.in = x; b.in_ps = x_ps; }
-  if (!b.in || !exact_takes(&b)) return MIE_EINVAL;
+  if (!b.in || !b.refresh || !exact_takes(&b)) return MIE_EINVAL;
   int s = mie_tiles_dilate(d->in_bits, d->N, d->Hin, d->Win, d->Hout, d->Wout, d->k, d->stride, d->pad, d->union_bits, d->out_bits, d->list,
                            d->stale, d->counts, d->flags, stream);
   if (s == MIE_OK && !direct)

@@ -45,11 +45,15 @@ struct ExactParams {
   int segs;    // segment accumulators
   unsigned spin_limit;
   int withhold_loads;      // self-test: the producers issue nothing, so the first wait runs out (MIE_OPT_TC_WITHHOLD_LOADS)
+  int slab_bufs;           // shared-memory slabs per epilogue set: output (+ reservoir (+ carry))
+  int slab_sets;           // ... and how many such buffers items take in turn (1 or 2)
+  unsigned div_tw, div_th; // magic numbers for divisions by the field's tiles per row and rows of tiles; 0: plain division
   mie_tail_job tail;
   PairTaps t;
+  TcParams c;              // a step: threshold, carry, stale tiles, own-tiles mode
 };
 struct ExactMaps {
-  CUtensorMap in[4], w, out, res;
+  CUtensorMap in[4], w, out, res, emitted;
 };
 
 __device__ __forceinline__ void tmem_ld16_async(unsigned taddr, unsigned *r) {
@@ -81,20 +85,20 @@ __host__ __device__ constexpr unsigned exact_segs(int cb) { return cb == 64 ? 2u
 // halo together, one commit for both the filter producer and the epilogue.  The issuing warp is what paces the kernel: the
 // instructions of a 3x3 chunk of 64 channels take 1930 clocks, a wait about 130 and a commit about 80 beside them.
 struct ExactIssue {
-  int bid, nblk, n_items, n_chunks, cin, tps, nviews;
+  int item0, item_step, n_items, n_chunks, cin, tps, nviews;
   unsigned tmem_base, a_base, b_base, row_bytes, halo_bytes, stage_bytes, stages, halos, segs, limit;
 };
-template <int CB>
+template <int CB, bool ALT>
 __device__ __forceinline__ void exact_issue(const ExactIssue a, const PairTapTable &t, unsigned long long *b_full, unsigned long long *done,
-    unsigned long long *a_ready, unsigned long long *a_empty, unsigned long long *seg_empty, volatile int *abort_flag) {
+    unsigned long long *a_ready, unsigned long long *a_empty, unsigned long long *seg_empty, unsigned long long *item_full, volatile int *abort_flag) {
   constexpr unsigned tap_units = CB * 64 >> 4;
   const unsigned id_hi = make_idesc_f16_pair(2 * CB), id_lo = make_idesc_f16_pair(CB);
   const unsigned long long b_tmpl = make_smem_desc_64(0), a_tmpl = make_smem_desc(0, a.row_bytes);
   const unsigned long long b_hi = b_tmpl & 0xFFFFFFFF00000000ull, a_hi = a_tmpl & 0xFFFFFFFF00000000ull;
   const unsigned lo_flags = (unsigned)(b_tmpl & 0xFFFF0000ull);
-  unsigned bs = 0, bpar = 0, as = 0, apar = 0, seg = 0, seg_par = 1, stage_addr = a.b_base;
+  unsigned bs = 0, bpar = 0, as = 0, apar = 0, seg = 0, seg_par = 1, stage_addr = a.b_base, turn = 0;
 #pragma unroll 1
-  for (int item = a.bid; item < a.n_items; item += a.nblk) {
+  for (int item = a.item0; item < a.n_items; item += a.item_step) {
 #pragma unroll 1
     for (int chunk = 0; chunk < a.n_chunks; ++chunk) {
       const unsigned nks = (unsigned)min(2, (a.cin - chunk * 32 + 15) >> 4);
@@ -126,13 +130,13 @@ __device__ __forceinline__ void exact_issue(const ExactIssue a, const PairTapTab
         if (++as == a.halos) { as = 0; apar ^= 1u; }
       }
     }
+    if (ALT) { pair_commit(&item_full[turn]); turn ^= 1u; }
   }
 }
 
 // One pixel's channels [co, co + HW) with FP32 instructions, for what two FP16 parts cannot hold (SplitShared, `winv`): the same sums as
 // the FP32 kernel's, padding multiplied as zeros like there.  Bounded by its loads (about 0.5 ms for an item of 256 channels and 5x5
 // taps), which no finite field of ordinary values comes to.
-template <int HW>
 __device__ __noinline__ void exact_fp32_quad(const ExactParams &p, int n, int oy, int ox, int c, float4 &out) {
   out = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
@@ -153,24 +157,135 @@ __device__ __forceinline__ void exact_fp32(const ExactParams &p, int n, int oy, 
 #pragma unroll
   for (int h = 0; h < HW / 4; ++h) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid && co + 4 * h < p.cout) exact_fp32_quad<HW>(p, n, oy, ox, co + 4 * h, v);
+    if (valid && co + 4 * h < p.cout) exact_fp32_quad(p, n, oy, ox, co + 4 * h, v);
     acc[4 * h] = v.x; acc[4 * h + 1] = v.y; acc[4 * h + 2] = v.z; acc[4 * h + 3] = v.w;
   }
 }
 
-// HW: channels per epilogue set (CB = 2 HW channels per block)
-template <int HW>
+// A step's activation at one pixel: acc, the convolution's channels; the pixel's rows of the reservoir, output and carry slabs.  Groups of 16
+// channels are sent when one of them moved by more than the threshold; returns whether one was.
+struct ExactRow {
+  unsigned res, out, em, sw;
+};
+template <int HW, int ACT>
+__device__ __forceinline__ bool exact_step(const ExactParams &p, const float *acc, const ExactRow r, const float *addend, int co) {
+  auto f = [&](float4 v) { return make_float4(tc_act<ACT>(p.act, v.x), tc_act<ACT>(p.act, v.y), tc_act<ACT>(p.act, v.z), tc_act<ACT>(p.act, v.w)); };
+  bool sent = false;
+#pragma unroll
+  for (int g = 0; g < HW / 16; ++g) {
+    float4 o[4], x[4];
+    float top = 0.0f;
+    auto at = [&](int i) { return (unsigned)(4 * g + i ^ (int)r.sw) << 4; };
+    if (ACT != MIE_ACT_NONE)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = lds4(r.res + at(i));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int h = 4 * g + i;
+      o[i] = make_float4(acc[4 * h], acc[4 * h + 1], acc[4 * h + 2], acc[4 * h + 3]);
+      if (addend && co + 4 * h < p.cout) o[i] = f4add(o[i], *reinterpret_cast<const float4 *>(addend + co + 4 * h));
+      if (ACT != MIE_ACT_NONE) {
+        const float4 b = p.c.emitted ? lds4(r.em + at(i)) : f(x[i]);
+        x[i] = f4add(x[i], o[i]);
+        const float4 y = f(x[i]);
+        o[i] = make_float4(y.x - b.x, y.y - b.y, y.z - b.z, y.w - b.w);
+        sts4(r.res + at(i), x[i]);
+      }
+      if (co + 4 * h < p.cout) top = fmaxf(top, fmaxf(fmaxf(fabsf(o[i].x), fabsf(o[i].y)), fmaxf(fabsf(o[i].z), fabsf(o[i].w))));
+    }
+    const bool flag = top > p.c.thr, withheld = (p.c.thr > 0.0f || p.c.emitted) && !flag;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sts4(r.out + at(i), withheld ? make_float4(0.f, 0.f, 0.f, 0.f) : o[i]);
+    sent |= flag;
+  }
+  return sent;
+}
+
+// The same from tensor memory, where an item's one or two segments all are (c: columns of the first): eight channels at a time in a loop
+// that the instruction cache holds.  As straight code over registers the epilogue of 32 channels ran at 20 clocks an instruction and
+// set the pace of the whole kernel (8 x 32 -> 32 at 480x640: 574 us; two items in hand, still straight, 472).
+// STEP false: the dense pass, out = f(reservoir = conv + bias).
+__device__ __forceinline__ void tmem_ld8_async(unsigned taddr, unsigned *r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+template <int HW, bool STEP, int ACT>
+__device__ __forceinline__ bool exact_finish(const ExactParams &p, unsigned c, unsigned n_seg, float inv0, float inv1, bool wide, const ExactRow r,
+                                             const float4 *col, int n, int oy, int ox, bool valid, int64_t pix, int co) {
+  constexpr unsigned CB = HW, HB = HW / 2;
+  auto f = [&](float4 v) { return make_float4(tc_act<ACT>(p.act, v.x), tc_act<ACT>(p.act, v.y), tc_act<ACT>(p.act, v.z), tc_act<ACT>(p.act, v.w)); };
+  const float *addend = p.addend && valid ? p.addend + pix * p.addend_ps + co : nullptr;
+  const bool thresholded = STEP && (p.c.thr > 0.0f || p.c.emitted);
+  bool sent = !STEP;
+  float top = 0.0f;
+#pragma unroll 1
+  for (unsigned g = 0; g < HW / 8; ++g) {
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
+#pragma unroll 1
+    for (unsigned j = 0; j < n_seg; ++j) {
+      const unsigned at = c + j * 3u * CB, ch = 8u * g, hi = at + ch / HB * CB + ch % HB;
+      const float inv = j ? inv1 : inv0;
+      unsigned a[8], b[8], d[8];
+      tmem_ld8_async(hi, a);
+      tmem_ld8_async(hi + HB, b);
+      tmem_ld8_async(at + 2u * CB + ch, d);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(fmaf(__uint_as_float(b[i]) + __uint_as_float(d[i]), SPLIT_LO, __uint_as_float(a[i])), inv, acc[i]);
+    }
+#pragma unroll
+    for (unsigned i = 0; i < 2; ++i) {
+      const unsigned h = 2u * g + i, at = (h ^ r.sw) << 4;
+      const int ch = (int)(4u * h);
+      const bool real = co + ch < p.cout;
+      const float4 w = lds4(smem_u32(col + h));
+      float4 v = make_float4(acc[4 * i] * w.x, acc[4 * i + 1] * w.y, acc[4 * i + 2] * w.z, acc[4 * i + 3] * w.w);
+      if (wide || w.x != w.x || w.y != w.y || w.z != w.z || w.w != w.w) {
+        v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (valid && real) exact_fp32_quad(p, n, oy, ox, co + ch, v);
+      }
+      if (!STEP && p.bias) v = f4add(v, lds4(smem_u32(col + HW / 4 + h)));
+      if (addend && real) v = f4add(v, *reinterpret_cast<const float4 *>(addend + ch));
+      if (!STEP) {
+        if (ACT != MIE_ACT_NONE) sts4(r.res + at, v);
+        v = f(v);
+      } else if (ACT != MIE_ACT_NONE) {
+        const float4 x = lds4(r.res + at), xn = f4add(x, v), b = p.c.emitted ? lds4(r.em + at) : f(x), y = f(xn);
+        v = make_float4(y.x - b.x, y.y - b.y, y.z - b.z, y.w - b.w);
+        sts4(r.res + at, xn);
+      }
+      sts4(r.out + at, v);
+      if (STEP && real) top = fmaxf(top, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
+    if (STEP && (g & 1u)) {      // a group of 16 channels is complete
+      const bool flag = top > p.c.thr;
+      if (thresholded && !flag)
+#pragma unroll
+        for (unsigned i = 0; i < 4; ++i) sts4(r.out + (((2u * g - 2u + i) ^ r.sw) << 4), make_float4(0.f, 0.f, 0.f, 0.f));
+      sent |= flag;
+      top = 0.0f;
+    }
+  }
+  return sent;
+}
+
+// HW: channels that a thread of the epilogue finishes.  ALT: the two sets of epilogue warps take items in turn (CB = HW channels per
+// block), else halves of each item's channels (CB = 2 HW).  STEP: a step (incremental activation, threshold, carry) instead of the dense
+// pass.
+template <int HW, bool STEP, bool ALT>
 __global__ void __launch_bounds__(EXACT_THREADS, 1)
 conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__ ExactMaps maps) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int CB = 2 * HW;
-  constexpr unsigned half_bytes = HW * 64u, tap_bytes = 2u * half_bytes;   // this block's rows of one tap: [hi | lo] of its half of the channels
+  constexpr int CB = ALT ? HW : 2 * HW, HB = CB / 2;      // HB: filter rows of a tap in this block, of either part
+  constexpr unsigned half_bytes = HB * 64u, tap_bytes = 2u * half_bytes;   // this block's rows of one tap: [hi | lo] of its half of the channels
   const unsigned row_bytes = (unsigned)p.wp * 128u;
   const unsigned halo_bytes = ((unsigned)p.wp * 2u * row_bytes + 1023u) & ~1023u;
   const unsigned stage_bytes = tap_bytes * (unsigned)p.tps;
   __shared__ unsigned long long b_full[EXACT_MAX_STAGES], done[EXACT_MAX_STAGES], a_full[EXACT_MAX_HALOS], a_ready[EXACT_MAX_HALOS],
-      a_empty[EXACT_MAX_HALOS], seg_empty[5];
+      a_empty[EXACT_MAX_HALOS], seg_empty[5], slab_full[2][2], item_full[2];
   __shared__ SplitShared s_split;
   __shared__ PairTapTable s_tap;
   __shared__ float4 s_col[2][2][HW / 4];      // per epilogue set: inverse scales and biases of its channels
@@ -187,7 +302,10 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
   if (tid == 0) {
     for (int s = 0; s < p.stages; ++s) { mbar_init(&b_full[s], 1); mbar_init(&done[s], 1); }
     for (int s = 0; s < p.halos; ++s) { mbar_init(&a_full[s], 1); mbar_init(&a_ready[s], 2 * SPLIT_WARPS); mbar_init(&a_empty[s], 1); }
-    for (int b = 0; b < p.segs; ++b) mbar_init(&seg_empty[b], 16);
+    for (int b = 0; b < p.segs; ++b) mbar_init(&seg_empty[b], ALT ? 8 : 16);
+    if (ALT) { mbar_init(&item_full[0], 1); mbar_init(&item_full[1], 1); }
+    if (STEP)
+      for (int b = 0; b < 4; ++b) mbar_init(&slab_full[b >> 1][b & 1], 2);
     for (unsigned u = 0; u < SPLIT_RING; ++u) mbar_init(&s_split.inv_full[u], 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -208,8 +326,9 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
   grid_dependency_wait();
   grid_dependency_trigger();
 
-  const int n_active = __shfl_sync(0xffffffffu, min(p.counts[0], p.max_tiles), 0);
-  const int n_cblk = p.cout_pad / CB, n_items = ((n_active + 3) >> 2) * n_cblk;
+  const int n_cblk = p.cout_pad / CB;
+  const int n_active = __shfl_sync(0xffffffffu, min(p.counts[0], p.max_tiles), 0);     // uniform, for the compiler too
+  const int n_items = ((n_active + 3) >> 2) * n_cblk;
   const unsigned b_base = smem_u32(smem), a_base = b_base + (((unsigned)p.stages * stage_bytes + 1023u) & ~1023u);
   const int nv = p.t.nviews;
 
@@ -222,7 +341,7 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
   } else if (warp == 1) {
     // =========================== filter producer: hi and lo rows of a tap ===========================
     const PairRing ring = {b_full, done, b_base, stage_bytes, (unsigned)p.stages};
-    pair_produce_filter(work, ring, p.t, p.tps, tap_bytes, (int)crank * HW, CB, &s_abort, [](int u) { return u; }, [&](int) { return 2u * tap_bytes; },
+    pair_produce_filter(work, ring, p.t, p.tps, tap_bytes, (int)crank * HB, CB, &s_abort, [](int u) { return u; }, [&](int) { return 2u * tap_bytes; },
                         [&](int, int tap, unsigned dst, unsigned bar, int row, int chunk) {
                           tma_load_4d_pair(dst, &maps.w, bar, 0, row, chunk, tap);
                           tma_load_4d_pair(dst + half_bytes, &maps.w, bar, 0, p.cout_pad + row, chunk, tap);
@@ -232,13 +351,13 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
     if (crank == 0u) {
       const ExactIssue a = {bid, nblk, n_items, p.n_chunks, p.cin, p.tps, nv, tmem_base, a_base, b_base, row_bytes, halo_bytes, stage_bytes, (unsigned)p.stages,
                             (unsigned)p.halos, (unsigned)p.segs, p.spin_limit};
-      exact_issue<CB>(a, s_tap, b_full, done, a_ready, a_empty, seg_empty, &s_abort);
+      exact_issue<CB, ALT>(a, s_tap, b_full, done, a_ready, a_empty, seg_empty, item_full, &s_abort);
     }
   } else if (warp >= 12) {
     // =========================== halos as two FP16 parts ===========================
     pair_split_halos(work, halos, a_ready, 2 * p.wp * p.wp, p.wp, n_active, tid - 384, s_split, &s_abort);
   } else if (warp >= 4) {
-    // =========================== epilogue: set `set` takes channels [set * HW, set * HW + HW) of the block ===========================
+    // =========================== epilogue: set `set` takes channels [set * HW, set * HW + HW) of the block, or every other item ===========================
     const int q = warp & 3, set = (warp - 4) >> 2;
     const int slot = (lane >> 3) & 1, prow = 2 * q + (lane >> 4), pcol = lane & 7;
     const unsigned lane_base = tmem_base + ((unsigned)(q * 32) << 16);
@@ -246,90 +365,181 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
     // 128 bytes (piece ^ (row & 7)) or 64 bytes (piece ^ (row / 2 & 3))
     constexpr unsigned SLAB = 128u * HW * 4u;
     const int row = slot * 64 + prow * 8 + pcol, sw = HW == 32 ? row & 7 : (row >> 1) & 3;
-    const unsigned slab = a_base + (unsigned)p.halos * halo_bytes + (unsigned)set * (p.act != MIE_ACT_NONE ? 2u : 1u) * SLAB;
-    const unsigned out_row = slab + (unsigned)row * (HW * 4u), res_row = out_row + SLAB;
-    const bool chief = q == 0 && elect_one();
-    unsigned seg = 0, stage = 0, stage_par = 0, unit = 0;
+    // output | reservoir | carry, once or twice
+    const unsigned set_bytes = (unsigned)p.slab_bufs * SLAB, slabs = a_base + (unsigned)p.halos * halo_bytes + (unsigned)(set * p.slab_sets) * set_bytes;
+    // the copies of slot s are issued by lane 8 s (whose pixel lies in it) of warp s of the set
+    const bool chief = q < 2 && lane == 8 * q, has_res = p.act != MIE_ACT_NONE;
+    if constexpr (STEP) tc_zero_stale(p.c, ntiles_total, THo, TWo, tid - 128, 256);
+    // units and segments of an item; with ALT a set skips the other one's
+    const int units = p.n_chunks * nv;
+    unsigned n_seg = 0;
+    for (int v = 0; v < nv; ++v) n_seg += (unsigned)((p.t.first[v + 1] - p.t.first[v] + p.tps - 1) / p.tps);
+    n_seg *= (unsigned)p.n_chunks;
+    unsigned seg = ALT ? (unsigned)set * n_seg : 0u, stage = 0, stage_par = 0, unit = ALT ? (unsigned)(set * units) : 0u, item_idx = 0;
     bool ok = true;
-    for (int item = bid; item < n_items && ok; item += nblk) {
-      // What the end of the item needs from global memory is asked for here and first looked at behind the segments: with a chain of
-      // loads at the end (list, scales, biases, list again) it took 5000 clocks, in which no segment is taken and the issuer stands
-      // still.
-      const int quad = item / n_cblk, cb = item - quad * n_cblk, co = cb * CB + set * HW;
-      const int e = 4 * quad + 2 * (int)crank + slot, at_col = q * 32 + lane;
-      const int listed = e < n_active ? p.list[e] : -1;
-      const float col = at_col < HW ? __ldg(p.winv + co + at_col) : (at_col < 2 * HW && p.bias && co + at_col - HW < p.cout) ? __ldg(p.bias + co + at_col - HW) : 0.0f;
-      float acc[HW];
-      bool wide = false;
-#pragma unroll
-      for (int i = 0; i < HW; ++i) acc[i] = 0.0f;
-      for (int cu = 0; cu < p.n_chunks * nv && ok; ++cu, ++unit) {
-        const int v = nv == 1 ? 0 : cu % nv;
-        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&s_split.inv_full[unit % SPLIT_RING], (unit / SPLIT_RING) & 1u, &s_abort, p.spin_limit)))) break;
-        const float inv = s_split.inv[unit % SPLIT_RING];
-        for (int left = p.t.first[v + 1] - p.t.first[v]; left > 0; left -= p.tps) {
-          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&done[stage], stage_par, &s_abort, p.spin_limit)))) break;
-          tc_fence_after();
-          const unsigned c = lane_base + seg * (3u * CB), own = c + (unsigned)set * CB;      // [hi | mid] columns of this set's channels
-          tmem_add_split<HW>(own, own + HW, c + 2u * CB + (unsigned)set * HW, inv, acc);
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&seg_empty[seg]), 0));
-          if (++seg == (unsigned)p.segs) seg = 0;
-          if (++stage == (unsigned)p.stages) { stage = 0; stage_par ^= 1u; }
-        }
-        wide |= inv != inv;
+    const int first = ALT ? bid + set * nblk : bid, step = ALT ? 2 * nblk : nblk;
+    auto column = [&](int item) { return (n_cblk == 1 ? 0 : item % n_cblk) * CB + (ALT ? 0 : set * HW); };
+    auto entry = [&](int item) {      // this lane's tile of an item
+      const int e = 4 * (n_cblk == 1 ? item : item / n_cblk) + 2 * (int)crank + slot, t = item < n_items && e < n_active ? p.list[e] : -1;
+      return t < ntiles_total ? t : -1;
+    };
+    auto place = [&](int t, int &x, int &y, int &n) {
+      const int r = p.div_tw ? (int)__umulhi((unsigned)t, p.div_tw) : t / TWo;
+      n = p.div_th ? (int)__umulhi((unsigned)r, p.div_th) : r / THo;
+      x = (t - r * TWo) * 8; y = (r - n * THo) * 8;
+    };
+    auto buffer = [&](unsigned idx) { return slabs + (p.slab_sets == 2 ? idx & 1u : 0u) * set_bytes; };
+    auto slab_bar = [&](unsigned idx) { return &slab_full[set][p.slab_sets == 2 ? idx & 1u : 0u]; };
+    // a chief asks for its tile's state for item `idx`, once the stores that last used the buffer have read it
+    auto fetch_state = [&](int item, int t, unsigned idx) {
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      const int co = column(item);
+      const unsigned bar = smem_u32(slab_bar(idx)), at = buffer(idx) + SLAB + (unsigned)slot * (SLAB / 2);
+      const unsigned bytes = has_res && co < p.cout && t >= 0 ? (SLAB / 2) * (p.c.emitted ? 2u : 1u) : 0u;
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+      if (bytes) {
+        int x, y, n;
+        place(t, x, y, n);
+        tma_load_4d_raw(at, &maps.res, bar, co, x, y, n);
+        if (p.c.emitted) tma_load_4d_raw(at + SLAB, &maps.emitted, bar, co, x, y, n);
       }
-      const int t = listed < ntiles_total ? listed : -1;
-      const int tx = (t >= 0) ? (t % TWo) * 8 : 0, ty = (t >= 0) ? ((t / TWo) % THo) * 8 : 0, n = (t >= 0) ? t / (TWo * THo) : 0;
+    };
+    int listed = entry(first);
+    if (STEP && chief && first < n_items) fetch_state(first, listed, 0u);
+    __syncwarp();
+    for (int item = first; item < n_items && ok; item += step, ++item_idx) {
+      // What the end of the item needs from global memory is asked for here and first looked at behind the segments.  The end of an
+      // item is what bounds layers of few units per item (32 -> 32 3x3: the nine taps take 1500 clocks, the end took 6500 with the
+      // state asked for at the item's start, divisions, one thread for all copies, and a load and a store in turn).
+      const int co = column(item), at_col = q * 32 + lane, t = listed;
+      listed = entry(item + step);
+      const float col = at_col < HW ? __ldg(p.winv + co + at_col) : (at_col < 2 * HW && p.bias && co + at_col - HW < p.cout) ? __ldg(p.bias + co + at_col - HW) : 0.0f;
+      int tx = 0, ty = 0, n = 0;
+      if (t >= 0) place(t, tx, ty, n);
       const bool valid = t >= 0 && ty + prow < p.hout && tx + pcol < p.wout;
       const int64_t pix = valid ? (int64_t)(n * p.hout + ty + prow) * p.wout + tx + pcol : 0;
-      if (at_col < 2 * HW) reinterpret_cast<float *>(s_col[set][at_col / HW])[at_col % HW] = col;
-      // a warp whose wait gave up goes on to the barrier of its set, where the four of them leave together;
-      // the slabs are free once the previous item's stores have read them
-      if (chief) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-      __syncwarp();
-      ok = set_all(1 + set, ok);
-      if (!ok) break;
+      const unsigned slab = buffer(item_idx), out_row = slab + (unsigned)row * (HW * 4u), res_row = out_row + SLAB, em_row = res_row + SLAB;
+      bool sent = false;
+      if constexpr (!ALT) {
+        float acc[HW];
+        bool wide = false;
 #pragma unroll
-      for (int h = 0; h < HW / 4; ++h) {
-        const float4 f = lds4(smem_u32(&s_col[set][0][h]));
-        acc[4 * h] *= f.x; acc[4 * h + 1] *= f.y; acc[4 * h + 2] *= f.z; acc[4 * h + 3] *= f.w;
-        wide |= f.x != f.x || f.y != f.y || f.z != f.z || f.w != f.w;
-      }
-      if (wide) exact_fp32<HW>(p, n, ty + prow, tx + pcol, valid, co, acc);
-#pragma unroll
-      for (int h = 0; h < HW / 4; ++h) {
-        const int c = co + 4 * h;
-        float4 v = make_float4(acc[4 * h], acc[4 * h + 1], acc[4 * h + 2], acc[4 * h + 3]);
-        if (p.bias) v = f4add(v, lds4(smem_u32(&s_col[set][1][h])));
-        if (p.addend && valid && c < p.cout) v = f4add(v, *reinterpret_cast<const float4 *>(p.addend + pix * p.addend_ps + c));
-        const unsigned at = (unsigned)(h ^ sw) << 4;
-        if (p.act != MIE_ACT_NONE) {
-          sts4(res_row + at, v);
-          v = p.act == MIE_ACT_RELU ? make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f))
-                                    : make_float4(tc_act_call(p.act, v.x), tc_act_call(p.act, v.y), tc_act_call(p.act, v.z), tc_act_call(p.act, v.w));
+        for (int i = 0; i < HW; ++i) acc[i] = 0.0f;
+        for (int cu = 0; cu < units && ok; ++cu, ++unit) {
+          const int v = nv == 1 ? 0 : cu % nv;
+          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&s_split.inv_full[unit % SPLIT_RING], (unit / SPLIT_RING) & 1u, &s_abort, p.spin_limit)))) break;
+          const float inv = s_split.inv[unit % SPLIT_RING];
+          for (int left = p.t.first[v + 1] - p.t.first[v]; left > 0; left -= p.tps) {
+            if (!(ok = __all_sync(0xffffffffu, mbar_wait(&done[stage], stage_par, &s_abort, p.spin_limit)))) break;
+            tc_fence_after();
+            const unsigned c = lane_base + seg * (3u * CB), own = c + (unsigned)set * CB;      // [hi | mid] columns of this set's channels
+            tmem_add_split<HW>(own, own + HW, c + 2u * CB + (unsigned)set * HW, inv, acc);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&seg_empty[seg]), 0));
+            if (++seg == (unsigned)p.segs) seg = 0;
+            if (++stage == (unsigned)p.stages) { stage = 0; stage_par ^= 1u; }
+          }
+          wide |= inv != inv;
         }
-        sts4(out_row + at, v);
+        if (at_col < 2 * HW) reinterpret_cast<float *>(s_col[set][at_col / HW])[at_col % HW] = col;
+        // a warp whose wait gave up goes on to the barrier of its set, where the four of them leave together
+        if (!STEP && chief) {      // the buffer is free once the stores of its last item have read it
+          if (p.slab_sets == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        }
+        if (STEP) {
+          if (chief && p.slab_sets == 2 && item + step < n_items) fetch_state(item + step, listed, item_idx + 1u);
+          __syncwarp();
+          if (ok) ok = mbar_wait(slab_bar(item_idx), (p.slab_sets == 2 ? item_idx >> 1 : item_idx) & 1u, &s_abort, p.spin_limit);
+        }
+        __syncwarp();
+        ok = set_all(1 + set, ok);
+        if (!ok) break;
+#pragma unroll
+        for (int h = 0; h < HW / 4; ++h) {
+          const float4 f = lds4(smem_u32(&s_col[set][0][h]));
+          acc[4 * h] *= f.x; acc[4 * h + 1] *= f.y; acc[4 * h + 2] *= f.z; acc[4 * h + 3] *= f.w;
+          wide |= f.x != f.x || f.y != f.y || f.z != f.z || f.w != f.w;
+        }
+        if (wide) exact_fp32<HW>(p, n, ty + prow, tx + pcol, valid, co, acc);
+        sent = valid;
+        if constexpr (!STEP) {
+#pragma unroll
+          for (int h = 0; h < HW / 4; ++h) {
+            const int c = co + 4 * h;
+            float4 v = make_float4(acc[4 * h], acc[4 * h + 1], acc[4 * h + 2], acc[4 * h + 3]);
+            if (p.bias) v = f4add(v, lds4(smem_u32(&s_col[set][1][h])));
+            if (p.addend && valid && c < p.cout) v = f4add(v, *reinterpret_cast<const float4 *>(p.addend + pix * p.addend_ps + c));
+            const unsigned at = (unsigned)(h ^ sw) << 4;
+            if (p.act != MIE_ACT_NONE) {
+              sts4(res_row + at, v);
+              v = p.act == MIE_ACT_RELU ? make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f))
+                                        : make_float4(tc_act_call(p.act, v.x), tc_act_call(p.act, v.y), tc_act_call(p.act, v.z), tc_act_call(p.act, v.w));
+            }
+            sts4(out_row + at, v);
+          }
+        } else {
+          // one stretch of code per activation: what is run once per item runs out of the instruction cache
+          const ExactRow r = {res_row, out_row, em_row, (unsigned)sw};
+          const float *ad = p.addend && valid ? p.addend + pix * p.addend_ps : nullptr;
+          if (p.act == MIE_ACT_RELU) sent = exact_step<HW, MIE_ACT_RELU>(p, acc, r, ad, co);
+          else if (p.act == MIE_ACT_NONE) sent = exact_step<HW, MIE_ACT_NONE>(p, acc, r, ad, co);
+          else sent = exact_step<HW, MIE_ACT_SIGMOID>(p, acc, r, ad, co);
+          sent = sent && valid;
+        }
+      } else {
+        ok = __all_sync(0xffffffffu, mbar_wait(&item_full[set], item_idx & 1u, &s_abort, p.spin_limit));
+        float inv[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const unsigned u = unit + (n_seg == 2u ? (unsigned)(j * units) >> 1 : 0u);
+          ok = __all_sync(0xffffffffu, ok && mbar_wait(&s_split.inv_full[u % SPLIT_RING], (u / SPLIT_RING) & 1u, &s_abort, p.spin_limit));
+          inv[j] = s_split.inv[u % SPLIT_RING];
+        }
+        unit += 2u * (unsigned)units;
+        if (at_col < 2 * HW) reinterpret_cast<float *>(s_col[set][at_col / HW])[at_col % HW] = col;
+        // a warp whose wait gave up goes on to the barrier of its set, where the four of them leave together
+        if (!STEP && chief) {      // the buffer is free once the stores of its last item have read it
+          if (p.slab_sets == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        }
+        if (STEP) {
+          if (chief && p.slab_sets == 2 && item + step < n_items) fetch_state(item + step, listed, item_idx + 1u);
+          __syncwarp();
+          if (ok) ok = mbar_wait(slab_bar(item_idx), (p.slab_sets == 2 ? item_idx >> 1 : item_idx) & 1u, &s_abort, p.spin_limit);
+        }
+        __syncwarp();
+        ok = set_all(1 + set, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const ExactRow r = {res_row, out_row, em_row, (unsigned)sw};
+        const bool wide = inv[0] != inv[0] || inv[1] != inv[1];
+        const unsigned c = lane_base + seg * (3u * CB);
+        if (p.act == MIE_ACT_RELU) sent = exact_finish<HW, STEP, MIE_ACT_RELU>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
+        else if (p.act == MIE_ACT_NONE) sent = exact_finish<HW, STEP, MIE_ACT_NONE>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
+        else sent = exact_finish<HW, STEP, MIE_ACT_SIGMOID>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
+        sent = sent && valid;
+        tc_fence_before();
+        __syncwarp();
+        for (unsigned j = 0; j < n_seg; ++j)
+          if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&seg_empty[seg + j]), 0));
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");
-      // the tiles of both slots lie in every warp (lanes 0 and 8)
-      const int t0 = __shfl_sync(0xffffffffu, t, 0), t1 = __shfl_sync(0xffffffffu, t, 8), x0 = __shfl_sync(0xffffffffu, tx, 0), x1 = __shfl_sync(0xffffffffu, tx, 8),
-                y0 = __shfl_sync(0xffffffffu, ty, 0), y1 = __shfl_sync(0xffffffffu, ty, 8), n0 = __shfl_sync(0xffffffffu, n, 0), n1 = __shfl_sync(0xffffffffu, n, 8);
-      if (chief && co < p.cout) {
-        if (t0 >= 0) {
-          tma_store_slab(slab, &maps.out, co, x0, y0, n0);
-          if (p.act != MIE_ACT_NONE) tma_store_slab(slab + SLAB, &maps.res, co, x0, y0, n0);
+      if (chief) {
+        if (co < p.cout && t >= 0) {
+          const unsigned half = (unsigned)slot * (SLAB / 2);
+          tma_store_slab(slab + half, &maps.out, co, tx, ty, n);
+          if (has_res) tma_store_slab(slab + SLAB + half, &maps.res, co, tx, ty, n);
+          if (STEP && p.c.emitted) tma_add_slab(slab + half, &maps.emitted, co, tx, ty, n);   // the carry advances by what was sent
         }
-        if (t1 >= 0) {
-          tma_store_slab(slab + SLAB / 2, &maps.out, co, x1, y1, n1);
-          if (p.act != MIE_ACT_NONE) tma_store_slab(slab + SLAB + SLAB / 2, &maps.res, co, x1, y1, n1);
-        }
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");      // (also without a copy: the waits count groups)
       }
-      // every pixel written is marked; ballot bytes: [tile 0 row 2q][tile 1 row 2q][tile 0 row 2q+1][tile 1 row 2q+1]
-      const unsigned bal = __ballot_sync(0xffffffffu, valid);
+      if (STEP && chief && p.slab_sets == 1 && item + step < n_items) fetch_state(item + step, listed, item_idx + 1u);
+      __syncwarp();
+      // the pixels sent (dense: every pixel written); ballot bytes: [tile 0 row 2q][tile 1 row 2q][tile 0 row 2q+1][tile 1 row 2q+1]
+      const unsigned bal = __ballot_sync(0xffffffffu, sent);
       if ((lane == 0 || lane == 8) && t >= 0) {
         const unsigned rows = ((bal >> lane) & 0xFFu) | (((bal >> (16 + lane)) & 0xFFu) << 8);
         if (rows) atomicOr(p.out_bits32 + 2 * (size_t)t + (q >> 1), rows << ((q & 1) * 16));
@@ -363,7 +573,8 @@ static inline int64_t exact_scales_at(int cin, int cout_pad, int k) { return (in
 // How a launch divides its columns and its shared memory; `stages` < 2: no split of it fits.
 struct ExactShape {
   PairTaps t;
-  int wp, cb, tps, stages, halos, segs;
+  int wp, cb, hw, tps, stages, halos, segs, slab_bufs, slab_sets;   // hw: channels of an epilogue thread
+  bool alt;
   size_t smem;
 };
 static ExactShape exact_shape(const mie_conv_args *a) {
@@ -376,16 +587,27 @@ static ExactShape exact_shape(const mie_conv_args *a) {
   if (a->cout_pad % 64 == 0 &&
       (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 100 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 75)
     h.cb = 64;
-  const int halo_bytes = (h.wp * 2 * h.wp * 128 + 1023) & ~1023, slab_bytes = 2 * (a->act != MIE_ACT_NONE ? 2 : 1) * 128 * (h.cb / 2) * 4;
-  const int budget = 222 * 1024 - slab_bytes;
   // Taps of a segment: its truncation grows with its additions, one per 16 channels and tap, the FP32 kernel's rounding with the whole
-  // reduction.  The longest whose error is not above the FP32 kernel's, nor above that of the two TF32 parts that stood here, for
+  // reduction.  Dense: the longest whose error is not above the FP32 kernel's, nor above that of the two TF32 parts that stood here, for
   // rectified inputs (segments of 3 / 5 / 9 taps over the FP32 kernel's error: 125 products 0.84 / 0.91 / 1.16, 288 0.75 / 0.99 / 1.68, 576
-  // 0.53 / 0.70 / 1.22, 1152 0.40 / 0.52 / 0.88, 1600 0.36 / 0.47 / 0.71, 2304 0.29 / 0.36 / 0.60).
-  const int depth = a->cin * a->k * a->k, most = depth < 100 ? 2 : depth < 400 ? (a->cin > 16 ? 3 : 5) : depth < 1600 ? 5 : 9;
-  int taps = 0;
+  // 0.53 / 0.70 / 1.22, 1152 0.40 / 0.52 / 0.88, 1600 0.36 / 0.47 / 0.71, 2304 0.29 / 0.36 / 0.60).  A step's result is a change, whose
+  // error is a fraction of the state's, and its three blocks of TF32 channels were never summed in segments at all.
+  const int depth = a->cin * a->k * a->k;
+  const int most = !a->refresh ? 9 : depth < 100 ? 2 : depth < 400 ? (a->cin > 16 ? 3 : 5) : depth < 1600 ? 5 : 9;
+  int taps = 0, n_seg = 0;
   for (int v = 0; v < h.t.nviews; ++v) taps = std::max(taps, h.t.first[v + 1] - h.t.first[v]);
   h.tps = divup(taps, divup(taps, most));
+  for (int v = 0; v < h.t.nviews; ++v) n_seg += divup(h.t.first[v + 1] - h.t.first[v], h.tps);
+  n_seg *= divup(a->cin, 32);
+  // Items of one or two segments are bound by what follows them, a chain of about 7000 clocks: two of them are in hand at once then
+  // (all segments of both in tensor memory).
+  h.alt = h.cb == 32 && n_seg <= 2;
+  h.hw = h.alt ? 32 : h.cb / 2;
+  h.slab_bufs = 1 + (a->act != MIE_ACT_NONE) + (a->emitted != nullptr);
+  // two buffers of slabs where they are small: the state of an item then arrives, and its results leave, while another is computed
+  h.slab_sets = h.hw == 16 ? 2 : 1;
+  const int halo_bytes = (h.wp * 2 * h.wp * 128 + 1023) & ~1023, slab_bytes = 2 * h.slab_sets * h.slab_bufs * 128 * h.hw * 4;
+  const int budget = 222 * 1024 - slab_bytes;
   // Units of a single stage (3x3) need halo buffers more than stages: load, split and instructions of a unit are three links of a chain
   // (res 256 -> 256: three halos and two stages 144 us, two and three 157).  Longer ones need the filter ahead (64 -> 32 5x5: 787 us with
   // three halos and four stages, 939 with four and two).
@@ -395,19 +617,22 @@ static ExactShape exact_shape(const mie_conv_args *a) {
   while (h.tps > 1 && budget - h.halos * halo_bytes < 2 * h.tps * h.cb * 64) --h.tps;
   const int stage_bytes = h.tps * h.cb * 64;
   h.stages = std::min((budget - h.halos * halo_bytes) / stage_bytes, EXACT_MAX_STAGES);
-  h.segs = std::min(h.stages, (int)exact_segs(h.cb));      // the epilogue learns of a segment from its stage's barrier
+  // ... two items' worth with `alt`: an item's barrier is not signalled again before its set has looked at it
+  h.segs = h.alt ? 2 * n_seg : std::min(h.stages, (int)exact_segs(h.cb));      // the epilogue learns of a segment from its stage's barrier
   h.smem = (size_t)((h.stages * stage_bytes + 1023) & ~1023) + (size_t)h.halos * halo_bytes + slab_bytes + 1024;
   return h;
 }
 
+// A dense evaluation (`refresh`), or a step of a layer in split precision, that the kernel takes.
 bool exact_takes(const mie_conv_args *a) {
   // a field one pixel wide or high has no odd columns or rows: that parity view of stride 2 would be empty, and a tensor map
   // cannot say so
   if (a->stride == 2 && (a->hin == 1 || a->win == 1)) return false;
-  return a->refresh && !a->head && a->wpacked_exact && a->k >= 3 && a->k <= 7 && (a->k & 1) && (a->stride == 1 || a->stride == 2) && !a->in2 && !a->accum &&
+  if (a->refresh ? a->head != nullptr : (a->bias || ((a->thr > 0.0f || a->emitted) && !g_opt_tc_thresholded))) return false;
+  return a->wpacked_exact && a->k >= 3 && a->k <= 7 && (a->k & 1) && (a->stride == 1 || a->stride == 2) && !a->in2 && !a->accum &&
          a->in_ps % 4 == 0 && aligned16(a->in) && aligned16(a->wpacked_exact) && a->cout % 4 == 0 && a->out_ps % 4 == 0 &&
          aligned16(a->out) && (!a->res || (a->res_ps % 4 == 0 && aligned16(a->res))) && (!a->addend || (a->addend_ps % 4 == 0 && aligned16(a->addend))) &&
-         a->cout_pad % 32 == 0 && exact_shape(a).stages >= 2;
+         (!a->emitted || (a->emitted_ps % 4 == 0 && aligned16(a->emitted))) && a->cout_pad % 32 == 0 && exact_shape(a).stages >= 2;
 }
 
 // fw: the filter in fp32, entry (tap, ci, co) at fw[tap * fw_tap + ci * fw_ci + co]
@@ -426,7 +651,11 @@ int launch_conv_exact(const mie_conv_args *a, const float *fw, int64_t fw_tap, i
   p.out = a->out; p.out_ps = a->out_ps; p.out_bits32 = reinterpret_cast<unsigned int *>(a->out_bits);
   p.act = a->act; p.res = a->res; p.res_ps = a->res_ps; p.addend = a->addend; p.addend_ps = a->addend_ps; p.bias = a->bias;
   p.tail = tail_for_kernel(a->tail);
-  p.t = h.t; p.wp = h.wp; p.cb = h.cb; p.tps = h.tps; p.stages = h.stages; p.halos = h.halos; p.segs = h.segs;
+  p.t = h.t; p.wp = h.wp; p.cb = h.cb; p.tps = h.tps; p.stages = h.stages; p.halos = h.halos; p.segs = h.segs; p.slab_bufs = h.slab_bufs; p.slab_sets = h.slab_sets;
+  // n / d = high word of n * ceil(2^32 / d), exact while n * d < 2^32
+  const unsigned tw = (unsigned)divup(a->wout, 8), th = (unsigned)divup(a->hout, 8);
+  auto magic = [&](unsigned d) { return d > 1 && (uint64_t)a->n * tw * th * d < (1ull << 32) ? (unsigned)(((1ull << 32) + d - 1) / d) : 0u; };
+  p.div_tw = magic(tw); p.div_th = magic(th);
   const size_t smem = h.smem;
   const int quads = divup(a->max_tiles, 4), clusters_max = MIE_SM_COUNT / 2;
 
@@ -449,26 +678,45 @@ int launch_conv_exact(const mie_conv_args *a, const float *fw, int64_t fw_tap, i
     if (!tc_encode(&maps.w, 4, a->wpacked_exact, dims, str, box_w, CU_TENSOR_MAP_SWIZZLE_64B)) return MIE_EINVAL;
   }
   {
-    // epilogue slabs: half a block's channels of one tile
-    const cuuint32_t box[4] = {(cuuint32_t)(p.cb / 2), 8, 8, 1};
-    const CUtensorMapSwizzle sw = p.cb == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+    // epilogue slabs: a set's channels of one tile
+    const cuuint32_t box[4] = {(cuuint32_t)h.hw, 8, 8, 1};
+    const CUtensorMapSwizzle sw = h.hw == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
     auto slab_map = [&](CUtensorMap *m, const float *base, int64_t ps) {
       const cuuint64_t dims[4] = {(cuuint64_t)a->cout, (cuuint64_t)a->wout, (cuuint64_t)a->hout, (cuuint64_t)a->n};
       const cuuint64_t str[3] = {(cuuint64_t)ps * 4, (cuuint64_t)a->wout * ps * 4, (cuuint64_t)a->hout * a->wout * ps * 4};
       return tc_encode(m, 4, base, dims, str, box, sw);
     };
-    if (!slab_map(&maps.out, a->out, a->out_ps) || (a->act != MIE_ACT_NONE && !slab_map(&maps.res, a->res, a->res_ps))) return MIE_EINVAL;
+    if (!slab_map(&maps.out, a->out, a->out_ps) || (a->act != MIE_ACT_NONE && !slab_map(&maps.res, a->res, a->res_ps)) ||
+        (a->emitted && !slab_map(&maps.emitted, a->emitted, a->emitted_ps)))
+      return MIE_EINVAL;
   }
-  const int64_t items = (int64_t)quads * (a->cout_pad / p.cb);
-  const int clusters = (int)(items < clusters_max ? items : clusters_max);
-  static int smem_set[2][MAX_DEVICES] = {{0}};
+  const int n_cblk = a->cout_pad / p.cb;
+  const int64_t items = (int64_t)quads * n_cblk;
+  int clusters = (int)(items < clusters_max ? items : clusters_max);
+  if (!a->refresh) {
+    TcParams &c = p.c;
+    c.thr = a->thr; c.emitted = a->emitted; c.stale = a->stale; c.counts = a->counts; c.max_tiles = a->max_tiles;
+    c.out = a->out; c.out_ps = a->out_ps; c.cout = a->cout; c.hout = a->hout; c.wout = a->wout;
+    if (a->head) {
+      // (a kernel that finds its own tiles was slower here: FireFlowNet's six layers 368 us a step, with the launches 346)
+      const mie_tail_job *j = a->head;
+      const int r = mie_tiles_dilate(j->in_bits, j->N, j->Hin, j->Win, j->Hout, j->Wout, j->k, j->stride, j->pad, j->union_bits, j->out_bits, j->list, j->stale,
+                                     j->counts, j->flags, st);
+      if (r != MIE_OK) return r;
+    }
+  }
+  static int smem_set[6][MAX_DEVICES] = {{0}};
   auto launch = [&](auto kernel, int i) {
     const int r = ensure_dynamic_smem(kernel, smem_set[i], smem);
     if (r != MIE_OK) return r;
     launch_chained_cluster(kernel, dim3((unsigned)(2 * clusters)), dim3(EXACT_THREADS), smem, st, 2, p, maps);
     return check_launch();
   };
-  return p.cb == 64 ? launch(conv_exact_kernel<32>, 1) : launch(conv_exact_kernel<16>, 0);
+  if (a->refresh)
+    return h.alt ? launch(conv_exact_kernel<32, false, true>, 0) : h.cb == 64 ? launch(conv_exact_kernel<32, false, false>, 1)
+                                                                              : launch(conv_exact_kernel<16, false, false>, 2);
+  return h.alt ? launch(conv_exact_kernel<32, true, true>, 3) : h.cb == 64 ? launch(conv_exact_kernel<32, true, false>, 4)
+                                                                           : launch(conv_exact_kernel<16, true, false>, 5);
 }
 
 // A field with a pixel stride or an address that TMA cannot read (5 bins of a voxel grid) as one it can: one read and one write.

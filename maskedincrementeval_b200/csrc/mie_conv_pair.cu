@@ -73,11 +73,6 @@ __device__ __forceinline__ void tmem_ld16_pair(unsigned taddr, unsigned taddr2, 
 __device__ __forceinline__ void tma_load_slab(unsigned smem_addr, const CUtensorMap *map, unsigned bar, int c0, int x, int y, int n) {
   tma_load_4d_raw(smem_addr, map, bar, c0, x, y, n);
 }
-__device__ __forceinline__ void tma_add_slab(unsigned smem_addr, const CUtensorMap *map, int c0, int x, int y, int n) {
-  asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-               ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_addr), "r"(c0), "r"(x), "r"(y), "r"(n) : "memory");
-}
-
 // One pixel, 16 channels (quads h0 .. h0 + 3 of a slab): v, the accumulator values; xs / es / os, shared addresses of the pixel's rows of the
 // reservoir, carry and output slabs (quad h of row r sits at h ^ (r & 7): the 128-byte swizzle of TMA).  Returns whether the
 // group was sent: a thresholded layer sends it when any of its channels moved by more than the threshold.
@@ -422,6 +417,18 @@ static int pair_block_width(const mie_conv_args *a) {
   return best;
 }
 
+// Own-tiles mode: the groups of n_cblk clusters that share the tiles out, or 0 for the separate dilation launch.
+// Not where several clusters finish a tile (kind 8, off by default): its word then goes through a scratch word and a
+// ticket per epilogue warp, which costs more than the launch it saves (gates 0 / 1 / 2, one stream: 27.8 / 25.6 / 24.0 us
+// against 23.6 / 23.1 / 22.2 us with the dilation launch).  Layers of 64 channels in two blocks keep the mode.
+// A group's share of the tiles must fit the list in its shared memory.
+int pair_own_groups(const mie_conv_args *a, int n_cblk, int clusters, int64_t ntiles) {
+  const int groups = clusters / n_cblk;
+  const int64_t pairs = ((int64_t)a->max_tiles + 1) / 2;
+  const int kind = n_cblk > 1 && a->cout_pad > 64 ? 8 : a->stride == 2 ? 1 : 4;
+  return (g_opt_own_kernels & kind) && groups >= 1 && 2 * ((pairs + groups - 1) / groups) <= OWN_MAX && a->max_tiles == ntiles ? groups : 0;
+}
+
 // Host-side rule; tc_eligible() has already accepted the layer.
 bool pair_takes(const mie_conv_args *a) { return a->k >= 3 && a->k <= 7; }
 
@@ -500,13 +507,9 @@ int launch_conv_pair(const mie_conv_args *a, cudaStream_t st) {
   const int64_t items = ((int64_t)a->max_tiles + 3) / 4 * n_cblk;
   int64_t clusters = items < MIE_SM_COUNT / 2 ? items : MIE_SM_COUNT / 2;
   if (a->own_tiles) {
-    // Not where several clusters finish a tile (kind 8, off by default): its word then goes through a scratch word and a
-    // ticket per epilogue warp, which costs more than the launch it saves (gates 0 / 1 / 2, one stream: 27.8 / 25.6 / 24.0 us
-    // against 23.6 / 23.1 / 22.2 us with the dilation launch).  Layers of 64 channels in two blocks keep the mode.
-    // Whole groups of n_cblk clusters; a group's share of the tiles must fit the list in its shared memory
-    const int64_t groups = clusters / n_cblk, sp = ((int64_t)a->max_tiles + 1) / 2;
     const int64_t ntiles = (int64_t)a->n * divup(a->hout, 8) * divup(a->wout, 8);
-    if ((g_opt_own_kernels & (n_cblk > 1 && a->cout_pad > 64 ? 8 : s == 2 ? 1 : 4)) && groups >= 1 && 2 * ((sp + groups - 1) / groups) <= OWN_MAX && a->max_tiles == ntiles) {
+    const int groups = pair_own_groups(a, n_cblk, (int)clusters, ntiles);
+    if (groups) {
       p.own = 1;
       p.head = *a->head;
       p.own_words = static_cast<unsigned long long *>(a->own_scratch);

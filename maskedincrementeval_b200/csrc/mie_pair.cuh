@@ -98,6 +98,11 @@ __device__ __forceinline__ void tma_store_slab(unsigned smem_addr, const CUtenso
                ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_addr), "r"(c0), "r"(x), "r"(y), "r"(n) : "memory");
 }
 
+__device__ __forceinline__ void tma_add_slab(unsigned smem_addr, const CUtensorMap *map, int c0, int x, int y, int n) {
+  asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+               ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_addr), "r"(c0), "r"(x), "r"(y), "r"(n) : "memory");
+}
+
 // Waits for three barriers at once (a barrier may be named twice): one round of their latency where three waits take three.
 __device__ __forceinline__ bool mbar_wait3(unsigned b0, unsigned p0, unsigned b1, unsigned p1, unsigned b2, unsigned p2, volatile int *abort_flag, unsigned limit) {
   for (unsigned it = 0; it < limit; ++it) {
@@ -345,6 +350,18 @@ __device__ __forceinline__ void sts4_if(unsigned addr, float4 v, bool on) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n\t}"
                ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"((unsigned)on) : "memory");
 }
+// The smallest magnitude but zero of the rows in `live` that start at r0 and r1.
+__device__ __noinline__ unsigned split_least(unsigned r0, unsigned r1, unsigned live) {
+  unsigned least = 0x7FFFFFFFu;
+  for (int it = 0; live >> it; ++it) {
+    if (!(live >> it & 1u)) continue;
+    const float4 a = lds4(r0 + (unsigned)(it * SPLIT_PASS * 128)), b = lds4(r1 + (unsigned)(it * SPLIT_PASS * 128));
+    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { const unsigned u = __float_as_uint(x[j]) & 0x7FFFFFFFu; if (u) least = min(least, u); }
+  }
+  return least;
+}
 __device__ __forceinline__ void pair_split_halos(const PairWork &w, const PairRing &r, unsigned long long *ready, int rows, int wp, int n_active, int t,
                                                  SplitShared &sh, volatile int *abort_flag) {
   const int lane = t & 31, cw = t >> 5, c = lane & 3;
@@ -388,15 +405,7 @@ __device__ __forceinline__ void pair_split_halos(const PairWork &w, const PairRi
       const unsigned mb = __float_as_uint(m);
       bool wide = false;
       if (mb >= 0x46800000u) {      // 2^14 or more: is it too much for what lies beside it?
-        unsigned least = 0x7FFFFFFFu;
-        auto scan = [&](const float *x) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) { const unsigned u = __float_as_uint(x[j]) & 0x7FFFFFFFu; if (u) least = min(least, u); }
-        };
-#pragma unroll
-        for (int it = 0; it < SPLIT_REGS; ++it) scan(v[it]);
-#pragma unroll 1
-        for (int it = SPLIT_REGS; it < passes; ++it) { float x[8]; read(it, x); scan(x); }
+        unsigned least = split_least(base + rd0, base + rd1, live);
         least = __reduce_min_sync(0xffffffffu, least);
         if (lane == 0) sh.least[cw] = least;
         set_all<32 * SPLIT_WARPS>(3, true);

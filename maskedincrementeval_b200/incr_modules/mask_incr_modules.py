@@ -424,7 +424,7 @@ class nnConvIncr(nn.Conv2d):
 
     def load_state_dict(self, state_dict: 'OrderedDict[str, torch.Tensor]', strict: bool = True):
         r = nn.Conv2d.load_state_dict(self, state_dict, strict=strict)
-        if self._packed:
+        if self._packed or self._packed_exact:
             fl.filter_epoch[0] += 1
         self._packed.clear()
         self._packed_exact.clear()
@@ -435,6 +435,8 @@ class nnConvIncr(nn.Conv2d):
         ver = (self.weight._version, self.weight.device, self.weight.data_ptr())
         hit = self._packed_exact.get(cin)
         if hit is None or hit[0] is not self.weight or hit[1] != ver:
+            if hit is not None:
+                fl.filter_epoch[0] += 1
             hit = self._packed_exact[cin] = (self.weight, ver, fl.pack_conv_weights_exact(self.weight[:, :cin]))
         return hit[2]
 
@@ -454,6 +456,19 @@ class nnConvIncr(nn.Conv2d):
             return True
         return (getattr(self, "precision", None) == "split" and cin * self._k * self._k >= 256
                 and self._k in (1, 3, 5, 7) and self._s in (1, 2))
+
+    def _split_copy(self, x_incr: Masked, d: torch.Tensor, m: TileMask, cin_limit: Optional[int]):
+        """The three channel blocks of an input in split precision, and how many channels they hold."""
+        n, cin, hin, win = d.shape
+        c3 = 3 * ((cin + 7) // 8 * 8)
+        d3 = self._scratch.get("split", (n, c3, hin, win), torch.float32, d.device, channels_last=True)
+        sb = self._scratch.get("split.bits", (fl.n_tiles(n, hin, win),), torch.int64, d.device)
+        # the producer of the delta (the driver's input-delta kernel) writes the copy itself once asked to
+        if not fl.split_made(d, d3):
+            fl.split_tf32(d, m, d3, sb)
+            if x_incr[1] is m and cin_limit is None:
+                fl.request_split(d, d3, sb)
+        return d3, c3
 
     def _filter_version(self, bn: "Optional[nn.BatchNorm2d]"):
         ver = (self.weight._version, self.weight.device, self.weight.data_ptr())
@@ -561,17 +576,14 @@ class nnConvIncr(nn.Conv2d):
         thresholded = activation is not None and (activation.thr() > 0.0 or
                                                   (config.carry and activation.emitted is not None))
         split = self._split_input(cin) and (config.tc_thresholded or not thresholded) and not refresh
+        # ... from two FP16 parts per operand, made inside the kernel, where it takes the layer (below); from three channel blocks of
+        # TF32 numbers elsewhere: 1x1 layers, layers with a folded batch-norm, and narrow inputs, whose three blocks fit one
+        # chunk (the 5-channel 5x5 head of eight 480x640 streams: 308 us, 440 in FP16 parts)
+        exact = split and bn is None and cin > 8 and self._k >= 3
+        split = split and not exact
         wbuf, cp, op, wtc = self._weights(cin_limit, split, bn)
         if split:
-            c3 = 3 * ((cin + 7) // 8 * 8)
-            d3 = sc.get("split", (n, c3, hin, win), torch.float32, d.device, channels_last=True)
-            sb = sc.get("split.bits", (fl.n_tiles(n, hin, win),), torch.int64, d.device)
-            # the producer of the delta (the driver's input-delta kernel) writes the copy itself once asked to
-            if not fl.split_made(d, d3):
-                fl.split_tf32(d, m, d3, sb)
-                if x_incr[1] is m and cin_limit is None:
-                    fl.request_split(d, d3, sb)
-            d, cin = d3, c3
+            d, cin = self._split_copy(x_incr, d, m, cin_limit)
         a = plan.args
         union = None
         a.in2, a.in2_ps = None, 0
@@ -620,7 +632,7 @@ class nnConvIncr(nn.Conv2d):
                                                plan.counts.data_ptr(), plan.flags.data_ptr(), st), "tiles_dilate")
             fl.offer_tail(job)
         a.in_, a.in_ps, a.cin = d.data_ptr(), fl.pixel_stride(d), cin
-        a.wpacked_exact, a.in_lo = None, None
+        a.wpacked_exact = None
         a.wpacked, a.cin_pad, a.cout, a.cout_pad = wbuf.data_ptr(), cp, self.out_channels, op
         a.wpacked_tc = wtc.data_ptr() if (wtc is not None and config.tensor_cores == "auto" and not refresh) else None
         a.refresh = 1 if refresh else 0
@@ -650,6 +662,14 @@ class nnConvIncr(nn.Conv2d):
             a.in_, a.in_ps, a.wpacked_exact = aligned.data_ptr(), fl.pixel_stride(aligned), wx.data_ptr()
             if not nat.lib.mie_conv_is_exact(C.byref(a)):
                 a.in_, a.in_ps, a.wpacked_exact = d.data_ptr(), fl.pixel_stride(d), None
+        if exact:
+            wx = self._weights_exact(cin)
+            a.wpacked_exact = wx.data_ptr()
+            if not nat.lib.mie_conv_is_exact(C.byref(a)):
+                exact, split, a.wpacked_exact = False, True, None
+                wbuf, cp, op, wtc = self._weights(cin_limit, True, bn)
+                d, cin = self._split_copy(x_incr, d, m, cin_limit)
+                a.in_, a.in_ps, a.cin, a.wpacked, a.cin_pad, a.wpacked_tc = d.data_ptr(), fl.pixel_stride(d), cin, wbuf.data_ptr(), cp, wtc.data_ptr()
         self.last_used_tensor_cores = bool(nat.lib.mie_conv_uses_tensor_cores(C.byref(a)))
         self.last_cluster_size = int(nat.lib.mie_conv_cluster_size(C.byref(a)))
         if split and not self.last_used_tensor_cores:
@@ -664,7 +684,7 @@ class nnConvIncr(nn.Conv2d):
         if (plain and not split and not config.kfenced_step and not config.tail_dilation and not a.accum and (x_incr[1] is None or x_incr[1] is m)
                 and d is x_incr[0] and (activation is None or type(activation).thr is nnReservedActivation.thr) and a.in_ % 16 == 0):
             self._prepared[kind] = _PreparedCall(self, activation, plan, d, m, x_incr[1] is None, not a.head, a.thr > 0.0 or bool(a.emitted),
-                                                 (wbuf, wtc))
+                                                 (wbuf, wtc, wx if exact else None))
         if (refresh and a.wpacked_exact and not a.head and not config.tail_dilation and second is None and x_incr[1] is m and x_incr[0].data_ptr() == d.data_ptr()
                 and (activation is None or activation.emitted is None) and (addend is None or type(addend[1]) is TileMask)):
             self._prepared_refresh[kind] = _PreparedRefresh(self, activation, plan, d, m, addend, (wbuf, wx))
@@ -709,6 +729,10 @@ class nnConvIncr(nn.Conv2d):
         for key, hit in list(self._packed.items()):      # filters that the steps after this pass may not use any more
             if hit[0][0] is not self.weight or hit[1] != self._filter_version(hit[0][1]):
                 del self._packed[key]
+                fl.filter_epoch[0] += 1
+        for key, hit in list(self._packed_exact.items()):
+            if hit[0] is not self.weight or hit[1] != self._filter_version(None):
+                del self._packed_exact[key]
                 fl.filter_epoch[0] += 1
         return nn.Conv2d.forward(self, x)
 

@@ -357,3 +357,60 @@ def test_upsample_and_concat_of_ragged_channel_counts(dev, c):
         up, mu = INCR.upsample2x([x, m], None, sc, pad4=True)
         assert float((up - F.interpolate(want, scale_factor=2, mode="bilinear", align_corners=False)).abs().max()) <= 1e-6
         assert float((up * (1 - mu.pixel_mask().float())).abs().max()) == 0.0
+
+
+# Steps in split precision (two FP16 parts per operand) against the FP32 kernel: cin, cout, k, stride, n, h, w, addend.  Items of one and two
+# segments in blocks of 32 channels, longer ones, blocks of 64, partial chunks, slabs and tiles, odd extents at stride 2, more items
+# than blocks
+@pytest.mark.parametrize("case", [(32, 32, 3, 1, 2, 104, 208, False), (64, 32, 3, 1, 1, 41, 50, False), (96, 32, 3, 1, 1, 24, 40, True), (32, 20, 5, 1, 1, 33, 44, False),
+                                  (36, 64, 3, 2, 1, 33, 41, False), (64, 64, 5, 1, 1, 104, 100, False), (16, 40, 7, 1, 1, 24, 40, False),
+                                  (256, 256, 3, 1, 1, 17, 23, True), (32, 96, 3, 1, 1, 8, 8, False)])
+@pytest.mark.parametrize("act,thr", [("relu", 0.0), ("tanh", 0.0), (None, 0.0), ("relu", 0.02), ("sigmoid", 0.02)])
+def test_split_precision_steps_against_fp32(dev, case, act, thr):
+    from maskedincrementeval_b200 import fields as fl, _native as nat
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    cin, cout, k, s, n, h, w, with_addend = case
+    if act == "sigmoid" and cout % 16:
+        pytest.skip("the FP32 kernel counts a partial group's missing channels, whose sigmoid is not 0, as changed")
+    old = fl.config.tensor_cores
+    out = {}
+    try:
+        for mode in ("auto", "off"):
+            fl.config.tensor_cores = mode
+            torch.manual_seed(15)
+            layer = ConvLayerIncr(cin, cout, k, s, k // 2, activation=act).to(dev).eval()
+            layer.conv2d.precision = "split"
+            a = layer.activation
+            g = torch.Generator(device=dev).manual_seed(16)
+            x = cl(torch.randn(n, cin, h, w, generator=g, device=dev))
+            steps = []
+            with torch.no_grad():
+                y = layer.forward_refresh_reservoirs(x)
+                if a is not None:
+                    a.threshold = thr
+                for frac in (0.05, 0.0, 1.0, 0.3):
+                    on = torch.rand(n, 1, h, w, generator=g, device=dev) < frac
+                    d = cl(torch.randn(n, cin, h, w, generator=g, device=dev) * on)
+                    ad = [cl(torch.randn(y.shape, generator=g, device=dev) * (torch.rand(n, 1, *y.shape[2:], generator=g, device=dev) < 0.1)), None] if with_addend else None
+                    dy, m = layer.conv2d.forward_fused([d, None], a, ad)
+                    if mode == "auto":
+                        assert nat.lib.mie_conv_is_exact(C.byref(layer.conv2d._plan(n, h, w, dev).args))
+                    steps.append((dy.clone(), m.pixel_mask().clone()))
+            out[mode] = steps, None if a is None else a.in_res.reservoir.clone(), None if a is None or a.emitted is None else a.emitted.clone()
+    finally:
+        fl.config.tensor_cores = old
+    # the FP32 kernel adds cin * k * k products one by one: a rounding of at most 2^-24 of a partial sum (below 4 here: weights are below
+    # 1 / sqrt(cin k k)) each, in either direction
+    tol = 4 * 2.0 ** -24 * (cin * k * k) ** 0.5
+    (sa, ra, ea), (so, ro, eo) = out["auto"], out["off"]
+    for (dy, m), (want, wm) in zip(sa, so):
+        assert torch.equal(m, (dy != 0).any(1, keepdim=True).to(torch.uint8))
+        if thr == 0.0:
+            assert float((dy - want).abs().max()) <= tol and float((m != wm).float().mean()) <= 1e-3
+    if ra is not None:
+        assert float((ra - ro).abs().max()) <= tol
+    if thr > 0.0:      # what has been sent lies within the threshold of the output, and is what the carry says
+        f = torch.relu if act == "relu" else torch.sigmoid
+        assert float((ea - f(ra)).abs().max()) <= thr + tol
+        differ = float(((ea - eo).abs() > tol).float().mean())
+        assert differ <= 1e-3, differ      # changes that lie at the threshold

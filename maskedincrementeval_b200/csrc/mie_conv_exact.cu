@@ -62,24 +62,36 @@ __device__ __forceinline__ void tmem_ld16_async(unsigned taddr, unsigned *r) {
                  "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                : "r"(taddr));
 }
-// acc[i] += inv * (hi[i] + 2^-11 (mid[i] + low[i])): the columns of a segment's three products, 16 at a time
-template <int N>
-__device__ __forceinline__ void tmem_add_split(unsigned hi, unsigned mid, unsigned low, float inv, float *acc) {
+// FULL: the low parts are multiplied too (lo x lo).  The second instruction then has N = 64 columns like the first, 43 clocks instead of 39,
+// and a segment a third more columns to read (64 -> 32 5x5 at 8 x 480x640: 874 us against 831), for the 2^-24 of a product that is
+// dropped elsewhere.  Taken by thin layers, where few products meet and the FP32 kernel is what they are measured against (16 -> 24 3x3,
+// error of the change over that kernel's, 0.5 / 5 / 40 % active: 1.04 / 0.90 / 0.93, without 1.21 / 1.01 / 0.96; of the state 1.01 / 0.97 /
+// 0.94).  Blocks of 32 channels only.
+// hi + 2^-11 (mid + low + 2^-11 last): the products of a segment
+__device__ __forceinline__ float split_sum(unsigned hi, unsigned mid, unsigned low, unsigned last, bool full) {
+  float v = __uint_as_float(mid) + __uint_as_float(low);
+  if (full) v = fmaf(__uint_as_float(last), SPLIT_LO, v);
+  return fmaf(v, SPLIT_LO, __uint_as_float(hi));
+}
+// acc[i] += inv * (the sum of a segment's products), 16 columns at a time
+template <int N, bool FULL>
+__device__ __forceinline__ void tmem_add_split(unsigned hi, unsigned mid, unsigned low, unsigned last, float inv, float *acc) {
 #pragma unroll
   for (int g = 0; g < N; g += 16) {
-    unsigned a[16], b[16], c[16];
+    unsigned a[16], b[16], c[16], d[16];
     tmem_ld16_async(hi + g, a);
     tmem_ld16_async(mid + g, b);
     tmem_ld16_async(low + g, c);
+    if (FULL) tmem_ld16_async(last + g, d);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-      acc[g + i] = fmaf(fmaf(__uint_as_float(b[i]) + __uint_as_float(c[i]), SPLIT_LO, __uint_as_float(a[i])), inv, acc[g + i]);
+    for (int i = 0; i < 16; ++i) acc[g + i] = fmaf(split_sum(a[i], b[i], c[i], FULL ? d[i] : 0u, FULL), inv, acc[g + i]);
   }
 }
 
-// Segment accumulators in 512 columns, 3 CB each: [hi x hi | hi x lo] per epilogue set, then lo x hi.
-__host__ __device__ constexpr unsigned exact_segs(int cb) { return cb == 64 ? 2u : 5u; }
+// Segment accumulators in 512 columns: [hi x hi | hi x lo] of either half of the channels, then lo x hi, or [lo x hi | lo x lo] like the first.
+__host__ __device__ constexpr unsigned exact_cols(int cb, bool full) { return (full ? 4u : 3u) * (unsigned)cb; }
+__host__ __device__ constexpr unsigned exact_segs(int cb, bool full) { return 512u / exact_cols(cb, full); }
 
 // The MMA issuer.  A ring stage of the filter is a segment: one wait for its operands, its accumulator and (first stage) the
 // halo together, one commit for both the filter producer and the epilogue.  The issuing warp is what paces the kernel: the
@@ -88,11 +100,11 @@ struct ExactIssue {
   int item0, item_step, n_items, n_chunks, cin, tps, nviews;
   unsigned tmem_base, a_base, b_base, row_bytes, halo_bytes, stage_bytes, stages, halos, segs, limit;
 };
-template <int CB, bool ALT>
+template <int CB, bool ALT, bool FULL>
 __device__ __forceinline__ void exact_issue(const ExactIssue a, const PairTapTable &t, unsigned long long *b_full, unsigned long long *done,
     unsigned long long *a_ready, unsigned long long *a_empty, unsigned long long *seg_empty, unsigned long long *item_full, volatile int *abort_flag) {
   constexpr unsigned tap_units = CB * 64 >> 4;
-  const unsigned id_hi = make_idesc_f16_pair(2 * CB), id_lo = make_idesc_f16_pair(CB);
+  const unsigned id_hi = make_idesc_f16_pair(2 * CB), id_lo = make_idesc_f16_pair(FULL ? 2 * CB : CB);
   const unsigned long long b_tmpl = make_smem_desc_64(0), a_tmpl = make_smem_desc(0, a.row_bytes);
   const unsigned long long b_hi = b_tmpl & 0xFFFFFFFF00000000ull, a_hi = a_tmpl & 0xFFFFFFFF00000000ull;
   const unsigned lo_flags = (unsigned)(b_tmpl & 0xFFFF0000ull);
@@ -111,7 +123,7 @@ __device__ __forceinline__ void exact_issue(const ExactIssue a, const PairTapTab
         for (int i = t.first[v]; i < end; i += a.tps) {
           const int nt = min(a.tps, end - i);
           unsigned b_lo = lo_flags | (stage_addr >> 4), off = (unsigned)t.off[i];
-          const unsigned d = a.tmem_base + seg * (3u * CB);
+          const unsigned d = a.tmem_base + seg * exact_cols(CB, FULL);
           const unsigned bbar = smem_u32(&b_full[bs]);
           if (!mbar_wait3(abar, ap, bbar, bpar, smem_u32(&seg_empty[seg]), seg_par, abort_flag, a.limit)) return;
           tc_fence_after();
@@ -209,7 +221,7 @@ __device__ __forceinline__ void tmem_ld8_async(unsigned taddr, unsigned *r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
-template <int HW, bool STEP, int ACT>
+template <int HW, bool STEP, bool FULL, int ACT>
 __device__ __forceinline__ bool exact_finish(const ExactParams &p, unsigned c, unsigned n_seg, float inv0, float inv1, bool wide, const ExactRow r,
                                              const float4 *col, int n, int oy, int ox, bool valid, int64_t pix, int co) {
   constexpr unsigned CB = HW, HB = HW / 2;
@@ -225,15 +237,16 @@ __device__ __forceinline__ bool exact_finish(const ExactParams &p, unsigned c, u
     for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
 #pragma unroll 1
     for (unsigned j = 0; j < n_seg; ++j) {
-      const unsigned at = c + j * 3u * CB, ch = 8u * g, hi = at + ch / HB * CB + ch % HB;
+      const unsigned at = c + j * exact_cols(CB, FULL), ch = 8u * g, hi = at + ch / HB * CB + ch % HB;
       const float inv = j ? inv1 : inv0;
-      unsigned a[8], b[8], d[8];
+      unsigned a[8], b[8], d[8], e[8];
       tmem_ld8_async(hi, a);
       tmem_ld8_async(hi + HB, b);
-      tmem_ld8_async(at + 2u * CB + ch, d);
+      tmem_ld8_async(FULL ? hi + 2u * CB : at + 2u * CB + ch, d);
+      if (FULL) tmem_ld8_async(hi + 2u * CB + HB, e);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = fmaf(fmaf(__uint_as_float(b[i]) + __uint_as_float(d[i]), SPLIT_LO, __uint_as_float(a[i])), inv, acc[i]);
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(split_sum(a[i], b[i], d[i], FULL ? e[i] : 0u, FULL), inv, acc[i]);
     }
 #pragma unroll
     for (unsigned i = 0; i < 2; ++i) {
@@ -274,7 +287,7 @@ __device__ __forceinline__ bool exact_finish(const ExactParams &p, unsigned c, u
 // HW: channels that a thread of the epilogue finishes.  ALT: the two sets of epilogue warps take items in turn (CB = HW channels per
 // block), else halves of each item's channels (CB = 2 HW).  STEP: a step (incremental activation, threshold, carry) instead of the dense
 // pass.
-template <int HW, bool STEP, bool ALT>
+template <int HW, bool STEP, bool ALT, bool FULL>
 __global__ void __launch_bounds__(EXACT_THREADS, 1)
 conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__ ExactMaps maps) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -351,7 +364,7 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
     if (crank == 0u) {
       const ExactIssue a = {bid, nblk, n_items, p.n_chunks, p.cin, p.tps, nv, tmem_base, a_base, b_base, row_bytes, halo_bytes, stage_bytes, (unsigned)p.stages,
                             (unsigned)p.halos, (unsigned)p.segs, p.spin_limit};
-      exact_issue<CB, ALT>(a, s_tap, b_full, done, a_ready, a_empty, seg_empty, item_full, &s_abort);
+      exact_issue<CB, ALT, FULL>(a, s_tap, b_full, done, a_ready, a_empty, seg_empty, item_full, &s_abort);
     }
   } else if (warp >= 12) {
     // =========================== halos as two FP16 parts ===========================
@@ -432,8 +445,9 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
           for (int left = p.t.first[v + 1] - p.t.first[v]; left > 0; left -= p.tps) {
             if (!(ok = __all_sync(0xffffffffu, mbar_wait(&done[stage], stage_par, &s_abort, p.spin_limit)))) break;
             tc_fence_after();
-            const unsigned c = lane_base + seg * (3u * CB), own = c + (unsigned)set * CB;      // [hi | mid] columns of this set's channels
-            tmem_add_split<HW>(own, own + HW, c + 2u * CB + (unsigned)set * HW, inv, acc);
+            // [hi | mid] columns of this set's channels, and [lo x hi | lo x lo] or lo x hi alone
+            const unsigned c = lane_base + seg * exact_cols(CB, FULL), own = c + (unsigned)set * CB, low = c + 2u * CB + (unsigned)set * (FULL ? CB : HW);
+            tmem_add_split<HW, FULL>(own, own + HW, low, low + HW, inv, acc);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&seg_empty[seg]), 0));
@@ -515,10 +529,10 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
         tc_fence_after();
         const ExactRow r = {res_row, out_row, em_row, (unsigned)sw};
         const bool wide = inv[0] != inv[0] || inv[1] != inv[1];
-        const unsigned c = lane_base + seg * (3u * CB);
-        if (p.act == MIE_ACT_RELU) sent = exact_finish<HW, STEP, MIE_ACT_RELU>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
-        else if (p.act == MIE_ACT_NONE) sent = exact_finish<HW, STEP, MIE_ACT_NONE>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
-        else sent = exact_finish<HW, STEP, MIE_ACT_SIGMOID>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
+        const unsigned c = lane_base + seg * exact_cols(CB, FULL);
+        if (p.act == MIE_ACT_RELU) sent = exact_finish<HW, STEP, FULL, MIE_ACT_RELU>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
+        else if (p.act == MIE_ACT_NONE) sent = exact_finish<HW, STEP, FULL, MIE_ACT_NONE>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
+        else sent = exact_finish<HW, STEP, FULL, MIE_ACT_SIGMOID>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
         sent = sent && valid;
         tc_fence_before();
         __syncwarp();
@@ -574,7 +588,7 @@ static inline int64_t exact_scales_at(int cin, int cout_pad, int k) { return (in
 struct ExactShape {
   PairTaps t;
   int wp, cb, hw, tps, stages, halos, segs, slab_bufs, slab_sets;   // hw: channels of an epilogue thread
-  bool alt;
+  bool alt, full;
   size_t smem;
 };
 static ExactShape exact_shape(const mie_conv_args *a) {
@@ -584,7 +598,8 @@ static ExactShape exact_shape(const mie_conv_args *a) {
   // 64 channels per block unless blocks of 32, which take 0.75 of its time, need fewer rounds for it (5x5: 305 and 245 clocks per tap and
   // 32 channels, 3x3 430 and 300)
   h.cb = 32;
-  if (a->cout_pad % 64 == 0 &&
+  h.full = !a->refresh && a->cin * a->k * a->k < 256;
+  if (!h.full && a->cout_pad % 64 == 0 &&
       (int64_t)divup(quads * (a->cout_pad / 64), clusters_max) * 100 <= (int64_t)divup(quads * (a->cout_pad / 32), clusters_max) * 75)
     h.cb = 64;
   // Taps of a segment: its truncation grows with its additions, one per 16 channels and tap, the FP32 kernel's rounding with the whole
@@ -618,7 +633,7 @@ static ExactShape exact_shape(const mie_conv_args *a) {
   const int stage_bytes = h.tps * h.cb * 64;
   h.stages = std::min((budget - h.halos * halo_bytes) / stage_bytes, EXACT_MAX_STAGES);
   // ... two items' worth with `alt`: an item's barrier is not signalled again before its set has looked at it
-  h.segs = h.alt ? 2 * n_seg : std::min(h.stages, (int)exact_segs(h.cb));      // the epilogue learns of a segment from its stage's barrier
+  h.segs = h.alt ? 2 * n_seg : std::min(h.stages, (int)exact_segs(h.cb, h.full));      // the epilogue learns of a segment from its stage's barrier
   h.smem = (size_t)((h.stages * stage_bytes + 1023) & ~1023) + (size_t)h.halos * halo_bytes + slab_bytes + 1024;
   return h;
 }
@@ -705,7 +720,7 @@ int launch_conv_exact(const mie_conv_args *a, const float *fw, int64_t fw_tap, i
       if (r != MIE_OK) return r;
     }
   }
-  static int smem_set[6][MAX_DEVICES] = {{0}};
+  static int smem_set[8][MAX_DEVICES] = {{0}};
   auto launch = [&](auto kernel, int i) {
     const int r = ensure_dynamic_smem(kernel, smem_set[i], smem);
     if (r != MIE_OK) return r;
@@ -713,10 +728,11 @@ int launch_conv_exact(const mie_conv_args *a, const float *fw, int64_t fw_tap, i
     return check_launch();
   };
   if (a->refresh)
-    return h.alt ? launch(conv_exact_kernel<32, false, true>, 0) : h.cb == 64 ? launch(conv_exact_kernel<32, false, false>, 1)
-                                                                              : launch(conv_exact_kernel<16, false, false>, 2);
-  return h.alt ? launch(conv_exact_kernel<32, true, true>, 3) : h.cb == 64 ? launch(conv_exact_kernel<32, true, false>, 4)
-                                                                           : launch(conv_exact_kernel<16, true, false>, 5);
+    return h.alt ? launch(conv_exact_kernel<32, false, true, false>, 0) : h.cb == 64 ? launch(conv_exact_kernel<32, false, false, false>, 1)
+                                                                                     : launch(conv_exact_kernel<16, false, false, false>, 2);
+  if (h.full) return h.alt ? launch(conv_exact_kernel<32, true, true, true>, 6) : launch(conv_exact_kernel<16, true, false, true>, 7);
+  return h.alt ? launch(conv_exact_kernel<32, true, true, false>, 3) : h.cb == 64 ? launch(conv_exact_kernel<32, true, false, false>, 4)
+                                                                                  : launch(conv_exact_kernel<16, true, false, false>, 5);
 }
 
 // A field with a pixel stride or an address that TMA cannot read (5 bins of a voxel grid) as one it can: one read and one write.

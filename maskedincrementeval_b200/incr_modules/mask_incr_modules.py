@@ -457,6 +457,13 @@ class nnConvIncr(nn.Conv2d):
         return (getattr(self, "precision", None) == "split" and cin * self._k * self._k >= 256
                 and self._k in (1, 3, 5, 7) and self._s in (1, 2))
 
+    def _thin(self, cin: int) -> bool:
+        """3x3 layers of 16 channels, too shallow for TF32 numbers on the tensor cores, run in split precision there as well: no less
+        precise than the FP32 kernel (one K-slice of 16 channels is one instruction a tap, so that nothing is truncated inside a
+        tap; with 12 channels the FP32 kernel's sums are too short to match, with 20 the second slice truncates) and faster
+        (16 -> 24 on 97x131 a step of 15 us, 32 on the FP32 kernel)."""
+        return config.tensor_cores == "auto" and cin == 16 and self._k == 3 and self.out_channels % 4 == 0
+
     def _split_copy(self, x_incr: Masked, d: torch.Tensor, m: TileMask, cin_limit: Optional[int]):
         """The three channel blocks of an input in split precision, and how many channels they hold."""
         n, cin, hin, win = d.shape
@@ -576,10 +583,10 @@ class nnConvIncr(nn.Conv2d):
         thresholded = activation is not None and (activation.thr() > 0.0 or
                                                   (config.carry and activation.emitted is not None))
         split = self._split_input(cin) and (config.tc_thresholded or not thresholded) and not refresh
-        # ... from two FP16 parts per operand, made inside the kernel, where it takes the layer (below); from three channel blocks of
+        # ... from two FP16 parts per operand, made inside the kernel, where it takes the layer (below; layers of _thin() too); from three channel blocks of
         # TF32 numbers elsewhere: 1x1 layers, layers with a folded batch-norm, and narrow inputs, whose three blocks fit one
         # chunk (the 5-channel 5x5 head of eight 480x640 streams: 308 us, 440 in FP16 parts)
-        exact = split and bn is None and cin > 8 and self._k >= 3
+        exact = bn is None and self._k >= 3 and (split and cin > 8 or not split and self._thin(cin) and not refresh and (config.tc_thresholded or not thresholded))
         split = split and not exact
         wbuf, cp, op, wtc = self._weights(cin_limit, split, bn)
         if split:
@@ -666,7 +673,9 @@ class nnConvIncr(nn.Conv2d):
             wx = self._weights_exact(cin)
             a.wpacked_exact = wx.data_ptr()
             if not nat.lib.mie_conv_is_exact(C.byref(a)):
-                exact, split, a.wpacked_exact = False, True, None
+                exact, a.wpacked_exact = False, None
+            if not exact and self._split_input(cin):
+                split = True
                 wbuf, cp, op, wtc = self._weights(cin_limit, True, bn)
                 d, cin = self._split_copy(x_incr, d, m, cin_limit)
                 a.in_, a.in_ps, a.cin, a.wpacked, a.cin_pad, a.wpacked_tc = d.data_ptr(), fl.pixel_stride(d), cin, wbuf.data_ptr(), cp, wtc.data_ptr()

@@ -364,7 +364,8 @@ def test_upsample_and_concat_of_ragged_channel_counts(dev, c):
 # than blocks
 @pytest.mark.parametrize("case", [(32, 32, 3, 1, 2, 104, 208, False), (64, 32, 3, 1, 1, 41, 50, False), (96, 32, 3, 1, 1, 24, 40, True), (32, 20, 5, 1, 1, 33, 44, False),
                                   (36, 64, 3, 2, 1, 33, 41, False), (64, 64, 5, 1, 1, 104, 100, False), (16, 40, 7, 1, 1, 24, 40, False),
-                                  (256, 256, 3, 1, 1, 17, 23, True), (32, 96, 3, 1, 1, 8, 8, False)])
+                                  (256, 256, 3, 1, 1, 17, 23, True), (32, 96, 3, 1, 1, 8, 8, False),
+                                  (16, 24, 3, 1, 1, 97, 131, False), (16, 64, 3, 2, 2, 33, 47, True), (16, 128, 3, 1, 1, 9, 9, False)])
 @pytest.mark.parametrize("act,thr", [("relu", 0.0), ("tanh", 0.0), (None, 0.0), ("relu", 0.02), ("sigmoid", 0.02)])
 def test_split_precision_steps_against_fp32(dev, case, act, thr):
     from maskedincrementeval_b200 import fields as fl, _native as nat
@@ -379,7 +380,7 @@ def test_split_precision_steps_against_fp32(dev, case, act, thr):
             fl.config.tensor_cores = mode
             torch.manual_seed(15)
             layer = ConvLayerIncr(cin, cout, k, s, k // 2, activation=act).to(dev).eval()
-            layer.conv2d.precision = "split"
+            layer.conv2d.precision = "split" if cin != 16 or k != 3 else None      # (3x3 layers of 16 channels run so by themselves)
             a = layer.activation
             g = torch.Generator(device=dev).manual_seed(16)
             x = cl(torch.randn(n, cin, h, w, generator=g, device=dev))

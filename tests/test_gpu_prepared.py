@@ -335,3 +335,68 @@ def test_a_captured_step_follows_new_parameters(dev, refresh, how):
         del taken
     finally:
         fl.config.refresh = old
+
+
+def _double_head(net):
+    with torch.no_grad():
+        conv = next(m for m in net.modules() if isinstance(m, torch.nn.Conv2d))
+        conv.weight.mul_(2.0)
+
+
+def _replace_parameter(net):
+    conv = [m for m in net.modules() if isinstance(m, torch.nn.Conv2d)][1]
+    conv.weight = torch.nn.Parameter(conv.weight.detach() * 0.5)
+
+
+def _replace_bias(net):
+    conv = [m for m in net.modules() if isinstance(m, torch.nn.Conv2d)][2]
+    conv.bias = torch.nn.Parameter(conv.bias.detach() + 0.25)
+
+
+def _replace_activation(net):
+    from maskedincrementeval_b200.incr_modules.mask_incr_modules import nnReservedActivation
+    acts = [m for m in net.modules() if isinstance(m, nnReservedActivation) and m.op is torch.relu]
+    acts[1].op = torch.tanh
+
+
+def _new_reservoir(net):
+    from maskedincrementeval_b200.incr_modules.mask_incr_modules import nnReservedActivation
+    acts = [m for m in net.modules() if isinstance(m, nnReservedActivation) and m.in_res.reservoir is not None]
+    acts[0].in_res.reservoir = acts[0].in_res.reservoir.clone(memory_format=torch.channels_last)
+
+
+def _fp32_kernels(net):
+    from maskedincrementeval_b200 import fields as fl
+    fl.config.tensor_cores = "off"
+
+
+@pytest.mark.parametrize("change", [None, _double_head, _replace_parameter, _replace_bias, _replace_activation, _new_reservoir, _fp32_kernels])
+def test_a_replayed_dense_pass_is_an_eager_one(dev, change):
+    """IncrementalRunner replays the dense pass once three in a row found the model alike; a change of any input of the pass, and
+    steps in between, give what a runner that never replays gives."""
+    from maskedincrementeval_b200 import fields as fl
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import E2VIDRecurrentIncr
+    from maskedincrementeval_b200.runtime import IncrementalRunner
+    torch.manual_seed(21)
+    net = E2VIDRecurrentIncr(dict(num_bins=5, skip_type="sum", recurrent_block_type="convlstm", num_encoders=3, base_num_channels=8,
+                                  num_residual_blocks=1, norm=None, use_upsample_conv=True, compat="exact")).to(dev).eval()
+    g = torch.Generator(device=dev).manual_seed(22)
+    frames = [torch.randn(1, 5, 40, 56, generator=g, device=dev).contiguous(memory_format=torch.channels_last) for _ in range(3)]
+    old = fl.config.tensor_cores
+    try:
+        run = IncrementalRunner(net)
+        for i in range(7):
+            run.refresh(frames[i % 3])
+        assert run._pass_graph is not None
+        if change is not None:
+            change(net)
+        run.refresh(frames[1])
+        outs = [run.refresh(frames[2]).clone()] + [run.step(f).clone() for f in frames]
+        outs.append(run.refresh(frames[0]).clone())
+        eager = IncrementalRunner(net, use_graph=False)
+        want = [eager.refresh(frames[2]).clone()] + [eager.step(f).clone() for f in frames]
+        want.append(eager.refresh(frames[0]).clone())
+    finally:
+        fl.config.tensor_cores = old
+    for y, w in zip(outs, want):
+        assert torch.equal(y, w)

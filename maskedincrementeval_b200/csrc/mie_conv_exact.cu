@@ -37,7 +37,7 @@ struct ExactParams {
   const float *fw; int64_t fw_tap, fw_ci; int fw_vec;                // filter entry (tap, ci, co) at fw[tap * fw_tap + ci * fw_ci + co]
   const float *winv;                                                 // inverse scale of every output channel's filter; NaN: fallback
   int cin, cout, cout_pad, n_chunks, n, hout, wout;
-  const int32_t *list; int32_t *counts; int max_tiles;
+  const int32_t *list; int32_t *counts; int max_tiles;               // list null (dense pass): every tile
   float *out; int64_t out_ps; unsigned int *out_bits32;
   int act; float *res; int64_t res_ps; const float *addend; int64_t addend_ps; const float *bias;
   int cb, stages, halos, wp;
@@ -340,7 +340,8 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
   grid_dependency_trigger();
 
   const int n_cblk = p.cout_pad / CB;
-  const int n_active = __shfl_sync(0xffffffffu, min(p.counts[0], p.max_tiles), 0);     // uniform, for the compiler too
+  // (no list: every tile, and nothing to wait for)
+  const int n_active = __shfl_sync(0xffffffffu, p.list ? min(p.counts[0], p.max_tiles) : ntiles_total, 0);     // uniform, for the compiler too
   const int n_items = ((n_active + 3) >> 2) * n_cblk;
   const unsigned b_base = smem_u32(smem), a_base = b_base + (((unsigned)p.stages * stage_bytes + 1023u) & ~1023u);
   const int nv = p.t.nviews;
@@ -393,7 +394,7 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
     const int first = ALT ? bid + set * nblk : bid, step = ALT ? 2 * nblk : nblk;
     auto column = [&](int item) { return (n_cblk == 1 ? 0 : item % n_cblk) * CB + (ALT ? 0 : set * HW); };
     auto entry = [&](int item) {      // this lane's tile of an item
-      const int e = 4 * (n_cblk == 1 ? item : item / n_cblk) + 2 * (int)crank + slot, t = item < n_items && e < n_active ? p.list[e] : -1;
+      const int e = 4 * (n_cblk == 1 ? item : item / n_cblk) + 2 * (int)crank + slot, t = item >= n_items || e >= n_active ? -1 : p.list ? p.list[e] : e;
       return t < ntiles_total ? t : -1;
     };
     auto place = [&](int t, int &x, int &y, int &n) {

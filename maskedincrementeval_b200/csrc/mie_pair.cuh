@@ -172,7 +172,7 @@ __device__ __forceinline__ void pair_produce_halos(const PairWork &w, const Pair
     bool have[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      int tile = __shfl_sync(0xffffffffu, e + i < n_active ? lst[e + i] : -1, 0);
+      int tile = __shfl_sync(0xffffffffu, e + i >= n_active ? -1 : LOCAL && !lst ? e + i : lst[e + i], 0);      // no list: every tile
       have[i] = e + i < n_active;
       // an entry outside the field is reported and skipped by the epilogue; here tile 0 stands in for it
       if (have[i] && (tile < 0 || tile >= ntiles_total)) {

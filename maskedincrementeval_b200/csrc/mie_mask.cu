@@ -290,6 +290,88 @@ __global__ void __launch_bounds__(256) tiles_dilate_kernel(
   }
 }
 
+// The same for large fields, in blocks of 1024.
+constexpr int DILATE_LARGE = 12288, DILATE_LARGE_THREADS = 1024;      // 9600 tiles: 10.3 us either way, 14400 12.8 and 11.3, 38400 40.3 and 18.8
+__global__ void __launch_bounds__(DILATE_LARGE_THREADS) tiles_dilate_large_kernel(
+    const uint64_t *__restrict__ in_bits, int N, int Hin, int Win, int Hout, int Wout, int k, int stride, int pad,
+    const uint64_t *__restrict__ union_bits, uint64_t *__restrict__ out_bits, int32_t *__restrict__ list,
+    int32_t *__restrict__ stale, int32_t *__restrict__ counts, uint8_t *__restrict__ flags) {
+  grid_dependency_wait();
+  grid_dependency_trigger();
+  const int ntiles = N * ((Hout + 7) >> 3) * ((Wout + 7) >> 3);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < ntiles) flags[t] = dilate_flag(t, in_bits, Hin, Win, Hout, Wout, k, stride, pad, union_bits, out_bits);
+  // the block that finishes last compacts both lists in ascending order
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = (atomicAdd(&counts[2], 1) == (int)gridDim.x - 1);
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // A run of consecutive tiles per warp, 128 at a time: count them, scan the counts over the block, write the tiles out.  Bound by
+  // latency.  (38400 tiles: a sweep of the whole block over 256 tiles at a time took 75 us, a chunk of 150 tiles per thread of 256,
+  // whose stores fall into 256 places, 40; this 19.)
+  __shared__ int s_wa[DILATE_LARGE_THREADS / 32], s_wb[DILATE_LARGE_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int run = ((ntiles + DILATE_LARGE_THREADS / 32 - 1) / (DILATE_LARGE_THREADS / 32) + 127) & ~127, lo = min(warp * run, ntiles), hi = min(lo + run, ntiles);
+  const bool vec = (reinterpret_cast<uintptr_t>(flags) & 3) == 0;
+  auto four = [&](int i) {      // the flag bytes of tiles i .. i + 3
+    if (vec && i + 4 <= hi) return __ldcg(reinterpret_cast<const unsigned *>(flags + i));
+    unsigned f = 0;
+    for (int k = 0; k < 4; ++k)
+      if (i + k < hi) f |= (unsigned)__ldcg(flags + i + k) << (8 * k);
+    return f;
+  };
+  int ca = 0, cs = 0;
+#pragma unroll 4
+  for (int i = lo + 4 * lane; i < hi; i += 128) {
+    const unsigned f = four(i);
+    ca += __popc(f & 0x01010101u);
+    cs += __popc(f & 0x02020202u);
+  }
+  ca = __reduce_add_sync(0xffffffffu, ca);
+  cs = __reduce_add_sync(0xffffffffu, cs);
+  if (lane == 0) { s_wa[warp] = ca; s_wb[warp] = cs; }
+  __syncthreads();
+  int oa = 0, os = 0;
+  int na = 0, ns = 0;
+#pragma unroll
+  for (int w = 0; w < DILATE_LARGE_THREADS / 32; ++w) {
+    if (w == warp) { oa = na; os = ns; }
+    na += s_wa[w];
+    ns += s_wb[w];
+  }
+  unsigned next = lo + 4 * lane < hi ? four(lo + 4 * lane) : 0u;
+  for (int base = lo; base < hi; base += 128) {
+    const int i = base + 4 * lane;
+    const unsigned f = next;
+    next = i + 128 < hi ? four(i + 128) : 0u;
+    const int mine = __popc(f & 0x01010101u) | __popc(f & 0x02020202u) << 16;
+    int upto = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int below = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto += below;
+    }
+    const int all = __shfl_sync(0xffffffffu, upto, 31);
+    int at = oa + ((upto - mine) & 0xFFFF), as = os + ((upto - mine) >> 16);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned b = f >> (8 * k);
+      if (b & 1u) list[at++] = i + k;
+      else if ((b & 2u) && stale) stale[as++] = i + k;
+    }
+    oa += all & 0xFFFF;
+    os += all >> 16;
+  }
+  if (threadIdx.x == 0) {
+    counts[0] = na;
+    counts[1] = stale ? ns : 0;
+    counts[2] = 0;
+  }
+}
+
 // Up to DILATE_SMALL_MAX tiles: one block keeps the flags in shared memory and compacts them itself -- no
 // ticket, no fence, no round trip through global memory (the deeper levels of a UNet at batch 1 are this small;
 // at 1452 tiles one block measured slower than the multi-block kernel).
@@ -328,7 +410,11 @@ extern "C" int mie_tiles_dilate(const uint64_t *in_bits, int N, int Hin, int Win
                                                                        union_bits, out_bits, list, stale, counts);
     return check_launch();
   }
-  launch_chained(tiles_dilate_kernel, dim3(divup(ntiles, 256)), dim3(256), 0, (cudaStream_t)stream, 
+  if (ntiles >= DILATE_LARGE)
+    launch_chained(tiles_dilate_large_kernel, dim3(divup(ntiles, DILATE_LARGE_THREADS)), dim3(DILATE_LARGE_THREADS), 0, (cudaStream_t)stream, 
+      in_bits, N, Hin, Win, Hout, Wout, k, stride, pad, union_bits, out_bits, list, stale, counts, flags);
+  else
+    launch_chained(tiles_dilate_kernel, dim3(divup(ntiles, 256)), dim3(256), 0, (cudaStream_t)stream, 
       in_bits, N, Hin, Win, Hout, Wout, k, stride, pad, union_bits, out_bits, list, stale, counts, flags);
   return check_launch();
 }

@@ -415,3 +415,9 @@ def test_split_precision_steps_against_fp32(dev, case, act, thr):
         assert float((ea - f(ra)).abs().max()) <= thr + tol
         differ = float(((ea - eo).abs() > tol).float().mean())
         assert differ <= 1e-3, differ      # changes that lie at the threshold
+
+
+# fields on both sides of the size from which the lists are compacted by warps: 12288 tiles, ragged edges, runs that end inside a warp's
+@pytest.mark.parametrize("n,h,w", [(3, 504, 512), (3, 512, 512), (1, 891, 895), (5, 411, 397)])
+def test_dilation_of_fields_around_the_large_kernels_limit(dev, n, h, w):
+    test_dilation_of_large_fields(dev, n, h, w)

@@ -7,7 +7,7 @@
 //     hi(input) x [hi(filter) | lo(filter)]  ->  N = 2 CB columns,      lo(input) x hi(filter)  ->  N = CB columns.
 // With two TF32 numbers per operand, which is what stood here before, an instruction takes 8 channels from the same 32 bytes,
 // the input had to be split by a pass of its own (one read and two writes of every layer's input through HBM) and twice the operand
-// bytes crossed L2: eight E2Depth streams 480x640 13.5 ms, now 9.2.
+// bytes crossed L2: eight E2Depth streams 480x640 13.5 ms, with FP16 parts 9.2.
 // (Splitting an operand: Markidis et al., 2018; scaled FP16 parts, and sums kept outside the tensor core because it truncates:
 // Ootomo and Yokota, 2022.)
 // What keeps the result at fp32 level is where the sums are rounded: the tensor core truncates each time it adds to an

@@ -441,9 +441,9 @@ class nnConvIncr(nn.Conv2d):
         return hit[2]
 
     def _split_input(self, cin: int) -> bool:
-        """Whether this layer runs on the tensor cores in split precision: input [d, d - tf32(d), d] against the
-        filter blocks [W, W, W - tf32(W)] (three times the channels), which is the fp32 convolution up to the dropped
-        lo*lo term.  Taken by
+        """Whether this layer runs on the tensor cores in split precision: the fp32 convolution up to the dropped lo*lo term, from two
+        FP16 parts per operand or as input [d, d - tf32(d), d] against the filter blocks [W, W, W - tf32(W)] (three times
+        the channels; ``forward_fused`` decides).  Taken by
           * narrow-input layers (the 5-bin voxel head): the raw O(1) input delta must not be truncated to TF32 (it
             random-walks in the first reservoir) and neither may the filter be rounded (the input changes by its full
             scale between frames);

@@ -232,6 +232,7 @@ __device__ __forceinline__ bool exact_finish(const ExactParams &p, unsigned c, u
   float top = 0.0f;
 #pragma unroll 1
   for (unsigned g = 0; g < HW / 8; ++g) {
+    __syncwarp();      // (lanes may have parted over the FP32 fallback; the loads from tensor memory are the warp's)
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.0f;

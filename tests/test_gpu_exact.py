@@ -154,7 +154,7 @@ def test_dense_pass_on_non_finite_values(dev, case, where):
 # Values that lie far apart in one halo: what two FP16 numbers with a common scale hold is computed on the tensor cores, the rest with FP32
 # instructions.  Every output against the sum of its products' magnitudes: fp32 sums of cin * k * k terms, or (below 2^17) a step
 # of 2^-49 of the largest value times the filter's entries (below 0.05).  (At 40000 some halos lie below 2^14.)
-@pytest.mark.parametrize("case", [(48, 32, 3, 1, 24, 40), (64, 64, 7, 1, 17, 23), (5, 32, 5, 2, 33, 40)])
+@pytest.mark.parametrize("case", [(48, 32, 3, 1, 24, 40), (64, 64, 7, 1, 17, 23), (5, 32, 5, 2, 33, 40), (16, 36, 3, 1, 41, 50)])
 @pytest.mark.parametrize("big,small", [(1.0, 1e-3), (1e-30, 1e-33), (16383.0, 1e-6), (40000.0, 1e-6), (1e6, 1e-9), (1e20, 1.0), (1e31, 1e30), (1e36, 0.2)])
 def test_dense_pass_on_values_far_apart(dev, case, big, small):
     from maskedincrementeval_b200.incr_modules._algebra import NATIVE
@@ -421,3 +421,35 @@ def test_split_precision_steps_against_fp32(dev, case, act, thr):
 @pytest.mark.parametrize("n,h,w", [(3, 504, 512), (3, 512, 512), (1, 891, 895), (5, 411, 397)])
 def test_dilation_of_fields_around_the_large_kernels_limit(dev, n, h, w):
     test_dilation_of_large_fields(dev, n, h, w)
+
+
+# Deltas that FP16 parts cannot hold, in steps: two items in hand (16 and 32 channels), one (64 -> 32), blocks of 64.  Against the FP32 kernel:
+# the same infinities and NaN, and the same state elsewhere up to fp32 sums of cin * 9 products
+@pytest.mark.parametrize("cin,cout", [(16, 36), (32, 32), (96, 32), (64, 64)])
+@pytest.mark.parametrize("odd", [float("inf"), float("nan"), 3e30, 1e5])
+def test_steps_on_values_far_apart(dev, cin, cout, odd):
+    from maskedincrementeval_b200 import fields as fl, _native as nat
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    old = fl.config.tensor_cores
+    out = {}
+    try:
+        for mode in ("auto", "off"):
+            fl.config.tensor_cores = mode
+            torch.manual_seed(17)
+            layer = ConvLayerIncr(cin, cout, 3, 1, 1, activation="relu").to(dev).eval()
+            layer.conv2d.precision = "split" if cin != 16 else None
+            g = torch.Generator(device=dev).manual_seed(18)
+            with torch.no_grad():
+                layer.forward_refresh_reservoirs(cl(torch.randn(1, cin, 41, 50, generator=g, device=dev)))
+                d = torch.randn(1, cin, 41, 50, generator=g, device=dev) * (1e-6 if odd == 1e5 else 0.2)
+                d[0, 3, 7::13, 5::17] = odd
+                layer([cl(d), None])
+                assert mode == "off" or nat.lib.mie_conv_is_exact(C.byref(layer.conv2d._plan(1, 41, 50, dev).args))
+            out[mode] = layer.activation.in_res.reservoir.clone()
+    finally:
+        fl.config.tensor_cores = old
+    got, want = out["auto"], out["off"]
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+    fine = want.isfinite()
+    assert bool(fine.any())
+    assert float(((got - want).abs()[fine] / want.abs()[fine].clamp(min=1.0)).max()) <= 1e-5

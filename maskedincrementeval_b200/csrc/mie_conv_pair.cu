@@ -95,7 +95,8 @@ __device__ __forceinline__ bool pair_group(const TcParams &p, const float *v, un
       sts4(xs + ((h ^ sw) << 4), xn);
     }
     const float thr = THR ? p.thr : 0.0f;
-    flag |= fabsf(o[i].x) > thr || fabsf(o[i].y) > thr || fabsf(o[i].z) > thr || fabsf(o[i].w) > thr;
+    // (of a quad past the last channel the slabs hold zeros, and f(0) - 0 is not zero for a sigmoid that is measured against the carry)
+    if (h < nq) flag |= fabsf(o[i].x) > thr || fabsf(o[i].y) > thr || fabsf(o[i].z) > thr || fabsf(o[i].w) > thr;
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) sts4(os + (((h0 + i) ^ sw) << 4), (THR && !flag) ? make_float4(0.f, 0.f, 0.f, 0.f) : o[i]);

@@ -339,6 +339,8 @@ class UNetRecurrentIncr(BaseUNetIncr):
     """Recurrent UNet (reference ``:382-468``): head conv5x5, ``num_encoders`` strided conv + ConvLSTM encoders,
     residual blocks, upsampling decoders with summed skips, 1x1 prediction and a final activation."""
 
+    PASS_IS_KERNELS = True      # the dense pass under NATIVE: IncrementalRunner may replay it
+
     def __init__(self, num_input_channels, num_output_channels=1, skip_type='sum',
                  recurrent_block_type='convlstm', activation='sigmoid', num_encoders=4, base_num_channels=32,
                  num_residual_blocks=2, norm=None, use_upsample_conv=True, compat: Optional[str] = None):
@@ -404,6 +406,8 @@ class E2VIDRecurrentIncr(nn.Module):
 
     DEFAULTS = dict(skip_type='sum', num_encoders=4, base_num_channels=32, num_residual_blocks=2, norm=None,
                     use_upsample_conv=True, recurrent_block_type='convlstm')
+
+    PASS_IS_KERNELS = True      # the dense pass under NATIVE: IncrementalRunner may replay it
 
     def __init__(self, config):
         super().__init__()

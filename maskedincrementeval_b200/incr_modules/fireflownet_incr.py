@@ -13,6 +13,8 @@ from .mask_incr_modules import nnConvIncr, set_precision  # noqa: F401  (nnConvI
 
 
 class FireFlowNetIncr(nn.Module):
+    PASS_IS_KERNELS = True      # the dense pass under NATIVE: IncrementalRunner may replay it
+
     def __init__(self, unet_kwargs, num_bins, compat: Optional[str] = None, precision: Optional[str] = "split"):
         super().__init__()
         base_num_channels = unet_kwargs["base_num_channels"]

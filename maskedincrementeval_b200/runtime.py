@@ -22,6 +22,11 @@ from . import fields as fl
 from .fields import TileMask
 
 
+# Modules whose dense pass is known, and the methods that make it up: one set on an object may do anything.
+_PLAIN_MODULES = (__package__ + ".", "torch.nn.")
+_PASS_METHODS = ("forward_refresh_reservoirs", "refresh_native", "forward_fused", "_run", "forward")
+
+
 def _deltas_of(out) -> List:
     """The list of ``[delta, mask]`` outputs in whatever structure the network returns."""
     if isinstance(out, dict):
@@ -157,9 +162,14 @@ class IncrementalRunner:
     # A refresh of one 260x346 stream is some forty short kernels, enqueued one by one in twice the time that they take
     # (910 us a pass; the kernels 450).
     def _may_record_pass(self, x) -> bool:
-        c = fl.config
+        # Only networks that say of themselves that their pass is launches of the library's kernels alone (``PASS_IS_KERNELS``), and
+        # only where it is: PyTorch's dense operators follow switches, and a subclass may do what a replay would not do again.
+        from .incr_modules._algebra import NATIVE, dense_ops
+        c, net = fl.config, self.model
         return (self.use_graph and not self.feedback and self._x_prev is not None and x.is_cuda and x.dtype == torch.float32
-                and x.shape == self._x_prev.shape and c.refresh == "native" and not c.tail_dilation and not c.kfenced_step)
+                and x.shape == self._x_prev.shape and c.refresh == "native" and not c.tail_dilation and not c.kfenced_step
+                and "PASS_IS_KERNELS" in type(net).__dict__ and dense_ops(getattr(net, "unetrecurrent", net), x) is NATIVE
+                and all(type(m).__module__.startswith(_PLAIN_MODULES) and m.__dict__.keys().isdisjoint(_PASS_METHODS) for m in net.modules()))
 
     def _pass_state(self, x):
         """Everything a dense pass of this model is decided by: objects (by identity) and plain values; and the objects, which whoever

@@ -400,3 +400,58 @@ def test_a_replayed_dense_pass_is_an_eager_one(dev, change):
         fl.config.tensor_cores = old
     for y, w in zip(outs, want):
         assert torch.equal(y, w)
+
+
+def _flow_net(dev, cls=None):
+    from maskedincrementeval_b200.incr_modules.fireflownet_incr import FireFlowNetIncr
+    torch.manual_seed(23)
+    return (cls or FireFlowNetIncr)(dict(base_num_channels=16, kernel_size=3, mask_output=False), 2, compat="exact").to(dev).eval()
+
+
+def _frames(dev, channels, h, w):
+    g = torch.Generator(device=dev).manual_seed(24)
+    return [cl(torch.randn(1, channels, h, w, generator=g, device=dev)) for _ in range(3)]
+
+
+def test_a_dense_pass_on_the_library_follows_its_switches(dev, monkeypatch):
+    """The delayed EV-FlowNet's dense pass runs on PyTorch's operators, which follow switches of their own: it is not replayed."""
+    from maskedincrementeval_b200.incr_modules.delayedevflownet_incr import DelayedEVFlowNetIncr
+    from maskedincrementeval_b200.runtime import IncrementalRunner
+    torch.manual_seed(25)
+    net = DelayedEVFlowNetIncr(dict(base_num_channels=32, kernel_size=3, mask_output=False), 2, compat="exact").to(dev).eval()
+    frames = _frames(dev, 2, 64, 64)
+    monkeypatch.setattr(torch.backends.cudnn, "allow_tf32", True)
+    run = IncrementalRunner(net)
+    for i in range(7):
+        run.refresh(frames[i % 3])
+    monkeypatch.setattr(torch.backends.cudnn, "allow_tf32", False)
+    got = [y.clone() for y in run.refresh(frames[0])]
+    with torch.no_grad():
+        want = net.forward_refresh_reservoirs(frames[0])["flow"]
+    assert all(torch.equal(y, w) for y, w in zip(got, want))
+
+
+def test_a_dense_pass_that_does_more_than_launch_kernels_is_run(dev):
+    """A subclass may count its passes or read from the device in them; so may a method set on an object."""
+    from maskedincrementeval_b200.incr_modules.fireflownet_incr import FireFlowNetIncr
+    from maskedincrementeval_b200.runtime import IncrementalRunner
+    seen = []
+
+    class Counting(FireFlowNetIncr):
+        def forward_refresh_reservoirs(self, x):
+            out = super().forward_refresh_reservoirs(x)
+            seen.append(float(out["flow"][0].abs().max()))
+            return out
+
+    frames = _frames(dev, 2, 40, 56)
+    run = IncrementalRunner(_flow_net(dev, Counting))
+    for i in range(8):
+        y = run.refresh(frames[i % 3])
+        assert len(seen) == i + 1 and seen[-1] == float(y.abs().max())
+    net = _flow_net(dev)
+    whole, calls = net.E2._run, []
+    net.E2._run = lambda ops, x: (calls.append(1), whole(ops, x))[1]
+    run = IncrementalRunner(net)
+    for i in range(8):
+        run.refresh(frames[i % 3])
+    assert len(calls) == 8

@@ -20,6 +20,7 @@ import torch
 from . import _native as nat
 from . import fields as fl
 from .fields import TileMask
+from .incr_modules.mask_incr_functional import IncrementReserve
 
 
 # Modules whose dense pass is known, and the methods that make it up: one set on an object may do anything.
@@ -172,9 +173,11 @@ class IncrementalRunner:
                 and all(type(m).__module__.startswith(_PLAIN_MODULES) and m.__dict__.keys().isdisjoint(_PASS_METHODS) for m in net.modules()))
 
     def _pass_state(self, x):
-        """Everything a dense pass of this model is decided by: objects (by identity) and plain values; and the objects, which whoever
-        keeps the state holds on to, so that no other object can be given one of their ids."""
+        """What a dense pass of this model is decided by, and the objects whose ids that names (whoever keeps it holds on to them, so
+        that no other object can be given one of the ids).  Of every module: its attributes by identity; its tensors, those in
+        its buffers and state reserves among them, also by version or address; and its plans."""
         objects, values = [], [x.shape, x.device, fl.config.epoch, nat.option_epoch[0], fl.filter_epoch[0], torch.is_autocast_enabled()]
+        buffers = []      # what the pass clears for the steps behind it is all that exists by then
         for m in self.model.modules():
             d = m.__dict__
             objects += d.values()
@@ -183,14 +186,19 @@ class IncrementalRunner:
                 objects.append(p)
                 if p is not None:
                     values.append((p._version, p.data_ptr()))
-            for name in ("in_res", "x1_res", "x2_res", "mp_res"):
-                r = d.get(name)
-                if r is not None:
-                    t = r.reservoir
+            for v in d.values():
+                kind = type(v)
+                if kind is torch.Tensor:
+                    values.append((v.data_ptr(), v.shape, v.stride()))
+                elif kind is fl.Scratch:
+                    buffers += v._b.values()
+                elif kind is IncrementReserve:
+                    t = v.reservoir
                     values.append(None if t is None else (t.data_ptr(), t.shape, t.stride()))
-            for p in d.get("_plans", {}).values():
-                objects += (p, p.tail)
-                values.append(p.needs_clear)
+            for v in d.get("_plans", {}).values():
+                objects += (v, v.tail)
+                values.append(v.needs_clear)
+        objects += buffers
         return (tuple(map(id, objects)), values), objects
 
     def _record_pass(self, x, key, refs) -> None:

@@ -130,3 +130,29 @@ def test_install_aliases():
     import sys
     for k in [k for k in sys.modules if k == "ext" or k.startswith("ext.") or k == "incr_modules" or k.startswith("incr_modules.")]:
         del sys.modules[k]
+
+
+def test_what_a_recorded_dense_pass_holds_for():
+    """The state that IncrementalRunner compares before it replays a dense pass: a state buffer of any name, a buffer made since, a
+    replaced parameter or attribute make it another one; looking does not."""
+    from maskedincrementeval_b200.incr_modules.event_representation_incr import BasicBlockIncr
+    from maskedincrementeval_b200.runtime import IncrementalRunner
+    net = BasicBlockIncr(8)
+    for reserve in (net.res_in, net.res_in2):
+        reserve.update_reservoir(torch.zeros(1, 8, 16, 16))
+    net._scratch = fl.Scratch()
+    net._extra = torch.zeros(4)
+    run, x = IncrementalRunner(net), torch.zeros(1, 8, 16, 16)
+
+    def differs(change):
+        (before, kept), _ = run._pass_state(x), change()
+        return before != run._pass_state(x)[0] and bool(kept)
+
+    assert not differs(lambda: None)
+    assert differs(lambda: setattr(net.res_in, "reservoir", net.res_in.reservoir.clone()))
+    assert differs(lambda: setattr(net.res_in2, "reservoir", net.res_in2.reservoir.clone()))
+    assert differs(lambda: net._scratch.get("new", (4,), torch.float32, "cpu"))
+    assert differs(lambda: net._extra.set_(torch.zeros(4)))
+    assert differs(lambda: torch.nn.init.zeros_(net.conv1.weight))
+    assert differs(lambda: setattr(net.relu, "op", torch.tanh))
+    assert not differs(lambda: None)

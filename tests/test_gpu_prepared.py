@@ -455,3 +455,40 @@ def test_a_dense_pass_that_does_more_than_launch_kernels_is_run(dev):
     for i in range(8):
         run.refresh(frames[i % 3])
     assert len(calls) == 8
+
+
+@pytest.mark.parametrize("thr", [0.0, 3e-2])
+@pytest.mark.parametrize("name", ["e2depth", "fireflow"])
+def test_steps_behind_replayed_dense_passes(dev, name, thr):
+    """Dense passes alone until one is recorded, then steps, whose buffers are made only now, passes and steps in turn: what a runner
+    without graphs gives."""
+    from maskedincrementeval_b200 import fields as fl
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import E2VIDRecurrentIncr
+    from maskedincrementeval_b200.runtime import IncrementalRunner
+
+    def net():
+        if name == "fireflow":
+            return _flow_net(dev)
+        torch.manual_seed(26)
+        return E2VIDRecurrentIncr(dict(num_bins=5, skip_type="sum", recurrent_block_type="convlstm", num_encoders=3, base_num_channels=16,
+                                       num_residual_blocks=1, norm=None, use_upsample_conv=True, compat="exact")).to(dev).eval()
+
+    fl.config.threshold = thr
+    frames = _frames(dev, 5 if name == "e2depth" else 2, 40, 56)
+    runners = [IncrementalRunner(net(), use_graph=g) for g in (True, False)]
+
+    def both(call, *a):
+        y, want = (getattr(r, call)(*a) for r in runners)
+        assert torch.equal(y, want), call
+
+    for i in range(6):
+        both("refresh", frames[i % 3])
+    assert runners[0]._pass_graph is not None
+    for i in range(4):
+        both("step", frames[i % 3])
+    for round_ in range(7):
+        both("refresh", frames[round_ % 3])
+        if round_ % 2:
+            for i in range(3):
+                both("step", frames[(round_ + i) % 3])
+    assert runners[0]._pass_graph is not None

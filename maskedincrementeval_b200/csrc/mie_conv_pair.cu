@@ -95,8 +95,13 @@ __device__ __forceinline__ bool pair_group(const TcParams &p, const float *v, un
       sts4(xs + ((h ^ sw) << 4), xn);
     }
     const float thr = THR ? p.thr : 0.0f;
-    // (of a quad past the last channel the slabs hold zeros, and f(0) - 0 is not zero for a sigmoid that is measured against the carry)
-    if (h < nq) flag |= fabsf(o[i].x) > thr || fabsf(o[i].y) > thr || fabsf(o[i].z) > thr || fabsf(o[i].w) > thr;
+    flag |= fabsf(o[i].x) > thr || fabsf(o[i].y) > thr || fabsf(o[i].z) > thr || fabsf(o[i].w) > thr;
+  }
+  // Of a quad past the last channel the slabs hold zeros, and f(0) - 0 is not zero for a sigmoid that is measured against the carry.
+  if (THR && nq - h0 < 4) {
+    flag = false;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) flag |= h0 + i < nq && (fabsf(o[i].x) > p.thr || fabsf(o[i].y) > p.thr || fabsf(o[i].z) > p.thr || fabsf(o[i].w) > p.thr);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) sts4(os + (((h0 + i) ^ sw) << 4), (THR && !flag) ? make_float4(0.f, 0.f, 0.f, 0.f) : o[i]);

@@ -97,6 +97,7 @@ class IncrementalRunner:
         self._pass_key = None      # ... the state it holds for, and what keeps its ids from being given to other objects
         self._pass_refs = None
         self._pass_seen = 0        # eager passes in a row that found the state in _pass_key
+        self._pass_tried = False   # ... and whether one has been recorded since, or was to be
         self._passes = 0           # passes at this input shape
 
     # -- device-side error status ----------------------------------------------------------------
@@ -117,8 +118,9 @@ class IncrementalRunner:
         key = refs = None
         if self._passes > 2 and self._may_record_pass(x):
             key, refs = self._pass_state(x)
+        replay = key is not None and self._pass_graph is not None and key == self._pass_key
         self.check()
-        if key is not None and self._pass_graph is not None and key == self._pass_key:
+        if replay:
             self._x_in.copy_(x)
             self._pass_graph.replay()
             self._frame = 1
@@ -149,7 +151,7 @@ class IncrementalRunner:
             self._pipe = None
             self._eager_steps = 0
             self._heads, self._head_of, self._heads_known = [], {}, False
-            self._pass_graph, self._pass_key, self._pass_refs, self._pass_seen, self._passes = None, None, None, 0, 1
+            self._pass_graph, self._pass_key, self._pass_refs, self._pass_seen, self._pass_tried, self._passes = None, None, None, 0, False, 1
         else:
             self._x_prev.copy_(x)
             for dst, src in zip(self._y, ys):
@@ -169,8 +171,7 @@ class IncrementalRunner:
         c, net = fl.config, self.model
         return (self.use_graph and not self.feedback and self._x_prev is not None and x.is_cuda and x.dtype == torch.float32
                 and x.shape == self._x_prev.shape and c.refresh == "native" and not c.tail_dilation and not c.kfenced_step
-                and "PASS_IS_KERNELS" in type(net).__dict__ and dense_ops(getattr(net, "unetrecurrent", net), x) is NATIVE
-                and all(type(m).__module__.startswith(_PLAIN_MODULES) and m.__dict__.keys().isdisjoint(_PASS_METHODS) for m in net.modules()))
+                and "PASS_IS_KERNELS" in type(net).__dict__ and dense_ops(getattr(net, "unetrecurrent", net), x) is NATIVE)
 
     def _pass_state(self, x):
         """What a dense pass of this model is decided by, and the objects whose ids that names (whoever keeps it holds on to them, so
@@ -204,19 +205,26 @@ class IncrementalRunner:
     def _record_pass(self, x, key, refs) -> None:
         """After an eager pass that found the model as ``key`` says: record one if two before it found it so too."""
         if key != self._pass_key:
-            self._pass_graph, self._pass_key, self._pass_refs, self._pass_seen = None, key, refs, 1
+            self._pass_graph, self._pass_key, self._pass_refs, self._pass_seen, self._pass_tried = None, key, refs, 1, False
             return
         self._pass_seen += 1
-        if self._pass_seen < 3 or self._pass_state(x)[0] != key:
+        if self._pass_seen < 3 or self._pass_tried or self._pass_state(x)[0] != key:
+            return
+        self._pass_tried = True      # a recording that comes to nothing is not tried again in this state
+        if not all(type(m).__module__.startswith(_PLAIN_MODULES) and m.__dict__.keys().isdisjoint(_PASS_METHODS) for m in self.model.modules()):
             return
         torch.cuda.synchronize(x.device)
         g = torch.cuda.CUDAGraph()
-        with torch.no_grad(), torch.cuda.graph(g):
-            out = self.model.forward_refresh_reservoirs(self._x_in, None) if self.takes_states else \
-                self.model.forward_refresh_reservoirs(self._x_in)
-            self._x_prev.copy_(self._x_in)
-            for dst, src in zip(self._y, _dense_of(out)):
-                dst.copy_(src)
+        try:
+            # (thread-local: another thread, a loader's for instance, may allocate meanwhile)
+            with torch.cuda.device(x.device), torch.no_grad(), torch.cuda.graph(g, capture_error_mode="thread_local"):
+                out = self.model.forward_refresh_reservoirs(self._x_in, None) if self.takes_states else \
+                    self.model.forward_refresh_reservoirs(self._x_in)
+                self._x_prev.copy_(self._x_in)
+                for dst, src in zip(self._y, _dense_of(out)):
+                    dst.copy_(src)
+        except Exception:      # the eager pass in front has given this call's result; passes go on like that
+            return
         # (the recording ran the pass's host side once more: it has to have left everything as it was)
         self._pass_graph = g if self._pass_state(x)[0] == key else None
 

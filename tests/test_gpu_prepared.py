@@ -492,3 +492,35 @@ def test_steps_behind_replayed_dense_passes(dev, name, thr):
             for i in range(3):
                 both("step", frames[(round_ + i) % 3])
     assert runners[0]._pass_graph is not None
+
+
+def test_a_dense_pass_that_cannot_be_recorded(dev, monkeypatch):
+    """A recording that fails costs nothing but the attempt: passes go on one by one, and the next attempt is made for another state."""
+    from maskedincrementeval_b200.runtime import IncrementalRunner
+    frames, net, tried = _frames(dev, 2, 40, 56), _flow_net(dev), []
+
+    class Refused(torch.cuda.graph):
+        def __enter__(self):
+            tried.append(self.capture_error_mode)
+            raise RuntimeError("refused")
+
+    run, eager = IncrementalRunner(net), IncrementalRunner(_flow_net(dev), use_graph=False)
+
+    def passes(count):
+        for i in range(count):
+            assert torch.equal(run.refresh(frames[i % 3]), eager.refresh(frames[i % 3]))
+
+    with monkeypatch.context() as m:
+        m.setattr(torch.cuda, "graph", Refused)
+        passes(9)
+        assert tried == ["thread_local"] and run._pass_graph is None
+        for r in (run, eager):
+            _double_head(r.model)
+        passes(9)
+        assert len(tried) == 2
+    for r in (run, eager):
+        _double_head(r.model)
+    passes(7)
+    assert run._pass_graph is not None
+    passes(2)
+    assert torch.equal(run.step(frames[1]), eager.step(frames[1]))

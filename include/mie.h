@@ -245,9 +245,10 @@ int mie_conv_step(const mie_conv_args *args /* host */, uint64_t *mask_bits, flo
                   void *stream);
 
 /* One dense evaluation of a layer in fp32 precision on the tensor cores in one call: of every output tile (max_tiles has to be
- * their number for that; else of those that mie_tiles_dilate lists as `dilate` describes), on the field x; where x or its pixel stride is not 16-byte aligned, on a copy of it (mie_pad_field) that
+ * their number for that; else of those that mie_tiles_dilate lists as `dilate` describes), on the field x; where x or its pixel
+ * stride is not 16-byte aligned, on a copy of it (mie_pad_field) that
  * is made in args->in with pixel stride args->in_ps.  No list is made when every tile is taken: `list` and counts[0..2] then
- * stay as they are. */
+ * stay as they are, while `dilate` is checked all the same.  Tile words are written whole and need no clearing. */
 int mie_conv_refresh_step(const mie_conv_args *args /* host */, const float *x, int64_t x_ps, const mie_tail_job *dilate /* host */,
                           void *stream);
 

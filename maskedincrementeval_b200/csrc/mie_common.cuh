@@ -178,6 +178,8 @@ __device__ void block_ordered_compact2(Flag flag, int n, int32_t *listA, int32_t
   *nb = s_bb;
 }
 
+int dilate_check(const mie_tail_job &j);      // what mie_tiles_dilate refuses (mie_mask.cu)
+
 // ---------------------------------------------------------------------------------------------
 // dilated output-tile set of a convolution: the per-tile test shared by the dilation kernels and the tail job
 // ---------------------------------------------------------------------------------------------

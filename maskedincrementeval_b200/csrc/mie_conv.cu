@@ -796,10 +796,11 @@ extern "C" int mie_conv_refresh_step(const mie_conv_args *a, const float *x, int
   int s = conv_check(&b);
   if (s != MIE_OK) return s;
   // Every output tile has to be listed, so no list is made: the kernel takes the tiles as they come.  The tile words need no clearing
-  // either, since every pixel of the field is marked.  (With the launch a pass over one 260x346 stream took 653 us, without it 607; eight 480x640 streams 9340 and 8784.)
-  if ((int64_t)b.n * divup(b.hout, 8) * divup(b.wout, 8) == b.max_tiles && !b.tail)
+  // either: the kernel writes them whole.  (With the launch a pass over one 260x346 stream took 653 us, without it 607; eight 480x640 streams 9340 and 8784.)
+  if ((int64_t)b.n * divup(b.hout, 8) * divup(b.wout, 8) == b.max_tiles && !b.tail) {
+    if ((s = dilate_check(*d)) != MIE_OK) return s;
     b.list = nullptr;
-  else
+  } else
     s = mie_tiles_dilate(d->in_bits, d->N, d->Hin, d->Win, d->Hout, d->Wout, d->k, d->stride, d->pad, d->union_bits, d->out_bits, d->list, d->stale, d->counts, d->flags,
                          stream);
   if (s == MIE_OK && !direct)

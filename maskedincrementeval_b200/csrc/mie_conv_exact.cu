@@ -558,7 +558,9 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
       const unsigned bal = __ballot_sync(0xffffffffu, sent);
       if ((lane == 0 || lane == 8) && t >= 0) {
         const unsigned rows = ((bal >> lane) & 0xFFu) | (((bal >> (16 + lane)) & 0xFFu) << 8);
-        if (rows) atomicOr(p.out_bits32 + 2 * (size_t)t + (q >> 1), rows << ((q & 1) * 16));
+        // (dense: every column block has the same rows to say, and says them whatever stood there)
+        if (!STEP) reinterpret_cast<unsigned short *>(p.out_bits32)[4 * (size_t)t + q] = (unsigned short)rows;
+        else if (rows) atomicOr(p.out_bits32 + 2 * (size_t)t + (q >> 1), rows << ((q & 1) * 16));
       }
     }
     if (chief) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");

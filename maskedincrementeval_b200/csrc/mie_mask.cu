@@ -396,13 +396,19 @@ __global__ void __launch_bounds__(1024) tiles_dilate_small_kernel(
   }
 }
 
+int mie::dilate_check(const mie_tail_job &j) {
+  if (!j.in_bits || !j.list || !j.counts || !j.flags || j.N <= 0 || j.Hin <= 0 || j.Win <= 0 || j.Hout <= 0 || j.Wout <= 0) return MIE_EINVAL;
+  if (j.k < 1 || j.k > 7 || j.stride < 1 || j.stride > 2 || j.pad < 0 || j.pad > j.k) return MIE_EUNSUPPORTED;
+  return j.out_bits && !j.stale ? MIE_EINVAL : MIE_OK;
+}
+
 extern "C" int mie_tiles_dilate(const uint64_t *in_bits, int N, int Hin, int Win, int Hout, int Wout, int k,
                                 int stride, int pad, const uint64_t *union_bits, uint64_t *out_bits,
                                 int32_t *list, int32_t *stale, int32_t *counts, uint8_t *flags, void *stream) {
-  if (!in_bits || !list || !counts || !flags || N <= 0 || Hin <= 0 || Win <= 0 || Hout <= 0 || Wout <= 0)
-    return MIE_EINVAL;
-  if (k < 1 || k > 7 || stride < 1 || stride > 2 || pad < 0 || pad > k) return MIE_EUNSUPPORTED;
-  if (out_bits && !stale) return MIE_EINVAL;
+  {
+    const int s = dilate_check({in_bits, N, Hin, Win, Hout, Wout, k, stride, pad, union_bits, out_bits, list, stale, counts, flags});
+    if (s != MIE_OK) return s;
+  }
   const int ntiles = N * divup(Hout, 8) * divup(Wout, 8);
   if (ntiles <= DILATE_SMALL_MAX) {
     const int threads = ntiles <= 256 ? 256 : (ntiles <= 512 ? 512 : 1024);

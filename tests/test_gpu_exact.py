@@ -486,3 +486,25 @@ def test_thresholded_sigmoid_of_partial_groups(dev, cout, stride):
         both = (dy != 0) & (want != 0)
         assert not bool(both.any()) or float((dy - want)[both].abs().max()) <= 2e-4
         assert float((m != wm).float().mean()) <= 0.01 and float(((dy != 0) != (want != 0)).float().mean()) <= 0.01
+
+
+# ragged and whole tiles, one column block and three, both widths of block
+@pytest.mark.parametrize("cin,cout,h,w", [(32, 32, 41, 50), (64, 96, 9, 9), (64, 64, 104, 100), (48, 36, 16, 24)])
+def test_dense_step_writes_whole_tile_words(dev, cin, cout, h, w):
+    """mie_conv_refresh_step makes no list: the tile words it finds may hold anything, and a bad dilation is refused as ever."""
+    from maskedincrementeval_b200 import fields as fl, _native as nat
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    torch.manual_seed(27)
+    c, x = ConvLayerIncr(cin, cout, 3, 1, 1, activation="relu").to(dev).eval(), cl(torch.randn(2, cin, h, w, device=dev))
+    with torch.no_grad():
+        y, m = NATIVE.conv(c.conv2d, NATIVE.lift(x), c.activation)
+        want, plan = y.clone(), c.conv2d._plan(2, h, w, dev)
+        plan.out_bits.fill_(-1)
+        taken = next(iter(c.conv2d._prepared_refresh.values()))
+        nat.check(nat.lib.mie_conv_refresh_step(C.byref(taken.args), x.data_ptr(), cin, C.addressof(taken.job.c), nat.stream_ptr(dev)), "refresh_step")
+        assert torch.equal(plan.out_bits, fl.full_mask(2, h, w, dev).bits) and torch.equal(plan.out, want)
+        for field, value, status in (("k", 9, nat.EUNSUPPORTED), ("N", 0, nat.EINVAL), ("flags", None, nat.EINVAL)):
+            bad = type(taken.job.c).from_buffer_copy(taken.job.c)
+            setattr(bad, field, value)
+            assert nat.lib.mie_conv_refresh_step(C.byref(taken.args), x.data_ptr(), cin, C.addressof(bad), nat.stream_ptr(dev)) == status

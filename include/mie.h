@@ -305,9 +305,9 @@ int mie_activation_increment(float *X, const float *in_incr, float *out_incr, in
  * (pointops_functional.py:13-14); out_incr [N,Cout,Hout,Wout] channels-last, every element is
  * written (the reference hands in torch.empty, pointops_functional.py:29).  pad = k/2.
  * Layers with Cin >= 48, k >= 3 and Cout a multiple of 4 run in fp32 precision on the tensor cores, the others on the
- * FP32 kernels (also where a pointer is not 16-byte aligned, and stride 2 on fields one pixel wide or high).
+ * FP32 kernels (also where out_incr is not 16-byte aligned, and stride 2 on fields one pixel wide or high).
  * workspace: device scratch of mie_conv_increment_workspace_bytes(...) bytes, 256-byte aligned; for the layers named it holds the
- * packed filter and two copies of the input. */
+ * packed filter and, where Cin is no multiple of 4 or x_incr not 16-byte aligned, a copy of the input (room for it in any case). */
 int64_t mie_conv_increment_workspace_bytes(int N, int cin, int H, int W, int cout, int k, int stride);
 int mie_conv_increment_ext(const float *x_incr, const void *mask, int mask_elem_size, const float *filter,
                            float *out_incr, int N, int cin, int H, int W, int cout, int k, int stride,

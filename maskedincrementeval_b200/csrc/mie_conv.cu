@@ -825,7 +825,7 @@ extern "C" int mie_conv_step(const mie_conv_args *a, uint64_t *mask_bits, float 
 namespace {
 struct IncWs {
   size_t bits_in, bits_out, counts, list, stale, flags, wpacked, wexact, copy, total;
-  int cp;      // channels of the input's copy, where it needs one
+  int cp;      // channels of the input's copy, which one that TMA cannot read as it lies needs
 };
 // fp32 precision on the tensor cores, for deltas of 48 channels or more: with fewer, the few products that meet at an isolated
 // active pixel leave the FP32 kernel the smaller error (5 channels 9e-8 against 5e-8, 16 1.0e-7 / 8e-8, 32 1.3e-7 / 1.1e-7; 48
@@ -856,7 +856,7 @@ IncWs inc_layout(int N, int cin, int H, int W, int cout, int k, int stride) {
     mie_conv_pack_dims_exact(cin, cout, k, &ne);
     o += up((size_t)ne * 4);
     w.copy = o;
-    if (cin % 4) o += up((size_t)N * H * W * w.cp * 4);
+    o += up((size_t)N * H * W * w.cp * 4);
   }
   w.total = o;
   return w;
@@ -924,7 +924,8 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   float *wx = reinterpret_cast<float *>(ws + L.wexact), *copy = reinterpret_cast<float *>(ws + L.copy);
   x.refresh = 1;
   x.wpacked_exact = wx;
-  if (cin % 4) { x.in = copy; x.in_ps = L.cp; }
+  const bool copied = cin % 4 || !aligned16(x_incr);
+  if (copied) { x.in = copy; x.in_ps = L.cp; }
   const bool exact = inc_exact(cin, cout, k) && exact_takes(&x);
   if (exact) {
     if ((s = pack_exact(filter, cout, cin, k, 1, wx, st)) != MIE_OK) return s;
@@ -937,6 +938,6 @@ extern "C" int mie_conv_increment_ext(const float *x_incr, const void *mask, int
   s = mie_tiles_dilate(bits_in, N, H, W, Ho, Wo, k, stride, pad, nullptr, nullptr, list, nullptr, counts, flags, stream);
   if (s != MIE_OK) return s;
   if (!exact) return mie_conv_tiles(&a, stream);
-  if (cin % 4 && (s = pad_field(x_incr, cin, cin, (int64_t)N * H * W, copy, nullptr, L.cp, counts, st)) != MIE_OK) return s;
+  if (copied && (s = pad_field(x_incr, cin, cin, (int64_t)N * H * W, copy, nullptr, L.cp, counts, st)) != MIE_OK) return s;
   return launch_conv_exact(&x, filter, cout, (int64_t)k * k * cout, st);
 }

@@ -508,3 +508,17 @@ def test_dense_step_writes_whole_tile_words(dev, cin, cout, h, w):
             bad = type(taken.job.c).from_buffer_copy(taken.job.c)
             setattr(bad, field, value)
             assert nat.lib.mie_conv_refresh_step(C.byref(taken.args), x.data_ptr(), cin, C.addressof(bad), nat.stream_ptr(dev)) == status
+
+
+@pytest.mark.parametrize("cin,offset", [(64, 1), (64, 2), (48, 3), (50, 1)])
+def test_extension_on_an_input_that_is_not_aligned(dev, cin, offset):
+    """An input at an odd address runs as one at an even address does: the same kernel, the same bits."""
+    from maskedincrementeval_b200.ext.pointops import pointops_functional as pf
+    g = torch.Generator(device=dev).manual_seed(28)
+    w = torch.randn(cin, 3, 3, 64, generator=g, device=dev) * 0.04
+    store = torch.randn(2 * 33 * 41 * cin + 4, generator=g, device=dev)
+    x = store[offset:offset + 2 * 33 * 41 * cin].view(2, 33, 41, cin).permute(0, 3, 1, 2)
+    assert x.data_ptr() % 16
+    y, _ = pf.functional_conv_module(x, w, mask=None, stride=(1, 1), padding=(1, 1))
+    want, _ = pf.functional_conv_module(x.clone(memory_format=torch.channels_last), w, mask=None, stride=(1, 1), padding=(1, 1))
+    assert torch.equal(y, want)

@@ -1,4 +1,5 @@
-// Dense evaluation (the refresh pass) in fp32 precision on the tensor cores, on CTA pairs like mie_conv_pair.cu.
+// Convolutions in fp32 precision on the tensor cores, on CTA pairs like mie_conv_pair.cu: the dense evaluation (the refresh pass), and
+// incremental steps of layers in split precision.
 //
 // Every operand is two FP16 numbers with a common power-of-two scale (mie_pair.cuh), together the fp32 value to 2^-24, and a
 // product is hi*hi + hi*lo + lo*hi; the dropped lo*lo is 2^-24 of it.  The halo arrives as fp32 and is split in shared memory by
@@ -19,7 +20,10 @@
 // What bounds it: operand reads and everything else that goes through shared memory (per tap and 32 channels, blocks of 64: 172 clocks
 // of its port for the instructions, which take 214 in the tensor core, 32 for the filter arriving, 35 to 70 for the
 // halo arriving and being split), then the epilogue's slabs on layers of few units (a chunk of a view) per item.
-// Epilogue: reservoir = conv + bias (+ addend), output = f(reservoir), every pixel of a listed tile marked.
+// Epilogue, dense: reservoir = conv + bias (+ addend), output = f(reservoir), every pixel of a tile marked.  A step: reservoir += conv
+// (+ addend), output = the change of f(reservoir), threshold, carry and marks as in the other step kernels.
+// What the parts do not hold (mie_pair.cuh) is multiplied with FP32 instructions, in functions that the ordinary course calls at most once an
+// item and keeps no registers for.
 #include <algorithm>
 #include "mie_pair.cuh"
 
@@ -35,7 +39,7 @@ constexpr int EXACT_MAX_HALOS = 4;
 struct ExactParams {
   const float *in; int64_t in_ps; int hin, win, k, stride, pad;      // read by the FP32 fallback only, like the filter below
   const float *fw; int64_t fw_tap, fw_ci; int fw_vec;                // filter entry (tap, ci, co) at fw[tap * fw_tap + ci * fw_ci + co]
-  const float *winv;                                                 // inverse scale of every output channel's filter; NaN: fallback
+  const float *winv;                                                 // inverse scale of every output channel's filter; NaN: not split
   int cin, cout, cout_pad, n_chunks, n, hout, wout;
   const int32_t *list; int32_t *counts; int max_tiles;               // list null (dense pass): every tile
   float *out; int64_t out_ps; unsigned int *out_bits32;
@@ -50,7 +54,7 @@ struct ExactParams {
   unsigned div_tw, div_th; // magic numbers for divisions by the field's tiles per row and rows of tiles; 0: plain division
   mie_tail_job tail;
   PairTaps t;
-  TcParams c;              // a step: threshold, carry, stale tiles, own-tiles mode
+  TcParams c;              // a step: threshold, carry, stale tiles
 };
 struct ExactMaps {
   CUtensorMap in[4], w, out, res, emitted;
@@ -146,32 +150,70 @@ __device__ __forceinline__ void exact_issue(const ExactIssue a, const PairTapTab
   }
 }
 
-// One pixel's channels [co, co + HW) with FP32 instructions, for what two FP16 parts cannot hold (SplitShared, `winv`): the same sums as
-// the FP32 kernel's, padding multiplied as zeros like there.  Bounded by its loads (about 0.5 ms for an item of 256 channels and 5x5
-// taps), which no finite field of ordinary values comes to.
-__device__ __noinline__ void exact_fp32_quad(const ExactParams &p, int n, int oy, int ox, int c, float4 &out) {
-  out = make_float4(0.f, 0.f, 0.f, 0.f);
+// ---- what two FP16 parts cannot hold, with FP32 instructions: out of line and on arrays in local memory, since what is run this seldom is
+// paid in instructions that are fetched, and what it keeps in registers by everything else ----
+// Adds to sums (HW channels from co on, in true units) the products of the values that were taken out of an item's unit cu (ring unit u), as
+// far as this thread's pixel and the taps of the unit's view reach them.  Returns whether there were any; reach: only that.
+template <int HW>
+__device__ __noinline__ bool exact_small(const ExactParams &p, const SplitShared &sh, unsigned u, int cu, int co, float *sums, bool reach) {
+  const SplitSmall &list = sh.small[u % SPLIT_RING];
+  const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) & 3, slot = (lane >> 3) & 1, prow = 2 * q + (lane >> 4), pcol = lane & 7;
+  const int nv = p.t.nviews, view = cu % nv, chunk = cu / nv, odd_y = p.stride == 2 ? view >> 1 : 0, odd_x = p.stride == 2 ? view & 1 : 0;
+  bool any = false;
+#pragma unroll 1
+  for (int i = 0; i < SPLIT_LISTED && list.at[i] != SPLIT_NONE; ++i) {
+    const int at = list.at[i];
+    // the tap that meets it at this pixel
+    const int ky = p.stride * (p.t.y0[view] + (at >> 9 & 15) - prow) + odd_y + p.pad, kx = p.stride * (p.t.x0[view] + (at >> 5 & 15) - pcol) + odd_x + p.pad;
+    if (at >> 13 != slot || ky < 0 || ky >= p.k || kx < 0 || kx >= p.k) continue;
+    any = true;
+    if (reach) continue;
+    const float *w = p.fw + (ky * p.k + kx) * p.fw_tap + (32 * chunk + (at & 31)) * p.fw_ci + co;
+#pragma unroll 4
+    for (int c = 0; c < HW; ++c)
+      if (co + c < p.cout) sums[c] += list.value[i] * __ldg(w + c);
+  }
+  return any;
+}
+
+// All channels of a pixel, where a halo or a channel's filter was not split: the same sums as the FP32 kernel's, padding multiplied as zeros
+// like there.  Infinities, NaN, values above 2^100, many values far apart and filters with entries too far apart come to this.  Bounded by
+// the latency of its loads, which the few KB of L1 beside the shared memory do not hold (64 -> 64 3x3 at 264x352, every halo: 3600 us, the FP32
+// kernel 285, split 36).  which: a bit per channel that is wanted.
+template <int HW>
+__device__ __noinline__ void exact_fp32(const ExactParams &p, int n, int oy, int ox, int co, unsigned which, float *sums) {
+  float acc[HW];
+#pragma unroll
+  for (int i = 0; i < HW; ++i) acc[i] = 0.0f;
 #pragma unroll 1
   for (int tap = 0; tap < p.k * p.k; ++tap) {
     const int iy = oy * p.stride - p.pad + tap / p.k, ix = ox * p.stride - p.pad + tap % p.k;
     const bool in = iy >= 0 && iy < p.hin && ix >= 0 && ix < p.win;
-    const float *x = p.in + (in ? ((int64_t)(n * p.hin + iy) * p.win + ix) * p.in_ps : 0), *w = p.fw + tap * p.fw_tap + c;
-#pragma unroll 4
-    for (int ci = 0; ci < p.cin; ++ci, w += p.fw_ci) {
-      const float xv = in ? __ldg(x + ci) : 0.0f;
-      const float4 f = p.fw_vec ? __ldg(reinterpret_cast<const float4 *>(w)) : make_float4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
-      out.x = fmaf(xv, f.x, out.x); out.y = fmaf(xv, f.y, out.y); out.z = fmaf(xv, f.z, out.z); out.w = fmaf(xv, f.w, out.w);
+    // (pixels are 16-byte aligned, a multiple of four channels apart; what lies behind the last channel is not used)
+    const float4 *x = reinterpret_cast<const float4 *>(p.in + (in ? ((int64_t)(n * p.hin + iy) * p.win + ix) * p.in_ps : 0));
+    const float *w = p.fw + tap * p.fw_tap + co;
+    float4 next = __ldg(x);
+#pragma unroll 1
+    for (int c4 = 0; c4 < p.cin; c4 += 4) {
+      const float4 now = next;
+      if (c4 + 4 < p.cin) next = __ldg(++x);
+#pragma unroll
+      for (int j = 0; j < 4; ++j, w += p.fw_ci) {
+        if (c4 + j >= p.cin) break;
+        const float xv = !in ? 0.0f : j == 0 ? now.x : j == 1 ? now.y : j == 2 ? now.z : now.w;
+#pragma unroll
+        for (int h = 0; h < HW; h += 4) {
+          float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (co + h < p.cout)
+            f = p.fw_vec ? __ldg(reinterpret_cast<const float4 *>(w + h)) : make_float4(__ldg(w + h), __ldg(w + h + 1), __ldg(w + h + 2), __ldg(w + h + 3));
+          acc[h] = fmaf(xv, f.x, acc[h]); acc[h + 1] = fmaf(xv, f.y, acc[h + 1]); acc[h + 2] = fmaf(xv, f.z, acc[h + 2]); acc[h + 3] = fmaf(xv, f.w, acc[h + 3]);
+        }
+      }
     }
   }
-}
-template <int HW>
-__device__ __forceinline__ void exact_fp32(const ExactParams &p, int n, int oy, int ox, bool valid, int co, float *acc) {
 #pragma unroll
-  for (int h = 0; h < HW / 4; ++h) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid && co + 4 * h < p.cout) exact_fp32_quad(p, n, oy, ox, co + 4 * h, v);
-    acc[4 * h] = v.x; acc[4 * h + 1] = v.y; acc[4 * h + 2] = v.z; acc[4 * h + 3] = v.w;
-  }
+  for (int i = 0; i < HW; ++i)
+    if (which >> i & 1u) sums[i] = acc[i];
 }
 
 // A step's activation at one pixel: acc, the convolution's channels; the pixel's rows of the reservoir, output and carry slabs.  Groups of 16
@@ -221,10 +263,94 @@ __device__ __forceinline__ void tmem_ld8_async(unsigned taddr, unsigned *r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
+// eight columns of segment j of channels 8 g on, as in exact_finish
+template <int HW, bool FULL>
+struct ExactColumns {
+  unsigned hi, mid, low, last;
+  __device__ __forceinline__ ExactColumns(unsigned c, unsigned j, unsigned g) {
+    const unsigned at = c + j * exact_cols(HW, FULL), ch = 8u * g;
+    hi = at + ch / (HW / 2) * HW + ch % (HW / 2);
+    mid = hi + HW / 2;
+    low = FULL ? hi + 2u * HW : at + 2u * HW + ch;
+    last = hi + 2u * HW + HW / 2;
+  }
+};
+__device__ __forceinline__ void tmem_st8(unsigned taddr, const float *v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+// An item (tile t of this thread, ring units unit .. unit + units - 1) of which the parts did not hold all, in front of exact_finish: its
+// finished sums take the place of the first segment's high columns, the other columns become zero.  exact_finish then has no
+// branch for it (a test and a call per four channels cost FireFlowNet's step 5 %, mostly in registers).  Called by a converged warp;
+// returns whether any of its pixels was concerned.
+template <int HW, bool FULL>
+__device__ __noinline__ bool exact_rare_item(const ExactParams &p, const SplitShared &sh, unsigned c, unsigned n_seg, unsigned unit, int units, unsigned odd, int t, int co) {
+  const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) & 3, TWo = (p.wout + 7) >> 3, THo = (p.hout + 7) >> 3;
+  const int n = t / (TWo * THo), oy = t / TWo % THo * 8 + 2 * q + (lane >> 4), ox = t % TWo * 8 + (lane & 7);
+  const bool valid = t >= 0 && oy < p.hout && ox < p.wout;
+  bool wide = odd != 0u, any = false;
+#pragma unroll 1
+  for (int cu = 0; cu < units; ++cu) {
+    const float scale = sh.inv[(unit + (unsigned)cu) % SPLIT_RING];
+    wide |= scale != scale;
+    if (valid && scale < 0.0f) any |= exact_small<HW>(p, sh, unit + (unsigned)cu, cu, co, nullptr, true);
+  }
+  if (!__any_sync(0xffffffffu, wide || any)) return false;
+  float sums[HW];
+#pragma unroll 1
+  for (unsigned g = 0; g < HW / 8; ++g) {
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
+#pragma unroll 1
+    for (unsigned j = 0; j < n_seg; ++j) {
+      const ExactColumns<HW, FULL> at(c, j, g);
+      const float inv = fabsf(sh.inv[(unit + (n_seg == 2u ? j * (unsigned)units >> 1 : 0u)) % SPLIT_RING]);
+      unsigned a[8], b[8], d[8], e[8];
+      tmem_ld8_async(at.hi, a);
+      tmem_ld8_async(at.mid, b);
+      tmem_ld8_async(at.low, d);
+      if (FULL) tmem_ld8_async(at.last, e);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(split_sum(a[i], b[i], d[i], FULL ? e[i] : 0u, FULL), inv, acc[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sums[8 * g + i] = acc[i] * __ldg(p.winv + co + 8 * g + i);
+  }
+  unsigned which = odd;
+  if (any)
+#pragma unroll 1
+    for (int cu = 0; cu < units; ++cu)
+      if (sh.inv[(unit + (unsigned)cu) % SPLIT_RING] < 0.0f) exact_small<HW>(p, sh, unit + (unsigned)cu, cu, co, sums, false);
+#pragma unroll 1
+  for (int cu = 0; cu < units; ++cu)
+    if (!(fabsf(sh.inv[(unit + (unsigned)cu) % SPLIT_RING]) > 0.0f)) which = ~0u;
+  if (valid && which) exact_fp32<HW>(p, n, oy, ox, co, which, sums);
+  __syncwarp();
+#pragma unroll 1
+  for (unsigned j = 0; j < n_seg; ++j)
+#pragma unroll 1
+    for (unsigned g = 0; g < HW / 8; ++g) {
+      const ExactColumns<HW, FULL> at(c, j, g);
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = j ? 0.0f : sums[8 * g + i];
+      tmem_st8(at.hi, v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = 0.0f;
+      tmem_st8(at.mid, v);
+      tmem_st8(at.low, v);
+      if (FULL) tmem_st8(at.last, v);
+    }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  return true;
+}
+
+// scales: the channels' inverse scales, four at a time, scale_step apart.
 template <int HW, bool STEP, bool FULL, int ACT>
-__device__ __forceinline__ bool exact_finish(const ExactParams &p, unsigned c, unsigned n_seg, float inv0, float inv1, bool wide, const ExactRow r,
-                                             const float4 *col, int n, int oy, int ox, bool valid, int64_t pix, int co) {
-  constexpr unsigned CB = HW, HB = HW / 2;
+__device__ __forceinline__ bool exact_finish(const ExactParams &p, unsigned c, unsigned n_seg, float inv0, float inv1, const float4 *scales, unsigned scale_step,
+                                             const ExactRow r, const float4 *col, bool valid, int64_t pix, int co) {
   auto f = [&](float4 v) { return make_float4(tc_act<ACT>(p.act, v.x), tc_act<ACT>(p.act, v.y), tc_act<ACT>(p.act, v.z), tc_act<ACT>(p.act, v.w)); };
   const float *addend = p.addend && valid ? p.addend + pix * p.addend_ps + co : nullptr;
   const bool thresholded = STEP && (p.c.thr > 0.0f || p.c.emitted);
@@ -232,19 +358,18 @@ __device__ __forceinline__ bool exact_finish(const ExactParams &p, unsigned c, u
   float top = 0.0f;
 #pragma unroll 1
   for (unsigned g = 0; g < HW / 8; ++g) {
-    __syncwarp();      // (lanes may have parted over the FP32 fallback; the loads from tensor memory are the warp's)
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
 #pragma unroll 1
     for (unsigned j = 0; j < n_seg; ++j) {
-      const unsigned at = c + j * exact_cols(CB, FULL), ch = 8u * g, hi = at + ch / HB * CB + ch % HB;
+      const ExactColumns<HW, FULL> at(c, j, g);
       const float inv = j ? inv1 : inv0;
       unsigned a[8], b[8], d[8], e[8];
-      tmem_ld8_async(hi, a);
-      tmem_ld8_async(hi + HB, b);
-      tmem_ld8_async(FULL ? hi + 2u * CB : at + 2u * CB + ch, d);
-      if (FULL) tmem_ld8_async(hi + 2u * CB + HB, e);
+      tmem_ld8_async(at.hi, a);
+      tmem_ld8_async(at.mid, b);
+      tmem_ld8_async(at.low, d);
+      if (FULL) tmem_ld8_async(at.last, e);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] = fmaf(split_sum(a[i], b[i], d[i], FULL ? e[i] : 0u, FULL), inv, acc[i]);
@@ -254,12 +379,8 @@ __device__ __forceinline__ bool exact_finish(const ExactParams &p, unsigned c, u
       const unsigned h = 2u * g + i, at = (h ^ r.sw) << 4;
       const int ch = (int)(4u * h);
       const bool real = co + ch < p.cout;
-      const float4 w = lds4(smem_u32(col + h));
+      const float4 w = lds4(smem_u32(scales + h * scale_step));
       float4 v = make_float4(acc[4 * i] * w.x, acc[4 * i + 1] * w.y, acc[4 * i + 2] * w.z, acc[4 * i + 3] * w.w);
-      if (wide || w.x != w.x || w.y != w.y || w.z != w.z || w.w != w.w) {
-        v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (valid && real) exact_fp32_quad(p, n, oy, ox, co + ch, v);
-      }
       if (!STEP && p.bias) v = f4add(v, lds4(smem_u32(col + HW / 4 + h)));
       if (addend && real) v = f4add(v, *reinterpret_cast<const float4 *>(addend + ch));
       if (!STEP) {
@@ -303,6 +424,8 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
   __shared__ SplitShared s_split;
   __shared__ PairTapTable s_tap;
   __shared__ float4 s_col[2][2][HW / 4];      // per epilogue set: inverse scales and biases of its channels
+  __shared__ float4 s_one;
+  __shared__ unsigned s_odd[2];               // ... and a bit for every channel whose filter was not split
   __shared__ unsigned s_tmem_base;
   __shared__ int s_abort;
 
@@ -322,6 +445,7 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
       for (int b = 0; b < 4; ++b) mbar_init(&slab_full[b >> 1][b & 1], 2);
     for (unsigned u = 0; u < SPLIT_RING; ++u) mbar_init(&s_split.inv_full[u], 1);
     s_abort = 0;
+    s_one = make_float4(1.f, 1.f, 1.f, 1.f);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 3) {
@@ -371,6 +495,8 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
   } else if (warp >= 12) {
     // =========================== halos as two FP16 parts ===========================
     pair_split_halos(work, halos, a_ready, 2 * p.wp * p.wp, p.wp, n_active, tid - 384, s_split, &s_abort);
+  } else if (warp == 3) {
+    pair_take_out(s_split, 2 * p.wp * p.wp, p.wp, lane);
   } else if (warp >= 4) {
     // =========================== epilogue: set `set` takes channels [set * HW, set * HW + HW) of the block, or every other item ===========================
     const int q = warp & 3, set = (warp - 4) >> 2;
@@ -419,6 +545,14 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
         if (p.c.emitted) tma_load_4d_raw(at + SLAB, &maps.emitted, bar, co, x, y, n);
       }
     };
+    // inverse scales and biases into shared memory, for behind the set's barrier
+    auto keep_column = [&](int at_col, float col) {
+      if (at_col < 2 * HW) reinterpret_cast<float *>(s_col[set][at_col / HW])[at_col % HW] = col;
+      if (q == 0) {
+        const unsigned odd = __ballot_sync(0xffffffffu, at_col < HW && col != col);
+        if (lane == 0) s_odd[set] = odd;
+      }
+    };
     int listed = entry(first);
     if (STEP && chief && first < n_items) fetch_state(first, listed, 0u);
     __syncwarp();
@@ -437,13 +571,14 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
       bool sent = false;
       if constexpr (!ALT) {
         float acc[HW];
-        bool wide = false;
+        float lost[HW];
+        bool wide = false, small = false;
 #pragma unroll
         for (int i = 0; i < HW; ++i) acc[i] = 0.0f;
         for (int cu = 0; cu < units && ok; ++cu, ++unit) {
           const int v = nv == 1 ? 0 : cu % nv;
           if (!(ok = __all_sync(0xffffffffu, mbar_wait(&s_split.inv_full[unit % SPLIT_RING], (unit / SPLIT_RING) & 1u, &s_abort, p.spin_limit)))) break;
-          const float inv = s_split.inv[unit % SPLIT_RING];
+          const float scale = s_split.inv[unit % SPLIT_RING], inv = fabsf(scale);
           for (int left = p.t.first[v + 1] - p.t.first[v]; left > 0; left -= p.tps) {
             if (!(ok = __all_sync(0xffffffffu, mbar_wait(&done[stage], stage_par, &s_abort, p.spin_limit)))) break;
             tc_fence_after();
@@ -456,9 +591,19 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
             if (++seg == (unsigned)p.segs) seg = 0;
             if (++stage == (unsigned)p.stages) { stage = 0; stage_par ^= 1u; }
           }
-          wide |= inv != inv;
+          if (__builtin_expect(!(scale > 0.0f), 0)) {
+            wide |= scale != scale;
+            if (scale < 0.0f && valid) {
+              if (!small)
+#pragma unroll 1
+                for (int i = 0; i < HW; ++i) lost[i] = 0.0f;
+              small = true;
+              exact_small<HW>(p, s_split, unit, cu, co, lost, false);
+            }
+            __syncwarp();
+          }
         }
-        if (at_col < 2 * HW) reinterpret_cast<float *>(s_col[set][at_col / HW])[at_col % HW] = col;
+        keep_column(at_col, col);
         // a warp whose wait gave up goes on to the barrier of its set, where the four of them leave together
         if (!STEP && chief) {      // the buffer is free once the stores of its last item have read it
           if (p.slab_sets == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -476,9 +621,16 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
         for (int h = 0; h < HW / 4; ++h) {
           const float4 f = lds4(smem_u32(&s_col[set][0][h]));
           acc[4 * h] *= f.x; acc[4 * h + 1] *= f.y; acc[4 * h + 2] *= f.z; acc[4 * h + 3] *= f.w;
-          wide |= f.x != f.x || f.y != f.y || f.z != f.z || f.w != f.w;
         }
-        if (wide) exact_fp32<HW>(p, n, ty + prow, tx + pcol, valid, co, acc);
+        const unsigned odd = s_odd[set];
+        if (__builtin_expect(valid && (small || wide || odd), 0)) {
+          float sums[HW];
+#pragma unroll
+          for (int i = 0; i < HW; ++i) sums[i] = small ? acc[i] + lost[i] : acc[i];
+          if (wide || odd) exact_fp32<HW>(p, n, ty + prow, tx + pcol, co, wide ? ~0u : odd, sums);
+#pragma unroll
+          for (int i = 0; i < HW; ++i) acc[i] = sums[i];
+        }
         sent = valid;
         if constexpr (!STEP) {
 #pragma unroll
@@ -507,14 +659,16 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
       } else {
         ok = __all_sync(0xffffffffu, mbar_wait(&item_full[set], item_idx & 1u, &s_abort, p.spin_limit));
         float inv[2];
+        bool noted = false;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const unsigned u = unit + (n_seg == 2u ? (unsigned)(j * units) >> 1 : 0u);
           ok = __all_sync(0xffffffffu, ok && mbar_wait(&s_split.inv_full[u % SPLIT_RING], (u / SPLIT_RING) & 1u, &s_abort, p.spin_limit));
-          inv[j] = s_split.inv[u % SPLIT_RING];
+          const float scale = s_split.inv[u % SPLIT_RING];
+          noted |= !(scale > 0.0f);
+          inv[j] = fabsf(scale);
         }
-        unit += 2u * (unsigned)units;
-        if (at_col < 2 * HW) reinterpret_cast<float *>(s_col[set][at_col / HW])[at_col % HW] = col;
+        keep_column(at_col, col);
         // a warp whose wait gave up goes on to the barrier of its set, where the four of them leave together
         if (!STEP && chief) {      // the buffer is free once the stores of its last item have read it
           if (p.slab_sets == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -530,12 +684,22 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
         if (!ok) break;
         tc_fence_after();
         const ExactRow r = {res_row, out_row, em_row, (unsigned)sw};
-        const bool wide = inv[0] != inv[0] || inv[1] != inv[1];
         const unsigned c = lane_base + seg * exact_cols(CB, FULL);
-        if (p.act == MIE_ACT_RELU) sent = exact_finish<HW, STEP, FULL, MIE_ACT_RELU>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
-        else if (p.act == MIE_ACT_NONE) sent = exact_finish<HW, STEP, FULL, MIE_ACT_NONE>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
-        else sent = exact_finish<HW, STEP, FULL, MIE_ACT_SIGMOID>(p, c, n_seg, inv[0], inv[1], wide, r, s_col[set][0], n, ty + prow, tx + pcol, valid, pix, co);
+        const float4 *scales = s_col[set][0];
+        unsigned scale_step = 1u;
+        const unsigned odd = s_odd[set];
+        if (__builtin_expect(noted || odd, 0)) {
+          if (exact_rare_item<HW, FULL>(p, s_split, c, n_seg, unit, units, odd, t, co)) {
+            inv[0] = inv[1] = 1.0f;
+            scales = &s_one; scale_step = 0u;
+          }
+        }
+        const float4 *own = s_col[set][0];
+        if (p.act == MIE_ACT_RELU) sent = exact_finish<HW, STEP, FULL, MIE_ACT_RELU>(p, c, n_seg, inv[0], inv[1], scales, scale_step, r, own, valid, pix, co);
+        else if (p.act == MIE_ACT_NONE) sent = exact_finish<HW, STEP, FULL, MIE_ACT_NONE>(p, c, n_seg, inv[0], inv[1], scales, scale_step, r, own, valid, pix, co);
+        else sent = exact_finish<HW, STEP, FULL, MIE_ACT_SIGMOID>(p, c, n_seg, inv[0], inv[1], scales, scale_step, r, own, valid, pix, co);
         sent = sent && valid;
+        unit += 2u * (unsigned)units;
         tc_fence_before();
         __syncwarp();
         for (unsigned j = 0; j < n_seg; ++j)
@@ -764,9 +928,11 @@ __global__ void __launch_bounds__(256) pad_field_kernel(const float *__restrict_
 }
 
 // [tap][chunk][hi: cout_pad rows | lo: cout_pad rows][32 FP16] <- w[cout][cin][ky][kx] (ihwo: stored [cin][ky][kx][cout]), zero padded, then
-// cout_pad inverse scales.  A channel's scale puts its largest entry into [2^14, 2^15).  NaN for a channel whose entries two FP16 numbers
+// cout_pad inverse scales.  A channel's scale puts its largest entry into [2^15, 2^16).  NaN for a channel whose entries two FP16 numbers
 // cannot hold: infinities, NaN, or entries above 2^10 (2^100 in any case) beside entries 2^-36 of them; its outputs are computed
-// with FP32 instructions.  (Below 2^10 what falls off is at most 2^-40 of an input.)  A block per NC channels, which it reads twice, the second time from the caches.
+// with FP32 instructions.  Of the others an entry below 2^-27 of the largest is held to 2^-52 of that, which is 2^-42 of an input at most.
+// (Such entries taken out, as the input's values are, cost 64 -> 64 3x3 at 264x352 67 us for 37 with one of them, and 440 with one input
+// channel of them, which a trained network may well have.)  A block per NC channels, which it reads twice, the second time from the caches.
 template <int NC>
 __global__ void __launch_bounds__(512) pack_weights_exact_kernel(const float *__restrict__ w, int cout, int cin, int k, int nch, int cout_pad, float *__restrict__ wp,
                                                                  int64_t scales_at, int ihwo) {
@@ -791,12 +957,12 @@ __global__ void __launch_bounds__(512) pack_weights_exact_kernel(const float *__
   __syncthreads();
   __half *out = reinterpret_cast<__half *>(wp);
   for (int cc = ihwo ? c : 0; cc < (ihwo ? c + 1 : NC); ++cc) {
-    const unsigned m = s_max[cc], e = min(max(m >> 23, 15u), 254u);
-    const float scale = __uint_as_float((268u - e) << 23);
+    const unsigned m = s_max[cc], e = split_exponent(m);
+    const float scale = split_scale(e);
     const int co = co0 + cc;
     if (first == 0 && co < cout_pad) {
       const bool wide = m > 0x71800000u || (m > 0x44800000u && (m >> 23) - (s_min[cc] >> 23) > 36u);
-      wp[scales_at + co] = wide ? __uint_as_float(0x7FC00000u) : __uint_as_float((e - 14u) << 23);
+      wp[scales_at + co] = wide ? __uint_as_float(0x7FC00000u) : split_inverse(e);
     }
     for (int i = first; i < nch * 32 * kk; i += step) {
       const int ci = i / kk, tap = i - ci * kk;

@@ -98,7 +98,7 @@ __device__ __forceinline__ bool pair_group(const TcParams &p, const float *v, un
     flag |= fabsf(o[i].x) > thr || fabsf(o[i].y) > thr || fabsf(o[i].z) > thr || fabsf(o[i].w) > thr;
   }
   // Of a quad past the last channel the slabs hold zeros, and f(0) - 0 is not zero for a sigmoid that is measured against the carry.
-  if (THR && nq - h0 < 4) {
+  if (THR && __builtin_expect(nq - h0 < 4, 0)) {
     flag = false;
 #pragma unroll
     for (int i = 0; i < 3; ++i) flag |= h0 + i < nq && (fabsf(o[i].x) > p.thr || fabsf(o[i].y) > p.thr || fabsf(o[i].z) > p.thr || fabsf(o[i].w) > p.thr);

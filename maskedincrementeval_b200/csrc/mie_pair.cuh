@@ -271,9 +271,14 @@ __device__ __forceinline__ void sts4(unsigned addr, float4 v) {
 // fp32 operands as two FP16 numbers each.  An operand v, scaled by a power of two s, is hi = fp16(s v) and lo = fp16(2^11 (s v - hi)),
 // rounded to nearest: together they hold v to 2^-24, as two TF32 numbers do, but an instruction takes 16 of them where it takes 8
 // TF32 numbers.  (A scaled FP16 split: Ootomo and Yokota, 2022.)  The input's scale is chosen for every halo in
-// shared memory, so that its largest value lies in [2^14, 2^15): a value keeps its 24 bits down to 2^-28 of that, and an absolute
-// step of 2^-49 of it below.  Halos for which that would not do -- an infinity, a NaN, values above 2^100, or above 2^14 beside
-// values 2^-36 of it -- are marked (inverse scale NaN), and the epilogue computes their pixels with FP32 instructions.
+// shared memory, so that its largest value lies in [2^15, 2^16) and does not round up to 2^16: a value is held to 2^-52 of that, which is 24
+// bits down to 2^-27 of it and 22 at 2^-29.  A few values smaller than that but zero, in whatever unit, are taken out of the halo and
+// listed, the halo's inverse scale gets a negative sign, and the epilogue multiplies them with FP32 instructions.  (Of normal values one halo
+// in 8000 has one, in the dense pass and in steps alike.  The line lies where FireFlowNet's step is not slower for it: from 2^-27 on, with
+// two such items a step, 336 us, from 2^-30 on 311, without 309; most of it is the fetching of instructions that are not at hand.)  Many such
+// values stay in the parts, down to 16 bits; a halo in which that is not enough, because values 2^-36 of the largest are among them, is marked
+// with a NaN, as are halos with an infinity, a NaN or values above 2^100, and the epilogue computes their pixels with FP32 instructions.  (To
+// compute all halos with many small values so, as a network with closed gates makes them, takes a hundred times as long as the layer.)
 // ---------------------------------------------------------------------------------------------------------------
 constexpr unsigned SPLIT_RING = 16;      // inverse scales kept: more than halo buffers and segment accumulators in flight
 constexpr float SPLIT_LO = 1.0f / 2048.0f;
@@ -304,14 +309,33 @@ __device__ __forceinline__ unsigned long long make_smem_desc_64(unsigned smem_ad
          (unsigned long long)1 << 46 | (unsigned long long)4 << 61;
 }
 
+// The exponent field that a largest magnitude (its bits) is scaled by; the scale and its inverse.
+__device__ __forceinline__ unsigned split_exponent(unsigned m) { return min(max((m + 0x1000u) >> 23, 16u), 254u); }
+__device__ __forceinline__ float split_scale(unsigned e) { return __uint_as_float((269u - e) << 23); }
+__device__ __forceinline__ float split_inverse(unsigned e) { return __uint_as_float((e - 15u) << 23); }
+
+// Two fp32 operations in an instruction.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
 __device__ __forceinline__ void split_fp16(const float *v, float scale, float4 &hi, float4 &lo) {      // eight channels
   unsigned h[4], l[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float a = v[2 * j] * scale, b = v[2 * j + 1] * scale;
-    const __half2 t = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(t);
-    const __half2 u = __floats2half2_rn((a - f.x) * 2048.0f, (b - f.y) * 2048.0f);
+    const float2 x = make_float2(v[2 * j], v[2 * j + 1]), a = mul2(x, make_float2(scale, scale));
+    const __half2 t = __float22half2_rn(a);
+    // (the scaling, by powers of two, and the differences are exact)
+    const float2 f = __half22float2(__hneg2(t)), r = mul2(fma2(x, make_float2(scale, scale), f), make_float2(2048.0f, 2048.0f));
+    const __half2 u = __float22half2_rn(r);
     h[j] = *reinterpret_cast<const unsigned *>(&t);
     l[j] = *reinterpret_cast<const unsigned *>(&u);
   }
@@ -324,15 +348,26 @@ __device__ __forceinline__ void split_fp16(const float *v, float scale, float4 &
 // takes eight channels: it reads pieces 2 c and 2 c + 1 of a row and writes pieces c and 4 + c; the eight rows of a warp are dealt such that
 // neighbouring lanes hold rows whose swizzles differ in bits 0 and 2, so that neither reads nor writes meet in a bank.
 // What it costs: one read and one write of the halo through shared memory (400 clocks of its port for a 3x3 layer's 25 KB), and a
-// chain of about 2200 clocks a unit (read 600, largest value of all warps 400, split and write 1100), beside the instructions of
-// the unit before.
+// chain of about 2200 clocks a unit (read 600, largest and smallest value of all warps 400, split and write 1100), beside the
+// instructions of the unit before.
 constexpr int SPLIT_WARPS = 8, SPLIT_PASS = 8 * SPLIT_WARPS;      // rows of a pass
 constexpr int SPLIT_REGS = 288 / SPLIT_PASS + (288 % SPLIT_PASS != 0);      // passes held in registers: halos up to 12 x 12; larger ones (7x7) read the rest twice
-struct SplitShared {
+constexpr int SPLIT_BELOW = 29;      // binades below the largest value from which values are taken out, if they are few
+constexpr int SPLIT_APART = 36;      // ... from which a halo with many such values is not split
+constexpr int SPLIT_LISTED = 4;
+struct SplitSmall {                          // values taken out, and where they stood: tile << 13 | halo row << 9 | halo column << 5 | channel
+  float value[SPLIT_LISTED];
+  unsigned short at[SPLIT_LISTED];           // (SPLIT_NONE behind the last one)
+};
+constexpr unsigned SPLIT_NONE = 0xFFFFu;
+struct __align__(16) SplitShared {
+  SplitSmall small[SPLIT_RING];              // of the units whose inverse scale is negative
   float red[2][SPLIT_WARPS];
-  unsigned least[SPLIT_WARPS];
-  float inv[SPLIT_RING];                       // inverse scale of a unit's halo (NaN: marked) ...
+  unsigned short least[2][SPLIT_WARPS];
+  float inv[SPLIT_RING];                       // inverse scale of a unit's halo (negative: values were taken out; NaN: not split) ...
   unsigned long long inv_full[SPLIT_RING];     // ... and that it is there
+  // the splitting warps' order to the one that takes values out: the halo, its exponent field | ring unit << 8 | tiles << 12 (~0: it may go)
+  unsigned take_base, take;
 };
 __device__ __forceinline__ float max3_abs(float a, float b, float c) {      // of magnitudes; a NaN stays
   float d;
@@ -350,23 +385,58 @@ __device__ __forceinline__ void sts4_if(unsigned addr, float4 v, bool on) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n\t}"
                ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"((unsigned)on) : "memory");
 }
-// The smallest magnitude but zero of the rows in `live` that start at r0 and r1.
-__device__ __noinline__ unsigned split_least(unsigned r0, unsigned r1, unsigned live) {
-  unsigned least = 0x7FFFFFFFu;
-  for (int it = 0; live >> it; ++it) {
-    if (!(live >> it & 1u)) continue;
-    const float4 a = lds4(r0 + (unsigned)(it * SPLIT_PASS * 128)), b = lds4(r1 + (unsigned)(it * SPLIT_PASS * 128));
-    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { const unsigned u = __float_as_uint(x[j]) & 0x7FFFFFFFu; if (u) least = min(least, u); }
-  }
-  return least;
+// How many threads of the splitting warps bring `yes`.
+__device__ __forceinline__ unsigned set_count(bool yes) {
+  unsigned r;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.popc.u32 %0, 3, %2, p;\n\t}" : "=r"(r) : "r"((unsigned)yes), "n"(32 * SPLIT_WARPS) : "memory");
+  return r;
 }
-__device__ __forceinline__ void pair_split_halos(const PairWork &w, const PairRing &r, unsigned long long *ready, int rows, int wp, int n_active, int t,
+// The splitting warps and the one that takes values out: an order is there, or carried out.
+__device__ __forceinline__ void split_meet() { asm volatile("bar.sync 4, %0;" ::"n"(32 * SPLIT_WARPS + 32) : "memory"); }
+// The warp that takes out of a halo the values below 2^-SPLIT_BELOW of its largest, but zero: lists them in ascending order and sets them to
+// zero.  A warp of its own: as a branch of the splitting warps it cost FireFlowNet's step 3 % without being run (registers, and the
+// instructions in between).
+__device__ __forceinline__ void pair_take_out(SplitShared &sh, int rows, int wp, int lane) {
+  for (;;) {
+    split_meet();
+    const unsigned order = sh.take, base = sh.take_base;
+    if (order == ~0u) return;
+    const int tiles = (int)(order >> 12);
+    const float thr = __uint_as_float(((order & 255u) - SPLIT_BELOW) << 23);
+    SplitSmall &list = sh.small[order >> 8 & 15u];
+    const int piece = lane & 7;
+    unsigned n = 0u;
+#pragma unroll 1
+    for (int r0 = 0; r0 < rows; r0 += 4) {
+      const int row = r0 + (lane >> 3), line = row / wp;
+      const bool live = row < rows && (line & 1) < tiles;
+      const unsigned at = base + (unsigned)row * 128u + (unsigned)((piece ^ (row & 7)) << 4);
+      const float4 v = lds4_if(at, live);
+      float x[4] = {v.x, v.y, v.z, v.w};
+      bool here = false;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool out = x[j] != 0.0f && fabsf(x[j]) < thr;
+        const unsigned all = __ballot_sync(0xffffffffu, out), i = n + __popc(all & ((1u << lane) - 1u));
+        if (out && i < (unsigned)SPLIT_LISTED) {
+          list.value[i] = x[j];
+          list.at[i] = (unsigned short)((line & 1) << 13 | (line >> 1) << 9 | (row - line * wp) << 5 | (4 * piece + j));
+        }
+        if (out) x[j] = 0.0f;
+        here |= out;
+        n += __popc(all);
+      }
+      sts4_if(at, make_float4(x[0], x[1], x[2], x[3]), here);
+    }
+    if (lane == 0 && n < (unsigned)SPLIT_LISTED) list.at[n] = (unsigned short)SPLIT_NONE;
+    split_meet();
+  }
+}
+template <int REGS>
+__device__ __forceinline__ void pair_split_halos_in(const PairWork &w, const PairRing &r, unsigned long long *ready, int rows, int wp, int n_active, int t,
                                                  SplitShared &sh, volatile int *abort_flag) {
-  const int lane = t & 31, cw = t >> 5, c = lane & 3;
-  const int row0 = cw * 8 + (int)((0x63724150u >> (4 * (lane >> 2))) & 7u);
-  const int sw = row0 & 7, passes = (rows + SPLIT_PASS - 1) / SPLIT_PASS;
+  const int lane = t & 31, cw = t >> 5, passes = (rows + SPLIT_PASS - 1) / SPLIT_PASS;
+  const int c = lane & 3, row0 = cw * 8 + (int)((0x63724150u >> (4 * (lane >> 2))) & 7u), sw = row0 & 7;
   const unsigned at = (unsigned)row0 * 128u, rd0 = at + (unsigned)((2 * c) ^ sw) * 16u, rd1 = at + (unsigned)((2 * c + 1) ^ sw) * 16u,
                  wr0 = at + (unsigned)(c ^ sw) * 16u, wr1 = at + (unsigned)((4 + c) ^ sw) * 16u;
   // which of the thread's rows hold input: of two tiles, or of the first alone (what lies in an absent tile's rows is none)
@@ -385,38 +455,66 @@ __device__ __forceinline__ void pair_split_halos(const PairWork &w, const PairRi
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
       };
       auto largest = [](const float *v, float m) { return max3_abs(max3_abs(max3_abs(max3_abs(m, v[0], v[1]), v[2], v[3]), v[4], v[5]), v[6], v[7]); };
-      float v[SPLIT_REGS][8], m = 0.0f;
+      // twice the smallest magnitude's bits less one: a zero is the largest number there is
+      auto smallest = [](const float *v, unsigned m) {
+        unsigned k[8];
 #pragma unroll
-      for (int it = 0; it < SPLIT_REGS; ++it) read(it, v[it]);
+        for (int j = 0; j < 8; ++j) k[j] = 2u * __float_as_uint(v[j]) - 1u;
+        return __vimin3_u32(__vimin3_u32(__vimin3_u32(__vimin3_u32(m, k[0], k[1]), k[2], k[3]), k[4], k[5]), k[6], k[7]);
+      };
+      float v[REGS][8], m = 0.0f;
+      unsigned least = 0xFFFFFFFFu;
 #pragma unroll
-      for (int it = 0; it < SPLIT_REGS; ++it) m = largest(v[it], m);
+      for (int it = 0; it < REGS; ++it) read(it, v[it]);
+#pragma unroll
+      for (int it = 0; it < REGS; ++it) { m = largest(v[it], m); least = smallest(v[it], least); }
 #pragma unroll 1
-      for (int it = SPLIT_REGS; it < passes; ++it) {
+      for (int it = REGS; it < passes; ++it) {
         float x[8];
         read(it, x);
         m = largest(x, m);
+        least = smallest(x, least);
       }
       m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));      // (of non-negative floats, NaN above all)
-      if (lane == 0) sh.red[unit & 1u][cw] = m;
+      least = __reduce_min_sync(0xffffffffu, least);
+      if (lane == 0) { sh.red[unit & 1u][cw] = m; sh.least[unit & 1u][cw] = (unsigned short)(least >> 16); }
       if (!set_all<32 * SPLIT_WARPS>(3, ok)) return;
       m = 0.0f;
 #pragma unroll
       for (int i = 0; i < SPLIT_WARPS; i += 2) m = max3_abs(m, sh.red[unit & 1u][i], sh.red[unit & 1u][i + 1]);
+      const uint4 l = *reinterpret_cast<const uint4 *>(sh.least[unit & 1u]);      // (a power of two counts as the binade below, which does no harm)
+      const unsigned l2 = __vminu2(__vminu2(l.x, l.y), __vminu2(l.z, l.w));
+      least = min(l2 & 0xFFFFu, l2 >> 16) >> 8;
       const unsigned mb = __float_as_uint(m);
-      bool wide = false;
-      if (mb >= 0x46800000u) {      // 2^14 or more: is it too much for what lies beside it?
-        unsigned least = split_least(base + rd0, base + rd1, live);
-        least = __reduce_min_sync(0xffffffffu, least);
-        if (lane == 0) sh.least[cw] = least;
-        set_all<32 * SPLIT_WARPS>(3, true);
+      const unsigned e = split_exponent(mb);
+      const float scale = split_scale(e);
+      float inv = split_inverse(e);
+      if (mb > 0x71800000u) {
+        inv = __uint_as_float(0x7FC00000u);
+      } else if (__builtin_expect(mb && e > SPLIT_BELOW && least < e - SPLIT_BELOW, 0)) {
+        // few enough for the list?
+        const float thr = __uint_as_float((e - SPLIT_BELOW) << 23);
+        unsigned few = 0u;
+#pragma unroll 1
+        for (int it = 0; it < passes; ++it) {
+          float x[8];
+          read(it, x);
 #pragma unroll
-        for (int i = 0; i < SPLIT_WARPS; ++i) least = min(least, sh.least[i]);
-        wide = mb > 0x71800000u || (mb >> 23) - (least >> 23) > 36u;
+          for (int j = 0; j < 8; ++j) few += x[j] != 0.0f && fabsf(x[j]) < thr;
+        }
+        if (set_count(few >= 1u) + set_count(few >= 2u) <= (unsigned)SPLIT_LISTED && !set_count(few >= 3u)) {
+          if (t == 0) { sh.take_base = base; sh.take = e | (unit % SPLIT_RING) << 8 | (unsigned)tiles << 12; }
+          split_meet();
+          split_meet();
+          inv = -inv;
+        } else if (e - least > SPLIT_APART) {
+          inv = __uint_as_float(0x7FC00000u);
+        }
+#pragma unroll
+        for (int it = 0; it < REGS; ++it) read(it, v[it]);
       }
-      const unsigned e = min(max(mb >> 23, 15u), 254u);
-      const float scale = __uint_as_float((268u - e) << 23);
       if (t == 0) {
-        sh.inv[unit % SPLIT_RING] = wide ? __uint_as_float(0x7FC00000u) : __uint_as_float((e - 14u) << 23);
+        sh.inv[unit % SPLIT_RING] = inv;
         mbar_arrive(&sh.inv_full[unit % SPLIT_RING]);
       }
       auto write = [&](int it, const float *x) {
@@ -426,9 +524,9 @@ __device__ __forceinline__ void pair_split_halos(const PairWork &w, const PairRi
         sts4_if(base + wr1 + (unsigned)(it * SPLIT_PASS * 128), lo, live >> it & 1u);
       };
 #pragma unroll
-      for (int it = 0; it < SPLIT_REGS; ++it) write(it, v[it]);
+      for (int it = 0; it < REGS; ++it) write(it, v[it]);
 #pragma unroll 1
-      for (int it = SPLIT_REGS; it < passes; ++it) {
+      for (int it = REGS; it < passes; ++it) {
         float x[8];
         read(it, x);
         __syncwarp();      // in place: the lanes of a row read before one of them writes
@@ -442,6 +540,15 @@ __device__ __forceinline__ void pair_split_halos(const PairWork &w, const PairRi
       if (++s == r.count) { s = 0; parity ^= 1u; }
     }
   }
+}
+// By the passes that the halo takes: one that reads no row costs as many instructions as one that does (3x3: a fifth).
+__device__ __forceinline__ void pair_split_halos(const PairWork &w, const PairRing &r, unsigned long long *ready, int rows, int wp, int n_active, int t,
+                                                 SplitShared &sh, volatile int *abort_flag) {
+  if (rows <= 3 * SPLIT_PASS) pair_split_halos_in<3>(w, r, ready, rows, wp, n_active, t, sh, abort_flag);
+  else if (rows <= 4 * SPLIT_PASS) pair_split_halos_in<4>(w, r, ready, rows, wp, n_active, t, sh, abort_flag);
+  else pair_split_halos_in<SPLIT_REGS>(w, r, ready, rows, wp, n_active, t, sh, abort_flag);
+  if (t == 0) sh.take = ~0u;      // (the splitting warps leave together, also where a wait gave up)
+  split_meet();
 }
 
 }  // namespace

@@ -151,20 +151,27 @@ def test_dense_pass_on_non_finite_values(dev, case, where):
         assert float(((got[big] - want[big]) / want[big]).abs().max()) <= 1e-5 if bool(big.any()) else True
 
 
-# Values that lie far apart in one halo: what two FP16 numbers with a common scale hold is computed on the tensor cores, the rest with FP32
-# instructions.  Every output against the sum of its products' magnitudes: fp32 sums of cin * k * k terms, or (below 2^17) a step
-# of 2^-49 of the largest value times the filter's entries (below 0.05).  (At 40000 some halos lie below 2^14.)
-@pytest.mark.parametrize("case", [(48, 32, 3, 1, 24, 40), (64, 64, 7, 1, 17, 23), (5, 32, 5, 2, 33, 40), (16, 36, 3, 1, 41, 50)])
-@pytest.mark.parametrize("big,small", [(1.0, 1e-3), (1e-30, 1e-33), (16383.0, 1e-6), (40000.0, 1e-6), (1e6, 1e-9), (1e20, 1.0), (1e31, 1e30), (1e36, 0.2)])
-def test_dense_pass_on_values_far_apart(dev, case, big, small):
+# Many values that lie far apart in one halo, in any unit: what two FP16 numbers with a common scale hold is computed on the tensor cores, the
+# rest with FP32 instructions.  Every output against the sum of its products' magnitudes: fp32 sums of cin * k * k terms, and (where no more
+# than 2^38 lies between them) a step of 2^-52 of the largest value times the filter's entries.
+FAR_APART = [(1.0, 1e-3), (1.0, 1e-8), (1.0, 1e-12), (1e-30, 1e-33), (1e-12, 1e-22), (16383.0, 1e-6), (1e4, 1e-6), (40000.0, 1e-6), (1e6, 1e-9), (1e20, 1.0),
+             (1e31, 1e30), (1e36, 0.2)]
+
+
+@pytest.mark.parametrize("case", [(48, 32, 3, 1, 24, 40), (64, 64, 7, 1, 17, 23), (5, 32, 5, 2, 33, 40), (16, 36, 3, 1, 41, 50), (40, 64, 5, 2, 35, 41)])
+@pytest.mark.parametrize("big,small", FAR_APART)
+@pytest.mark.parametrize("unit", [0.05, 1e6])
+def test_dense_pass_on_values_far_apart(dev, case, big, small, unit):
     from maskedincrementeval_b200.incr_modules._algebra import NATIVE
     from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
     cin, cout, k, s, h, w = case
+    if big * unit * cin * k * k > 1e37:
+        return      # beyond fp32
     torch.manual_seed(12)
     layer = ConvLayerIncr(cin, cout, k, s, k // 2, activation="relu").to(dev).eval()
     c = layer.conv2d
     with torch.no_grad():
-        c.weight.mul_(0.05 / c.weight.abs().max())
+        c.weight.mul_(unit / c.weight.abs().max())
         c.bias.zero_()
     x = cl(torch.randn(1, cin, h, w, device=dev).clamp_(-3, 3) * (small / 3))
     x[0, :, 3::11, 5::13] *= big / small
@@ -173,30 +180,81 @@ def test_dense_pass_on_values_far_apart(dev, case, big, small):
     with torch.no_grad():
         NATIVE.conv(c, NATIVE.lift(x), layer.activation)
     got = layer.activation.in_res.reservoir.double()
-    step = big * 2.0 ** -49 * 0.05 * cin * k * k if big < 2 ** 17 else 0.0
+    step = big * 2.0 ** -52 * unit * cin * k * k if big / small < 2.0 ** 38 else 0.0
     assert bool(got.isfinite().all())
     assert float(((got - want).abs() - 2e-6 * size).max()) <= step
 
 
-# the same for a filter whose entries lie far apart, and for one of tiny entries
-@pytest.mark.parametrize("big,small", [(1e6, 1e-6), (1e30, 1e-3), (1e-20, 1e-22), (900.0, 1e-3)])
-def test_dense_pass_on_filters_far_apart(dev, big, small):
+# A few small values beside large ones, in the dense pass and in steps, blocks and items of every form: as exact as any others (2e-6 as above), in
+# any unit.  (A large pixel and a small value per 12 x 12 pixels: no halo has more small ones than are listed.)
+@pytest.mark.parametrize("cin,cout,k,s", [(48, 32, 3, 1), (32, 32, 3, 1), (16, 24, 3, 1), (64, 64, 3, 1), (64, 64, 5, 1), (40, 64, 5, 2), (96, 36, 3, 2), (132, 64, 3, 1)])
+@pytest.mark.parametrize("big,small", [(1.0, 1e-9), (1.0, 1e-14), (1e-5, 1e-30), (16383.0, 1e-9), (1e6, 1e-3)])
+@pytest.mark.parametrize("step", [False, True])
+def test_a_few_small_values(dev, cin, cout, k, s, big, small, step):
+    from maskedincrementeval_b200 import _native as nat
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    torch.manual_seed(29)
+    h, w = 61, 90
+    layer = ConvLayerIncr(cin, cout, k, s, k // 2, activation=None if step else "relu").to(dev).eval()
+    c = layer.conv2d
+    c.precision = "split"
+    c.bias.data.zero_()
+    x = torch.zeros(1, cin, h, w, device=dev)
+    x[0, :, 3::12, 4::12] = big * torch.randn(1, 1, 1, device=dev) + big * torch.rand(cin, 5, 8, device=dev)
+    rows, cols = torch.arange(9, h, 12, device=dev), torch.arange(10, w, 12, device=dev)
+    for i, r in enumerate(rows):
+        for j, q in enumerate(cols):
+            x[0, (7 * i + 5 * j) % cin, r, q] = small * (1 + i) * (-1) ** j
+    x = cl(x)
+    want = F.conv2d(x.double(), c.weight.detach().double(), stride=s, padding=k // 2)
+    size = F.conv2d(x.double().abs(), c.weight.detach().double().abs(), stride=s, padding=k // 2)
+    for _ in range(2):      # (the order in which they are found must not matter)
+        with torch.no_grad():
+            if step:
+                y, m = layer([x, None])
+                assert nat.lib.mie_conv_is_exact(C.byref(c._plan(1, h, w, dev).args)) or cin * k * k < 256
+            else:
+                NATIVE.conv(c, NATIVE.lift(x), layer.activation)
+                y = layer.activation.in_res.reservoir
+        got = y.clone()
+        assert _ == 0 or torch.equal(got, first)
+        first = got
+        assert float(((got.double() - want).abs() - 2e-6 * size).max()) <= 0.0
+
+
+# the same for a filter whose entries lie far apart, and for one of tiny entries.  (At isolated pixels an output may be a sum of small
+# entries alone, which the parts hold to 2^-52 of the channel's largest entry where that lies below 2^10.)
+@pytest.mark.parametrize("big,small", [(1e6, 1e-6), (1e30, 1e-3), (1e-20, 1e-22), (900.0, 1e-3), (1.0, 1e-9), (1e-3, 1e-20)])
+@pytest.mark.parametrize("cin,cout,k,s", [(48, 64, 3, 1), (32, 32, 3, 1), (10, 36, 5, 2)])
+@pytest.mark.parametrize("isolated", [False, True])
+def test_dense_pass_on_filters_far_apart(dev, big, small, cin, cout, k, s, isolated):
+    from maskedincrementeval_b200.ext.pointops import pointops_functional as pf
     from maskedincrementeval_b200.incr_modules._algebra import NATIVE
     from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
     torch.manual_seed(13)
-    layer = ConvLayerIncr(48, 64, 3, 1, 1, activation="relu").to(dev).eval()
+    layer = ConvLayerIncr(cin, cout, k, s, k // 2, activation="relu").to(dev).eval()
     c = layer.conv2d
     with torch.no_grad():
         c.weight.normal_().clamp_(-3, 3).mul_(small / 3)
         c.weight[::5, :, 0, 0] *= big / small
         c.bias.zero_()
-    x = cl(torch.randn(1, 48, 21, 30, device=dev))
-    want = F.conv2d(x.double(), c.weight.detach().double(), padding=1)
-    size = F.conv2d(x.double().abs(), c.weight.detach().double().abs(), padding=1)
+    x = torch.randn(1, cin, 21, 30, device=dev)
+    if isolated:
+        on = torch.zeros(1, 1, 21, 30, device=dev)
+        on[:, :, 2::k, 1::k] = 1.0
+        x = x * on * (torch.rand(1, cin, 21, 30, device=dev) < 0.2)
+    x = cl(x)
+    want = F.conv2d(x.double(), c.weight.detach().double(), stride=s, padding=k // 2)
+    size = F.conv2d(x.double().abs(), c.weight.detach().double().abs(), stride=s, padding=k // 2)
+    step = F.conv2d(x.double().abs(), torch.full_like(c.weight, big * 2.0 ** -52 if big < 2 ** 10 else 0.0).double(), stride=s, padding=k // 2)
     with torch.no_grad():
         NATIVE.conv(c, NATIVE.lift(x), layer.activation)
-    got = layer.activation.in_res.reservoir.double()
-    assert float(((got - want).abs() / size).max()) <= 2e-6
+        got = [layer.activation.in_res.reservoir.double()]
+        if cin >= 48:
+            got.append(pf.functional_conv_module(x, c.conv2d_weights, mask=None, stride=(s, s), padding=(k // 2, k // 2))[0].double())
+    for y in got:
+        assert float(((y - want).abs() - 2e-6 * size - step).max()) <= 0.0
 
 
 def test_extension_on_a_silent_step(dev):
@@ -424,7 +482,7 @@ def test_dilation_of_fields_around_the_large_kernels_limit(dev, n, h, w):
 # Deltas that FP16 parts cannot hold, in steps: two items in hand (16 and 32 channels), one (64 -> 32), blocks of 64.  Against the FP32 kernel:
 # the same infinities and NaN, and the same state elsewhere up to fp32 sums of cin * 9 products
 @pytest.mark.parametrize("cin,cout", [(16, 36), (32, 32), (96, 32), (64, 64)])
-@pytest.mark.parametrize("odd", [float("inf"), float("nan"), 3e30, 1e5])
+@pytest.mark.parametrize("odd", [float("inf"), float("nan"), 3e30, 1e5, 1.0])
 def test_steps_on_values_far_apart(dev, cin, cout, odd):
     from maskedincrementeval_b200 import fields as fl, _native as nat
     from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
@@ -439,18 +497,21 @@ def test_steps_on_values_far_apart(dev, cin, cout, odd):
             g = torch.Generator(device=dev).manual_seed(18)
             with torch.no_grad():
                 layer.forward_refresh_reservoirs(cl(torch.randn(1, cin, 41, 50, generator=g, device=dev)))
-                d = torch.randn(1, cin, 41, 50, generator=g, device=dev) * (1e-6 if odd == 1e5 else 0.2)
+                d = torch.randn(1, cin, 41, 50, generator=g, device=dev) * {1e5: 1e-6, 1.0: 1e-11}.get(odd, 0.2)
                 d[0, 3, 7::13, 5::17] = odd
-                layer([cl(d), None])
+                dy, m = layer([cl(d), None])
                 assert mode == "off" or nat.lib.mie_conv_is_exact(C.byref(layer.conv2d._plan(1, 41, 50, dev).args))
-            out[mode] = layer.activation.in_res.reservoir.clone()
+            out[mode] = layer.activation.in_res.reservoir.clone(), dy.clone(), m.pixel_mask().clone()
     finally:
         fl.config.tensor_cores = old
-    got, want = out["auto"], out["off"]
-    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
-    fine = want.isfinite()
-    assert bool(fine.any())
-    assert float(((got - want).abs()[fine] / want.abs()[fine].clamp(min=1.0)).max()) <= 1e-5
+    for got, want in zip(out["auto"][:2], out["off"][:2]):
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+        fine = want.isfinite()
+        assert bool(fine.any())
+        assert float(((got - want).abs()[fine] / want.abs()[fine].clamp(min=1.0)).max()) <= 1e-5
+    # a pixel is marked where a finite change is not 0 (a NaN is above no threshold): few changes lie so close to 0 that the kernels differ
+    (_, dy, m), (_, _, wm) = out["auto"], out["off"]
+    assert torch.equal(m, ((dy != 0) & ~dy.isnan()).any(1, keepdim=True).to(torch.uint8)) and float((m != wm).float().mean()) <= 1e-2
 
 
 # A thresholded sigmoid on the TF32 kernel with partial groups of 16 channels and blocks that end in a group of none: what is sent, against

@@ -20,11 +20,14 @@ import torch
 from . import _native as nat
 from . import fields as fl
 from .fields import TileMask
+from .incr_modules._algebra import NATIVE, dense_ops
 from .incr_modules.mask_incr_functional import IncrementReserve
 
 
 # Modules whose dense pass is known, and the methods that make it up: one set on an object may do anything.
 _PLAIN_MODULES = (__package__ + ".", "torch.nn.")
+_MODULE_ATTRIBUTES = len(torch.nn.Module().__dict__)      # what a module's dictionary begins with, and no pass depends on
+_HOLDERS = frozenset((torch.Tensor, fl.Scratch, IncrementReserve))
 _PASS_METHODS = ("forward_refresh_reservoirs", "refresh_native", "forward_fused", "_run", "forward")
 
 
@@ -167,7 +170,6 @@ class IncrementalRunner:
     def _may_record_pass(self, x) -> bool:
         # Only networks that say of themselves that their pass is launches of the library's kernels alone (``PASS_IS_KERNELS``), and
         # only where it is: PyTorch's dense operators follow switches, and a subclass may do what a replay would not do again.
-        from .incr_modules._algebra import NATIVE, dense_ops
         c, net = fl.config, self.model
         return (self.use_graph and not self.feedback and self._x_prev is not None and x.is_cuda and x.dtype == torch.float32
                 and x.shape == self._x_prev.shape and c.refresh == "native" and not c.tail_dilation and not c.kfenced_step
@@ -179,26 +181,31 @@ class IncrementalRunner:
         its buffers and state reserves among them, also by version or address; and its plans."""
         objects, values = [], [x.shape, x.device, fl.config.epoch, nat.option_epoch[0], fl.filter_epoch[0], torch.is_autocast_enabled()]
         buffers = []      # what the pass clears for the steps behind it is all that exists by then
-        for m in self.model.modules():
-            d = m.__dict__
-            objects += d.values()
-            objects += d["_modules"].values()
-            for p in (*d["_parameters"].values(), *d["_buffers"].values()):
-                objects.append(p)
-                if p is not None:
-                    values.append((p._version, p.data_ptr()))
-            for v in d.values():
-                kind = type(v)
-                if kind is torch.Tensor:
-                    values.append((v.data_ptr(), v.shape, v.stride()))
-                elif kind is fl.Scratch:
+        stack = [self.model]
+        while stack:
+            d = stack.pop().__dict__
+            children = d["_modules"].values()
+            stack += [m for m in children if m is not None]
+            objects += children
+            for kind in ("_parameters", "_buffers"):
+                for p in d[kind].values():
+                    objects.append(p)
+                    if p is not None:
+                        values += (p._version, p.data_ptr())
+            own = list(d.values()) if next(iter(d)) != "training" else list(d.values())[_MODULE_ATTRIBUTES:]
+            objects += own
+            for v in [v for v in own if type(v) in _HOLDERS]:
+                if type(v) is torch.Tensor:
+                    values.append(v.data_ptr())
+                elif type(v) is fl.Scratch:
                     buffers += v._b.values()
-                elif kind is IncrementReserve:
+                else:
                     t = v.reservoir
-                    values.append(None if t is None else (t.data_ptr(), t.shape, t.stride()))
-            for v in d.get("_plans", {}).values():
-                objects += (v, v.tail)
-                values.append(v.needs_clear)
+                    values += (None,) if t is None else (t.data_ptr(), t.shape, t.stride())
+            if "_plans" in d:
+                for v in d["_plans"].values():
+                    objects += (v, v.tail)
+                    values.append(v.needs_clear)
         objects += buffers
         return (tuple(map(id, objects)), values), objects
 

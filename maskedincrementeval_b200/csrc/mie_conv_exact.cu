@@ -66,12 +66,13 @@ __device__ __forceinline__ void tmem_ld16_async(unsigned taddr, unsigned *r) {
                  "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                : "r"(taddr));
 }
-// FULL: the low parts are multiplied too (lo x lo).  The second instruction then has N = 64 columns like the first, 43 clocks instead of 39,
-// and a segment a third more columns to read (64 -> 32 5x5 at 8 x 480x640: 874 us against 831), for the 2^-24 of a product that is
-// dropped elsewhere.  Taken by thin layers, where few products meet and the FP32 kernel is what they are measured against (16 -> 24 3x3,
-// error of the change over that kernel's, 0.5 / 5 / 40 % active: 1.04 / 0.90 / 0.93, without 1.21 / 1.01 / 0.96; of the state 1.01 / 0.97 /
-// 0.94).  Blocks of 32 channels only.
-// hi + 2^-11 (mid + low + 2^-11 last): the products of a segment
+// hi + 2^-11 (mid + low + 2^-11 last): the products of a segment.
+// FULL: the low parts are multiplied too (lo x lo), and in layers of up to 16 channels third parts, which hold what two leave of an operand,
+// with the high ones (pair_mma_full).  The low accumulator then has N = 64 columns like the high one, and a segment a third more
+// columns to read (64 -> 32 5x5 at 8 x 480x640, lo x lo alone: 874 us against 831), for 2^-24 of a product.  Taken by thin layers, where few
+// products meet and the FP32 kernel is what they are measured against (16 -> 24 3x3, error of the change over that kernel's, 0.5 / 5 / 40 %
+// active: without 1.21 / 1.01 / 0.96, with lo x lo 1.04 / 0.90 / 0.93, with third parts 0.73 / 0.72 / 0.80; a step on 97x131 15.8 us without these,
+// 17.1 with).  Blocks of 32 channels only.
 __device__ __forceinline__ float split_sum(unsigned hi, unsigned mid, unsigned low, unsigned last, bool full) {
   float v = __uint_as_float(mid) + __uint_as_float(low);
   if (full) v = fmaf(__uint_as_float(last), SPLIT_LO, v);
@@ -108,7 +109,7 @@ template <int CB, bool ALT, bool FULL>
 __device__ __forceinline__ void exact_issue(const ExactIssue a, const PairTapTable &t, unsigned long long *b_full, unsigned long long *done,
     unsigned long long *a_ready, unsigned long long *a_empty, unsigned long long *seg_empty, unsigned long long *item_full, volatile int *abort_flag) {
   constexpr unsigned tap_units = CB * 64 >> 4;
-  const unsigned id_hi = make_idesc_f16_pair(2 * CB), id_lo = make_idesc_f16_pair(FULL ? 2 * CB : CB);
+  const unsigned id_hi = make_idesc_f16_pair(2 * CB), id_lo = make_idesc_f16_pair(CB);
   const unsigned long long b_tmpl = make_smem_desc_64(0), a_tmpl = make_smem_desc(0, a.row_bytes);
   const unsigned long long b_hi = b_tmpl & 0xFFFFFFFF00000000ull, a_hi = a_tmpl & 0xFFFFFFFF00000000ull;
   const unsigned lo_flags = (unsigned)(b_tmpl & 0xFFFF0000ull);
@@ -134,7 +135,8 @@ __device__ __forceinline__ void exact_issue(const ExactIssue a, const PairTapTab
           for (int k = 0; k < nt; ++k, b_lo += tap_units) {
             const unsigned a_lo = halo + off;
             off = (unsigned)t.off[i + k + 1];     // the next tap's, while this one is issued (the table has a spare entry)
-            pair_mma_split(d, d + 2u * CB, a_hi | a_lo, b_hi | b_lo, id_hi, id_lo, (unsigned)k, nks);
+            if (FULL) pair_mma_full(d, d + 2u * CB, a_hi | a_lo, b_hi | b_lo, id_hi, (unsigned)k, nks, (unsigned)(a.cin <= 16));
+            else pair_mma_split(d, d + 2u * CB, a_hi | a_lo, b_hi | b_lo, id_hi, id_lo, (unsigned)k, nks);
           }
           pair_commit(&done[bs]);
           if (++seg == a.segs) { seg = 0; seg_par ^= 1u; }
@@ -494,7 +496,8 @@ conv_exact_kernel(const __grid_constant__ ExactParams p, const __grid_constant__
     }
   } else if (warp >= 12) {
     // =========================== halos as two FP16 parts ===========================
-    pair_split_halos(work, halos, a_ready, 2 * p.wp * p.wp, p.wp, n_active, tid - 384, s_split, &s_abort);
+    if (FULL && p.cin <= 16) pair_split_halos<true>(work, halos, a_ready, 2 * p.wp * p.wp, p.wp, n_active, tid - 384, s_split, &s_abort);
+    else pair_split_halos<false>(work, halos, a_ready, 2 * p.wp * p.wp, p.wp, n_active, tid - 384, s_split, &s_abort);
   } else if (warp == 3) {
     pair_take_out(s_split, 2 * p.wp * p.wp, p.wp, lane);
   } else if (warp >= 4) {
@@ -966,11 +969,17 @@ __global__ void __launch_bounds__(512) pack_weights_exact_kernel(const float *__
     }
     for (int i = first; i < nch * 32 * kk; i += step) {
       const int ci = i / kk, tap = i - ci * kk;
-      const float v = co < cout && ci < cin ? entry(i, co) * scale : 0.0f;
-      const __half h = __float2half_rn(v);
+      // (up to 16 channels: what two parts leave lies in the hi rows where 16 channels further on would be)
+      const bool third = cin <= 16 && ci >= 16;
+      const float v = co < cout && (third ? ci - 16 : ci) < cin ? entry(third ? i - 16 * kk : i, co) * scale : 0.0f;
+      __half h = __float2half_rn(v);
+      if (third) {
+        const float r = (v - __half2float(h)) * 2048.0f;
+        h = __float2half_rn(r - __half2float(__float2half_rn(r)));
+      }
       const int64_t at = (((int64_t)tap * nch + (ci >> 5)) * 2 * cout_pad + co) * 32 + (ci & 31);
       out[at] = h;
-      out[at + (int64_t)cout_pad * 32] = __float2half_rn((v - __half2float(h)) * 2048.0f);
+      out[at + (int64_t)cout_pad * 32] = third ? __float2half_rn(0.0f) : __float2half_rn((v - __half2float(h)) * 2048.0f);
     }
   }
 }

@@ -301,6 +301,27 @@ __device__ __forceinline__ void pair_mma_split(unsigned d1, unsigned d2, unsigne
       ::"r"(d1), "r"(d2), "l"(a_desc), "l"(b_desc), "r"(id1), "r"(id2), "r"(accumulate), "r"(nks)
       : "memory");
 }
+// The same with every product that leaves 2^-35 of the largest: lo x [hi | lo], and where the channels are 16 at most (`third`) those of third
+// parts, which lie where the second K-slice would be (input: of lo, filter: of hi; scaled like lo).  id: of N = 2 CB columns.
+__device__ __forceinline__ void pair_mma_full(unsigned d1, unsigned d2, unsigned long long a_desc, unsigned long long b_desc, unsigned id, unsigned accumulate,
+                                              unsigned nks, unsigned third) {
+  asm volatile(
+      "{\n\t.reg .pred p, q, e, r1, r3;\n\t.reg .b64 a1, a2, a3, b1;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.eq.b32 q, 0, 0;\n\t"
+      "setp.gt.and.u32 r1, %6, 1, e;\n\t"
+      "setp.ne.and.b32 r3, %7, 0, e;\n\t"
+      "add.u64 a1, %2, 2;\n\tadd.u64 a2, %2, 4;\n\tadd.u64 a3, %2, 6;\n\tadd.u64 b1, %3, 2;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %2, %3, %4, p;\n\t"
+      "@r1 tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %4, q;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%1], a2, %3, %4, p;\n\t"
+      "@r1 tcgen05.mma.cta_group::2.kind::f16 [%1], a3, b1, %4, q;\n\t"
+      "@r3 tcgen05.mma.cta_group::2.kind::f16 [%1], %2, b1, %4, q;\n\t"
+      "@r3 tcgen05.mma.cta_group::2.kind::f16 [%1], a3, %3, %4, q;\n\t}"
+      ::"r"(d1), "r"(d2), "l"(a_desc), "l"(b_desc), "r"(id), "r"(accumulate), "r"(nks), "r"(third)
+      : "memory");
+}
 // Instruction descriptor: FP16 operands, both K-major, FP32 accumulator, M = 256.
 __device__ __forceinline__ unsigned make_idesc_f16_pair(int n) { return (1u << 4) | ((unsigned)(n >> 3) << 17) | (16u << 24); }
 // Rows of 64 bytes, 64-byte swizzle, 8-row groups 512 bytes apart.
@@ -327,8 +348,10 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
       : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
   return d;
 }
-__device__ __forceinline__ void split_fp16(const float *v, float scale, float4 &hi, float4 &lo) {      // eight channels
-  unsigned h[4], l[4];
+// Eight channels.  THIRD: also what two parts leave, scaled like lo (exact: two bits).
+template <bool THIRD>
+__device__ __forceinline__ void split_fp16(const float *v, float scale, float4 &hi, float4 &lo, float4 &third) {
+  unsigned h[4], l[4], m[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const float2 x = make_float2(v[2 * j], v[2 * j + 1]), a = mul2(x, make_float2(scale, scale));
@@ -338,9 +361,15 @@ __device__ __forceinline__ void split_fp16(const float *v, float scale, float4 &
     const __half2 u = __float22half2_rn(r);
     h[j] = *reinterpret_cast<const unsigned *>(&t);
     l[j] = *reinterpret_cast<const unsigned *>(&u);
+    if (THIRD) {
+      const float2 g = __half22float2(u);
+      const __half2 w = __floats2half2_rn(r.x - g.x, r.y - g.y);
+      m[j] = *reinterpret_cast<const unsigned *>(&w);
+    }
   }
   hi = make_float4(__uint_as_float(h[0]), __uint_as_float(h[1]), __uint_as_float(h[2]), __uint_as_float(h[3]));
   lo = make_float4(__uint_as_float(l[0]), __uint_as_float(l[1]), __uint_as_float(l[2]), __uint_as_float(l[3]));
+  if (THIRD) third = make_float4(__uint_as_float(m[0]), __uint_as_float(m[1]), __uint_as_float(m[2]), __uint_as_float(m[3]));
 }
 
 // The splitting warps (t: thread among theirs).  A halo lies in shared memory as `rows` rows of 128 bytes (32 fp32 channels of a
@@ -432,7 +461,8 @@ __device__ __forceinline__ void pair_take_out(SplitShared &sh, int rows, int wp,
     split_meet();
   }
 }
-template <int REGS>
+// THIRD: of halos of 16 channels at most third parts too, in the place of the channels that do not exist (pair_mma_full).
+template <int REGS, bool THIRD>
 __device__ __forceinline__ void pair_split_halos_in(const PairWork &w, const PairRing &r, unsigned long long *ready, int rows, int wp, int n_active, int t,
                                                  SplitShared &sh, volatile int *abort_flag) {
   const int lane = t & 31, cw = t >> 5, passes = (rows + SPLIT_PASS - 1) / SPLIT_PASS;
@@ -518,10 +548,12 @@ __device__ __forceinline__ void pair_split_halos_in(const PairWork &w, const Pai
         mbar_arrive(&sh.inv_full[unit % SPLIT_RING]);
       }
       auto write = [&](int it, const float *x) {
-        float4 hi, lo;
-        split_fp16(x, scale, hi, lo);
-        sts4_if(base + wr0 + (unsigned)(it * SPLIT_PASS * 128), hi, live >> it & 1u);
-        sts4_if(base + wr1 + (unsigned)(it * SPLIT_PASS * 128), lo, live >> it & 1u);
+        float4 hi, lo, third;
+        split_fp16<THIRD>(x, scale, hi, lo, third);
+        const unsigned by = (unsigned)(it * SPLIT_PASS * 128);
+        sts4_if(base + wr0 + by, hi, live >> it & 1u);
+        sts4_if(base + wr1 + by, lo, (!THIRD || c < 2) && live >> it & 1u);
+        if (THIRD) sts4_if(base + at + (unsigned)(((6 + c) & 7) ^ sw) * 16u + by, third, c < 2 && live >> it & 1u);
       };
 #pragma unroll
       for (int it = 0; it < REGS; ++it) write(it, v[it]);
@@ -542,11 +574,12 @@ __device__ __forceinline__ void pair_split_halos_in(const PairWork &w, const Pai
   }
 }
 // By the passes that the halo takes: one that reads no row costs as many instructions as one that does (3x3: a fifth).
+template <bool THIRD>
 __device__ __forceinline__ void pair_split_halos(const PairWork &w, const PairRing &r, unsigned long long *ready, int rows, int wp, int n_active, int t,
                                                  SplitShared &sh, volatile int *abort_flag) {
-  if (rows <= 3 * SPLIT_PASS) pair_split_halos_in<3>(w, r, ready, rows, wp, n_active, t, sh, abort_flag);
-  else if (rows <= 4 * SPLIT_PASS) pair_split_halos_in<4>(w, r, ready, rows, wp, n_active, t, sh, abort_flag);
-  else pair_split_halos_in<SPLIT_REGS>(w, r, ready, rows, wp, n_active, t, sh, abort_flag);
+  if (rows <= 3 * SPLIT_PASS) pair_split_halos_in<3, THIRD>(w, r, ready, rows, wp, n_active, t, sh, abort_flag);
+  else if (rows <= 4 * SPLIT_PASS) pair_split_halos_in<4, THIRD>(w, r, ready, rows, wp, n_active, t, sh, abort_flag);
+  else pair_split_halos_in<SPLIT_REGS, THIRD>(w, r, ready, rows, wp, n_active, t, sh, abort_flag);
   if (t == 0) sh.take = ~0u;      // (the splitting warps leave together, also where a wait gave up)
   split_meet();
 }

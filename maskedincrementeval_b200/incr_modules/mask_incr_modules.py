@@ -458,11 +458,12 @@ class nnConvIncr(nn.Conv2d):
                 and self._k in (1, 3, 5, 7) and self._s in (1, 2))
 
     def _thin(self, cin: int) -> bool:
-        """3x3 layers of 16 channels, too shallow for TF32 numbers on the tensor cores, run in split precision there as well: no less
-        precise than the FP32 kernel (one K-slice of 16 channels is one instruction a tap, so that nothing is truncated inside a
-        tap; with 12 channels the FP32 kernel's sums are too short to match, with 20 the second slice truncates) and faster
-        (16 -> 24 on 97x131 a step of 15 us, 32 on the FP32 kernel)."""
-        return config.tensor_cores == "auto" and cin == 16 and self._k == 3 and self.out_channels % 4 == 0
+        """3x3 layers of 12 to 16 channels, too shallow for TF32 numbers on the tensor cores, run in split precision there as well, with third
+        parts.  Error of a change against float64 over the FP32 kernel's, at 0.05 / 0.5 / 5 / 40 % active pixels: 16 channels 0.70 / 0.73 /
+        0.72 / 0.80, 12 0.82 / 0.83 / 0.82 / 0.90; of the state 0.82 to 0.96.  Not with 8 (up to 1.08: that kernel's sums are short), nor above
+        16 (20 channels 1.19 to 1.29: the third parts have their place where the second 16 channels would be).  And faster: 16 -> 24 on
+        97x131 a step of 17 us, 32 on the FP32 kernel."""
+        return config.tensor_cores == "auto" and 12 <= cin <= 16 and self._k == 3 and self.out_channels % 4 == 0
 
     def _split_copy(self, x_incr: Masked, d: torch.Tensor, m: TileMask, cin_limit: Optional[int]):
         """The three channel blocks of an input in split precision, and how many channels they hold."""

@@ -423,7 +423,7 @@ def test_upsample_and_concat_of_ragged_channel_counts(dev, c):
 @pytest.mark.parametrize("case", [(32, 32, 3, 1, 2, 104, 208, False), (64, 32, 3, 1, 1, 41, 50, False), (96, 32, 3, 1, 1, 24, 40, True), (32, 20, 5, 1, 1, 33, 44, False),
                                   (36, 64, 3, 2, 1, 33, 41, False), (64, 64, 5, 1, 1, 104, 100, False), (16, 40, 7, 1, 1, 24, 40, False),
                                   (256, 256, 3, 1, 1, 17, 23, True), (32, 96, 3, 1, 1, 8, 8, False),
-                                  (16, 24, 3, 1, 1, 97, 131, False), (16, 64, 3, 2, 2, 33, 47, True), (16, 128, 3, 1, 1, 9, 9, False)])
+                                  (16, 24, 3, 1, 1, 97, 131, False), (16, 64, 3, 2, 2, 33, 47, True), (12, 24, 3, 1, 1, 41, 50, False), (12, 40, 3, 2, 1, 33, 41, True), (16, 128, 3, 1, 1, 9, 9, False)])
 @pytest.mark.parametrize("act,thr", [("relu", 0.0), ("tanh", 0.0), (None, 0.0), ("relu", 0.02), ("sigmoid", 0.02)])
 def test_split_precision_steps_against_fp32(dev, case, act, thr):
     from maskedincrementeval_b200 import fields as fl, _native as nat
@@ -436,7 +436,7 @@ def test_split_precision_steps_against_fp32(dev, case, act, thr):
             fl.config.tensor_cores = mode
             torch.manual_seed(15)
             layer = ConvLayerIncr(cin, cout, k, s, k // 2, activation=act).to(dev).eval()
-            layer.conv2d.precision = "split" if cin != 16 or k != 3 else None      # (3x3 layers of 16 channels run so by themselves)
+            layer.conv2d.precision = "split" if cin not in (12, 16) or k != 3 else None      # (3x3 layers of 12 and 16 channels run so by themselves)
             a = layer.activation
             g = torch.Generator(device=dev).manual_seed(16)
             x = cl(torch.randn(n, cin, h, w, generator=g, device=dev))
@@ -583,3 +583,35 @@ def test_extension_on_an_input_that_is_not_aligned(dev, cin, offset):
     y, _ = pf.functional_conv_module(x, w, mask=None, stride=(1, 1), padding=(1, 1))
     want, _ = pf.functional_conv_module(x.clone(memory_format=torch.channels_last), w, mask=None, stride=(1, 1), padding=(1, 1))
     assert torch.equal(y, want)
+
+
+# Thin layers on both sides of the rule that gives them to the tensor cores: no step less precise than the FP32 kernel's, from isolated pixels
+# to dense changes, in the change and in the state
+@pytest.mark.parametrize("cin,taken", [(8, False), (12, True), (16, True), (20, False)])
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("frac", [0.0005, 0.005, 0.05, 0.4])
+def test_thin_layers_are_no_less_precise_than_fp32(dev, cin, taken, stride, frac):
+    from maskedincrementeval_b200 import fields as fl, _native as nat
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    old, err = fl.config.tensor_cores, {}
+    try:
+        for mode in ("auto", "off"):
+            fl.config.tensor_cores = mode
+            torch.manual_seed(30)
+            layer = ConvLayerIncr(cin, 24, 3, stride, 1, activation="relu").to(dev).eval()
+            c, g = layer.conv2d, torch.Generator(device=dev).manual_seed(31)
+            change = state = 0.0
+            for _ in range(4):
+                with torch.no_grad():
+                    layer.forward_refresh_reservoirs(cl(torch.randn(1, cin, 97, 131, generator=g, device=dev)))
+                    before = layer.activation.in_res.reservoir.double()
+                    d = cl(torch.randn(1, cin, 97, 131, generator=g, device=dev) * (torch.rand(1, 1, 97, 131, generator=g, device=dev) < frac))
+                    want = F.conv2d(d.double(), c.weight.double(), stride=stride, padding=1)
+                    change += float((c.forward_fused([d, None], None, None)[0].double() - want).square().sum())
+                    layer([d, None])
+                    assert bool(nat.lib.mie_conv_is_exact(C.byref(c._plan(1, 97, 131, dev).args))) == (taken and mode == "auto")
+                    state += float((layer.activation.in_res.reservoir.double() - before - want).square().sum())
+            err[mode] = change ** 0.5, state ** 0.5
+    finally:
+        fl.config.tensor_cores = old
+    assert err["auto"][0] <= err["off"][0] and err["auto"][1] <= err["off"][1], err

@@ -778,8 +778,8 @@ def run_ours(args):
                              "refresh_native_ms": time_native_refresh(),
                              "refresh_native_note": "the same dense pass on this library's kernels, in fp32 precision on the "
                                                     "tensor cores.  Eager launches, one pass per event pair with the L2 "
-                                                    "flushed before it: the device waits for the host, which enqueues some "
-                                                    "twenty short kernels (replayed back to back by IncrementalRunner: 0.6 ms)"}
+                                                    "flushed before it: the device waits for the host, which enqueues 23 "
+                                                    "short kernels (replayed back to back by IncrementalRunner: 0.6 ms)"}
             line["activity"] = activity_table(net, run, frames_dev[2 + Wm + K], dev)
             # the same frames with activation / ConvLSTM thresholds and carry: the sparsest setting of the threshold
             # study that stays inside the 2e-3 tolerance with these weights

@@ -274,7 +274,8 @@ int mie_conv_pack_dims(int cin, int cout, int k, int *cin_pad, int *cout_pad, in
  * the inverse scales behind them; n_floats floats, 16-byte aligned.
  * mie_pad_field: a dense field of `pixels` pixels with a pixel stride that the tensor cores' loads can follow (out_ps a
  * multiple of 4, >= C rounded up to 4, out 16-byte aligned; channels up to the next multiple of 4 are zero).
- * mie_split_exact: the same into hi, and zeros into lo (the form in which callers of earlier versions pass the input). */
+ * mie_split_exact: the same into hi, and zeros into lo (the form in which callers of earlier versions pass the input; this library
+ * has no use for it). */
 int mie_pad_field(const float *in, int64_t in_ps, int C, int64_t pixels, float *out, int64_t out_ps, void *stream);
 int mie_split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, void *stream);
 int mie_conv_pack_dims_exact(int cin, int cout, int k, int64_t *n_floats /* host */);

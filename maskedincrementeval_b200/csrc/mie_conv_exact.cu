@@ -1007,6 +1007,7 @@ int pad_field(const float *in, int64_t in_ps, int C, int64_t pixels, float *out,
 
 }  // namespace mie
 
+// (for callers of earlier versions)
 extern "C" int mie_split_exact(const float *in, int64_t in_ps, int C, int64_t pixels, float *hi, float *lo, int64_t out_ps, void *stream) {
   if (!lo) return MIE_EINVAL;
   return pad_field(in, in_ps, C, pixels, hi, lo, out_ps, nullptr, (cudaStream_t)stream);

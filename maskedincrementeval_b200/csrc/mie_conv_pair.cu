@@ -428,7 +428,7 @@ static int pair_block_width(const mie_conv_args *a) {
 // ticket per epilogue warp, which costs more than the launch it saves (gates 0 / 1 / 2, one stream: 27.8 / 25.6 / 24.0 us
 // against 23.6 / 23.1 / 22.2 us with the dilation launch).  Layers of 64 channels in two blocks keep the mode.
 // A group's share of the tiles must fit the list in its shared memory.
-int pair_own_groups(const mie_conv_args *a, int n_cblk, int clusters, int64_t ntiles) {
+static int pair_own_groups(const mie_conv_args *a, int n_cblk, int clusters, int64_t ntiles) {
   const int groups = clusters / n_cblk;
   const int64_t pairs = ((int64_t)a->max_tiles + 1) / 2;
   const int kind = n_cblk > 1 && a->cout_pad > 64 ? 8 : a->stride == 2 ? 1 : 4;

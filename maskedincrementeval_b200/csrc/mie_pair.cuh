@@ -564,8 +564,9 @@ __device__ __forceinline__ void pair_split_halos_in(const PairWork &w, const Pai
         __syncwarp();      // in place: the lanes of a row read before one of them writes
         write(it, x);
       }
-      // The instructions read it through the asynchronous proxy.  What the arrival orders is this block's shared memory alone, so the
-      // default (block) scope of its release is enough; with release.cluster it took 1300 clocks, as long as the splitting.
+      // The instructions read it through the asynchronous proxy, also those that the other block issues: each block's rows are read by its own
+      // SM's tensor core.  What the arrival orders is this block's shared memory alone, so the default (block) scope of its release is
+      // enough; with release.cluster it took 1300 clocks, as long as the splitting.
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&ready[s]), 0));

@@ -40,7 +40,6 @@ bool tc_encode(CUtensorMap *m, int rank, const void *base, const cuuint64_t *dim
 // The CTA-pair kernel (mie_conv_pair.cu).
 bool pair_takes(const mie_conv_args *a);
 int launch_conv_pair(const mie_conv_args *a, cudaStream_t st);
-int pair_own_groups(const mie_conv_args *a, int n_cblk, int clusters, int64_t ntiles);
 extern unsigned g_opt_spin_limit;   // MIE_OPT_TC_SPIN_LIMIT
 extern int g_opt_tc_thresholded;    // MIE_OPT_TC_THRESHOLDED
 extern int g_opt_withhold_loads;    // MIE_OPT_TC_WITHHOLD_LOADS

@@ -165,8 +165,8 @@ class IncrementalRunner:
         return self.output
 
     # -- the dense pass as a graph -------------------------------------------------------------------
-    # A refresh of one 260x346 stream is some forty short kernels, enqueued one by one in twice the time that they take
-    # (910 us a pass; the kernels 450).
+    # A refresh of one 260x346 stream is 23 short kernels and some copies, enqueued one by one in twice the time that they take (910 us
+    # a pass; the kernels 450).
     def _may_record_pass(self, x) -> bool:
         # Only networks that say of themselves that their pass is launches of the library's kernels alone (``PASS_IS_KERNELS``), and
         # only where it is: PyTorch's dense operators follow switches, and a subclass may do what a replay would not do again.

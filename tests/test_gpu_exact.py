@@ -615,3 +615,28 @@ def test_thin_layers_are_no_less_precise_than_fp32(dev, cin, taken, stride, frac
     finally:
         fl.config.tensor_cores = old
     assert err["auto"][0] <= err["off"][0] and err["auto"][1] <= err["off"][1], err
+
+
+def test_dense_evaluation_as_callers_of_earlier_versions_ask_for_it(dev):
+    """mie_split_exact and mie_conv_tiles with two input fields: the same as with the field itself."""
+    from maskedincrementeval_b200 import fields as fl, _native as nat
+    from maskedincrementeval_b200.incr_modules._algebra import NATIVE
+    from maskedincrementeval_b200.incr_modules.e2depth_incr import ConvLayerIncr
+    torch.manual_seed(32)
+    layer, n, h, w = ConvLayerIncr(5, 32, 5, 1, 2, activation="relu").to(dev).eval(), 2, 33, 41
+    x = cl(torch.randn(n, 5, h, w, device=dev))
+    with torch.no_grad():
+        y, m = NATIVE.conv(layer.conv2d, NATIVE.lift(x), layer.activation)
+        want, plan = y.clone(), layer.conv2d._plan(n, h, w, dev)
+        both = torch.full((2, n, h, w, 8), float("nan"), device=dev)
+        st = nat.stream_ptr(dev)
+        nat.check(nat.lib.mie_split_exact(x.data_ptr(), 5, 5, n * h * w, both[0].data_ptr(), both[1].data_ptr(), 8, st), "split_exact")
+        a = nat.ConvArgs.from_buffer_copy(next(iter(layer.conv2d._prepared_refresh.values())).args)
+        a.in_, a.in_lo, a.in_ps = both[0].data_ptr(), both[1].data_ptr(), 8
+        job = plan.tail.c
+        nat.check(nat.lib.mie_tiles_dilate(job.in_bits, job.N, job.Hin, job.Win, job.Hout, job.Wout, job.k, job.stride, job.pad, job.union_bits, job.out_bits,
+                                           job.list, job.stale, job.counts, job.flags, st), "tiles_dilate")
+        plan.out.zero_()
+        nat.check(nat.lib.mie_conv_tiles(C.byref(a), st), "conv_tiles")
+        assert torch.equal(both[0, ..., :5].permute(0, 3, 1, 2), x) and bool((both[0, ..., 5:8] == 0).all()) and bool((both[1] == 0).all())
+        assert torch.equal(plan.out, want) and torch.equal(plan.out_bits, fl.full_mask(n, h, w, dev).bits)
